@@ -38,11 +38,46 @@ struct DotsXY {  // <v0|v1>
     __host__ __device__ static constexpr int a(int) { return 0; }
     __host__ __device__ static constexpr int b(int) { return 1; }
 };
-struct DotsCG6 {  // <x|x>, <p|x>, <p|p>, <x|Hx>, <p|Hx>, <p|Hp> for (x, p, Hx, Hp)
-    static constexpr int K = 6;
+struct DotsXPG {  // <x|x>, <p|x>, <p|p>, <x|g>, <p|g> for (x, p, g or Hx)
+    static constexpr int K = 5;
     __host__ __device__ static constexpr int a(int k) { return (k == 0 || k == 3) ? 0 : 1; }
-    __host__ __device__ static constexpr int b(int k) { return k < 2 ? 0 : (k == 2 ? 1 : (k == 5 ? 3 : 2)); }
+    __host__ __device__ static constexpr int b(int k) { return k < 2 ? 0 : (k == 2 ? 1 : 2); }
 };
+
+// <psi|H psi> of one band from what an hpsi_device call left (HpsiDot): the
+// grid partials, and the nonlocal part sum_l uVunk(l)^2 / (iuV(l) dV) where
+// the partials lack it.  One warp, fixed order, the same value in every lane.
+struct HpsiSum {
+    const double* part;
+    int nch;
+    const double* uvunk;
+    const int* iuv;
+    int nzlma;
+    double dV;
+};
+
+__device__ __forceinline__ double hpsi_sum(const HpsiSum& h, int b, int lane) {
+    double v = warp_strided_sum(h.part + (long)b * h.nch, h.nch, 1, lane);
+    if (h.uvunk) {
+        const double* u = h.uvunk + (long)b * h.nzlma;
+        double t = 0.0;
+        for (int l = lane; l < h.nzlma; l += 32) {
+            const int s = h.iuv[l];  // +-1 as a rule; uVunk is zero where iuV is
+            const double q = u[l] * u[l];
+            t += s == 1 ? q : (s == -1 ? -q : (s == 0 ? 0.0 : q / s));
+        }
+        t /= h.dV;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        v += t;
+    }
+    return v;
+}
+
+static HpsiSum hpsi_sum_of(const HpsiDot& d) {
+    const Context& c = ctx();
+    return HpsiSum{d.part, d.nch, d.with_nl ? nullptr : d.uvunk, c.iuv, c.nzlma, c.dV};
+}
 
 // K dot products per band among up to 4 vectors, one read of each vector.
 template <typename T, int NV, class P>
@@ -93,12 +128,11 @@ __global__ void __launch_bounds__(VT) k_multidot(const T* v0, const T* v1, const
 // g = -c1 (hx - E x); partial |g|^2 (cg_module.f90:186-190)
 template <typename T>
 __global__ void __launch_bounds__(VT) k_cg_g(CGVec<T> v, long ld, long n, const double* __restrict__ E,
-                                             double* __restrict__ part, const int* __restrict__ active, int vec) {
+                                             double* __restrict__ part, int vec) {
     using G = Grp16<T>;
     constexpr int W = G::W;
     __shared__ double sh[VT / 32];
     const int b = blockIdx.y;
-    if (active && !active[b]) return;
     const T e = (T)E[b];
     double acc = 0.0;
     const long base = (long)blockIdx.x * VCHUNK, off = (long)b * ld;
@@ -242,14 +276,20 @@ __global__ void __launch_bounds__(VT) k_cg_p(CGVec<T> v, long ld, long n, const 
     }
 }
 
-// hx = u11 hx + u21 hp; g = -c1 (hx - W (u11 x + u21 p)); partial |g|^2 (:337-347)
-template <typename T>
-__device__ __forceinline__ T cg_upd1_elem(T& hx, T hp, T x, T p, T u11, T u21, T w) {
-    hx = u11 * hx + u21 * hp;
-    return (T)(-2.0) * (hx - w * (u11 * x + u21 * p));
+// g' = -c1 (hx' - W x') for hx' = u11 hx + u21 hp and x' = u11 x + u21 p
+// (cg_module.f90:337-347), with hx = E x - g / 2 put in:
+//   g' = u11 g - 2 (u11 (E - W) x + u21 (hp - W p)).
+// The terms are residual-sized where the literal form subtracts two vectors
+// of the size of H x, and hx itself is neither read nor written: five
+// vectors per step instead of six.  FIRST takes the literal form from hx (x
+// may come in unnormalised, then E is no Rayleigh quotient), also five.
+template <typename T, bool FIRST>
+__device__ __forceinline__ T cg_g_elem(T g, T hp, T x, T p, T u11, T u21, T w, T xe) {
+    if (FIRST) return (T)(-2.0) * (fma(u11, g, u21 * hp) - w * fma(u11, x, u21 * p));
+    return fma(u11, g, (T)(-2.0) * fma(xe, x, u21 * fma(-w, p, hp)));
 }
 
-template <typename T>
+template <typename T, bool FIRST>
 __global__ void __launch_bounds__(VT) k_cg_upd1(CGVec<T> v, long ld, long n, CGScal s, double* __restrict__ part,
                                                 const int* __restrict__ active, int vec) {
     using G = Grp16<T>;
@@ -258,30 +298,29 @@ __global__ void __launch_bounds__(VT) k_cg_upd1(CGVec<T> v, long ld, long n, CGS
     const int b = blockIdx.y;
     if (active && !active[b]) return;
     const long off = (long)b * ld, base = (long)blockIdx.x * VCHUNK;
-    const T u11 = (T)s.u11[b], u21 = (T)s.u21[b], w = (T)s.W[b];
+    const T u11 = (T)s.u11[b], u21 = (T)s.u21[b], w = (T)s.E[b];
+    const T xe = (T)(s.u11[b] * (s.E1[b] - s.E[b]));  // E1: the step's old quotient
+    const T* gin = FIRST ? v.hx : v.g;
     double acc = 0.0;
 #pragma unroll 4
     for (int j = 0; j < VITEMS / W; ++j) {
         const long i = base + ((long)j * VT + threadIdx.x) * W;
         if (vec && i + W <= n) {
-            T hx[W], hp[W], x[W], p[W], g[W];
-            G::load(v.hx + off + i, hx);
+            T hp[W], x[W], p[W], g[W];
             G::load(v.hp + off + i, hp);
             G::load(v.x + off + i, x);
             G::load(v.p + off + i, p);
+            G::load(gin + off + i, g);
 #pragma unroll
             for (int q = 0; q < W; ++q) {
-                g[q] = cg_upd1_elem(hx[q], hp[q], x[q], p[q], u11, u21, w);
+                g[q] = cg_g_elem<T, FIRST>(g[q], hp[q], x[q], p[q], u11, u21, w, xe);
                 acc = fma((double)g[q], (double)g[q], acc);
             }
-            G::store(v.hx + off + i, hx);
             G::store(v.g + off + i, g);
         } else {
             for (int q = 0; q < W && i + q < n; ++q) {
                 const long k = off + i + q;
-                T hx = v.hx[k];
-                const T g = cg_upd1_elem(hx, v.hp[k], v.x[k], v.p[k], u11, u21, w);
-                v.hx[k] = hx;
+                const T g = cg_g_elem<T, FIRST>(gin[k], v.hp[k], v.x[k], v.p[k], u11, u21, w, xe);
                 v.g[k] = g;
                 acc = fma((double)g, (double)g, acc);
             }
@@ -291,15 +330,13 @@ __global__ void __launch_bounds__(VT) k_cg_upd1(CGVec<T> v, long ld, long n, CGS
     if (threadIdx.x == 0) part[(long)b * gridDim.x + blockIdx.x] = r;
 }
 
-// x = u11 x + u21 p unless rejected (:366-369)
+// x = u11 x + u21 p unless rejected (:366-369), for the bands with pend set
 template <typename T>
-__global__ void __launch_bounds__(VT) k_cg_upd2(CGVec<T> v, long ld, long n, CGScal s,
-                                                const int* __restrict__ active, int vec) {
+__global__ void __launch_bounds__(VT) k_cg_upd2(CGVec<T> v, long ld, long n, CGScal s, int vec) {
     using G = Grp16<T>;
     constexpr int W = G::W;
     const int b = blockIdx.y;
-    if (active && !active[b]) return;
-    if (s.reject[b]) return;
+    if (!s.pend[b]) return;
     const long off = (long)b * ld, base = (long)blockIdx.x * VCHUNK;
     const T u11 = (T)s.u11[b], u21 = (T)s.u21[b];
 #pragma unroll 4
@@ -319,28 +356,113 @@ __global__ void __launch_bounds__(VT) k_cg_upd2(CGVec<T> v, long ld, long n, CGS
     }
 }
 
+// The end of a sweep: the x update that the last line step left pending (apply
+// != 0), x in FP64 to out64 and H x = E x - g / 2 to hx where they are given.
+template <typename T>
+__global__ void __launch_bounds__(VT) k_cg_end(CGVec<T> v, long ld, long n, CGScal s, int apply, T* __restrict__ hx,
+                                               double* __restrict__ out64, int vec) {
+    using G = Grp16<T>;
+    constexpr int W = G::W;
+    const int b = blockIdx.y;
+    const bool upd = apply && s.pend[b];
+    if (!upd && !hx && !out64) return;
+    const long off = (long)b * ld, base = (long)blockIdx.x * VCHUNK;
+    const T u11 = upd ? (T)s.u11[b] : (T)1, u21 = upd ? (T)s.u21[b] : (T)0, e = (T)s.E[b];
+#pragma unroll 4
+    for (int j = 0; j < VITEMS / W; ++j) {
+        const long i = base + ((long)j * VT + threadIdx.x) * W;
+        if (vec && i + W <= n) {
+            T x[W];
+            G::load(v.x + off + i, x);
+            if (upd) {
+                T p[W];
+                G::load(v.p + off + i, p);
+#pragma unroll
+                for (int q = 0; q < W; ++q) x[q] = cg_upd2_elem(x[q], p[q], u11, u21);
+                if (!out64) G::store(v.x + off + i, x);
+            }
+            if (out64) {
+#pragma unroll
+                for (int q = 0; q < W; q += 2)
+                    *reinterpret_cast<double2*>(out64 + off + i + q) = make_double2((double)x[q], (double)x[q + 1]);
+            }
+            if (hx) {
+                T g[W];
+                G::load(v.g + off + i, g);
+#pragma unroll
+                for (int q = 0; q < W; ++q) g[q] = fma(e, x[q], (T)(-0.5) * g[q]);
+                G::store(hx + off + i, g);
+            }
+        } else {
+            for (int q = 0; q < W && i + q < n; ++q) {
+                const long k = off + i + q;
+                T x = v.x[k];
+                if (upd) x = cg_upd2_elem(x, v.p[k], u11, u21);
+                if (out64)
+                    out64[k] = (double)x;
+                else if (upd)
+                    v.x[k] = x;
+                if (hx) hx[k] = fma(e, x, (T)(-0.5) * v.g[k]);
+            }
+        }
+    }
+}
+
 // ---------------------------------------------------- per-band scalars
-__global__ void s_init(CGScal s, int nb) {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per band; each kernel first adds the per-CTA partials it needs in
+// a fixed order, so no separate reduction launch stands between two vector
+// passes.
+constexpr int SB = 128;  // threads of a scalar CTA: four bands
+
+// start of a sweep: E = dV <x|H x>
+__global__ void __launch_bounds__(SB) s_start(CGScal s, HpsiSum h, int nb) {
+    const int b = blockIdx.x * (SB / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (b >= nb) return;
+    const double v = hpsi_sum(h, b, lane);
+    if (lane != 0) return;
+    s.E[b] = h.dV * v;
     s.E1[b] = 1e10;
     s.gkgk[b] = 0.0;
     s.active[b] = 1;
-    s.reject[b] = 0;
     s.pend[b] = 0;
     if (b == 0) *s.rej_any = 0;
     s.res[b] = 0.0;
 }
 
-// top of the icg loop (cg_module.f90:205-219): a band stops once its
-// Rayleigh quotient moved by less than tol_e in the last line step (the
-// reference's 1e-15, cg_module.f90:218, in FP64)
-__global__ void s_top(CGScal s, int nb, int last, double tol_e) {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb || !s.active[b]) return;
-    const double rb = s.rb[b];
-    s.res[b] = rb / 4.0;
-    if (rb < 0.0 || fabs(s.E[b] - s.E1[b]) < tol_e || last) s.active[b] = 0;
+// End of a line step and top of the next (cg_module.f90:359-365, 205-219): rb
+// = dV <g|g> from the partials; unless it is the first, the update is rejected
+// when the residual grew 1e8-fold.  A band stops once its Rayleigh quotient
+// moved by less than tol_e in the last line step (the reference's 1e-15,
+// cg_module.f90:218, in FP64); a rejected one stops here too, its quotient
+// being put back.
+__global__ void __launch_bounds__(SB) s_step(CGScal s, const double* __restrict__ part, int nch, double dV, int nb,
+                                             int first, int last, double tol_e, double* __restrict__ esp,
+                                             double* __restrict__ res) {
+    const int b = blockIdx.x * (SB / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (b >= nb) return;
+    const int act = s.active[b];
+    double rb = 0.0;
+    if (act) rb = dV * warp_strided_sum(part + (long)b * nch, nch, 1, lane);
+    if (lane != 0) return;
+    if (act) {
+        s.rb[b] = rb;
+        if (!first) {
+            const bool reject = rb / s.res[b] > 1e8;
+            if (reject) {
+                s.E[b] = s.E1[b];
+                *s.rej_any = 1;
+            }
+            s.pend[b] = !reject;
+        }
+        s.res[b] = rb / 4.0;
+        if (rb < 0.0 || fabs(s.E[b] - s.E1[b]) < tol_e || last) s.active[b] = 0;
+    } else {
+        s.pend[b] = 0;
+    }
+    if (last) {
+        esp[b] = s.E[b];
+        res[b] = s.res[b];
+    }
 }
 
 // The stopping tolerance of a line step.  FP64 bands use the reference's
@@ -420,53 +542,40 @@ __device__ void eig2(double a11, double a12, double a22, double b11, double b12,
     X[3] = y1 / u22; X[2] = (y0 - u12 * X[3]) / u11;
 }
 
-// 2x2 Rayleigh-Ritz, pair choice and sign fix (cg_module.f90:299-333)
-__global__ void s_eig(CGScal s, int nb) {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb || !s.active[b]) return;
-    const double* v = s.dots + 6L * b;  // xx, px, pp, xHx, pHx, pHp
+// 2x2 Rayleigh-Ritz, pair choice and sign fix (cg_module.f90:299-333) from the
+// five dots of the search-direction pass (the last two with g, or with H x in
+// the first step) and <p|H p>
+__global__ void __launch_bounds__(SB) s_eig(CGScal s, const double* __restrict__ part, int nch, HpsiSum h, int nb,
+                                            int first) {
+    const int b = blockIdx.x * (SB / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (b >= nb || !s.active[b]) return;  // uniform per warp
+    double v[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) v[k] = h.dV * warp_strided_sum(part + (long)b * nch * 5 + k, nch, 5, lane);
+    const double php = h.dV * hpsi_sum(h, b, lane);
+    if (lane != 0) return;
+    const double E = s.E[b];
     double W[2], X[4];
     int info;
-    eig2(v[3], v[4], v[5], v[0], v[1], v[2], W, X, &info);
+    const double xhx = first ? v[3] : fma(E, v[0], -0.5 * v[3]);
+    const double phx = first ? v[4] : fma(E, v[1], -0.5 * v[4]);
+    eig2(xhx, phx, php, v[0], v[1], v[2], W, X, &info);
     if (info != 0) {  // B not positive definite: keep x (no update)
-        W[0] = s.E[b]; X[0] = 1.0; X[1] = 0.0;
-    } else if (fabs(W[0] - s.E[b]) > 1e-1 && fabs(W[1] - s.E[b]) <= 1e-1) {
+        W[0] = E; X[0] = 1.0; X[1] = 0.0;
+    } else if (fabs(W[0] - E) > 1e-1 && fabs(W[1] - E) <= 1e-1) {
         X[0] = X[2]; X[1] = X[3]; W[0] = W[1];
     }
     if (X[0] < 0.0) { X[0] = -X[0]; X[1] = -X[1]; }
-    s.E1[b] = s.E[b];
+    s.E1[b] = E;
     s.E[b] = W[0];
-    s.W[b] = W[0];
     s.u11[b] = X[0];
     s.u21[b] = X[1];
-}
-
-__global__ void s_rej(CGScal s, int nb) {  // cg_module.f90:359-365
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb) return;
-    if (!s.active[b]) {
-        s.pend[b] = 0;
-        return;
-    }
-    s.reject[b] = 0;
-    if (s.rb[b] / s.res[b] > 1e8) {
-        s.E[b] = s.E1[b];
-        s.reject[b] = 1;
-        *s.rej_any = 1;
-    }
-    s.pend[b] = !s.reject[b];
 }
 
 template <typename T>
 __global__ void k_convert(const double* __restrict__ a, T* __restrict__ b, long n) {
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     for (; i < n; i += (long)gridDim.x * blockDim.x) b[i] = (T)a[i];
-}
-
-template <typename T>
-__global__ void k_convert_back(const T* __restrict__ a, double* __restrict__ b, long n) {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    for (; i < n; i += (long)gridDim.x * blockDim.x) b[i] = (double)a[i];
 }
 
 // sum_i (hx - e x)^2 per band (residual norms after the eigenvalues are known)
@@ -489,6 +598,13 @@ __global__ void __launch_bounds__(VT) k_resid(const double* __restrict__ x, cons
     if (threadIdx.x == 0) part[(long)b * gridDim.x + blockIdx.x] = s;
 }
 
+__global__ void __launch_bounds__(SB) s_esp(HpsiSum h, int nb, double* __restrict__ e) {
+    const int b = blockIdx.x * (SB / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (b >= nb) return;
+    const double v = hpsi_sum(h, b, lane);
+    if (lane == 0) e[b] = h.dV * v;
+}
+
 // e(n) = dV <x_n|H x_n> (esp_calc_module.f90:33-42) and, if res != NULL,
 // res(n) = dV |H x_n - e(n) x_n|^2, all FP64 (device pointers)
 int esp_device(const double* x, long ld, int nb, int spin, double* e, double* res) {
@@ -499,11 +615,12 @@ int esp_device(const double* x, long ld, int nb, int spin, double* e, double* re
     double *hx = nullptr, *part = nullptr;
     RS_CHECK(workspace_t("esp_hx", (size_t)ld * nb, &hx));
     RS_CHECK(workspace_t("esp_part", (size_t)nb * nchunk, &part));
-    RS_CHECK(hpsi_device<double>(x, hx, ld, nb, spin, nullptr));
+    HpsiDot dot;
+    dot.cap = hpsi_dot_cap(c.n1, c.n2, c.n3);
+    RS_CHECK(workspace_t("esp_dot", (size_t)nb * dot.cap, &dot.part));
+    RS_CHECK(hpsi_device<double>(x, hx, ld, nb, spin, nullptr, &dot));
     const dim3 vg(nchunk, nb);
-    const int gv = grp16_ok<double>(ld, {x, hx}) ? 1 : 0;
-    launch(k_multidot<double, 2, DotsXY>, vg, VT, 0, st, x, hx, nullptr, nullptr, ld, n, part, nullptr, gv);
-    launch(k_finish, div_up(nb, 128), 128, 0, st, part, nchunk, 1, nb, c.dV, e, nullptr);
+    launch(s_esp, div_up(nb, SB / 32), SB, 0, st, hpsi_sum_of(dot), nb, e);
     if (res) {
         launch(k_resid, vg, VT, 0, st, x, hx, ld, n, e, part);
         launch(k_finish, div_up(nb, 128), 128, 0, st, part, nchunk, 1, nb, c.dV, res, nullptr);
@@ -513,8 +630,11 @@ int esp_device(const double* x, long ld, int nb, int spin, double* e, double* re
 }
 
 // ------------------------------------------------------------ driver
+// hx_out (if given) receives the sweep's H x (in the CG workspace); out64 (if
+// given) the bands in FP64 in place of the update of x.
 template <typename T>
-static int cg_run(T* x, long ld, int mb, int spin, double* esp, double* res, int ncg, int mloop, int ipc) {
+static int cg_run(T* x, long ld, int mb, int spin, double* esp, double* res, int ncg, int mloop, int ipc,
+                  const T** hx_out = nullptr, double* out64 = nullptr) {
     Context& c = ctx();
     cudaStream_t st = c.stream;
     const long n = c.ml;
@@ -532,52 +652,53 @@ static int cg_run(T* x, long ld, int mb, int spin, double* esp, double* res, int
     v.r = base + 5 * vec;
     v.q = base + 6 * vec;
     double* scal = nullptr;
-    RS_CHECK(workspace_t("cg_scal", (size_t)mb * (20 + SS_STRIDE + SS_MAXM), &scal));
+    RS_CHECK(workspace_t("cg_scal", (size_t)mb * (13 + SS_MAXM), &scal));
     CGScal s{};
     s.E = scal; s.E1 = scal + mb; s.rb = scal + 2 * mb; s.gkgk = scal + 3 * mb; s.res = scal + 4 * mb;
-    s.u11 = scal + 5 * mb; s.u21 = scal + 6 * mb; s.W = scal + 7 * mb; s.rr0 = scal + 8 * mb;
-    s.rr1 = scal + 9 * mb; s.pa = scal + 10 * mb; s.pb = scal + 11 * mb; s.bk = scal + 12 * mb;
-    s.dots = scal + 13 * mb;  // 6 per band
-    double* ss = scal + 20 * mb;                 // s-step Gram / g-dot slots, SS_STRIDE per band
-    double* cz = ss + (size_t)SS_STRIDE * mb;    // s-step coefficients, SS_MAXM per band
+    s.u11 = scal + 5 * mb; s.u21 = scal + 6 * mb; s.rr0 = scal + 7 * mb; s.rr1 = scal + 8 * mb;
+    s.pa = scal + 9 * mb; s.pb = scal + 10 * mb; s.bk = scal + 11 * mb; s.dots = scal + 12 * mb;
+    double* cz = scal + 13 * (size_t)mb;  // s-step coefficients, SS_MAXM per band
     int* flags = nullptr;
-    RS_CHECK(workspace_t("cg_flags", (size_t)mb * 4 + 1, &flags));
-    s.active = flags; s.pc_active = flags + mb; s.reject = flags + 2 * mb; s.pend = flags + 3 * mb;
-    s.rej_any = flags + 4 * mb;
+    RS_CHECK(workspace_t("cg_flags", (size_t)mb * 3 + 1, &flags));
+    s.active = flags; s.pc_active = flags + mb; s.pend = flags + 2 * mb;
+    s.rej_any = flags + 3 * mb;
+    // per-CTA partials: <g|g> (also the literal preconditioner's dots), the
+    // five line-search dots, <psi|H psi>, the basis passes
+    HpsiDot hd;
+    hd.cap = hpsi_dot_cap(c.n1, c.n2, c.n3);
+    const int pcap = std::max(nchunk, 64);
     double* part = nullptr;
-    RS_CHECK(workspace_t("cg_part", (size_t)mb * nchunk * 8, &part));
+    RS_CHECK(workspace_t("cg_part", (size_t)mb * ((size_t)nchunk * 6 + hd.cap + (size_t)(SS_MAXM + 1) * 2 * pcap),
+                         &part));
+    double* pdots = part + (size_t)mb * nchunk;
+    hd.part = pdots + (size_t)mb * nchunk * 5;
+    double* pbasis = hd.part + (size_t)mb * hd.cap;
 
     const dim3 vg(nchunk, mb);
-    const int sb = div_up(mb, 128);
-    const double dV = c.dV;
-    const int gv = grp16_ok<T>(ld, {x, base}) ? 1 : 0;  // 16-byte element groups
+    const int sb = div_up(mb, 128), wb = div_up(mb, SB / 32);
+    const double dV = c.dV, tol = cg_stop_tol<T>();
+    const int gv = grp16_ok<T>(ld, {x, base, out64}) ? 1 : 0;  // 16-byte element groups
     PcArgs pa{c.n1, c.n2, c.n3, VT % c.n1, (VT / c.n1) % c.n2, VT / (c.n1 * c.n2),
               c.pc.c - 0.0, c.pc.c1, c.pc.c2, c.pc.c3};
     auto finish = [&](int K, double scale, double* out, const int* act) {
         launch(k_finish, div_up((long)mb * K, 128), 128, 0, st, part, nchunk, K, mb, scale, out, act);
     };
 
-    launch(s_init, sb, 128, 0, st, s, mb);
-    RS_CHECK(hpsi_device<T>(x, v.hx, ld, mb, spin, nullptr));
-    {
-        launch(k_multidot<T, 2, DotsXY>, vg, VT, 0, st, x, v.hx, nullptr, nullptr, ld, n, part, nullptr, gv);
-        finish(1, dV, s.E, nullptr);
-    }
-    launch(k_cg_g<T>, vg, VT, 0, st, v, ld, n, s.E, part, nullptr, gv);
-    finish(1, dV, s.rb, nullptr);
+    RS_CHECK(hpsi_device<T>(x, v.hx, ld, mb, spin, nullptr, &hd));
+    launch(s_start, wb, SB, 0, st, s, hpsi_sum_of(hd), mb);
+    launch(k_cg_g<T>, vg, VT, 0, st, v, ld, n, s.E, part, gv);
+    launch(s_step, wb, SB, 0, st, s, (const double*)part, nchunk, dV, mb, 1, ncg == 0, tol, esp, res);
     RS_LAUNCH();
 
     const bool sstep = ipc == 4 && mloop >= 1 && mloop <= SS_MAXM;
-    for (int icg = 1; icg <= ncg + 1; ++icg) {
-        const int last = icg == ncg + 1;
-        launch(s_top, sb, 128, 0, st, s, mb, last, cg_stop_tol<T>());
-        if (last) break;
+    for (int icg = 1; icg <= ncg; ++icg) {
         if (sstep) {
-            // --- preconditioner, rb = <Pg|g> dV and the search direction p
-            // in mloop + 2 passes (s-step form; w_j in r, q, Pg, hp, which
-            // are free until hpsi(p))
+            // --- preconditioner, rb = <Pg|g> dV, the search direction p and
+            // the dots of x, p, g in mloop + 2 passes (s-step form; w_j in r,
+            // q, Pg, hp, which are free until hpsi(p)).  The pass also makes
+            // the previous step's x update, as it reads the old p anyway.
             const SSVec<T> sv{{v.r, v.q, v.Pg, v.hp}};
-            RS_CHECK(sstep_precond<T>(v.g, sv, v.p, x, ld, mb, mloop, icg == 1, s, ss, cz, part, pa, dV));
+            RS_CHECK(sstep_precond<T>(v.g, icg == 1 ? v.hx : (const T*)nullptr, sv, v.p, x, ld, mb, mloop, s, cz, pbasis, pcap, pdots, pa, dV));
         } else {
             // --- preconditioning (Pgk = gk on entry)
             if (ipc == 4 && mloop > 0) {
@@ -599,37 +720,38 @@ static int cg_run(T* x, long ld, int mb, int spin, double* esp, double* res, int
                 RS_CUDA(cudaMemcpyAsync(v.Pg, v.g, vec * sizeof(T), cudaMemcpyDeviceToDevice, st));
             }
             RS_LAUNCH();
-            // --- rb = <Pg|g> dV; search direction
-            {
-                launch(k_multidot<T, 2, DotsXY>, vg, VT, 0, st, v.Pg, v.g, nullptr, nullptr, ld, n, part, s.active,
-                       gv);
-                finish(1, dV, s.rb, s.active);
-            }
+            // --- rb = <Pg|g> dV; search direction; dots of x, p, g
+            launch(k_multidot<T, 2, DotsXY>, vg, VT, 0, st, v.Pg, v.g, nullptr, nullptr, ld, n, part, s.active, gv);
+            finish(1, dV, s.rb, s.active);
             launch(s_p, sb, 128, 0, st, s, mb, icg == 1);
             launch(k_cg_p<T>, vg, VT, 0, st, v, ld, n, s.bk, icg == 1, s.active);
+            launch(k_multidot<T, 3, DotsXPG>, vg, VT, 0, st, x, v.p, icg == 1 ? v.hx : v.g, nullptr, ld, n,
+                   pdots, s.active, gv);
             RS_LAUNCH();
         }
-        RS_CHECK(hpsi_device<T>(v.p, v.hp, ld, mb, spin, s.active));
-        // --- six dots: <x|x>, <p|x>, <p|p>, <x|Hx>, <p|Hx>, <p|Hp>
-        {
-            launch(k_multidot<T, 4, DotsCG6>, vg, VT, 0, st, x, v.p, v.hx, v.hp, ld, n, part, s.active, gv);
-            finish(6, dV, s.dots, s.active);
-        }
-        launch(s_eig, sb, 128, 0, st, s, mb);
-        launch(k_cg_upd1<T>, vg, VT, 0, st, v, ld, n, s, part, s.active, gv);
-        finish(1, dV, s.rb, s.active);
-        launch(s_rej, sb, 128, 0, st, s, mb);
-        // s-step form: the x update waits for the next search-direction pass,
-        // which reads the old p anyway
-        if (!sstep) launch(k_cg_upd2<T>, vg, VT, 0, st, v, ld, n, s, s.active, gv);
+        RS_CHECK(hpsi_device<T>(v.p, v.hp, ld, mb, spin, s.active, &hd));
+        launch(s_eig, wb, SB, 0, st, s, (const double*)pdots, nchunk, hpsi_sum_of(hd), mb, icg == 1);
+        launch(icg == 1 ? k_cg_upd1<T, true> : k_cg_upd1<T, false>, vg, VT, 0, st, v, ld, n, s, part, s.active, gv);
+        launch(s_step, wb, SB, 0, st, s, (const double*)part, nchunk, dV, mb, 0, icg == ncg, tol, esp, res);
+        if (!sstep) launch(k_cg_upd2<T>, vg, VT, 0, st, v, ld, n, s, gv);
         RS_LAUNCH();
     }
-    if (sstep) {  // the last step's update
-        launch(k_cg_upd2<T>, vg, VT, 0, st, v, ld, n, s, (const int*)s.pend, gv);
-        RS_LAUNCH();
-    }
-    RS_CUDA(cudaMemcpyAsync(esp, s.E, sizeof(double) * mb, cudaMemcpyDeviceToDevice, st));
-    RS_CUDA(cudaMemcpyAsync(res, s.res, sizeof(double) * mb, cudaMemcpyDeviceToDevice, st));
+    T* hx = hx_out && ncg > 0 ? v.hx : nullptr;
+    if (hx_out) *hx_out = v.hx;
+    launch(k_cg_end<T>, vg, VT, 0, st, v, ld, n, s, sstep ? 1 : 0, hx, out64, gv);
+    RS_LAUNCH();
+    return RSDFT_OK;
+}
+
+// Whether the last sweep of mb bands rejected any update (cg_module.f90:
+// 359-365): its H x then belongs to another x and must be formed again.
+static int cg_rejected(int mb, int* rej) {
+    Context& c = ctx();
+    int* flags = nullptr;
+    RS_CHECK(workspace_t("cg_flags", (size_t)mb * 3 + 1, &flags));
+    *rej = 1;
+    RS_CUDA(cudaMemcpyAsync(rej, flags + 3 * mb, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    RS_CUDA(cudaStreamSynchronize(c.stream));
     return RSDFT_OK;
 }
 
@@ -641,20 +763,12 @@ int cg_device_f32(const double* unk, long ld, int mb, int spin, double* esp, dou
     RS_CHECK(workspace_t("cg_x32", (size_t)n, &x32));
     launch(k_convert<float>, 4 * c.num_sms, 256, 0, c.stream, unk, x32, n);
     RS_LAUNCH();
-    RS_CHECK(cg_run<float>(x32, ld, mb, spin, esp, res, ncg, mloop, ipc));
+    RS_CHECK(cg_run<float>(x32, ld, mb, spin, esp, res, ncg, mloop, ipc, hx_out));
     *x32_out = x32;
     if (hx_out) {
-        // the sweep's H x: the CG keeps hx = H x through its updates, except
-        // for a band whose update was rejected (cg_module.f90:359-365)
-        *hx_out = nullptr;
-        float* hx = nullptr;
-        int* flags = nullptr;
-        RS_CHECK(workspace_t("cg_vec", (size_t)ld * mb * 7, &hx));
-        RS_CHECK(workspace_t("cg_flags", (size_t)mb * 4 + 1, &flags));
         int rej = 1;
-        RS_CUDA(cudaMemcpyAsync(&rej, flags + 4 * mb, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-        RS_CUDA(cudaStreamSynchronize(c.stream));
-        if (rej == 0) *hx_out = hx;
+        RS_CHECK(cg_rejected(mb, &rej));
+        if (rej) *hx_out = nullptr;
     }
     return RSDFT_OK;
 }
@@ -689,15 +803,14 @@ int cg_device_f32_staged(const double* unk_host, double* unk_dev, long ld, int m
         float* xb = x32 + (size_t)b0 * ld;
         launch(k_convert<float>, 4 * c.num_sms, 256, 0, c.stream, (const double*)(unk_dev + (size_t)b0 * ld), xb, n);
         RS_LAUNCH();
-        RS_CHECK(cg_run<float>(xb, ld, nb, spin, esp + b0, res + b0, ncg, mloop, ipc));
+        const float* hx = nullptr;
+        RS_CHECK(cg_run<float>(xb, ld, nb, spin, esp + b0, res + b0, ncg, mloop, ipc, &hx));
         // this block's H x out of the CG workspace, and its rejection flag
-        float* hx = nullptr;
         int* flags = nullptr;
-        RS_CHECK(workspace_t("cg_vec", (size_t)ld * nb * 7, &hx));
-        RS_CHECK(workspace_t("cg_flags", (size_t)nb * 4 + 1, &flags));
+        RS_CHECK(workspace_t("cg_flags", (size_t)nb * 3 + 1, &flags));
         RS_CUDA(cudaMemcpyAsync(hx_all + (size_t)b0 * ld, hx, sizeof(float) * (size_t)n, cudaMemcpyDeviceToDevice,
                                 c.stream));
-        launch(k_or_flag, 1, 1, 0, c.stream, rej, (const int*)(flags + 4 * nb));
+        launch(k_or_flag, 1, 1, 0, c.stream, rej, (const int*)(flags + 3 * nb));
         RS_LAUNCH();
     }
     *x32_out = x32;
@@ -711,20 +824,11 @@ int cg_device_f32_staged(const double* unk_host, double* unk_dev, long ld, int m
 int cg_device(double* unk, long ld, int mb, int spin, double* esp, double* res, int ncg, int mloop, int ipc,
               int mode, const double** hx_out) {
     if (mode == RSDFT_MODE_FP64) {
-        RS_CHECK(cg_run<double>(unk, ld, mb, spin, esp, res, ncg, mloop, ipc));
+        RS_CHECK(cg_run<double>(unk, ld, mb, spin, esp, res, ncg, mloop, ipc, hx_out));
         if (hx_out) {
-            // as in cg_device_f32: the CG's hx is H x unless an update was
-            // rejected (cg_module.f90:359-365)
-            Context& c = ctx();
-            *hx_out = nullptr;
-            double* hx = nullptr;
-            int* flags = nullptr;
-            RS_CHECK(workspace_t("cg_vec", (size_t)ld * mb * 7, &hx));
-            RS_CHECK(workspace_t("cg_flags", (size_t)mb * 4 + 1, &flags));
             int rej = 1;
-            RS_CUDA(cudaMemcpyAsync(&rej, flags + 4 * mb, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-            RS_CUDA(cudaStreamSynchronize(c.stream));
-            if (rej == 0) *hx_out = hx;
+            RS_CHECK(cg_rejected(mb, &rej));
+            if (rej) *hx_out = nullptr;
         }
         return RSDFT_OK;
     }
@@ -734,10 +838,7 @@ int cg_device(double* unk, long ld, int mb, int spin, double* esp, double* res, 
     RS_CHECK(workspace_t("cg_x32", (size_t)n, &x32));
     launch(k_convert<float>, 4 * c.num_sms, 256, 0, c.stream, unk, x32, n);
     RS_LAUNCH();
-    RS_CHECK(cg_run<float>(x32, ld, mb, spin, esp, res, ncg, mloop, ipc));
-    launch(k_convert_back<float>, 4 * c.num_sms, 256, 0, c.stream, x32, unk, n);
-    RS_LAUNCH();
-    return RSDFT_OK;
+    return cg_run<float>(x32, ld, mb, spin, esp, res, ncg, mloop, ipc, nullptr, unk);
 }
 
 }  // namespace rsdft

@@ -41,7 +41,7 @@ inline bool grp16_ok(long ld, std::initializer_list<const void*> ptrs) {
 }
 
 struct CGScal {
-    double *E, *E1, *rb, *gkgk, *res, *u11, *u21, *W, *rr0, *rr1, *pa, *pb, *bk, *dots;
+    double *E, *E1, *rb, *gkgk, *res, *u11, *u21, *rr0, *rr1, *pa, *pb, *bk, *dots;
     int *active, *pc_active, *reject;
     int* pend;     // x = u11 x + u21 p still to be applied (s-step form: by the next p pass)
     int* rej_any;  // set when any band's update was rejected (its hx then no longer equals H x)
@@ -54,10 +54,22 @@ __device__ __forceinline__ T cg_upd2_elem(T x, T p, T u11, T u21) {
     return fma(u11, x, u21 * p);
 }
 
+// After the first line step the sweep keeps g = -2 (H x - E x) instead of H x:
+// every use of H x is E x - g / 2, so no vector for it is read or written.
 template <typename T>
 struct CGVec {
     T *x, *hx, *hp, *g, *Pg, *p, *r, *q;  // q = preconditioner search direction
 };
+
+// Fixed-order sum by one warp of n values p[0], p[stride], ...: lane l takes
+// l, l + 32, ..., then a shuffle tree; the result is valid in every lane.
+__device__ __forceinline__ double warp_strided_sum(const double* __restrict__ p, int n, int stride, int lane) {
+    double v = 0.0;
+    for (int c = lane; c < n; c += 32) v += p[(long)c * stride];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
 
 // 7-point operator of precond_cg_mat2_omp (cgpc_hprsdft_module.f90:
 // 290-340, E0 = 0) at point i = i1 + n1 (i2 + n2 i3), periodic.
@@ -114,19 +126,25 @@ __device__ __forceinline__ void pc_step(const PcArgs& pa, int& i1, int& i2, int&
 // stays well conditioned) A acts on coefficients as the tridiagonal
 //   A w_0 = d (w_0 + w_1),  A w_k = d w_k + (d/2)(w_{k+1} + w_{k-1}),
 // and every dot the recurrences need is a bilinear form in the Gram matrix
-// G_ij = <w_i, w_j> (i < mloop, j <= mloop).  So: mloop passes build the
-// basis and its Gram entries, the scalar recurrences of the reference run
+// G_ij = <w_i, w_j> (i < mloop, j <= mloop), which two dots per basis vector
+// determine (s_sstep).  So: mloop passes build the basis and its dots, the scalar recurrences of the reference run
 // per band on coefficient vectors (s_sstep), and one pass forms
 //   p = g + sum_j cz_j w_j + bk p
 // (Pg itself, the rb = <Pg|g> dot and cg_module.f90:247-261 folded in).
 // The result equals the reference's to rounding: the same Krylov
 // polynomial, evaluated in another basis.
 constexpr int SS_MAXM = 4;   // mloop handled by the s-step form
-constexpr int SS_STRIDE = 20;  // Gram / g-dot slots per band
 
 template <typename T>
 struct SSVec {
     T* w[SS_MAXM];
+};
+
+// per-CTA dot partials of the basis passes (pass k: nch[k] per band, two
+// values each, one in the last pass)
+struct SSPart {
+    const double* part[SS_MAXM + 1];
+    int nch[SS_MAXM + 1];
 };
 
 // off-diagonal part of the 7-point operator at point i
@@ -142,11 +160,13 @@ __device__ __forceinline__ T pc_offdiag(const T* __restrict__ f, long i, int i1,
 }
 
 // Preconditioner + search direction of one CG step in the s-step form:
-// p = Pg (first) or Pg + bk p, with rb = dV <Pg|g> and gkgk updated in s.
-// ss and cz hold SS_STRIDE and SS_MAXM doubles per band, part the per-CTA
-// partial sums (mb x nchunk x 8 doubles).
+// p = Pg (first) or Pg + bk p, with rb = dV <Pg|g> and gkgk updated in s, and
+// the line search's dots of x, p, g as per-CTA partials in dots (5 per chunk).
+// hx: H x in the first step, null later (k_ss_p).
+// cz holds SS_MAXM doubles per band, part (SS_MAXM + 1) x 2 x part_cap per
+// band.
 template <typename T>
-int sstep_precond(const T* g, const SSVec<T>& sv, T* p, T* x, long ld, int mb, int mloop, int first, const CGScal& s,
-                  double* ss, double* cz, double* part, const PcArgs& pa, double dV);
+int sstep_precond(const T* g, const T* hx, const SSVec<T>& sv, T* p, T* x, long ld, int mb, int mloop, const CGScal& s,
+                  double* cz, double* part, int part_cap, double* dots, const PcArgs& pa, double dV);
 
 }  // namespace rsdft

@@ -144,6 +144,8 @@ struct StencilArgs {
     const int* gpt_ptr;   // point-major CSR over sphere groups
     const int* gpt_grp;
     const T* gpt_uv4;
+    double* dot;          // optional: [band][ndot] partial sums of <psi|H psi> over the CTAs of a band
+    int ndot;
 };
 
 template <typename T, int MD, int TX>
@@ -177,6 +179,7 @@ __global__ void __launch_bounds__(TX * 16) k_stencil(StencilArgs<T> a, StencilCo
     }
     const T c0 = (T)cf.c0;
 
+    double dot = 0.0;
     T q[2 * MD + 1];
 #pragma unroll
     for (int k = 0; k < 2 * MD; ++k) q[k] = act ? __ldg(p + col + plane * pwrap(zs - MD + k, n3)) : (T)0;
@@ -212,9 +215,16 @@ __global__ void __launch_bounds__(TX * 16) k_stencil(StencilArgs<T> a, StencilCo
                 for (int k = s; k < e; ++k) v = v + __ldg(a.pt_uv + k) * (T)__ldg(un + __ldg(a.pt_lma + k));
             }
             h[j] = v;
+            dot = fma((double)q[MD], (double)v, dot);
         }
 #pragma unroll
         for (int k = 0; k < 2 * MD; ++k) q[k] = q[k + 1];
+    }
+    if (a.dot) {
+        __shared__ double red[NT / 32];
+        dot = block_sum<NT>(dot, red);
+        if (t == 0)
+            a.dot[(long)band * a.ndot + (long)zc * gridDim.x * gridDim.y + blockIdx.y * gridDim.x + blockIdx.x] = dot;
     }
 }
 
@@ -258,6 +268,7 @@ struct Pk<double> {
     __device__ static __forceinline__ t add(t a, t b) { return __dadd_rn(a, b); }
     __device__ static __forceinline__ t mul(t a, t b) { return __dmul_rn(a, b); }
     __device__ static __forceinline__ t splat(double v) { return v; }
+    __device__ static __forceinline__ void dot(t a, t b, double& s) { s = __fma_rn(a, b, s); }
     __device__ static __forceinline__ t of(const double* p) { return p[0]; }
     __device__ static __forceinline__ void get2(const double2& v, t* o) {
         o[0] = v.x;
@@ -277,6 +288,10 @@ struct Pk<float> {
     __device__ static __forceinline__ t add(t a, t b) { return __fadd2_rn(a, b); }
     __device__ static __forceinline__ t mul(t a, t b) { return __fmul2_rn(a, b); }
     __device__ static __forceinline__ t splat(float v) { return make_float2(v, v); }
+    __device__ static __forceinline__ void dot(t a, t b, double& s) {
+        s = __fma_rn((double)a.x, (double)b.x, s);
+        s = __fma_rn((double)a.y, (double)b.y, s);
+    }
     __device__ static __forceinline__ t of(const float* p) { return make_float2(p[0], p[1]); }
     __device__ static __forceinline__ void get2(const float4& v, t* o) {
         o[0] = make_float2(v.x, v.y);
@@ -296,12 +311,24 @@ struct Pk<float> {
 // part when the plane is one of the tile's own, and slot U + Md + 1 (the
 // output completed by this arrival) is written when hp is set.  NK packs per
 // thread, two per row.
-template <typename T, int MD, int NK, int BY, int U>
+//
+// DOT adds this plane's share of <psi|(T + Vloc) psi>.  Slot U holds
+// sum_m cz_m psi(P - m) when plane P arrives; over the periodic grid the pairs
+// (P, P - m) and (P, P + m) give equal sums, so the z part is twice
+// psi(P) acc[U] and the dot needs no value that is not in registers here.
+template <typename T, int MD, int NK, int BY, bool DOT, int U>
 __device__ __forceinline__ void push_body(typename Pk<T>::t (&acc)[2 * MD + 1][NK], const typename Pk<T>::t* c,
                                           const typename Pk<T>::t* in, bool inner, const CoefT<T>& cf, T* hp,
-                                          int n1) {
+                                          int n1, double& dot) {
     using P = Pk<T>;
     constexpr int Q = 2 * MD + 1;
+    if constexpr (DOT) {
+        if (inner) {
+#pragma unroll
+            for (int i = 0; i < NK; ++i)
+                P::dot(c[i], P::fma(P::splat((T)2), acc[U][i], in[i]), dot);
+        }
+    }
 #pragma unroll
     for (int i = 0; i < NK; ++i) {
         acc[(U + MD) % Q][i] = P::mul(P::splat(cf.cz[MD - 1]), c[i]);
@@ -321,14 +348,14 @@ __device__ __forceinline__ void push_body(typename Pk<T>::t (&acc)[2 * MD + 1][N
 
 // Runtime slot -> compile-time slot: only the short push runs per case, so
 // the loop body is not replicated 2 Md + 1 times.
-template <typename T, int MD, int NK, int BY>
+template <typename T, int MD, int NK, int BY, bool DOT>
 __device__ __forceinline__ void push_slot(int u, typename Pk<T>::t (&acc)[2 * MD + 1][NK], const typename Pk<T>::t* c,
                                           const typename Pk<T>::t* in, bool inner, const CoefT<T>& cf, T* hp,
-                                          int n1) {
+                                          int n1, double& dot) {
     constexpr int Q = 2 * MD + 1;
-#define RS_PUSH_CASE(K)                                                                  \
-    case K:                                                                              \
-        if constexpr (K < Q) push_body<T, MD, NK, BY, K>(acc, c, in, inner, cf, hp, n1); \
+#define RS_PUSH_CASE(K)                                                                            \
+    case K:                                                                                        \
+        if constexpr (K < Q) push_body<T, MD, NK, BY, DOT, K>(acc, c, in, inner, cf, hp, n1, dot); \
         break;
     switch (u) {
         RS_PUSH_CASE(0) RS_PUSH_CASE(1) RS_PUSH_CASE(2) RS_PUSH_CASE(3) RS_PUSH_CASE(4) RS_PUSH_CASE(5)
@@ -352,7 +379,7 @@ __device__ __forceinline__ void push_slot(int u, typename Pk<T>::t (&acc)[2 * MD
 // The 2 Md + 1 accumulators rotate through registers with compile-time
 // indices (a switch on the slot selects the push), so a stage is read only
 // while its own plane is current and the ring can stay shallow.
-template <typename T, int MD, int BY>
+template <typename T, int MD, int BY, bool DOT>
 __global__ void __launch_bounds__(384, 1) k_stencil_tma(const __grid_constant__ TmaMaps maps, StencilArgs<T> a,
                                                        const CoefT<T> cf, int TY, int RS, int S, int ncw,
                                                        int* __restrict__ err) {
@@ -452,6 +479,7 @@ __global__ void __launch_bounds__(384, 1) k_stencil_tma(const __grid_constant__ 
         for (int i = 0; i < NK; ++i) acc[q][i] = P::splat((T)0);
 
     bool ok = true;
+    double dot = 0.0;
     int s = 0, u = 0;
     uint32_t ph = 0;
     for (int k = 0; k < nk; ++k) {
@@ -523,12 +551,26 @@ __global__ void __launch_bounds__(384, 1) k_stencil_tma(const __grid_constant__ 
         // z pushes into the accumulator ring (slot = output arrival mod Q)
         // and, from arrival 2 Md on, the write of the completed output k - Md
         T* hp = (k >= 2 * MD && thr) ? hb + plane * (zs + k - 2 * MD) : nullptr;
-        push_slot<T, MD, NK, BY>(u, acc, c, in, inner, cf, hp, n1);
+        push_slot<T, MD, NK, BY, DOT>(u, acc, c, in, inner, cf, hp, n1, dot);
         if (++s == S) {
             s = 0;
             ph ^= 1u;
         }
         if (++u == Q) u = 0;
+    }
+    if constexpr (DOT) {
+        // fixed-order sum over the consumer warps
+        double* red = reinterpret_cast<double*>(empty + S);
+        if (!thr) dot = 0.0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        if (lane == 0) red[warp] = dot;
+        asm volatile("bar.sync 1, %0;" ::"r"(ncw * 32) : "memory");
+        if (t == 0) {
+            double v = 0.0;
+            for (int w = 0; w < ncw; ++w) v += red[w];
+            a.dot[(long)band * a.ndot + zc * gridDim.x + blockIdx.x] = v;
+        }
     }
     if (!ok) atomicExch(err, 1);
 }
@@ -641,14 +683,25 @@ static TmaGeom tma_geometry(int n1, int n2) {
             best.S = S;
             best.ncw = ncw;
             best.threads = threads;
-            best.smem = (size_t)S * stage + (size_t)S * 16;
+            best.smem = (size_t)S * stage + (size_t)S * 16 + 12 * sizeof(double);
         }
     }
     return best;
 }
 
+template <typename T, int MD, int BY, bool DOT>
+static int launch_tma_dot(const TmaMaps& maps, const StencilArgs<T>& a, const StencilCoef& cf, int nb,
+                          const TmaGeom& g, cudaStream_t st) {
+    RS_CHECK(set_smem_optin((const void*)k_stencil_tma<T, MD, BY, DOT>, 220 * 1024 + 8 * 16 + 12 * 8));
+    dim3 grid(a.n2 / g.TY, (unsigned)(nb * a.nzc));
+    launch(k_stencil_tma<T, MD, BY, DOT>, grid, g.threads, g.smem, st, maps, a, coef_as<T>(cf), g.TY, g.RS, g.S, g.ncw,
+           ctx().err_flag);
+    RS_LAUNCH();
+    return RSDFT_OK;
+}
+
 template <typename T, int MD, int BY>
-static int launch_tma(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStream_t st, bool* used) {
+static int launch_tma(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStream_t st, HpsiDot* dot, bool* used) {
     Context& c = ctx();
     *used = false;
     const TmaGeom g = tma_geometry<T, MD, BY>(a.n1, a.n2);
@@ -657,9 +710,13 @@ static int launch_tma(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStrea
     const int sms = c.num_sms > 0 ? c.num_sms : 148;
     const long base = (long)(a.n2 / g.TY) * nb;
     int nzc = (int)std::min<long>(std::max<long>(1, (sms + base - 1) / base), std::max(1, a.nzo / (4 * MD)));
-    while ((long)nb * nzc > 65535 && nzc > 1) --nzc;
+    while (((long)nb * nzc > 65535 || (dot && (a.n2 / g.TY) * nzc > dot->cap)) && nzc > 1) --nzc;
     a.zlen = div_up(a.nzo, nzc);
     a.nzc = div_up(a.nzo, a.zlen);
+    if (dot) {
+        a.ndot = (a.n2 / g.TY) * a.nzc;
+        if (a.ndot > dot->cap) return RSDFT_OK;
+    }
     TmaMaps maps;
     const CUtensorMapDataType dt = sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     const unsigned long long dims[4] = {(unsigned long long)a.n1, (unsigned long long)a.n2,
@@ -679,22 +736,25 @@ static int launch_tma(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStrea
         encode_tmap_4d(&maps.wrap, dt, a.psi, dims, strides, bw) != RSDFT_OK ||
         encode_tmap_4d(&maps.vloc, dt, a.vloc, vdims, vstrides, bm) != RSDFT_OK)
         return RSDFT_OK;  // not usable for this shape: the caller takes the general kernel
-    RS_CHECK(set_smem_optin((const void*)k_stencil_tma<T, MD, BY>, 220 * 1024 + 8 * 16));
-    dim3 grid(a.n2 / g.TY, (unsigned)(nb * a.nzc));
-    launch(k_stencil_tma<T, MD, BY>, grid, g.threads, g.smem, st, maps, a, coef_as<T>(cf), g.TY, g.RS, g.S, g.ncw,
-           c.err_flag);
-    RS_LAUNCH();
+    if (dot) {
+        dot->nch = a.ndot;
+        dot->with_nl = false;
+        a.dot = dot->part;
+        RS_CHECK((launch_tma_dot<T, MD, BY, true>(maps, a, cf, nb, g, st)));
+    } else {
+        RS_CHECK((launch_tma_dot<T, MD, BY, false>(maps, a, cf, nb, g, st)));
+    }
     *used = true;
     return RSDFT_OK;
 }
 
 template <typename T, int MD>
-static int launch_stencil_md2(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStream_t st) {
+static int launch_stencil_md2(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStream_t st, HpsiDot* dot) {
     const Context& c = ctx();
     bool used = false;
     // two rows per thread up to Md = 6; one above, where the 2 Md + 1
     // accumulators of two rows no longer fit the register budget
-    RS_CHECK((launch_tma<T, MD, (MD <= 6 ? 2 : 1)>(a, cf, nb, st, &used)));
+    RS_CHECK((launch_tma<T, MD, (MD <= 6 ? 2 : 1)>(a, cf, nb, st, dot, &used)));
     if (used) {
         if (a.gpt_ptr && c.nl_npt > 0) {
             constexpr int BCH = 32;
@@ -712,35 +772,46 @@ static int launch_stencil_md2(StencilArgs<T> a, const StencilCoef& cf, int nb, c
     const long base = (long)div_up(a.n1, tx) * div_up(a.n2, 16) * nb;
     const long want = 8L * (c.num_sms > 0 ? c.num_sms : 148);
     int nzc = (int)std::min<long>(std::max<long>(1, (want + base - 1) / base), std::max(1, a.nzo / 8));
-    while ((long)nb * nzc > 65535 && nzc > 1) --nzc;
+    const int nxy = div_up(a.n1, tx) * div_up(a.n2, 16);
+    while (((long)nb * nzc > 65535 || (dot && nxy * nzc > dot->cap)) && nzc > 1) --nzc;
     a.zlen = div_up(a.nzo, nzc);
     a.nzc = div_up(a.nzo, a.zlen);
+    if (dot) {
+        if (nxy * a.nzc > dot->cap) {
+            set_error("hpsi: %d partial sums per band exceed %d", nxy * a.nzc, dot->cap);
+            return RSDFT_EINVAL;
+        }
+        dot->nch = a.ndot = nxy * a.nzc;
+        dot->with_nl = true;
+        a.dot = dot->part;
+    }
     launch_stencil_md<T, MD>(a, cf, nb, st);
     RS_LAUNCH();
     return RSDFT_OK;
 }
 
 template <typename T>
-static int launch_stencil(StencilArgs<T> a, const StencilCoef& cf, int md, int nb, cudaStream_t st) {
+static int launch_stencil(StencilArgs<T> a, const StencilCoef& cf, int md, int nb, cudaStream_t st,
+                          HpsiDot* dot = nullptr) {
     if (a.nzo <= 0) {
         a.z0 = 0;
         a.nzo = a.n3;
     }
     switch (md) {
-        case 1: return launch_stencil_md2<T, 1>(a, cf, nb, st);
-        case 2: return launch_stencil_md2<T, 2>(a, cf, nb, st);
-        case 3: return launch_stencil_md2<T, 3>(a, cf, nb, st);
-        case 4: return launch_stencil_md2<T, 4>(a, cf, nb, st);
-        case 5: return launch_stencil_md2<T, 5>(a, cf, nb, st);
-        case 6: return launch_stencil_md2<T, 6>(a, cf, nb, st);
-        case 7: return launch_stencil_md2<T, 7>(a, cf, nb, st);
-        case 8: return launch_stencil_md2<T, 8>(a, cf, nb, st);
+        case 1: return launch_stencil_md2<T, 1>(a, cf, nb, st, dot);
+        case 2: return launch_stencil_md2<T, 2>(a, cf, nb, st, dot);
+        case 3: return launch_stencil_md2<T, 3>(a, cf, nb, st, dot);
+        case 4: return launch_stencil_md2<T, 4>(a, cf, nb, st, dot);
+        case 5: return launch_stencil_md2<T, 5>(a, cf, nb, st, dot);
+        case 6: return launch_stencil_md2<T, 6>(a, cf, nb, st, dot);
+        case 7: return launch_stencil_md2<T, 7>(a, cf, nb, st, dot);
+        case 8: return launch_stencil_md2<T, 8>(a, cf, nb, st, dot);
         default: set_error("Md=%d unsupported", md); return RSDFT_EUNSUP;
     }
 }
 
 template <typename T>
-int hpsi_device(const T* psi, T* hpsi, long ld, int nb, int spin, const int* band_active) {
+int hpsi_device(const T* psi, T* hpsi, long ld, int nb, int spin, const int* band_active, HpsiDot* dot) {
     Context& c = ctx();
     if (nb <= 0) return RSDFT_OK;
     if (nb > 65535) {
@@ -776,11 +847,12 @@ int hpsi_device(const T* psi, T* hpsi, long ld, int nb, int spin, const int* ban
     a.gpt_ptr = nl ? c.gpt_ptr : nullptr;
     a.gpt_grp = c.gpt_grp;
     a.gpt_uv4 = (const T*)(sizeof(T) == 8 ? (const void*)c.gpt_uv4 : (const void*)c.gpt_uv4_32);
-    return launch_stencil<T>(a, c.sc, c.md, nb, c.stream);
+    if (dot) dot->uvunk = uvunk;
+    return launch_stencil<T>(a, c.sc, c.md, nb, c.stream, dot);
 }
 
-template int hpsi_device<double>(const double*, double*, long, int, int, const int*);
-template int hpsi_device<float>(const float*, float*, long, int, int, const int*);
+template int hpsi_device<double>(const double*, double*, long, int, int, const int*, HpsiDot*);
+template int hpsi_device<float>(const float*, float*, long, int, int, const int*, HpsiDot*);
 
 }  // namespace rsdft
 

@@ -1,14 +1,36 @@
 // Internal (C++) entry points shared between the library's translation units.
 #pragma once
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace rsdft {
 
+// <psi|H psi> of an hpsi_device call, left as sums for the caller to finish in
+// a fixed order: per band, nch grid partials at part[band * nch], and unless
+// with_nl the nonlocal part sum_l uvunk(l)^2 / (iuV(l) dV) on top (uvunk:
+// nzlma values per band, null without projectors).  A skipped band's partials
+// are not written.
+struct HpsiDot {
+    double* part = nullptr;  // nb * cap values
+    int cap = 0;
+    int nch = 0;
+    bool with_nl = false;
+    const double* uvunk = nullptr;
+};
+
 // H psi for nb bands of leading dimension ld (device pointers).  Bands with
 // band_active[b] == 0 are skipped (output left untouched).
 template <typename T>
-int hpsi_device(const T* psi, T* hpsi, long ld, int nb, int spin, const int* band_active);
+int hpsi_device(const T* psi, T* hpsi, long ld, int nb, int spin, const int* band_active, HpsiDot* dot = nullptr);
+
+// most grid partials per band a launch over planes of n1 x n2 points makes
+// (the general stencil kernel's 16 x 16 tiles with the z split at its most)
+inline int hpsi_dot_cap(int n1, int n2, int n3) {
+    const int xy = ((n1 + 15) / 16) * ((n2 + 15) / 16);
+    return std::max(xy * std::max(1, n3 / 8), 64);
+}
 
 // Deterministic block sum (fixed shuffle tree + fixed warp order).  All
 // threads of the block must call it; the result is valid in thread 0.

@@ -3,6 +3,7 @@
 // cgvec.cuh) and the search-direction update folded into it
 // (cg_module.f90:232-261).
 #include <algorithm>
+#include <type_traits>
 
 #include "cgvec.cuh"
 #include "kernels.cuh"
@@ -12,13 +13,14 @@
 
 namespace rsdft {
 
-// Basis vector w_K (K = 0: r0 = g - A g, the reference's first residual).
-// STORE: write w_K; dots <w_K, w_j> for j <= K.  !STORE (K = mloop): w_K
-// only feeds dots: <w_K, w_j> and <w_j, g> for j < K.
+// Basis vector w_K (K = 0: r0 = g - A g, the reference's first residual) and
+// its dots: STORE, write w_K with <w_K, w_{K-1}> (K = 0: <g, w_0>) and
+// <w_K, w_K>; !STORE (K = mloop), only <S w_{K-1}, w_{K-1}> with S = B for
+// K = 1 and 2 B above.
 template <typename T, int K, bool STORE>
 __global__ void __launch_bounds__(VT) k_ss_basis(const T* __restrict__ g, SSVec<T> sv, long ld, long n, PcArgs pa,
                                                  double* __restrict__ part, const int* __restrict__ active) {
-    constexpr int D = K == 0 ? 1 : (STORE ? K + 1 : 2 * K);
+    constexpr int D = STORE ? 2 : 1;
     __shared__ double sh[D * (VT / 32)];
     const int b = blockIdx.y;
     if (active && !active[b]) return;
@@ -34,30 +36,20 @@ __global__ void __launch_bounds__(VT) k_ss_basis(const T* __restrict__ g, SSVec<
     for (int it = 0; it < VITEMS; ++it) {
         const long i = base + it * VT + threadIdx.x;
         if (i < n) {
+            const T si = src[i];
             T wk;
             if constexpr (K == 0) {
-                wk = src[i] - pc_apply<T>(src, i, i1, i2, i3, pa);
+                wk = si - pc_apply<T>(src, i, i1, i2, i3, pa);
             } else if constexpr (K == 1) {
                 wk = pc_offdiag<T>(src, i, i1, i2, i3, pa) * inv_d;
             } else {
-                wk = (T)2 * pc_offdiag<T>(src, i, i1, i2, i3, pa) * inv_d - sv.w[K >= 2 ? K - 2 : 0][off + i];
+                wk = (T)2 * pc_offdiag<T>(src, i, i1, i2, i3, pa) * inv_d;
+                if constexpr (STORE) wk -= sv.w[K >= 2 ? K - 2 : 0][off + i];
             }
-            if constexpr (STORE) sv.w[K < SS_MAXM ? K : 0][off + i] = wk;
-            if constexpr (K == 0) {
-                acc[0] = fma((double)wk, (double)wk, acc[0]);
-            } else {
-                double wj[K];
-#pragma unroll
-                for (int j = 0; j < K; ++j) wj[j] = (double)(j == K - 1 ? src[i] : sv.w[j][off + i]);
-#pragma unroll
-                for (int j = 0; j < K; ++j) acc[j] = fma((double)wk, wj[j], acc[j]);
-                if constexpr (STORE) {
-                    acc[K] = fma((double)wk, (double)wk, acc[K]);
-                } else {
-                    const double gg = (double)g[off + i];
-#pragma unroll
-                    for (int j = 0; j < K; ++j) acc[K + j] = fma(wj[j], gg, acc[K + j]);
-                }
+            acc[0] = fma((double)wk, (double)si, acc[0]);
+            if constexpr (STORE) {
+                sv.w[K < SS_MAXM ? K : 0][off + i] = wk;
+                acc[D - 1] = fma((double)wk, (double)wk, acc[D - 1]);
             }
         }
         pc_step(pa, i1, i2, i3);
@@ -69,38 +61,56 @@ __global__ void __launch_bounds__(VT) k_ss_basis(const T* __restrict__ g, SSVec<
     }
 }
 
-// fixed-order sum of the per-CTA partials into out[b * ostride + k]
-__global__ void k_finish_to(const double* __restrict__ part, int nchunk, int K, int nb, double* __restrict__ out,
-                            int ostride, const int* __restrict__ active) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nb * K) return;
-    int b = i / K, k = i - b * K;
-    if (active && !active[b]) return;
-    const double* p = part + (long)b * nchunk * K + k;
-    double s = 0.0;
-    for (int c = 0; c < nchunk; ++c) s += p[(long)c * K];
-    out[(long)b * ostride + k] = s;
-}
-
-// Per band: the reference's preconditioner recurrences on coefficient
-// vectors (early exit when |r0|^2 < 1e-24, cgpc_hprsdft_module.f90:186),
-// then rb = dV <Pg|g> = rb + dV sum_j cz_j <w_j|g> and the search-direction
-// scalars bk = rb / gkgk, gkgk = rb (cg_module.f90:232-250).
-__global__ void s_sstep(CGScal s, const double* __restrict__ ss, double* __restrict__ cz_out, int nb, int m,
-                        double d, double dV, int first) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb || !s.active[b]) return;
-    const double* S = ss + (long)b * SS_STRIDE;
-    double G[SS_MAXM + 1][SS_MAXM + 1] = {};
-    double gd[SS_MAXM] = {};
-    G[0][0] = S[0];
-    for (int k = 1; k < m; ++k)
-        for (int j = 0; j <= k; ++j) G[k][j] = G[j][k] = S[k * (k + 1) / 2 + j];
-    const int o = m * (m + 1) / 2;
-    for (int j = 0; j < m; ++j) {
-        G[m][j] = G[j][m] = S[o + j];
-        gd[j] = S[o + m + j];
+// Per band, one warp: sum the basis passes' partials (fixed order), expand
+// them into the Gram matrix, run the reference's preconditioner recurrences
+// on coefficient vectors (early exit when |r0|^2 < 1e-24,
+// cgpc_hprsdft_module.f90:186), then rb = dV <Pg|g> = rb + dV sum_j cz_j
+// <w_j|g> and the search-direction scalars bk = rb / gkgk, gkgk = rb
+// (cg_module.f90:232-250).
+//
+// w_j = T_j(B) w_0 with the Chebyshev polynomials T_j and B symmetric, so the
+// whole Gram matrix follows from the moments mu_k = <w_0, T_k(B) w_0>:
+//   <w_i, w_j> = (mu_{i+j} + mu_{|i-j|}) / 2,
+//   mu_{2k} = 2 <w_k, w_k> - mu_0,  mu_{2k+1} = 2 <w_{k+1}, w_k> - mu_1,
+// and, with B g = ((1 - d) g - w_0) / d (from w_0 = g - A g, A = d (I + B)),
+//   <g, w_1> = ((1 - d) <g, w_0> - mu_0) / d,
+//   <g, w_{j+1}> = 2 ((1 - d) <g, w_j> - mu_j) / d - <g, w_{j-1}>.
+// A basis pass therefore needs the dots of its source and its result only
+// (two per pass), and the last one a single dot of its source: it reads one
+// vector where a direct Gram matrix reads mloop + 1.
+__global__ void __launch_bounds__(128) s_sstep(CGScal s, SSPart pt, double* __restrict__ cz_out, int nb, int m,
+                                               double d, double dV, int first) {
+    const int b = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (b >= nb || !s.active[b]) return;  // uniform per warp
+    double S[2 * (SS_MAXM + 1)];
+#pragma unroll
+    for (int k = 0; k <= SS_MAXM; ++k) {
+        S[2 * k] = S[2 * k + 1] = 0.0;
+        if (k <= m) {
+            const int D = k < m ? 2 : 1;
+            const double* p = pt.part[k] + (long)b * pt.nch[k] * D;
+            S[2 * k] = warp_strided_sum(p, pt.nch[k], D, lane);
+            if (D == 2) S[2 * k + 1] = warp_strided_sum(p + 1, pt.nch[k], D, lane);
+        }
     }
+    if (lane != 0) return;
+    double mu[2 * SS_MAXM] = {}, gd[SS_MAXM] = {};
+    mu[0] = S[1];
+    gd[0] = S[0];
+    for (int k = 1; k <= m; ++k) {
+        // <w_k, w_{k-1}>; the last pass leaves <S w_{m-1}, w_{m-1}>
+        double c = S[2 * k];
+        if (k == m && k >= 2) c -= S[2 * (k - 1)];
+        mu[2 * k - 1] = k == 1 ? c : 2.0 * c - mu[1];
+        if (k < m) mu[2 * k] = 2.0 * S[2 * k + 1] - mu[0];
+    }
+    for (int j = 1; j < m; ++j) {
+        const double t = ((1.0 - d) * gd[j - 1] - mu[j - 1]) / d;
+        gd[j] = j == 1 ? t : 2.0 * t - gd[j - 2];
+    }
+    double G[SS_MAXM + 1][SS_MAXM + 1] = {};
+    for (int i = 0; i < m; ++i)
+        for (int j = 0; j <= m; ++j) G[i][j] = G[j][i] = 0.5 * (mu[i + j] + mu[i > j ? i - j : j - i]);
     double cz[SS_MAXM + 1] = {};
     double rr = G[0][0];
     if (!(rr < 1e-24)) {
@@ -138,70 +148,103 @@ __global__ void s_sstep(CGScal s, const double* __restrict__ ss, double* __restr
     for (int j = 0; j < SS_MAXM; ++j) cz_out[(long)b * SS_MAXM + j] = j < m ? cz[j] : 0.0;
 }
 
-// p = g + sum_j cz_j w_j (+ bk p after the first step)
-template <typename T>
-__global__ void __launch_bounds__(VT) k_ss_p(const T* __restrict__ g, SSVec<T> sv, T* __restrict__ p,
-                                             T* __restrict__ x, long ld, long n, const double* __restrict__ cz,
-                                             const double* __restrict__ bk_, int m, int first,
+// p = g + sum_j cz_j w_j (+ bk p after the first step), the previous step's x
+// update, and the line search's five dots of x, p and g (cg_module.f90:
+// 268-297): <x|x>, <p|x>, <p|p>, <x|g>, <p|g>.  All three vectors are in
+// registers here, so the dots cost no memory traffic; with g = -2 (H x - E x)
+// they give <x|Hx> = E <x|x> - <x|g> / 2 and <p|Hx> = E <p|x> - <p|g> / 2,
+// and <p|H p> comes from the H p kernels.  In the first step (hx given) the
+// last two dots are <x|Hx> and <p|Hx> themselves: x may come in unnormalised,
+// E is then no Rayleigh quotient and the identity would cancel (1.7e-12 in
+// the residuals of a band of norm 27, against 1e-15 this way).
+template <typename T, int M>
+__global__ void __launch_bounds__(VT) k_ss_p(const T* __restrict__ g, const T* __restrict__ hx, SSVec<T> sv,
+                                             T* __restrict__ p, T* __restrict__ x, long ld, long n, const double* __restrict__ cz,
+                                             const double* __restrict__ bk_,
                                              const int* __restrict__ active, const int* __restrict__ pend,
                                              const double* __restrict__ u11_, const double* __restrict__ u21_,
-                                             int vec) {
+                                             double* __restrict__ part, int vec) {
     using G = Grp16<T>;
     constexpr int W = G::W;
+    __shared__ double sh[5 * (VT / 32)];
     const int b = blockIdx.y;
-    const bool act = !active || active[b];
+    const bool act = active[b];
     const bool upd = pend && pend[b];  // the previous step's x update, which needs the old p
     if (!act && !upd) return;
     const long off = (long)b * ld, base = (long)blockIdx.x * VCHUNK;
-    T c[SS_MAXM];
+    T c[M];
 #pragma unroll
-    for (int j = 0; j < SS_MAXM; ++j) c[j] = (T)cz[(long)b * SS_MAXM + j];
+    for (int j = 0; j < M; ++j) c[j] = (T)cz[(long)b * SS_MAXM + j];
     const T bk = (T)bk_[b];
     const T u11 = upd ? (T)u11_[b] : (T)0, u21 = upd ? (T)u21_[b] : (T)0;
+    const bool first = hx != nullptr, old = upd || !first;
+    double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    auto elem = [&](T& xv, T& pv, T gv, T hv, const T* w) {
+        if (upd) xv = cg_upd2_elem(xv, pv, u11, u21);
+        T pg = gv;
+#pragma unroll
+        for (int j = 0; j < M; ++j) pg += c[j] * w[j];
+        pv = first ? pg : pg + bk * pv;
+        const double xd = (double)xv, pd = (double)pv, gd = (double)(first ? hv : gv);
+        acc[0] = fma(xd, xd, acc[0]);
+        acc[1] = fma(pd, xd, acc[1]);
+        acc[2] = fma(pd, pd, acc[2]);
+        acc[3] = fma(xd, gd, acc[3]);
+        acc[4] = fma(pd, gd, acc[4]);
+    };
 #pragma unroll 2
     for (int it = 0; it < VITEMS / W; ++it) {
         const long i = base + ((long)it * VT + threadIdx.x) * W;
         if (vec && i + W <= n) {
-            T pg[W], t[W];
-            if (upd || !first) G::load(p + off + i, t);
-            if (upd) {
-                T xv[W];
-                G::load(x + off + i, xv);
+            T pv[W], xv[W];
 #pragma unroll
-                for (int q = 0; q < W; ++q) xv[q] = cg_upd2_elem(xv[q], t[q], u11, u21);
+            for (int q = 0; q < W; ++q) pv[q] = (T)0;
+            if (old) G::load(p + off + i, pv);
+            G::load(x + off + i, xv);
+            if (!act) {
+#pragma unroll
+                for (int q = 0; q < W; ++q) xv[q] = cg_upd2_elem(xv[q], pv[q], u11, u21);
                 G::store(x + off + i, xv);
+                continue;
             }
-            if (!act) continue;
-            T pn[W];
+            T gv[W], hv[W], wv[M][W];
+            G::load(g + off + i, gv);
 #pragma unroll
-            for (int q = 0; q < W; ++q) pn[q] = t[q];
-            G::load(g + off + i, pg);
+            for (int q = 0; q < W; ++q) hv[q] = (T)0;
+            if (first) G::load(hx + off + i, hv);
 #pragma unroll
-            for (int j = 0; j < SS_MAXM; ++j) {
-                if (j < m) {
-                    G::load(sv.w[j] + off + i, t);
+            for (int j = 0; j < M; ++j) G::load(sv.w[j] + off + i, wv[j]);
 #pragma unroll
-                    for (int q = 0; q < W; ++q) pg[q] += c[j] * t[q];
-                }
+            for (int q = 0; q < W; ++q) {
+                T w[M];
+#pragma unroll
+                for (int j = 0; j < M; ++j) w[j] = wv[j][q];
+                elem(xv[q], pv[q], gv[q], hv[q], w);
             }
-            if (!first) {
-#pragma unroll
-                for (int q = 0; q < W; ++q) pg[q] += bk * pn[q];
-            }
-            G::store(p + off + i, pg);
+            if (upd) G::store(x + off + i, xv);
+            G::store(p + off + i, pv);
         } else {
             for (int q = 0; q < W && i + q < n; ++q) {
                 const long k = off + i + q;
-                const T po = (upd || !first) ? p[k] : (T)0;
-                if (upd) x[k] = cg_upd2_elem(x[k], po, u11, u21);
-                if (!act) continue;
-                T pg = g[k];
+                T pv = old ? p[k] : (T)0, xv = x[k];
+                if (!act) {
+                    x[k] = cg_upd2_elem(xv, pv, u11, u21);
+                    continue;
+                }
+                T w[M];
 #pragma unroll
-                for (int j = 0; j < SS_MAXM; ++j)
-                    if (j < m) pg += c[j] * sv.w[j][k];
-                p[k] = first ? pg : pg + bk * po;
+                for (int j = 0; j < M; ++j) w[j] = sv.w[j][k];
+                elem(xv, pv, g[k], first ? hx[k] : (T)0, w);
+                if (upd) x[k] = xv;
+                p[k] = pv;
             }
         }
+    }
+    if (!act) return;
+    block_sum_n<VT, 5>(acc, sh);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) part[((long)b * gridDim.x + blockIdx.x) * 5 + k] = acc[k];
     }
 }
 
@@ -234,26 +277,22 @@ static int launch_ss_fly(int m, dim3 vg, cudaStream_t st, const T* g, SSVec<T> s
 // One basis step as a z march over the 7-point operator, the hpsi stencil's
 // pattern with Md = 1: a CTA owns TY full-width rows of one band; a producer
 // warp streams each source plane (TY + 2 rows, periodic y wrap split into
-// boxes) into a ring of S shared-memory stages, together with TY-row tiles of
-// the operands the step's epilogue needs at the plane that completes there
-// (w_0 .. w_{K-2}, and g for the last step).  Consumer threads own VX x 2
+// boxes) into a ring of S shared-memory stages, together with the TY-row tile
+// of w_{K-2} at the plane that completes there (K >= 2, not the last step).  Consumer threads own VX x 2
 // points, push the z contributions into 3 rotating accumulators, and at the
 // completed plane form w_K, store it and add the step's dot products; the
 // CTA's dot partials are summed in a fixed order at the end.  Every vector
 // element is read once from memory.
 struct PcMaps {
     CUtensorMap full, edge, mid, wrap;  // source boxes of TY + 2, TY + 1, TY, 1 rows
-    CUtensorMap aux[SS_MAXM];           // epilogue operands, TY rows
+    CUtensorMap aux[1];                 // epilogue operand, TY rows
 };
 
 template <int K, bool STORE>
 struct PcStep {
-    static constexpr int NA = (K >= 2 ? K - 1 : 0) + (STORE ? 0 : 1);  // w_0..w_{K-2}, then g
-    static constexpr int D = K == 0 ? 1 : (STORE ? K + 1 : 2 * K);
-    // CTAs per SM: the first two steps have no epilogue operands and few
-    // dots, so two CTAs (<= 85 registers, half the stage ring each) fit and
-    // hide the per-plane latency better
-    static constexpr int CTAS = K <= 1 ? 2 : 1;
+    static constexpr int NA = (STORE && K >= 2) ? 1 : 0;  // w_{K-2}
+    static constexpr int D = STORE ? 2 : 1;
+    static constexpr int CTAS = 2;  // CTAs per SM (<= 85 registers, half the stage ring each)
 };
 
 __device__ __forceinline__ int pc_pwrap(int i, int n) {
@@ -453,26 +492,13 @@ __global__ void __launch_bounds__(384, PcStep<K, STORE>::CTAS) k_pc_tma(const __
                     const int i = r * VX + e;
                     if constexpr (K == 0)
                         wk[e] = -o[i];
-                    else if constexpr (K == 1)
+                    else if constexpr (K == 1 || !STORE)
                         wk[e] = o[i];
                     else
-                        wk[e] = o[i] - av[K >= 2 ? K - 2 : 0][e];
+                        wk[e] = o[i] - av[0][e];
                     const double wd = (double)wk[e];
-                    if constexpr (K == 0) {
-                        dots[0] = fma(wd, wd, dots[0]);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < K - 1; ++j) dots[j] = fma(wd, (double)av[j][e], dots[j]);
-                        dots[K - 1] = fma(wd, (double)cprev[i], dots[K - 1]);
-                        if constexpr (STORE) {
-                            dots[K] = fma(wd, wd, dots[K]);
-                        } else {
-                            const double gg = (double)av[NA - 1][e];
-#pragma unroll
-                            for (int j = 0; j < K - 1; ++j) dots[K + j] = fma((double)av[j][e], gg, dots[K + j]);
-                            dots[2 * K - 1] = fma((double)cprev[i], gg, dots[2 * K - 1]);
-                        }
-                    }
+                    dots[0] = fma(wd, (double)cprev[i], dots[0]);
+                    if constexpr (STORE) dots[D - 1] = fma(wd, wd, dots[D - 1]);
                 }
                 if constexpr (STORE) {
                     if (thr) *reinterpret_cast<V*>(ob + zo + (long)r * n1) = VT::make(wk);
@@ -611,10 +637,7 @@ template <typename T>
 static int pc_tma_dispatch(int K, bool store, const T* g, const SSVec<T>& sv, const PcArgs& pa, long ld, int mb,
                            const int* active, double* part, int part_cap, int* nchunk, bool* used) {
     const T* src = K == 0 ? g : sv.w[K - 1];
-    const T* aux[SS_MAXM] = {};
-    int na = 0;
-    for (int j = 0; j + 2 <= K; ++j) aux[na++] = sv.w[j];
-    if (!store) aux[na++] = g;
+    const T* aux[1] = {K >= 2 ? sv.w[K - 2] : nullptr};
     T* wout = store ? sv.w[K] : nullptr;
 #define RS_PC_CASE(KK, ST)                                                                              \
     if (K == KK && store == ST)                                                                         \
@@ -633,47 +656,54 @@ static int pc_tma_dispatch(int K, bool store, const T* g, const SSVec<T>& sv, co
 }
 
 template <typename T>
-int sstep_precond(const T* g, const SSVec<T>& sv, T* p, T* x, long ld, int mb, int mloop, int first, const CGScal& s,
-                  double* ss, double* cz, double* part, const PcArgs& pa, double dV) {
+int sstep_precond(const T* g, const T* hx, const SSVec<T>& sv, T* p, T* x, long ld, int mb, int mloop, const CGScal& s,
+                  double* cz, double* part, int part_cap, double* dots, const PcArgs& pa, double dV) {
     const Context& c = ctx();
     cudaStream_t st = c.stream;
     const long n = c.ml;
     const int nchunk = div_up(n, VCHUNK);
     const dim3 vg(nchunk, mb);
-    const int sb = div_up(mb, 128);
-    auto finish_to = [&](int K, double* out, int nch) {
-        launch(k_finish_to, div_up((long)mb * K, 128), 128, 0, st, part, nch, K, mb, out, SS_STRIDE, s.active);
-    };
+    SSPart pt{};
     // basis steps: TMA z march where the shape allows, element-wise otherwise
     for (int k = 0; k <= mloop; ++k) {
         const bool store = k < mloop;
-        const int D = k == 0 ? 1 : (store ? k + 1 : 2 * k);
-        double* out = ss + (store ? k * (k + 1) / 2 : mloop * (mloop + 1) / 2);
+        double* out = part + (size_t)k * 2 * part_cap * mb;
         bool used = false;
         int nch = 0;
-        RS_CHECK(pc_tma_dispatch<T>(k, store, g, sv, pa, ld, mb, s.active, part, nchunk, &nch, &used));
+        RS_CHECK(pc_tma_dispatch<T>(k, store, g, sv, pa, ld, mb, s.active, out, part_cap, &nch, &used));
         if (!used) {
             if (k == 0)
-                launch(k_ss_basis<T, 0, true>, vg, VT, 0, st, g, sv, ld, n, pa, part, s.active);
+                launch(k_ss_basis<T, 0, true>, vg, VT, 0, st, g, sv, ld, n, pa, out, s.active);
             else if (store)
-                RS_CHECK(launch_ss_store<T>(k, vg, st, g, sv, ld, n, pa, part, s.active));
+                RS_CHECK(launch_ss_store<T>(k, vg, st, g, sv, ld, n, pa, out, s.active));
             else
-                RS_CHECK(launch_ss_fly<T>(k, vg, st, g, sv, ld, n, pa, part, s.active));
+                RS_CHECK(launch_ss_fly<T>(k, vg, st, g, sv, ld, n, pa, out, s.active));
             nch = nchunk;
         }
-        finish_to(D, out, nch);
+        pt.part[k] = out;
+        pt.nch[k] = nch;
     }
-    launch(s_sstep, sb, 128, 0, st, s, ss, cz, mb, mloop, pa.d, dV, first);
-    const int gv = grp16_ok<T>(ld, {g, p, x, sv.w[0], sv.w[1], sv.w[2], sv.w[3]}) ? 1 : 0;
-    launch(k_ss_p<T>, vg, VT, 0, st, g, sv, p, x, ld, n, cz, s.bk, mloop, first, s.active,
-           (const int*)(first ? nullptr : s.pend), (const double*)s.u11, (const double*)s.u21, gv);
+    launch(s_sstep, div_up(mb, 4), 128, 0, st, s, pt, cz, mb, mloop, pa.d, dV, hx ? 1 : 0);
+    const int gv = grp16_ok<T>(ld, {g, hx, p, x, sv.w[0], sv.w[1], sv.w[2], sv.w[3]}) ? 1 : 0;
+    auto launch_p = [&](auto M) {
+        launch(k_ss_p<T, decltype(M)::value>, vg, VT, 0, st, g, hx, sv, p, x, ld, n, (const double*)cz,
+               (const double*)s.bk, (const int*)s.active, (const int*)(hx ? nullptr : s.pend),
+               (const double*)s.u11, (const double*)s.u21, dots, gv);
+    };
+    switch (mloop) {
+        case 1: launch_p(std::integral_constant<int, 1>{}); break;
+        case 2: launch_p(std::integral_constant<int, 2>{}); break;
+        case 3: launch_p(std::integral_constant<int, 3>{}); break;
+        case 4: launch_p(std::integral_constant<int, 4>{}); break;
+        default: set_error("s-step mloop %d", mloop); return RSDFT_EUNSUP;
+    }
     RS_LAUNCH();
     return RSDFT_OK;
 }
 
-template int sstep_precond<double>(const double*, const SSVec<double>&, double*, double*, long, int, int, int,
-                                   const CGScal&, double*, double*, double*, const PcArgs&, double);
-template int sstep_precond<float>(const float*, const SSVec<float>&, float*, float*, long, int, int, int,
-                                  const CGScal&, double*, double*, double*, const PcArgs&, double);
+template int sstep_precond<double>(const double*, const double*, const SSVec<double>&, double*, double*, long, int,
+                                   int, const CGScal&, double*, double*, int, double*, const PcArgs&, double);
+template int sstep_precond<float>(const float*, const float*, const SSVec<float>&, float*, float*, long, int, int,
+                                  const CGScal&, double*, double*, int, double*, const PcArgs&, double);
 
 }  // namespace rsdft

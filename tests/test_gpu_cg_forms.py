@@ -1,0 +1,43 @@
+"""CG sweep against the oracle where its kernels change form: the basis passes by TMA (even widths) and element-wise
+(odd ones), every s-step order, the literal preconditioner above it, no preconditioner, no line step, and bands that
+come in unnormalised (the first step then takes its dots from H x, not from g)."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+from rsdft_b200 import api
+from rsdft_b200.cell import Workload, build_cell
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12  # the FP64 form's bar; measured 1e-14 .. 2e-13
+
+
+def rel(a, b):
+    return float(np.abs(a - b).max() / np.abs(b).max())
+
+
+@pytest.mark.parametrize("n,nb,mloop,ncg,scale", [
+    (12, 16, 3, 4, 1.0), (12, 5, 1, 3, 1.0), (12, 3, 2, 2, 30.0), (16, 7, 4, 4, 1.0), (15, 9, 3, 4, 1.0),
+    (13, 1, 4, 2, 1.0), (12, 4, 5, 3, 1.0), (12, 4, 0, 3, 1.0), (14, 6, 3, 0, 1.0), (15, 2, 2, 1, 30.0),
+])
+def test_cg_forms(gpu, n, nb, mloop, ncg, scale):
+    c = build_cell(Workload("cg_forms", 1, n, nb, nb, 0.03, 2000 + n))
+    gpu.setup(c)
+    o = O.Oracle(c)
+    q = np.linalg.qr(c.psi0(nb))[0] * (scale / np.sqrt(c.dV))
+    q = np.asfortranarray(q)
+    ru, resp, rres, _ = o.conjugate_gradient(q, ncg, mloop)
+    u = torch.from_numpy(np.ascontiguousarray(q.T)).cuda().t()
+    esp = torch.zeros(nb, dtype=torch.float64, device="cuda")
+    res = torch.zeros_like(esp)
+    gpu.conjugate_gradient(1, c.ML, nb, 1, 1, u, esp, res, ncg=ncg, mloop=mloop)
+    gpu.synchronize()
+    assert rel(u.cpu().numpy(), ru) <= TOL
+    assert rel(esp.cpu().numpy(), resp) <= TOL
+    assert rel(res.cpu().numpy(), rres) <= TOL
+    # the FP32 form of the same sweep: eps(FP32) = 6e-8 per operation, a few line steps
+    x = torch.from_numpy(np.ascontiguousarray(q.T)).cuda().t()
+    gpu.conjugate_gradient(1, c.ML, nb, 1, 1, x, esp, res, ncg=ncg, mloop=mloop, mode=api.MODE_MIXED_BF16X3)
+    gpu.synchronize()
+    assert rel(x.cpu().numpy(), ru) <= 1e-4
