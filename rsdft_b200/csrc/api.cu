@@ -277,7 +277,7 @@ int rsdft_gpu_finalize(void) {
     c.regs.clear();
     void* ptrs[] = {c.err_flag, c.vloc, c.vloc32, c.lma_ptr, c.jjp, c.uv, c.uv32, c.iuv, c.amap, c.duv,
                     c.grp_lma0, c.grp_cnt, c.pt_ptr, c.pt_lma, c.pt_uv, c.pt_uv32,
-                    c.gpt_ptr, c.gpt_grp, c.gpt_uv4, c.gpt_uv4_32, c.nl_pts, c.nl_ptr};
+                    c.gpt_ptr, c.gpt_grp, c.gpt_uv4, c.gpt_uv4_32, c.nl_pts, c.nl_ptr, c.atom_ptr, c.atom_lma};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (c.solver) cusolverDnDestroy(c.solver);
@@ -514,11 +514,18 @@ int rsdft_gpu_set_nonlocal(int nzlma, const int* lma_ptr, const int* jjp, const 
     RS_CHECK(upload(&c.pt_lma, plma.data(), plma.size()));
     RS_CHECK(upload(&c.pt_uv, puv.data(), puv.size()));
     RS_CHECK(upload(&c.pt_uv32, puv32.data(), puv32.size()));
+    // the projectors of each atom, for the force sums
+    std::vector<int> aptr(std::max(natom, 0) + 1, 0), alma(nzlma);
+    for (int l = 0; l < nzlma; ++l) aptr[hamap[l] + 1]++;
+    std::partial_sum(aptr.begin(), aptr.end(), aptr.begin());
+    std::vector<int> apos(aptr.begin(), aptr.end() - 1);
+    for (int l = 0; l < nzlma; ++l) alma[apos[hamap[l]]++] = l;
+    RS_CHECK(upload(&c.atom_ptr, aptr.data(), aptr.size()));
+    RS_CHECK(upload(&c.atom_lma, alma.data(), alma.size()));
     c.nzlma = nzlma;
     c.natom = natom;
     c.nnz = nnz;
     c.ngroup = (int)g0.size();
-    c.h_amap = hamap;
     c.nl_set = true;
     return RSDFT_OK;
 }

@@ -110,7 +110,8 @@ struct Context {
     int nl_npt = 0;             // grid points covered by at least one sphere
     int* nl_pts = nullptr;      // nl_npt: those points, ascending
     int* nl_ptr = nullptr;      // nl_npt+1: their first entry in the group CSR
-    std::vector<int> h_amap;
+    int* atom_ptr = nullptr;    // natom+1: the projectors of each atom, ascending
+    int* atom_lma = nullptr;    // nzlma
 
     // workspace
     std::map<std::string, Buf> ws;

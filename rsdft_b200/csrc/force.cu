@@ -9,182 +9,253 @@
 //   dL/dR_ak  = sum_n sum_{lma in a} iuV dV [(chi.dk uV)(uV.psi) + (chi.uV)(dk uV.psi)]
 // With chi_n = occ_n dV psi_n the second line is dE/dR = -F.
 //
-// k_nl_grad gathers psi (and chi) once per sphere for the 4 projector
-// contractions of every projector in the sphere group (one warp per band),
-// reduces with a fixed shuffle tree and accumulates the band sum of each
-// projector in a fixed order (CTA loops over its bands), then k_atom_sum adds
-// the projectors of each atom in order: bit-reproducible.
+// k_nl_grad takes a sphere group (up to 4 projectors on one point list) x
+// FG_BANDS bands per CTA: the group's point indices and 16 values per point
+// (uV and its three derivatives of each projector) are staged in shared
+// memory once and every warp gathers two vectors at a time (two bands, or one
+// band and its cotangent) against them, 32 dot products in registers.  A
+// butterfly leaves dot product i in lane i, so the products t d and the sum
+// over the warp's bands need no further reduction.  Warps, band chunks and
+// the projectors of an atom are added in a fixed order: bit-reproducible.
+// The bound is the gather of psi (a sphere's rows are ~9 points, so it pulls
+// most of the array's lines).  216-atom cell, 480 bands: 857 us per call with
+// one CTA per sphere (216 CTAs, the 16 values re-read from L2 for every
+// band), 258 us this way.
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernels.cuh"
 
 namespace rsdft {
 
-constexpr int FW = 8;  // warps per CTA
+constexpr int FW = 8;         // warps per CTA
+constexpr int FG_BANDS = 32;  // bands per CTA
+constexpr int FG_CH = 512;    // sphere points staged at a time
 
-// per projector: out[lma*3 + k] = sum over bands of the contribution
+// part[chunk][lma * 3 + k] = the chunk's band sum of each projector
 template <bool CHI>
 __global__ void __launch_bounds__(FW * 32) k_nl_grad(const double* __restrict__ psi, const double* __restrict__ chi,
                                                      long ld, int nb, const double* __restrict__ occ, double cscale,
                                                      const int* __restrict__ grp_lma0, const int* __restrict__ grp_cnt,
                                                      const int* __restrict__ lma_ptr, const int* __restrict__ jjp,
                                                      const double* __restrict__ uv, const double* __restrict__ duv,
-                                                     const int* __restrict__ iuv, double dV,
-                                                     double* __restrict__ out, int* __restrict__ err) {
-    __shared__ double sh[FW][4][3];
+                                                     const int* __restrict__ iuv, double dV, int nzlma,
+                                                     double* __restrict__ part, int* __restrict__ err) {
+    extern __shared__ __align__(16) double fg_sm[];  // 16 x FG_CH values, FG_CH indices
+    double(*s_c)[FG_CH] = reinterpret_cast<double(*)[FG_CH]>(fg_sm);
+    int* s_j = reinterpret_cast<int*>(fg_sm + 16 * FG_CH);
+    __shared__ double sh[FW][16];
+    constexpr int BPW = CHI ? 1 : 2;  // bands a warp takes at a time
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = blockIdx.x;
     const int l0 = grp_lma0[g], cnt = grp_cnt[g];
     const int js = lma_ptr[l0], n = lma_ptr[l0 + 1] - js;
-    int off[4];
+    long off[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) off[q] = q < cnt ? lma_ptr[l0 + q] : js;
-    double tot[4][3];
+    const int b0 = blockIdx.y * FG_BANDS, b1 = min(nb, b0 + FG_BANDS);
+    const int nrep = (FG_BANDS + FW * BPW - 1) / (FW * BPW);
+    // dot product i = 16 w + 4 q + c of vector w: c = 0 uV, c = 1..3 its
+    // derivatives, projector q; lane i owns it after the reduction
+    double tot = 0.0;
+    int staged = -1;
+    for (int r = 0; r < nrep; ++r) {
+        const int bw = b0 + (r * FW + warp) * BPW;
+        const double* v[2];
+        bool act[2];
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) tot[q][k] = 0.0;
-    for (int b = warp; b < nb; b += FW) {
-        const double o = occ ? occ[b] : 1.0;
-        if (!CHI && o == 0.0) continue;
-        const double* p = psi + (long)b * ld;
-        const double* x = CHI ? chi + (long)b * ld : nullptr;
-        // per projector: t = uV.psi, d_k = duV_k.psi (and the chi versions)
-        double t[4], d[4][3], tc[4], dc[4][3];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            t[q] = 0.0;
-            tc[q] = 0.0;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) d[q][k] = dc[q][k] = 0.0;
+        for (int w = 0; w < 2; ++w) {
+            const int b = CHI ? bw : bw + w;
+            act[w] = b < b1 && (CHI || !occ || occ[b] != 0.0);
+            v[w] = (CHI && w == 1 ? chi : psi) + (long)(act[w] ? b : 0) * ld;
         }
-        for (int j = lane; j < n; j += 32) {
-            const int jj = jjp[js + j];
-            if (!RS_DCHECK(jj >= 0 && jj < ld, CK_NL_GRAD_POINT, jj, err)) continue;
-            const double v = __ldg(p + jj);
-            const double xv = CHI ? __ldg(x + jj) : 0.0;
+        double acc[32];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                if (q < cnt) {
-                    const long e = off[q] + j;
-                    const double u = __ldg(uv + e);
-                    const double d0 = __ldg(duv + 3 * e), d1 = __ldg(duv + 3 * e + 1), d2 = __ldg(duv + 3 * e + 2);
-                    t[q] = fma(u, v, t[q]);
-                    d[q][0] = fma(d0, v, d[q][0]);
-                    d[q][1] = fma(d1, v, d[q][1]);
-                    d[q][2] = fma(d2, v, d[q][2]);
-                    if (CHI) {
-                        tc[q] = fma(u, xv, tc[q]);
-                        dc[q][0] = fma(d0, xv, dc[q][0]);
-                        dc[q][1] = fma(d1, xv, dc[q][1]);
-                        dc[q][2] = fma(d2, xv, dc[q][2]);
+        for (int i = 0; i < 32; ++i) acc[i] = 0.0;
+        for (int c0 = 0; c0 < n; c0 += FG_CH) {
+            const int m = min(FG_CH, n - c0);
+            if (staged != c0) {  // the same for every thread
+                __syncthreads();
+                for (int i = threadIdx.x; i < m; i += FW * 32) {
+                    s_j[i] = jjp[js + c0 + i];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const long e = off[q] + c0 + i;
+                        s_c[4 * q][i] = q < cnt ? uv[e] : 0.0;
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) s_c[4 * q + 1 + k][i] = q < cnt ? duv[3 * e + k] : 0.0;
                     }
                 }
+                __syncthreads();
+                staged = c0;
             }
-        }
+#pragma unroll 2
+            for (int j = lane; j < m; j += 32) {
+                const int jj = s_j[j];
+                const bool in = RS_DCHECK(jj >= 0 && jj < ld, CK_NL_GRAD_POINT, jj, err);
+                double x[2];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+                for (int w = 0; w < 2; ++w) x[w] = act[w] && in ? __ldg(v[w] + jj) : 0.0;
 #pragma unroll
-            for (int s = 16; s > 0; s >>= 1) {
-                t[q] += __shfl_xor_sync(0xffffffffu, t[q], s);
-#pragma unroll
-                for (int k = 0; k < 3; ++k) d[q][k] += __shfl_xor_sync(0xffffffffu, d[q][k], s);
-                if (CHI) {
-                    tc[q] += __shfl_xor_sync(0xffffffffu, tc[q], s);
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) dc[q][k] += __shfl_xor_sync(0xffffffffu, dc[q][k], s);
+                for (int i = 0; i < 16; ++i) {
+                    const double u = s_c[i][j];
+                    acc[i] = fma(u, x[0], acc[i]);
+                    acc[16 + i] = fma(u, x[1], acc[16 + i]);
                 }
             }
         }
+        // 32 sums over 32 lanes: at each step a lane keeps the half of the
+        // values whose index has its own bit, so lane i ends with sum i
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (q < cnt) {
-                const double w = iuv[l0 + q] * dV;
+        for (int s = 16; s >= 1; s >>= 1) {
+            const bool upper = (lane & s) != 0;
 #pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    if (CHI)
-                        tot[q][k] += w * (dc[q][k] * t[q] + tc[q] * d[q][k]);
-                    else
-                        tot[q][k] += cscale * o * w * t[q] * d[q][k];
-                }
+            for (int j = 0; j < s; ++j) {
+                const double give = upper ? acc[j] : acc[j + s], keep = upper ? acc[j + s] : acc[j];
+                acc[j] = keep + __shfl_xor_sync(0xffffffffu, give, s);
             }
         }
+        const double d = acc[0];
+        const int q = (lane >> 2) & 3;
+        const double wq = q < cnt ? iuv[l0 + q] * dV : 0.0;
+        double c;
+        if (CHI) {  // (chi.duV)(uV.psi) + (chi.uV)(duV.psi), one half per lane half
+            c = wq * d * __shfl_sync(0xffffffffu, d, (lane ^ 16) & ~3);
+        } else {
+            const int b = bw + (lane >> 4);
+            const double t = __shfl_sync(0xffffffffu, d, lane & ~3);
+            c = b < b1 && occ[b] != 0.0 ? cscale * occ[b] * wq * t * d : 0.0;
+        }
+        c += __shfl_xor_sync(0xffffffffu, c, 16);
+        if (bw < b1) tot += c;
     }
-    if (lane == 0) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-            for (int k = 0; k < 3; ++k) sh[warp][q][k] = tot[q][k];
-    }
+    if (lane < 16) sh[warp][lane] = tot;
     __syncthreads();
-    if (threadIdx.x < 12) {
-        const int q = threadIdx.x / 3, k = threadIdx.x % 3;
+    if (threadIdx.x < 16 && (threadIdx.x & 3) != 0) {
+        const int q = threadIdx.x >> 2, k = (threadIdx.x & 3) - 1;
         if (q < cnt) {
             double s = 0.0;
-            for (int w = 0; w < FW; ++w) s += sh[w][q][k];
-            out[(long)(l0 + q) * 3 + k] = s;
+#pragma unroll
+            for (int w = 0; w < FW; ++w) s += sh[w][threadIdx.x];
+            part[((long)blockIdx.y * nzlma + l0 + q) * 3 + k] = s;
         }
     }
 }
 
-__global__ void k_atom_sum(const double* __restrict__ per_lma, const int* __restrict__ atom_ptr,
+// f(3 a + k): the projectors of atom a in order, each over its band chunks in
+// order; one warp per atom component (the lanes take the chunks)
+__global__ void k_atom_sum(const double* __restrict__ part, int nchunk, int nzlma, const int* __restrict__ atom_ptr,
                            const int* __restrict__ atom_lma, int natom, double* __restrict__ f) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (i >= natom * 3) return;
-    int a = i / 3, k = i % 3;
+    const int a = i / 3, k = i % 3;
     double s = 0.0;
-    for (int e = atom_ptr[a]; e < atom_ptr[a + 1]; ++e) s += per_lma[(long)atom_lma[e] * 3 + k];
-    f[i] = s;
+    for (int e = atom_ptr[a]; e < atom_ptr[a + 1]; ++e)
+        for (int y = lane; y < nchunk; y += 32) s += part[((long)y * nzlma + atom_lma[e]) * 3 + k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) f[i] = s;
 }
 
 // dL/dV(r) = sum_n chi_n(r) psi_n(r), chi_n = occ_n dV psi_n when chi == NULL
-__global__ void k_vloc_adjoint(const double* __restrict__ psi, const double* __restrict__ chi, long ld, int nb,
-                               const double* __restrict__ occ, double dV, long n, double* __restrict__ out) {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double s = 0.0;
-    if (chi) {
-        for (int b = 0; b < nb; ++b) s = fma(__ldg(chi + (long)b * ld + i), __ldg(psi + (long)b * ld + i), s);
-    } else {
-        for (int b = 0; b < nb; ++b) {
-            const double o = occ[b];
-            if (o == 0.0) continue;
-            const double v = __ldg(psi + (long)b * ld + i);
-            s = fma(o * dV * v, v, s);
+// A thread takes W consecutive points (16-byte loads when the layout allows).
+// The bands that take part (occ != 0; all of them with chi) are listed in
+// shared memory first, so that a trip over four of them is four independent
+// loads with no branch between them; their terms are added in band order.
+constexpr int VA_LIST = 1024;  // bands listed at a time
+
+template <int W, bool CHI>
+__global__ void __launch_bounds__(256) k_vloc_adjoint(const double* __restrict__ psi, const double* __restrict__ chi,
+                                                      long ld, int nb, const double* __restrict__ occ, double dV,
+                                                      long n, double* __restrict__ out) {
+    __shared__ int s_b[VA_LIST];
+    __shared__ double s_o[VA_LIST];
+    __shared__ int s_n;
+    const long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * W;
+    const bool in = i < n;  // n is a multiple of W
+    constexpr int U = 4;
+    double s[W];
+#pragma unroll
+    for (int e = 0; e < W; ++e) s[e] = 0.0;
+    auto load = [](const double* p, double (&v)[W]) {
+        if constexpr (W == 2) {
+            const double2 t = __ldg(reinterpret_cast<const double2*>(p));
+            v[0] = t.x;
+            v[1] = t.y;
+        } else {
+            v[0] = __ldg(p);
         }
+    };
+    for (int b0 = 0; b0 < nb; b0 += VA_LIST) {
+        __syncthreads();
+        if (threadIdx.x < 32) {  // one warp lists the bands in order
+            int cnt = 0;
+            for (int b = b0; b < min(nb, b0 + VA_LIST); b += 32) {
+                const int bb = b + (int)threadIdx.x;
+                const double o = bb < nb ? (CHI ? 1.0 : occ[bb]) : 0.0;
+                const unsigned m = __ballot_sync(0xffffffffu, o != 0.0);
+                if (o != 0.0) {
+                    const int at = cnt + __popc(m & ((1u << threadIdx.x) - 1u));
+                    s_b[at] = bb;
+                    s_o[at] = o * dV;
+                }
+                cnt += __popc(m);
+            }
+            if (threadIdx.x == 0) s_n = cnt;
+        }
+        __syncthreads();
+        if (!in) continue;
+        const int cnt = s_n;
+        int q = 0;
+        auto trip = [&](auto NU) {
+            constexpr int N = decltype(NU)::value;
+            double v[N][W], x[N][W];
+#pragma unroll
+            for (int u = 0; u < N; ++u) {
+                load(psi + (long)s_b[q + u] * ld + i, v[u]);
+                if (CHI) load(chi + (long)s_b[q + u] * ld + i, x[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < N; ++u)
+#pragma unroll
+                for (int e = 0; e < W; ++e)
+                    s[e] = CHI ? fma(x[u][e], v[u][e], s[e]) : fma(s_o[q + u] * v[u][e], v[u][e], s[e]);
+        };
+        for (; q + U <= cnt; q += U) trip(std::integral_constant<int, U>{});
+        for (; q < cnt; ++q) trip(std::integral_constant<int, 1>{});
     }
-    out[i] = s;
+    if (!in) return;
+#pragma unroll
+    for (int e = 0; e < W; ++e) out[i + e] = s[e];
 }
 
-static int atom_tables(int** aptr, int** alma) {
-    Context& c = ctx();
-    std::vector<int> cnt(c.natom + 1, 0), lst(c.nzlma);
-    for (int l = 0; l < c.nzlma; ++l) cnt[c.h_amap[l] + 1]++;
-    for (int a = 0; a < c.natom; ++a) cnt[a + 1] += cnt[a];
-    std::vector<int> pos(cnt.begin(), cnt.end() - 1);
-    for (int l = 0; l < c.nzlma; ++l) lst[pos[c.h_amap[l]]++] = l;
-    RS_CHECK(workspace_t("atom_ptr", cnt.size(), aptr));
-    RS_CHECK(workspace_t("atom_lma", lst.size() + 1, alma));
-    RS_CUDA(cudaMemcpyAsync(*aptr, cnt.data(), cnt.size() * sizeof(int), cudaMemcpyHostToDevice, c.stream));
-    RS_CUDA(cudaMemcpyAsync(*alma, lst.data(), lst.size() * sizeof(int), cudaMemcpyHostToDevice, c.stream));
-    RS_CUDA(cudaStreamSynchronize(c.stream));
+static int vloc_adjoint(const double* psi, const double* chi, long ld, int nb, const double* occ, double dV, long n,
+                        double* out) {
+    cudaStream_t st = ctx().stream;
+    const bool vec = n % 2 == 0 && ld % 2 == 0 && reinterpret_cast<uintptr_t>(psi) % 16 == 0 &&
+                     reinterpret_cast<uintptr_t>(chi) % 16 == 0;
+    auto kern = vec ? (chi ? k_vloc_adjoint<2, true> : k_vloc_adjoint<2, false>)
+                    : (chi ? k_vloc_adjoint<1, true> : k_vloc_adjoint<1, false>);
+    launch(kern, div_up(n, (vec ? 2 : 1) * 256L), 256, 0, st, psi, chi, ld, nb, occ, dV, n, out);
+    RS_LAUNCH();
     return RSDFT_OK;
 }
 
 static int nl_grad(const double* psi, const double* chi, long ld, int nb, const double* occ, double cscale,
                    double* f_dev) {
     Context& c = ctx();
-    double* per = nullptr;
-    int *aptr, *alma;
-    RS_CHECK(workspace_t("force_lma", (size_t)c.nzlma * 3, &per));
-    RS_CHECK(atom_tables(&aptr, &alma));
-    if (chi)
-        launch(k_nl_grad<true>, c.ngroup, FW * 32, 0, c.stream, psi, chi, ld, nb, occ, cscale, c.grp_lma0, c.grp_cnt,
-                                                            c.lma_ptr, c.jjp, c.uv, c.duv, c.iuv, c.dV, per, c.err_flag);
-    else
-        launch(k_nl_grad<false>, c.ngroup, FW * 32, 0, c.stream, psi, chi, ld, nb, occ, cscale, c.grp_lma0, c.grp_cnt,
-                                                             c.lma_ptr, c.jjp, c.uv, c.duv, c.iuv, c.dV, per, c.err_flag);
+    const int nchunk = div_up(nb, FG_BANDS);
+    double* part = nullptr;
+    RS_CHECK(workspace_t("force_part", (size_t)c.nzlma * 3 * nchunk, &part));
+    const size_t smem = FG_CH * (16 * sizeof(double) + sizeof(int));
+    auto kern = chi ? k_nl_grad<true> : k_nl_grad<false>;
+    RS_CHECK(set_smem_optin((const void*)kern, (int)smem));
+    launch(kern, dim3(c.ngroup, nchunk), FW * 32, smem, c.stream, psi, chi, ld, nb, occ, cscale,
+           (const int*)c.grp_lma0, (const int*)c.grp_cnt, (const int*)c.lma_ptr, (const int*)c.jjp,
+           (const double*)c.uv, (const double*)c.duv, (const int*)c.iuv, c.dV, c.nzlma, part, c.err_flag);
     RS_LAUNCH();
-    launch(k_atom_sum, div_up(c.natom * 3, 128), 128, 0, c.stream, per, aptr, alma, c.natom, f_dev);
+    launch(k_atom_sum, div_up(c.natom * 3, 4), 128, 0, c.stream, (const double*)part, nchunk, c.nzlma,
+           (const int*)c.atom_ptr, (const int*)c.atom_lma, c.natom, f_dev);
     RS_LAUNCH();
     return RSDFT_OK;
 }
@@ -242,8 +313,7 @@ int rsdft_gpu_hpsi_adjoint(const double* psi, const double* chi, long ld, int nb
     if (occ) RS_CHECK(stage_in(occ, sizeof(double) * nb, "adj_occ", (void**)&docc));
     if (dl_dv) {
         RS_CHECK(workspace_t("adj_dv", (size_t)c.ml, &gv));
-        launch(k_vloc_adjoint, div_up(c.ml, 256), 256, 0, c.stream, dp, dc, ld, nb, docc, c.dV, c.ml, gv);
-        RS_LAUNCH();
+        RS_CHECK(vloc_adjoint(dp, dc, ld, nb, docc, c.dV, c.ml, gv));
         RS_CHECK(stage_out(dl_dv, gv, sizeof(double) * c.ml));
     }
     if (dl_dr) {
@@ -275,9 +345,7 @@ int rsdft_gpu_calc_density(const double* unk, long ld, int mb, const double* occ
     RS_CHECK(stage_in(occ, sizeof(double) * mb, "adj_occ", (void**)&docc));
     RS_CHECK(workspace_t("adj_dv", (size_t)c.ml, &dr));
     // the V-part adjoint with unit volume element: sum_n occ_n psi_n^2
-    launch(k_vloc_adjoint, div_up(c.ml, 256), 256, 0, c.stream, dp, (const double*)nullptr, ld, mb,
-           (const double*)docc, 1.0, c.ml, dr);
-    RS_LAUNCH();
+    RS_CHECK(vloc_adjoint(dp, nullptr, ld, mb, docc, 1.0, c.ml, dr));
     RS_CHECK(stage_out(rho, dr, sizeof(double) * c.ml));
     (void)sp;
     return RSDFT_OK;

@@ -28,7 +28,8 @@ def test_cg_forms(gpu, n, nb, mloop, ncg, scale):
     q = np.linalg.qr(c.psi0(nb))[0] * (scale / np.sqrt(c.dV))
     q = np.asfortranarray(q)
     ru, resp, rres, _ = o.conjugate_gradient(q, ncg, mloop)
-    u = torch.from_numpy(np.ascontiguousarray(q.T)).cuda().t()
+    u = api.fortran_empty(c.ML, nb)
+    u.copy_(torch.from_numpy(q))
     esp = torch.zeros(nb, dtype=torch.float64, device="cuda")
     res = torch.zeros_like(esp)
     gpu.conjugate_gradient(1, c.ML, nb, 1, 1, u, esp, res, ncg=ncg, mloop=mloop)
@@ -37,7 +38,8 @@ def test_cg_forms(gpu, n, nb, mloop, ncg, scale):
     assert rel(esp.cpu().numpy(), resp) <= TOL
     assert rel(res.cpu().numpy(), rres) <= TOL
     # the FP32 form of the same sweep: eps(FP32) = 6e-8 per operation, a few line steps
-    x = torch.from_numpy(np.ascontiguousarray(q.T)).cuda().t()
+    x = api.fortran_empty(c.ML, nb)
+    x.copy_(torch.from_numpy(q))
     gpu.conjugate_gradient(1, c.ML, nb, 1, 1, x, esp, res, ncg=ncg, mloop=mloop, mode=api.MODE_MIXED_BF16X3)
     gpu.synchronize()
     assert rel(x.cpu().numpy(), ru) <= 1e-4
