@@ -95,9 +95,10 @@ __global__ void __launch_bounds__(VT) k_multidot(const T* v0, const T* v1, const
     double acc[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) acc[k] = 0.0;
-    const long base = (long)blockIdx.x * VCHUNK;
+    const int items = vec_items(n);
+    const long base = (long)blockIdx.x * (VT * items);
 #pragma unroll 4
-    for (int j = 0; j < VITEMS / W; ++j) {
+    for (int j = 0; j < items / W; ++j) {
         const long i = base + ((long)j * VT + threadIdx.x) * W;
         T vv[NV][W];
         if (vec && i + W <= n) {
@@ -126,7 +127,7 @@ __global__ void __launch_bounds__(VT) k_multidot(const T* v0, const T* v1, const
 }
 
 // g = -c1 (hx - E x); partial |g|^2 (cg_module.f90:186-190)
-template <typename T>
+template <typename T, int IT>
 __global__ void __launch_bounds__(VT) k_cg_g(CGVec<T> v, long ld, long n, const double* __restrict__ E,
                                              double* __restrict__ part, int vec) {
     using G = Grp16<T>;
@@ -135,9 +136,10 @@ __global__ void __launch_bounds__(VT) k_cg_g(CGVec<T> v, long ld, long n, const 
     const int b = blockIdx.y;
     const T e = (T)E[b];
     double acc = 0.0;
-    const long base = (long)blockIdx.x * VCHUNK, off = (long)b * ld;
+    const int items = vec_items<IT>(n);
+    const long base = (long)blockIdx.x * (VT * items), off = (long)b * ld;
 #pragma unroll 4
-    for (int j = 0; j < VITEMS / W; ++j) {
+    for (int j = 0; j < items / W; ++j) {
         const long i = base + ((long)j * VT + threadIdx.x) * W;
         if (vec && i + W <= n) {
             T hx[W], x[W], g[W];
@@ -168,13 +170,14 @@ __global__ void __launch_bounds__(VT) k_pc0(CGVec<T> v, long ld, long n, PcArgs 
     __shared__ double sh[VT / 32];
     const int b = blockIdx.y;
     if (active && !active[b]) return;
-    const long off = (long)b * ld, base = (long)blockIdx.x * VCHUNK;
+    const int items = vec_items(n);
+    const long off = (long)b * ld, base = (long)blockIdx.x * (VT * items);
     const T* g = v.g + off;
     double acc = 0.0;
     int i1, i2, i3;
     pc_coords(base + threadIdx.x, pa, i1, i2, i3);
-#pragma unroll 8
-    for (int it = 0; it < VITEMS; ++it) {
+#pragma unroll 4
+    for (int it = 0; it < items; ++it) {
         const long i = base + it * VT + threadIdx.x;
         if (i < n) {
             const T gi = g[i];
@@ -198,13 +201,14 @@ __global__ void __launch_bounds__(VT) k_pc1(CGVec<T> v, long ld, long n, PcArgs 
     __shared__ double sh[VT / 32];
     const int b = blockIdx.y;
     if (active && !active[b]) return;
-    const long off = (long)b * ld, base = (long)blockIdx.x * VCHUNK;
+    const int items = vec_items(n);
+    const long off = (long)b * ld, base = (long)blockIdx.x * (VT * items);
     const T* q = v.q + off;
     double acc = 0.0;
     int i1, i2, i3;
     pc_coords(base + threadIdx.x, pa, i1, i2, i3);
-#pragma unroll 8
-    for (int it = 0; it < VITEMS; ++it) {
+#pragma unroll 4
+    for (int it = 0; it < items; ++it) {
         const long i = base + it * VT + threadIdx.x;
         if (i < n) {
             const T f = pc_apply<T>(q, i, i1, i2, i3, pa);
@@ -224,11 +228,12 @@ __global__ void __launch_bounds__(VT) k_pc2(CGVec<T> v, long ld, long n, const d
     __shared__ double sh[VT / 32];
     const int b = blockIdx.y;
     if (active && !active[b]) return;
-    const long off = (long)b * ld, base = (long)blockIdx.x * VCHUNK;
+    const int items = vec_items(n);
+    const long off = (long)b * ld, base = (long)blockIdx.x * (VT * items);
     const T a = (T)pa_[b];
     double acc = 0.0;
-#pragma unroll 8
-    for (int it = 0; it < VITEMS; ++it) {
+#pragma unroll 4
+    for (int it = 0; it < items; ++it) {
         const long i = base + it * VT + threadIdx.x;
         if (i < n) {
             const T qi = v.q[off + i];
@@ -252,10 +257,11 @@ __global__ void __launch_bounds__(VT) k_pc3(CGVec<T> v, long ld, long n, const d
                                             const int* __restrict__ active) {
     const int b = blockIdx.y;
     if (active && !active[b]) return;
-    const long off = (long)b * ld, base = (long)blockIdx.x * VCHUNK;
+    const int items = vec_items(n);
+    const long off = (long)b * ld, base = (long)blockIdx.x * (VT * items);
     const T bb = (T)pb_[b];
-#pragma unroll 8
-    for (int it = 0; it < VITEMS; ++it) {
+#pragma unroll 4
+    for (int it = 0; it < items; ++it) {
         const long i = base + it * VT + threadIdx.x;
         if (i < n) v.q[off + i] = v.r[off + i] + bb * v.q[off + i];
     }
@@ -267,10 +273,11 @@ __global__ void __launch_bounds__(VT) k_cg_p(CGVec<T> v, long ld, long n, const 
                                              int first, const int* __restrict__ active) {
     const int b = blockIdx.y;
     if (active && !active[b]) return;
-    const long off = (long)b * ld, base = (long)blockIdx.x * VCHUNK;
+    const int items = vec_items(n);
+    const long off = (long)b * ld, base = (long)blockIdx.x * (VT * items);
     const T bk = (T)bk_[b];
-#pragma unroll 8
-    for (int it = 0; it < VITEMS; ++it) {
+#pragma unroll 4
+    for (int it = 0; it < items; ++it) {
         const long i = base + it * VT + threadIdx.x;
         if (i < n) v.p[off + i] = first ? v.Pg[off + i] : v.Pg[off + i] + bk * v.p[off + i];
     }
@@ -289,7 +296,7 @@ __device__ __forceinline__ T cg_g_elem(T g, T hp, T x, T p, T u11, T u21, T w, T
     return fma(u11, g, (T)(-2.0) * fma(xe, x, u21 * fma(-w, p, hp)));
 }
 
-template <typename T, bool FIRST>
+template <typename T, bool FIRST, int IT>
 __global__ void __launch_bounds__(VT) k_cg_upd1(CGVec<T> v, long ld, long n, CGScal s, double* __restrict__ part,
                                                 const int* __restrict__ active, int vec) {
     using G = Grp16<T>;
@@ -297,13 +304,14 @@ __global__ void __launch_bounds__(VT) k_cg_upd1(CGVec<T> v, long ld, long n, CGS
     __shared__ double sh[VT / 32];
     const int b = blockIdx.y;
     if (active && !active[b]) return;
-    const long off = (long)b * ld, base = (long)blockIdx.x * VCHUNK;
+    const int items = vec_items<IT>(n);
+    const long off = (long)b * ld, base = (long)blockIdx.x * (VT * items);
     const T u11 = (T)s.u11[b], u21 = (T)s.u21[b], w = (T)s.E[b];
     const T xe = (T)(s.u11[b] * (s.E1[b] - s.E[b]));  // E1: the step's old quotient
     const T* gin = FIRST ? v.hx : v.g;
     double acc = 0.0;
 #pragma unroll 4
-    for (int j = 0; j < VITEMS / W; ++j) {
+    for (int j = 0; j < items / W; ++j) {
         const long i = base + ((long)j * VT + threadIdx.x) * W;
         if (vec && i + W <= n) {
             T hp[W], x[W], p[W], g[W];
@@ -337,10 +345,11 @@ __global__ void __launch_bounds__(VT) k_cg_upd2(CGVec<T> v, long ld, long n, CGS
     constexpr int W = G::W;
     const int b = blockIdx.y;
     if (!s.pend[b]) return;
-    const long off = (long)b * ld, base = (long)blockIdx.x * VCHUNK;
+    const int items = vec_items(n);
+    const long off = (long)b * ld, base = (long)blockIdx.x * (VT * items);
     const T u11 = (T)s.u11[b], u21 = (T)s.u21[b];
 #pragma unroll 4
-    for (int j = 0; j < VITEMS / W; ++j) {
+    for (int j = 0; j < items / W; ++j) {
         const long i = base + ((long)j * VT + threadIdx.x) * W;
         if (vec && i + W <= n) {
             T x[W], p[W];
@@ -358,7 +367,7 @@ __global__ void __launch_bounds__(VT) k_cg_upd2(CGVec<T> v, long ld, long n, CGS
 
 // The end of a sweep: the x update that the last line step left pending (apply
 // != 0), x in FP64 to out64 and H x = E x - g / 2 to hx where they are given.
-template <typename T>
+template <typename T, int IT>
 __global__ void __launch_bounds__(VT) k_cg_end(CGVec<T> v, long ld, long n, CGScal s, int apply, T* __restrict__ hx,
                                                double* __restrict__ out64, int vec) {
     using G = Grp16<T>;
@@ -366,10 +375,11 @@ __global__ void __launch_bounds__(VT) k_cg_end(CGVec<T> v, long ld, long n, CGSc
     const int b = blockIdx.y;
     const bool upd = apply && s.pend[b];
     if (!upd && !hx && !out64) return;
-    const long off = (long)b * ld, base = (long)blockIdx.x * VCHUNK;
+    const int items = vec_items<IT>(n);
+    const long off = (long)b * ld, base = (long)blockIdx.x * (VT * items);
     const T u11 = upd ? (T)s.u11[b] : (T)1, u21 = upd ? (T)s.u21[b] : (T)0, e = (T)s.E[b];
 #pragma unroll 4
-    for (int j = 0; j < VITEMS / W; ++j) {
+    for (int j = 0; j < items / W; ++j) {
         const long i = base + ((long)j * VT + threadIdx.x) * W;
         if (vec && i + W <= n) {
             T x[W];
@@ -583,11 +593,12 @@ __global__ void __launch_bounds__(VT) k_resid(const double* __restrict__ x, cons
                                               long n, const double* __restrict__ e, double* __restrict__ part) {
     __shared__ double sh[VT / 32];
     const int b = blockIdx.y;
-    const long off = (long)b * ld, base = (long)blockIdx.x * VCHUNK;
+    const int items = vec_items(n);
+    const long off = (long)b * ld, base = (long)blockIdx.x * (VT * items);
     const double eb = e[b];
     double acc = 0.0;
-#pragma unroll 8
-    for (int it = 0; it < VITEMS; ++it) {
+#pragma unroll 4
+    for (int it = 0; it < items; ++it) {
         const long i = base + it * VT + threadIdx.x;
         if (i < n) {
             const double r = hx[off + i] - eb * x[off + i];
@@ -611,7 +622,7 @@ int esp_device(const double* x, long ld, int nb, int spin, double* e, double* re
     Context& c = ctx();
     cudaStream_t st = c.stream;
     const long n = c.ml;
-    const int nchunk = div_up(n, VCHUNK);
+    const int nchunk = vec_chunks(n, nb, c.num_sms > 0 ? c.num_sms : 148);
     double *hx = nullptr, *part = nullptr;
     RS_CHECK(workspace_t("esp_hx", (size_t)ld * nb, &hx));
     RS_CHECK(workspace_t("esp_part", (size_t)nb * nchunk, &part));
@@ -631,14 +642,17 @@ int esp_device(const double* x, long ld, int nb, int spin, double* e, double* re
 
 // ------------------------------------------------------------ driver
 // hx_out (if given) receives the sweep's H x (in the CG workspace); out64 (if
-// given) the bands in FP64 in place of the update of x.
+// given) the bands in FP64 in place of the update of x.  plan_mb: the band count
+// that launch geometry and partial sums are chosen for, the whole set's when x
+// is a block of it (0: mb).
 template <typename T>
 static int cg_run(T* x, long ld, int mb, int spin, double* esp, double* res, int ncg, int mloop, int ipc,
-                  const T** hx_out = nullptr, double* out64 = nullptr) {
+                  const T** hx_out = nullptr, double* out64 = nullptr, int plan_mb = 0) {
+    if (plan_mb == 0) plan_mb = mb;
     Context& c = ctx();
     cudaStream_t st = c.stream;
     const long n = c.ml;
-    const int nchunk = div_up(n, VCHUNK);
+    const int nchunk = vec_chunks(n, plan_mb, c.num_sms > 0 ? c.num_sms : 148);
     const size_t vec = (size_t)ld * mb;
     CGVec<T> v{};
     v.x = x;
@@ -666,6 +680,7 @@ static int cg_run(T* x, long ld, int mb, int spin, double* esp, double* res, int
     // five line-search dots, <psi|H psi>, the basis passes
     HpsiDot hd;
     hd.cap = hpsi_dot_cap(c.n1, c.n2, c.n3);
+    hd.plan_nb = plan_mb;
     const int pcap = std::max(nchunk, 64);
     double* part = nullptr;
     RS_CHECK(workspace_t("cg_part", (size_t)mb * ((size_t)nchunk * 6 + hd.cap + (size_t)(SS_MAXM + 1) * 2 * pcap),
@@ -675,6 +690,7 @@ static int cg_run(T* x, long ld, int mb, int spin, double* esp, double* res, int
     double* pbasis = hd.part + (size_t)mb * hd.cap;
 
     const dim3 vg(nchunk, mb);
+    const bool full = vec_full(n, nchunk);
     const int sb = div_up(mb, 128), wb = div_up(mb, SB / 32);
     const double dV = c.dV, tol = cg_stop_tol<T>();
     const int gv = grp16_ok<T>(ld, {x, base, out64}) ? 1 : 0;  // 16-byte element groups
@@ -686,7 +702,7 @@ static int cg_run(T* x, long ld, int mb, int spin, double* esp, double* res, int
 
     RS_CHECK(hpsi_device<T>(x, v.hx, ld, mb, spin, nullptr, &hd));
     launch(s_start, wb, SB, 0, st, s, hpsi_sum_of(hd), mb);
-    launch(k_cg_g<T>, vg, VT, 0, st, v, ld, n, s.E, part, gv);
+    launch(full ? k_cg_g<T, 32> : k_cg_g<T, 0>, vg, VT, 0, st, v, ld, n, s.E, part, gv);
     launch(s_step, wb, SB, 0, st, s, (const double*)part, nchunk, dV, mb, 1, ncg == 0, tol, esp, res);
     RS_LAUNCH();
 
@@ -698,7 +714,7 @@ static int cg_run(T* x, long ld, int mb, int spin, double* esp, double* res, int
             // q, Pg, hp, which are free until hpsi(p)).  The pass also makes
             // the previous step's x update, as it reads the old p anyway.
             const SSVec<T> sv{{v.r, v.q, v.Pg, v.hp}};
-            RS_CHECK(sstep_precond<T>(v.g, icg == 1 ? v.hx : (const T*)nullptr, sv, v.p, x, ld, mb, mloop, s, cz, pbasis, pcap, pdots, pa, dV));
+            RS_CHECK(sstep_precond<T>(v.g, icg == 1 ? v.hx : (const T*)nullptr, sv, v.p, x, ld, mb, plan_mb, mloop, s, cz, pbasis, pcap, pdots, pa, dV));
         } else {
             // --- preconditioning (Pgk = gk on entry)
             if (ipc == 4 && mloop > 0) {
@@ -731,14 +747,16 @@ static int cg_run(T* x, long ld, int mb, int spin, double* esp, double* res, int
         }
         RS_CHECK(hpsi_device<T>(v.p, v.hp, ld, mb, spin, s.active, &hd));
         launch(s_eig, wb, SB, 0, st, s, (const double*)pdots, nchunk, hpsi_sum_of(hd), mb, icg == 1);
-        launch(icg == 1 ? k_cg_upd1<T, true> : k_cg_upd1<T, false>, vg, VT, 0, st, v, ld, n, s, part, s.active, gv);
+        launch(icg == 1 ? (full ? k_cg_upd1<T, true, 32> : k_cg_upd1<T, true, 0>)
+                        : (full ? k_cg_upd1<T, false, 32> : k_cg_upd1<T, false, 0>),
+               vg, VT, 0, st, v, ld, n, s, part, s.active, gv);
         launch(s_step, wb, SB, 0, st, s, (const double*)part, nchunk, dV, mb, 0, icg == ncg, tol, esp, res);
         if (!sstep) launch(k_cg_upd2<T>, vg, VT, 0, st, v, ld, n, s, gv);
         RS_LAUNCH();
     }
     T* hx = hx_out && ncg > 0 ? v.hx : nullptr;
     if (hx_out) *hx_out = v.hx;
-    launch(k_cg_end<T>, vg, VT, 0, st, v, ld, n, s, sstep ? 1 : 0, hx, out64, gv);
+    launch(full ? k_cg_end<T, 32> : k_cg_end<T, 0>, vg, VT, 0, st, v, ld, n, s, sstep ? 1 : 0, hx, out64, gv);
     RS_LAUNCH();
     return RSDFT_OK;
 }
@@ -804,7 +822,7 @@ int cg_device_f32_staged(const double* unk_host, double* unk_dev, long ld, int m
         launch(k_convert<float>, 4 * c.num_sms, 256, 0, c.stream, (const double*)(unk_dev + (size_t)b0 * ld), xb, n);
         RS_LAUNCH();
         const float* hx = nullptr;
-        RS_CHECK(cg_run<float>(xb, ld, nb, spin, esp + b0, res + b0, ncg, mloop, ipc, &hx));
+        RS_CHECK(cg_run<float>(xb, ld, nb, spin, esp + b0, res + b0, ncg, mloop, ipc, &hx, nullptr, mb));
         // this block's H x out of the CG workspace, and its rejection flag
         int* flags = nullptr;
         RS_CHECK(workspace_t("cg_flags", (size_t)nb * 3 + 1, &flags));

@@ -11,9 +11,32 @@
 
 namespace rsdft {
 
-constexpr int VT = 256;           // threads per vector CTA
-constexpr int VITEMS = 32;        // elements per thread
-constexpr int VCHUNK = VT * VITEMS;
+constexpr int VT = 256;  // threads per vector CTA
+
+// Chunks per band of the vector kernels.  A thread takes 32 points of its
+// CTA's chunk where the bands alone fill the GPU, and down to 4 for a small
+// block, until there are about eight CTAs per SM: there the CTA's chain of
+// dependent trips is the whole time (search-direction pass at 24^3 x 32:
+// 15.6 us at 32 points, 5.5 us at 4).
+inline int vec_chunks(long n, int nb, int sms) {
+    int items = 32;
+    while (items > 4 && (n + (long)VT * items - 1) / ((long)VT * items) * nb < 8L * sms) items /= 2;
+    return (int)((n + (long)VT * items - 1) / ((long)VT * items));
+}
+
+// whether a launch over nchunk chunks has 32 points per thread; the hot
+// kernels are compiled for that (IT = 32) and for a run-time count (IT = 0),
+// which costs them 1 to 3 %
+inline bool vec_full(long n, int nchunk) { return (n + VT * 32L - 1) / (VT * 32L) == nchunk; }
+
+// points per thread of a launch with gridDim.x chunks over n points
+template <int IT = 0>
+__device__ __forceinline__ int vec_items(long n) {
+    if (IT > 0) return IT;
+    int items = 4;
+    while ((long)VT * items * gridDim.x < n) items *= 2;
+    return items;
+}
 
 // 16-byte element groups of the vector kernels: a thread takes W = 16 /
 // sizeof(T) consecutive elements per step (one vector access per stream);
@@ -162,11 +185,12 @@ __device__ __forceinline__ T pc_offdiag(const T* __restrict__ f, long i, int i1,
 // Preconditioner + search direction of one CG step in the s-step form:
 // p = Pg (first) or Pg + bk p, with rb = dV <Pg|g> and gkgk updated in s, and
 // the line search's dots of x, p, g as per-CTA partials in dots (5 per chunk).
-// hx: H x in the first step, null later (k_ss_p).
+// hx: H x in the first step, null later (k_ss_p).  plan_mb: the band count the
+// launch geometry is chosen for.
 // cz holds SS_MAXM doubles per band, part (SS_MAXM + 1) x 2 x part_cap per
 // band.
 template <typename T>
-int sstep_precond(const T* g, const T* hx, const SSVec<T>& sv, T* p, T* x, long ld, int mb, int mloop, const CGScal& s,
-                  double* cz, double* part, int part_cap, double* dots, const PcArgs& pa, double dV);
+int sstep_precond(const T* g, const T* hx, const SSVec<T>& sv, T* p, T* x, long ld, int mb, int plan_mb, int mloop,
+                  const CGScal& s, double* cz, double* part, int part_cap, double* dots, const PcArgs& pa, double dV);
 
 }  // namespace rsdft

@@ -630,6 +630,18 @@ __global__ void __launch_bounds__(128) k_nl_scatter(T* __restrict__ hpsi, long l
     }
 }
 
+// Bands per scatter thread: 32, so that a point's entries are read from L1 for
+// 15 of 16 band pairs, and fewer for a small block, down to one pair, until
+// there are eight CTAs per SM (a thread's pairs are a serial chain: 24^3 x 32
+// takes 16.6 us at 32 bands per thread, 2.8 us at 4).
+static int scatter_chunk(int nb) {
+    const Context& c = ctx();
+    const long sms = c.num_sms > 0 ? c.num_sms : 148;
+    int bch = 32;
+    while (bch > SC_BU && (long)div_up(c.nl_npt, 128) * div_up(nb, bch) < 8 * sms) bch /= 2;
+    return bch;
+}
+
 template <typename T, int MD, int TX>
 static void launch_stencil_tx(const StencilArgs<T>& a, const StencilCoef& cf, int nb, cudaStream_t st) {
     dim3 grid(div_up(a.n1, TX), div_up(a.n2, 16), nb * a.nzc);
@@ -652,19 +664,25 @@ static void launch_stencil_md(const StencilArgs<T>& a, const StencilCoef& cf, in
 // read), ring depth S >= 3, consumer warps ncw, one producer warp, at most
 // 384 threads (the register budget of the 2 Md + 1 accumulators).
 struct TmaGeom {
-    int TY = 0, RS = 0, S = 0, ncw = 0, threads = 0;
+    int TY = 0, RS = 0, S = 0, ncw = 0, threads = 0, nzc = 1;
     size_t smem = 0;
 };
 
+// The tile height and z split of least march_cost.  A plane costs about 500
+// cycles of latency plus 1.1 x its shared-memory wavefronts (window loads and
+// TMA fill); a halo plane, which feeds the z accumulators only, a quarter.
+// That reproduces 2140 cycles per plane at 72^3 FP64 (TY = 18) and 1940 FP32
+// (TY = 36), and 26 us for 24^3 x 32 bands in one z chunk (measured 27.6),
+// which the split takes to 12.5 us.
 template <typename T, int MD, int BY>
-static TmaGeom tma_geometry(int n1, int n2) {
+static TmaGeom tma_geometry(int n1, int n2, int nz, int nb, int sms, int dot_cap) {
     TmaGeom best;
     constexpr int VX = 16 / (int)sizeof(T);
     constexpr int MDX = (MD + VX - 1) / VX * VX;
     const int RS = (int)((((size_t)n1 * sizeof(T) + 127) / 128) * 128 / sizeof(T));
     if (n1 % VX != 0 || n1 < MDX || RS > 256 || n2 < MD) return best;
     const size_t budget = 220 * 1024;
-    double best_score = -1.0;
+    double best_cost = 0.0;
     for (int TY = BY; TY <= std::min(n2, 256 - 2 * MD); TY += BY) {
         if (n2 % TY != 0 || TY < MD || !(TY == n2 || n2 >= TY + MD)) continue;
         const int ncw = ((n1 / VX) * (TY / BY) + 31) / 32;
@@ -673,16 +691,23 @@ static TmaGeom tma_geometry(int n1, int n2) {
         const size_t stage = (size_t)(2 * TY + 2 * MD) * RS * sizeof(T);
         const int S = (int)std::min<size_t>(budget / (stage + 16), 8);
         if (S < 3) continue;
-        // halo overhead first, then busy threads, then ring depth
-        const double used = (double)((n1 / VX) * (TY / BY)) / threads;
-        const double score = 100.0 * TY / (TY + 2 * MD) + 10.0 * used + 0.1 * S;
-        if (score > best_score) {
-            best_score = score;
+        const int tiles = n2 / TY;
+        const int zmax = std::min({std::max(1, nz / 4), 65535 / nb, dot_cap / tiles});
+        if (zmax < 1) continue;
+        // window loads per thread: BY + 2 Md rows, 2 MDX / VX vectors of each
+        // own row, Vloc
+        const double loads = BY + 2 * MD + BY * (2.0 * MDX / VX) + BY;
+        const double t = 500.0 + 1.1 * (4.0 * loads * ncw + (2.0 * TY + 2 * MD) * RS * sizeof(T) / 128.0);
+        int nzc = 1;
+        const double cost = march_cost((long)tiles * nb, nz, 2 * MD, zmax, sms, t, 0.25 * t, &nzc);
+        if (best.TY == 0 || cost <= 1.05 * best_cost) {  // the taller tile at a near tie
+            best_cost = best.TY == 0 ? cost : std::min(cost, best_cost);
             best.TY = TY;
             best.RS = RS;
             best.S = S;
             best.ncw = ncw;
             best.threads = threads;
+            best.nzc = nzc;
             best.smem = (size_t)S * stage + (size_t)S * 16 + 12 * sizeof(double);
         }
     }
@@ -704,19 +729,14 @@ template <typename T, int MD, int BY>
 static int launch_tma(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStream_t st, HpsiDot* dot, bool* used) {
     Context& c = ctx();
     *used = false;
-    const TmaGeom g = tma_geometry<T, MD, BY>(a.n1, a.n2);
+    const int sms = c.num_sms > 0 ? c.num_sms : 148;
+    const TmaGeom g = tma_geometry<T, MD, BY>(a.n1, a.n2, a.nzo, dot && dot->plan_nb ? dot->plan_nb : nb, sms,
+                                                dot ? dot->cap : 1 << 20);
     if (g.TY == 0) return RSDFT_OK;
     if (reinterpret_cast<uintptr_t>(a.hpsi) % 16 != 0 || (a.ld * sizeof(T)) % 16 != 0) return RSDFT_OK;
-    const int sms = c.num_sms > 0 ? c.num_sms : 148;
-    const long base = (long)(a.n2 / g.TY) * nb;
-    int nzc = (int)std::min<long>(std::max<long>(1, (sms + base - 1) / base), std::max(1, a.nzo / (4 * MD)));
-    while (((long)nb * nzc > 65535 || (dot && (a.n2 / g.TY) * nzc > dot->cap)) && nzc > 1) --nzc;
-    a.zlen = div_up(a.nzo, nzc);
+    a.zlen = div_up(a.nzo, g.nzc);
     a.nzc = div_up(a.nzo, a.zlen);
-    if (dot) {
-        a.ndot = (a.n2 / g.TY) * a.nzc;
-        if (a.ndot > dot->cap) return RSDFT_OK;
-    }
+    if (dot) a.ndot = (a.n2 / g.TY) * a.nzc;
     TmaMaps maps;
     const CUtensorMapDataType dt = sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     const unsigned long long dims[4] = {(unsigned long long)a.n1, (unsigned long long)a.n2,
@@ -757,9 +777,9 @@ static int launch_stencil_md2(StencilArgs<T> a, const StencilCoef& cf, int nb, c
     RS_CHECK((launch_tma<T, MD, (MD <= 6 ? 2 : 1)>(a, cf, nb, st, dot, &used)));
     if (used) {
         if (a.gpt_ptr && c.nl_npt > 0) {
-            constexpr int BCH = 32;
-            dim3 grid(div_up(c.nl_npt, 128), div_up(nb, BCH));
-            launch(k_nl_scatter<T>, grid, 128, 0, st, a.hpsi, a.ld, nb, BCH, (const int*)c.nl_pts,
+            const int bch = scatter_chunk(nb);
+            dim3 grid(div_up(c.nl_npt, 128), div_up(nb, bch));
+            launch(k_nl_scatter<T>, grid, 128, 0, st, a.hpsi, a.ld, nb, bch, (const int*)c.nl_pts,
                    (const int*)c.nl_ptr, c.nl_npt, a.gpt_grp, a.gpt_uv4, a.uvunk, a.nzlma, a.band_active,
                    c.err_flag);
             RS_LAUNCH();
@@ -769,7 +789,7 @@ static int launch_stencil_md2(StencilArgs<T> a, const StencilCoef& cf, int nb, c
     // general shapes (odd widths, very wide rows): register-queue kernel with
     // per-plane halo loads and the nonlocal scatter fused
     const int tx = (a.n1 % 32 == 0 || a.n1 > 24) ? 32 : (a.n1 % 24 == 0 ? 24 : 16);
-    const long base = (long)div_up(a.n1, tx) * div_up(a.n2, 16) * nb;
+    const long base = (long)div_up(a.n1, tx) * div_up(a.n2, 16) * (dot && dot->plan_nb ? dot->plan_nb : nb);
     const long want = 8L * (c.num_sms > 0 ? c.num_sms : 148);
     int nzc = (int)std::min<long>(std::max<long>(1, (want + base - 1) / base), std::max(1, a.nzo / 8));
     const int nxy = div_up(a.n1, tx) * div_up(a.n2, 16);
@@ -981,9 +1001,9 @@ extern "C" int rsdft_gpu_op_nonlocal_add(const double* uvunk, double* htpsi, lon
     double* dh;
     bool sh;
     RS_CHECK(wf_acquire(htpsi, ld, nb, "ham_out", &dh, &sh));
-    constexpr int BCH = 32;
-    dim3 grid(div_up(c.nl_npt, 128), div_up(nb, BCH));
-    launch(k_nl_scatter<double>, grid, 128, 0, c.stream, dh, ld, nb, BCH, (const int*)c.nl_pts, (const int*)c.nl_ptr,
+    const int bch = scatter_chunk(nb);
+    dim3 grid(div_up(c.nl_npt, 128), div_up(nb, bch));
+    launch(k_nl_scatter<double>, grid, 128, 0, c.stream, dh, ld, nb, bch, (const int*)c.nl_pts, (const int*)c.nl_ptr,
            c.nl_npt, (const int*)c.gpt_grp, (const double*)c.gpt_uv4, (const double*)du, c.nzlma, (const int*)nullptr,
            c.err_flag);
     RS_LAUNCH();

@@ -11,10 +11,13 @@ namespace rsdft {
 // a fixed order: per band, nch grid partials at part[band * nch], and unless
 // with_nl the nonlocal part sum_l uvunk(l)^2 / (iuV(l) dV) on top (uvunk:
 // nzlma values per band, null without projectors).  A skipped band's partials
-// are not written.
+// are not written.  plan_nb: the band count the launch geometry, and with it the
+// grouping of the partials, is chosen for (0: the call's own), so that a set of
+// bands taken in blocks gives the bits of one call.
 struct HpsiDot {
     double* part = nullptr;  // nb * cap values
     int cap = 0;
+    int plan_nb = 0;
     int nch = 0;
     bool with_nl = false;
     const double* uvunk = nullptr;
@@ -72,6 +75,29 @@ __device__ __forceinline__ void block_sum_n(double (&v)[K], double* sh) {
         }
     }
     __syncthreads();
+}
+
+// Cost in SM cycles of a z march over nz output planes by nwork (tile, band)
+// pairs, each split into up to zmax z chunks: a CTA spends t_in cycles on each
+// of its planes, t_halo on each of `extra` halo planes and about 2000 on
+// start-up and the last stores, and conc CTAs run at a time.  Whole waves,
+// since the CTAs are equally long; 0.5 % per halo plane against each further
+// chunk (72^3 x 480 FP32, Md = 6, in two chunks: a model gain of 2 % without
+// that, a measured loss of 3 %).  *nzc receives the best split:
+// a small block is split until its CTAs fill the GPU, a large one only where
+// that evens out the last wave.
+inline double march_cost(long nwork, int nz, int extra, int zmax, long conc, double t_in, double t_halo, int* nzc) {
+    double best = 0.0;
+    for (int c = 1; c <= std::min(zmax, 12); ++c) {
+        const int zlen = (nz + c - 1) / c, n = (nz + zlen - 1) / zlen;
+        const double cost = (double)((nwork * n + conc - 1) / conc) * (zlen * t_in + extra * t_halo + 2000.0) *
+                            (1.0 + 0.005 * extra * (n - 1));
+        if (c == 1 || cost < best) {
+            best = cost;
+            *nzc = n;
+        }
+    }
+    return best;
 }
 
 // Symmetric-positive-definite orthonormalisation (CholeskyQR2 in the dV

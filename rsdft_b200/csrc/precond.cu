@@ -24,7 +24,8 @@ __global__ void __launch_bounds__(VT) k_ss_basis(const T* __restrict__ g, SSVec<
     __shared__ double sh[D * (VT / 32)];
     const int b = blockIdx.y;
     if (active && !active[b]) return;
-    const long off = (long)b * ld, base = (long)blockIdx.x * VCHUNK;
+    const int items = vec_items(n);
+    const long off = (long)b * ld, base = (long)blockIdx.x * (VT * items);
     const T* src = K == 0 ? g + off : sv.w[K > 0 ? K - 1 : 0] + off;
     const T inv_d = (T)(1.0 / pa.d);
     double acc[D];
@@ -32,8 +33,8 @@ __global__ void __launch_bounds__(VT) k_ss_basis(const T* __restrict__ g, SSVec<
     for (int k = 0; k < D; ++k) acc[k] = 0.0;
     int i1, i2, i3;
     pc_coords(base + threadIdx.x, pa, i1, i2, i3);
-#pragma unroll 8
-    for (int it = 0; it < VITEMS; ++it) {
+#pragma unroll 4
+    for (int it = 0; it < items; ++it) {
         const long i = base + it * VT + threadIdx.x;
         if (i < n) {
             const T si = src[i];
@@ -78,25 +79,26 @@ __global__ void __launch_bounds__(VT) k_ss_basis(const T* __restrict__ g, SSVec<
 // A basis pass therefore needs the dots of its source and its result only
 // (two per pass), and the last one a single dot of its source: it reads one
 // vector where a direct Gram matrix reads mloop + 1.
-__global__ void __launch_bounds__(128) s_sstep(CGScal s, SSPart pt, double* __restrict__ cz_out, int nb, int m,
-                                               double d, double dV, int first) {
+// The order m is a template parameter, so that the small arrays stay in
+// registers (6.3 us a launch; 14.8 with run-time loops over local memory).
+template <int m>
+__global__ void __launch_bounds__(128) s_sstep(CGScal s, SSPart pt, double* __restrict__ cz_out, int nb, double d,
+                                               double dV, int first) {
     const int b = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (b >= nb || !s.active[b]) return;  // uniform per warp
-    double S[2 * (SS_MAXM + 1)];
+    double S[2 * (m + 1)];
 #pragma unroll
-    for (int k = 0; k <= SS_MAXM; ++k) {
-        S[2 * k] = S[2 * k + 1] = 0.0;
-        if (k <= m) {
-            const int D = k < m ? 2 : 1;
-            const double* p = pt.part[k] + (long)b * pt.nch[k] * D;
-            S[2 * k] = warp_strided_sum(p, pt.nch[k], D, lane);
-            if (D == 2) S[2 * k + 1] = warp_strided_sum(p + 1, pt.nch[k], D, lane);
-        }
+    for (int k = 0; k <= m; ++k) {
+        const int D = k < m ? 2 : 1;
+        const double* p = pt.part[k] + (long)b * pt.nch[k] * D;
+        S[2 * k] = warp_strided_sum(p, pt.nch[k], D, lane);
+        S[2 * k + 1] = D == 2 ? warp_strided_sum(p + 1, pt.nch[k], D, lane) : 0.0;
     }
     if (lane != 0) return;
-    double mu[2 * SS_MAXM] = {}, gd[SS_MAXM] = {};
+    double mu[2 * m] = {}, gd[m] = {};
     mu[0] = S[1];
     gd[0] = S[0];
+#pragma unroll
     for (int k = 1; k <= m; ++k) {
         // <w_k, w_{k-1}>; the last pass leaves <S w_{m-1}, w_{m-1}>
         double c = S[2 * k];
@@ -104,48 +106,63 @@ __global__ void __launch_bounds__(128) s_sstep(CGScal s, SSPart pt, double* __re
         mu[2 * k - 1] = k == 1 ? c : 2.0 * c - mu[1];
         if (k < m) mu[2 * k] = 2.0 * S[2 * k + 1] - mu[0];
     }
+#pragma unroll
     for (int j = 1; j < m; ++j) {
         const double t = ((1.0 - d) * gd[j - 1] - mu[j - 1]) / d;
         gd[j] = j == 1 ? t : 2.0 * t - gd[j - 2];
     }
-    double G[SS_MAXM + 1][SS_MAXM + 1] = {};
+    double G[m + 1][m + 1] = {};
+#pragma unroll
     for (int i = 0; i < m; ++i)
-        for (int j = 0; j <= m; ++j) G[i][j] = G[j][i] = 0.5 * (mu[i + j] + mu[i > j ? i - j : j - i]);
-    double cz[SS_MAXM + 1] = {};
+    #pragma unroll
+    for (int j = 0; j <= m; ++j) G[i][j] = G[j][i] = 0.5 * (mu[i + j] + mu[i > j ? i - j : j - i]);
+    double cz[m + 1] = {};
     double rr = G[0][0];
     if (!(rr < 1e-24)) {
-        double r[SS_MAXM + 1] = {}, q[SS_MAXM + 1] = {}, ft[SS_MAXM + 1];
+        double r[m + 1] = {}, q[m + 1] = {}, ft[m + 1];
         r[0] = q[0] = 1.0;
-        for (int il = 1; il <= m; ++il) {
+    #pragma unroll
+    for (int il = 1; il <= m; ++il) {
             // ft = A q in the basis
-            for (int i = 0; i <= m; ++i) ft[i] = d * q[i];
+        #pragma unroll
+    for (int i = 0; i <= m; ++i) ft[i] = d * q[i];
             ft[1] += d * q[0];
-            for (int j = 1; j < m; ++j) {
+        #pragma unroll
+    for (int j = 1; j < m; ++j) {
                 ft[j + 1] += 0.5 * d * q[j];
                 ft[j - 1] += 0.5 * d * q[j];
             }
             double pAp = 0.0;
-            for (int i = 0; i <= m; ++i)
-                for (int j = 0; j <= m; ++j) pAp += q[i] * G[i][j] * ft[j];
+        #pragma unroll
+    for (int i = 0; i <= m; ++i)
+            #pragma unroll
+    for (int j = 0; j <= m; ++j) pAp += q[i] * G[i][j] * ft[j];
             const double a = rr / pAp;
-            for (int i = 0; i <= m; ++i) cz[i] += a * q[i];
+        #pragma unroll
+    for (int i = 0; i <= m; ++i) cz[i] += a * q[i];
             if (il == m) break;
-            for (int i = 0; i <= m; ++i) r[i] -= a * ft[i];
+        #pragma unroll
+    for (int i = 0; i <= m; ++i) r[i] -= a * ft[i];
             double rn = 0.0;
-            for (int i = 0; i <= m; ++i)
-                for (int j = 0; j <= m; ++j) rn += r[i] * G[i][j] * r[j];
+        #pragma unroll
+    for (int i = 0; i <= m; ++i)
+            #pragma unroll
+    for (int j = 0; j <= m; ++j) rn += r[i] * G[i][j] * r[j];
             const double bb = rn / rr;
             rr = rn;
-            for (int i = 0; i <= m; ++i) q[i] = r[i] + bb * q[i];
+        #pragma unroll
+    for (int i = 0; i <= m; ++i) q[i] = r[i] + bb * q[i];
         }
     }
     double gz = 0.0;
+#pragma unroll
     for (int j = 0; j < m; ++j) gz += cz[j] * gd[j];
     const double rb = s.rb[b] + dV * gz;
     s.rb[b] = rb;
     s.bk[b] = first ? 0.0 : rb / s.gkgk[b];
     s.gkgk[b] = rb;
-    for (int j = 0; j < SS_MAXM; ++j) cz_out[(long)b * SS_MAXM + j] = j < m ? cz[j] : 0.0;
+#pragma unroll
+    for (int j = 0; j < SS_MAXM; ++j) cz_out[(long)b * SS_MAXM + j] = j < m ? cz[j < m ? j : 0] : 0.0;
 }
 
 // p = g + sum_j cz_j w_j (+ bk p after the first step), the previous step's x
@@ -157,7 +174,7 @@ __global__ void __launch_bounds__(128) s_sstep(CGScal s, SSPart pt, double* __re
 // last two dots are <x|Hx> and <p|Hx> themselves: x may come in unnormalised,
 // E is then no Rayleigh quotient and the identity would cancel (1.7e-12 in
 // the residuals of a band of norm 27, against 1e-15 this way).
-template <typename T, int M>
+template <typename T, int M, int IT>
 __global__ void __launch_bounds__(VT) k_ss_p(const T* __restrict__ g, const T* __restrict__ hx, SSVec<T> sv,
                                              T* __restrict__ p, T* __restrict__ x, long ld, long n, const double* __restrict__ cz,
                                              const double* __restrict__ bk_,
@@ -171,7 +188,8 @@ __global__ void __launch_bounds__(VT) k_ss_p(const T* __restrict__ g, const T* _
     const bool act = active[b];
     const bool upd = pend && pend[b];  // the previous step's x update, which needs the old p
     if (!act && !upd) return;
-    const long off = (long)b * ld, base = (long)blockIdx.x * VCHUNK;
+    const int items = vec_items<IT>(n);
+    const long off = (long)b * ld, base = (long)blockIdx.x * (VT * items);
     T c[M];
 #pragma unroll
     for (int j = 0; j < M; ++j) c[j] = (T)cz[(long)b * SS_MAXM + j];
@@ -193,7 +211,7 @@ __global__ void __launch_bounds__(VT) k_ss_p(const T* __restrict__ g, const T* _
         acc[4] = fma(pd, gd, acc[4]);
     };
 #pragma unroll 2
-    for (int it = 0; it < VITEMS / W; ++it) {
+    for (int it = 0; it < items / W; ++it) {
         const long i = base + ((long)it * VT + threadIdx.x) * W;
         if (vec && i + W <= n) {
             T pv[W], xv[W];
@@ -538,19 +556,20 @@ __global__ void __launch_bounds__(384, PcStep<K, STORE>::CTAS) k_pc_tma(const __
 }
 
 // Geometry of k_pc_tma: TY (even, divides n2, n2 == TY or n2 >= TY + 1), row
-// pitch RS (n1 rounded up to 128 bytes), ring depth S (2..8), consumer warps.
+// pitch RS (n1 rounded up to 128 bytes), ring depth S (2..8), consumer warps
+// and the z split.  Chosen by march_cost as for the H psi stencil.
 struct PcGeom {
-    int TY = 0, RS = 0, S = 0, ncw = 0, threads = 0;
+    int TY = 0, RS = 0, S = 0, ncw = 0, threads = 0, nzc = 1;
     size_t smem = 0;
 };
 
 template <typename T>
-static PcGeom pc_geometry(int n1, int n2, int na, int d, int ctas) {
+static PcGeom pc_geometry(int n1, int n2, int n3, int mb, int sms, int part_cap, int na, int d, int ctas) {
     PcGeom best;
     constexpr int VX = 16 / (int)sizeof(T);
     const int RS = (int)((((size_t)n1 * sizeof(T) + 127) / 128) * 128 / sizeof(T));
     if (n1 % VX != 0 || n1 < VX || RS > 256 || n2 < 2) return best;
-    double best_score = -1.0;
+    double best_cost = 0.0;
     for (int TY = 2; TY <= std::min(n2, 254); TY += 2) {
         if (n2 % TY != 0 || !(TY == n2 || n2 >= TY + 1)) continue;
         const int ncw = ((n1 / VX) * (TY / 2) + 31) / 32;
@@ -562,15 +581,25 @@ static PcGeom pc_geometry(int n1, int n2, int na, int d, int ctas) {
         if (budget <= fixed) continue;
         const int S = (int)std::min<size_t>((budget - fixed) / (stage + 16), 8);
         if (S < 2) continue;
-        const double used = (double)((n1 / VX) * (TY / 2)) / threads;
-        const double score = 100.0 * TY / (TY + 2) + 10.0 * used + 2.0 * std::min(S, 4);
-        if (score > best_score) {
-            best_score = score;
+        const int tiles = n2 / TY;
+        const int zmax = std::min({std::max(1, n3 / 4), 65535 / mb, part_cap / tiles});
+        int nzc = 1;
+        if (zmax < 1) continue;
+        // cycles per plane: shared-memory wavefronts (window and epilogue
+        // loads, TMA fill) or the SM's share of HBM, times the CTAs sharing it
+        const double row = RS * sizeof(T);
+        const double lds = 1.1 * (ncw * 4.0 * (8 + 2 * na) + (TY + 2 + na * TY) * row / 128.0);
+        const double hbm = (TY + 2 + (na + 1) * TY) * row / 23.0;
+        const double t = 400.0 + ctas * std::max(lds, hbm);
+        const double cost = march_cost((long)tiles * mb, n3, 2, zmax, (long)ctas * sms, t, 0.3 * t, &nzc);
+        if (best.TY == 0 || cost <= 1.05 * best_cost) {  // the taller tile at a near tie
+            best_cost = best.TY == 0 ? cost : std::min(cost, best_cost);
             best.TY = TY;
             best.RS = RS;
             best.S = S;
             best.ncw = ncw;
             best.threads = threads;
+            best.nzc = nzc;
             best.smem = (size_t)S * stage + (size_t)S * 16 + fixed;
         }
     }
@@ -581,22 +610,18 @@ static PcGeom pc_geometry(int n1, int n2, int na, int d, int ctas) {
 // pointers do not suit it (the caller then takes the element-wise kernels).
 template <typename T, int K, bool STORE>
 static int pc_tma_step(const T* src, const T* const* aux, T* wout, const PcArgs& pa, long ld, int mb,
-                       const int* active, double* part, int part_cap, int* nchunk, bool* used) {
+                       int plan_mb, const int* active, double* part, int part_cap, int* nchunk, bool* used) {
     Context& c = ctx();
     *used = false;
     constexpr int NA = PcStep<K, STORE>::NA;
     constexpr int D = PcStep<K, STORE>::D;
     const int n1 = pa.n1, n2 = pa.n2, n3 = pa.n3;
-    const PcGeom g = pc_geometry<T>(n1, n2, NA, D, PcStep<K, STORE>::CTAS);
+    const int sms = c.num_sms > 0 ? c.num_sms : 148;
+    const PcGeom g = pc_geometry<T>(n1, n2, n3, plan_mb, sms, part_cap, NA, D, PcStep<K, STORE>::CTAS);
     if (g.TY == 0 || (ld * sizeof(T)) % 16 != 0) return RSDFT_OK;
     if (STORE && reinterpret_cast<uintptr_t>(wout) % 16 != 0) return RSDFT_OK;
-    const int sms = c.num_sms > 0 ? c.num_sms : 148;
-    const long base = (long)(n2 / g.TY) * mb;
-    int nzc = (int)std::min<long>(std::max<long>(1, (sms + base - 1) / base), std::max(1, n3 / 4));
-    while (((long)mb * nzc > 65535 || (n2 / g.TY) * nzc > part_cap) && nzc > 1) --nzc;
-    const int zlen = div_up(n3, nzc);
-    nzc = div_up(n3, zlen);
-    if ((n2 / g.TY) * nzc > part_cap) return RSDFT_OK;  // partials would not fit
+    const int zlen = div_up(n3, g.nzc);
+    const int nzc = div_up(n3, zlen);
     PcMaps maps;
     const CUtensorMapDataType dt = sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     const unsigned long long dims[4] = {(unsigned long long)n1, (unsigned long long)n2, (unsigned long long)n3,
@@ -635,13 +660,13 @@ static int pc_tma_step(const T* src, const T* const* aux, T* wout, const PcArgs&
 // basis step K of the s-step form through the TMA kernel (runtime K)
 template <typename T>
 static int pc_tma_dispatch(int K, bool store, const T* g, const SSVec<T>& sv, const PcArgs& pa, long ld, int mb,
-                           const int* active, double* part, int part_cap, int* nchunk, bool* used) {
+                           int plan_mb, const int* active, double* part, int part_cap, int* nchunk, bool* used) {
     const T* src = K == 0 ? g : sv.w[K - 1];
     const T* aux[1] = {K >= 2 ? sv.w[K - 2] : nullptr};
     T* wout = store ? sv.w[K] : nullptr;
 #define RS_PC_CASE(KK, ST)                                                                              \
     if (K == KK && store == ST)                                                                         \
-        return pc_tma_step<T, KK, ST>(src, aux, wout, pa, ld, mb, active, part, part_cap, nchunk, used);
+        return pc_tma_step<T, KK, ST>(src, aux, wout, pa, ld, mb, plan_mb, active, part, part_cap, nchunk, used);
     RS_PC_CASE(0, true)
     RS_PC_CASE(1, true)
     RS_PC_CASE(2, true)
@@ -656,12 +681,12 @@ static int pc_tma_dispatch(int K, bool store, const T* g, const SSVec<T>& sv, co
 }
 
 template <typename T>
-int sstep_precond(const T* g, const T* hx, const SSVec<T>& sv, T* p, T* x, long ld, int mb, int mloop, const CGScal& s,
-                  double* cz, double* part, int part_cap, double* dots, const PcArgs& pa, double dV) {
+int sstep_precond(const T* g, const T* hx, const SSVec<T>& sv, T* p, T* x, long ld, int mb, int plan_mb, int mloop,
+                  const CGScal& s, double* cz, double* part, int part_cap, double* dots, const PcArgs& pa, double dV) {
     const Context& c = ctx();
     cudaStream_t st = c.stream;
     const long n = c.ml;
-    const int nchunk = div_up(n, VCHUNK);
+    const int nchunk = vec_chunks(n, plan_mb, c.num_sms > 0 ? c.num_sms : 148);
     const dim3 vg(nchunk, mb);
     SSPart pt{};
     // basis steps: TMA z march where the shape allows, element-wise otherwise
@@ -670,7 +695,7 @@ int sstep_precond(const T* g, const T* hx, const SSVec<T>& sv, T* p, T* x, long 
         double* out = part + (size_t)k * 2 * part_cap * mb;
         bool used = false;
         int nch = 0;
-        RS_CHECK(pc_tma_dispatch<T>(k, store, g, sv, pa, ld, mb, s.active, out, part_cap, &nch, &used));
+        RS_CHECK(pc_tma_dispatch<T>(k, store, g, sv, pa, ld, mb, plan_mb, s.active, out, part_cap, &nch, &used));
         if (!used) {
             if (k == 0)
                 launch(k_ss_basis<T, 0, true>, vg, VT, 0, st, g, sv, ld, n, pa, out, s.active);
@@ -683,10 +708,11 @@ int sstep_precond(const T* g, const T* hx, const SSVec<T>& sv, T* p, T* x, long 
         pt.part[k] = out;
         pt.nch[k] = nch;
     }
-    launch(s_sstep, div_up(mb, 4), 128, 0, st, s, pt, cz, mb, mloop, pa.d, dV, hx ? 1 : 0);
     const int gv = grp16_ok<T>(ld, {g, hx, p, x, sv.w[0], sv.w[1], sv.w[2], sv.w[3]}) ? 1 : 0;
     auto launch_p = [&](auto M) {
-        launch(k_ss_p<T, decltype(M)::value>, vg, VT, 0, st, g, hx, sv, p, x, ld, n, (const double*)cz,
+        constexpr int MM = decltype(M)::value;
+        launch(s_sstep<MM>, div_up(mb, 4), 128, 0, st, s, pt, cz, mb, pa.d, dV, hx ? 1 : 0);
+        launch(vec_full(n, nchunk) ? k_ss_p<T, MM, 32> : k_ss_p<T, MM, 0>, vg, VT, 0, st, g, hx, sv, p, x, ld, n, (const double*)cz,
                (const double*)s.bk, (const int*)s.active, (const int*)(hx ? nullptr : s.pend),
                (const double*)s.u11, (const double*)s.u21, dots, gv);
     };
@@ -702,8 +728,8 @@ int sstep_precond(const T* g, const T* hx, const SSVec<T>& sv, T* p, T* x, long 
 }
 
 template int sstep_precond<double>(const double*, const double*, const SSVec<double>&, double*, double*, long, int,
-                                   int, const CGScal&, double*, double*, int, double*, const PcArgs&, double);
-template int sstep_precond<float>(const float*, const float*, const SSVec<float>&, float*, float*, long, int, int,
+                                   int, int, const CGScal&, double*, double*, int, double*, const PcArgs&, double);
+template int sstep_precond<float>(const float*, const float*, const SSVec<float>&, float*, float*, long, int, int, int,
                                   const CGScal&, double*, double*, int, double*, const PcArgs&, double);
 
 }  // namespace rsdft
