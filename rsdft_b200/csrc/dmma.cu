@@ -40,7 +40,7 @@ struct DmmaArgs {
     long K;
     long kchunk;      // K values per split (blockIdx.y), a multiple of DM_BK
     double alpha, beta;
-    double* partial;  // split-K: raw tile sums [split][tile][BM][BN]; C unused
+    double* partial;  // split-K: raw tile sums [split][tile][BM][BN], C unused; null: C written
     int sym;          // only tiles tm <= tn (a symmetric product)
     int ntm, ntiles;
 };
@@ -219,33 +219,59 @@ __global__ void __launch_bounds__(32 * WM * WN, CPS) k_dmma(DmmaArgs g) {
         }
 }
 
-// C(i, j) = alpha * sum over splits (fixed order) of the raw tile sums;
-// symmetric products read tiles below the diagonal transposed from the upper
-// ones; symmetrize returns alpha/2 (G + G^T).
-template <int BM, int BN>
-__global__ void k_dmma_reduce(const double* __restrict__ P, int nsplit, int ntiles, int ntm, int sym, int m,
-                              double alpha, int symmetrize, double* __restrict__ C, long ldc) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y;
-    if (i >= m) return;
-    auto fetch = [&](int r, int c) {
-        int tm = r / BM, tn = c / BN;
-        if (sym && tm > tn) {
-            const int t = r;
-            r = c;
-            c = t;
-            tm = r / BM;
-            tn = c / BN;
-        }
-        const int t = sym ? tn * (tn + 1) / 2 + tm : tm + tn * ntm;
-        const size_t off = (size_t)t * (BM * BN) + (size_t)(r - tm * BM) * BN + (c - tn * BN);
-        double s = 0.0;
-        for (int z = 0; z < nsplit; ++z) s += P[(size_t)z * ntiles * (BM * BN) + off];
-        return s;
-    };
-    double v = fetch(i, j);
-    if (symmetrize) v = 0.5 * (v + fetch(j, i));
-    C[(long)j * ldc + i] = alpha * v;
+// C(i, j) = alpha * sum over splits of the raw tile sums; a symmetric product
+// holds the tiles on and above the diagonal and the mirror image is written
+// along with them; symmetrize returns alpha/2 (G + G^T).  A block takes 32
+// elements along a tile's contiguous dimension; each of its 32 warps adds every
+// 32nd split and the warps' sums are added in order (24^3 x 32: 61 us when a
+// thread added 296 splits by itself with its neighbours a tile row apart,
+// about 5 us this way).
+template <int BT>
+__global__ void __launch_bounds__(1024) k_dmma_reduce(const double* __restrict__ P, int nsplit, int ntiles, int ntm,
+                                                      int sym, int m, int n, double alpha, int symmetrize,
+                                                      double* __restrict__ C, long ldc) {
+    __shared__ double sh[2][32][33];
+    constexpr int CB = BT / 32;  // column blocks of a tile
+    const int cx = threadIdx.x, y = threadIdx.y;
+    const int t = blockIdx.x / (BT * CB), rest = blockIdx.x % (BT * CB);
+    const int r = rest / CB, c = rest % CB * 32 + cx;
+    int tm, tn;
+    if (sym) {
+        tn = 0;
+        for (int u = t; u > tn; ++tn) u -= tn + 1;
+        tm = t - tn * (tn + 1) / 2;
+    } else {
+        tm = t % ntm;
+        tn = t / ntm;
+    }
+    const int i = tm * BT + r, j = tn * BT + c;
+    if (i >= m || j - cx >= n) return;  // uniform: the whole block is outside
+    // the transposed element is another one only on a diagonal tile of a
+    // symmetric product, or anywhere in a full one
+    const bool both = symmetrize && (!sym || tm == tn);
+    const size_t zs = (size_t)ntiles * (BT * BT);
+    const double* p = P + (size_t)t * (BT * BT) + (size_t)r * BT + c;
+    const double* q = P + (size_t)(sym ? t : tn + tm * ntm) * (BT * BT) + (size_t)c * BT + r;
+    double s = 0.0, u = 0.0;
+#pragma unroll 4
+    for (int z = y; z < nsplit; z += 32) {
+        s += p[z * zs];
+        if (both) u += q[z * zs];
+    }
+    sh[0][y][cx] = s;
+    sh[1][y][cx] = u;
+    __syncthreads();
+    if (y > 0 || j >= n) return;
+    const int nz = min(nsplit, 32);
+    double v = 0.0, w = 0.0;
+    for (int z = 0; z < nz; ++z) {
+        v += sh[0][z][cx];
+        w += sh[1][z][cx];
+    }
+    if (both) v = 0.5 * (v + w);
+    v *= alpha;
+    C[(long)j * ldc + i] = v;
+    if (sym && tm < tn) C[(long)i * ldc + j] = v;
 }
 
 template <int BM, int BN, int WM, int WN, bool KMAJOR, int CPS>
@@ -276,12 +302,32 @@ bool vec_ok(const DmmaArgs& g) {
 
 }  // namespace
 
+// One Gram product with BT x BT tiles, at most `slots` CTAs resident.
+template <int BT, int WM, int WN, int CPS>
+static int gram_tiles(DmmaArgs g, double alpha, int symmetrize, double* C, long ldc) {
+    Context& c = ctx();
+    g.ntm = div_up(g.M, BT);
+    g.ntiles = g.sym ? g.ntm * (g.ntm + 1) / 2 : g.ntm * div_up(g.N, BT);
+    // whole waves of CTAs: the largest split count with tiles x splits <= two
+    // waves, at least eight K blocks each (a CTA's pipeline fill), K split
+    // evenly
+    const long slots = (long)CPS * (c.num_sms > 0 ? c.num_sms : 148);
+    const long kblocks = (g.K + DM_BK - 1) / DM_BK;
+    int nsplit = (int)std::max<long>(1, std::min<long>((kblocks + 7) / 8, 2 * slots / g.ntiles));
+    g.kchunk = ((kblocks + nsplit - 1) / nsplit) * DM_BK;
+    nsplit = (int)((g.K + g.kchunk - 1) / g.kchunk);
+    RS_CHECK(workspace_t("dmma_partials", (size_t)nsplit * g.ntiles * BT * BT, &g.partial));
+    RS_CHECK((launch_dmma<BT, BT, WM, WN, true, CPS>(g, nsplit, vec_ok(g))));
+    launch(k_dmma_reduce<BT>, g.ntiles * BT * (BT / 32), dim3(32, 32), 0, c.stream, (const double*)g.partial,
+           nsplit, g.ntiles, g.ntm, g.sym, g.M, g.N, alpha, symmetrize, C, ldc);
+    RS_LAUNCH();
+    return RSDFT_OK;
+}
+
 // Tall Gram: C (m x n, column-major, ldc) = alpha A^T B for A (K x m), B
 // (K x n) column-major with leading dimension ld, K = kdim (the grid).
 int dmma_gram(const double* A, const double* B, long ld, long kdim, int m, int n, double alpha, int symmetrize,
               double* C, long ldc, bool symmetric_product) {
-    Context& c = ctx();
-    constexpr int BM = 128, BN = 128;
     DmmaArgs g{};
     g.A = A;
     g.lda = ld;
@@ -290,28 +336,22 @@ int dmma_gram(const double* A, const double* B, long ld, long kdim, int m, int n
     g.M = m;
     g.N = n;
     g.K = kdim;
-    g.ntm = div_up(m, BM);
-    const int ntn = div_up(n, BN);
     // upper tiles only for a symmetric product: A^T A, or A^T (H A) of a
     // symmetric operator (its lower tiles equal the upper ones to rounding;
     // the diagonal tiles are symmetrised by the reduction)
     g.sym = (m == n && (A == B || (symmetric_product && symmetrize))) ? 1 : 0;
-    g.ntiles = g.sym ? g.ntm * (g.ntm + 1) / 2 : g.ntm * ntn;
-    // whole waves of CTAs (one per SM: 123 KB of stages): the largest split
-    // count with tiles x splits <= 2 x SMs, K split evenly
-    const int sms = c.num_sms > 0 ? c.num_sms : 148;
-    const long kblocks = (kdim + DM_BK - 1) / DM_BK;
-    int nsplit = (int)std::max<long>(1, std::min<long>(kblocks, (2L * sms) / g.ntiles));
-    g.kchunk = ((kblocks + nsplit - 1) / nsplit) * DM_BK;
-    nsplit = (int)((kdim + g.kchunk - 1) / g.kchunk);
-    double* P = nullptr;
-    RS_CHECK(workspace_t("dmma_partials", (size_t)nsplit * g.ntiles * BM * BN, &P));
-    g.partial = P;
-    RS_CHECK((launch_dmma<BM, BN, 4, 4, true, 1>(g, nsplit, vec_ok(g))));
-    launch(k_dmma_reduce<BM, BN>, dim3(div_up(m, 128), n), 128, 0, c.stream, (const double*)P, nsplit, g.ntiles,
-           g.ntm, g.sym, m, alpha, symmetrize, C, ldc);
-    RS_LAUNCH();
-    return RSDFT_OK;
+    // Tile edge: the work is the tiles' area, padding included, and 64 x 64
+    // tiles (half the reuse of an operand in registers) run at about 0.85 of
+    // the rate of 128 x 128 ones: 160 bands, symmetric, take 3 tiles of 128^2
+    // or 6 of 64^2, 390 us and 185 us.  Up to 32 bands one 32 x 32 tile does.
+    const int mx = std::max(m, n);
+    if (mx <= 32) return gram_tiles<32, 2, 2, 4>(g, alpha, symmetrize, C, ldc);
+    auto area = [&](long t) {
+        const long a = div_up(m, t), b = div_up(n, t);
+        return (double)(g.sym ? a * (a + 1) / 2 : a * b) * t * t;
+    };
+    if (area(64) < 0.85 * area(128)) return gram_tiles<64, 2, 4, 2>(g, alpha, symmetrize, C, ldc);
+    return gram_tiles<128, 4, 4, 1>(g, alpha, symmetrize, C, ldc);
 }
 
 // General product C = alpha op(A) B + beta C (column-major; op = A or A^T),
