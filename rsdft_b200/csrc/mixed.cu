@@ -127,71 +127,44 @@ __global__ void k_split_small_tf32(const double* __restrict__ V, int mb, int ldv
     }
 }
 
-// slices[s][b][k] = term s of psi(k, b): same layout as psi (K-major per
-// band).  grid (ceil(ml / 2048), nb): 8 consecutive k per thread, read as
-// 16-byte pairs and written as one 16-byte group per slice when vec is set
-// (ml % 8 == 0, ld even, 16-byte aligned bases).
-template <typename TI>
-__global__ void __launch_bounds__(256) k_split_cols(const TI* __restrict__ psi, long ld, int nb, long ml,
-                                                    __nv_bfloat16* __restrict__ out, int vec) {
-    const long n = ml * nb;
-    const int b = blockIdx.y;
-    const long k0 = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
-    if (k0 >= ml) return;
-    const TI* src = psi + (long)b * ld + k0;
-    __nv_bfloat16* o = out + (long)b * ml + k0;
-    if (vec && k0 + 8 <= ml) {
-        __nv_bfloat16 h[8], m[8], l[8];
-        constexpr int W = 16 / (int)sizeof(TI);  // elements per 16-byte load
-#pragma unroll
-        for (int q = 0; q < 8 / W; ++q) {
-            TI v[W];
-            Vec16<TI>::get(*reinterpret_cast<const typename Vec16<TI>::t*>(src + W * q), v);
-#pragma unroll
-            for (int e = 0; e < W; ++e) split_bf16((double)v[e], h[W * q + e], m[W * q + e], l[W * q + e]);
-        }
-        *reinterpret_cast<uint4*>(o) = *reinterpret_cast<const uint4*>(h);
-        *reinterpret_cast<uint4*>(o + n) = *reinterpret_cast<const uint4*>(m);
-        *reinterpret_cast<uint4*>(o + 2 * n) = *reinterpret_cast<const uint4*>(l);
-        return;
-    }
-    for (long k = 0; k < 8 && k0 + k < ml; ++k) {
-        __nv_bfloat16 h, m, l;
-        split_bf16((double)src[k], h, m, l);
-        o[k] = h;
-        o[n + k] = m;
-        o[2 * n + k] = l;
-    }
-}
+// slices[s][kb][b][32] = term s of psi(32 kb .., b): the K blocks of all bands
+// side by side, zero past ml.  A tile of a Gram product (128 bands of one K
+// block) is then one contiguous 8 KB piece, and a tile of a rotation's B
+// operand (32 bands x 256 grid points) eight 2 KB pieces.  With the bands as
+// rows of the grid's length instead, every 64-byte row of a tile lies in
+// another page; at 96^3 x 1088 the Gram products ran at 355 TFLOP/s that way
+// against 880 at 72^3 x 480, 1020 this way.  A warp takes one K block
+// of eight bands: 128- or 256-byte reads per band, 512-byte writes.
+constexpr int SPC_KB = 8;  // K blocks (warps) per CTA
+constexpr int SPC_B = 8;   // bands per warp
 
-// slices[s][i][m] = term s of psi(i, m), m fastest, padded to mbk (zeros):
-// the transpose that makes the band index the K dimension of a rotation
 template <typename TI>
-__global__ void k_split_rows(const TI* __restrict__ psi, long ld, int nb, long ml, int mbk,
-                             __nv_bfloat16* __restrict__ out) {
-    __shared__ double tile[32][33];
-    const long i0 = (long)blockIdx.x * 32;
-    const int m0 = blockIdx.y * 32;
-    const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
-    for (int r = ty; r < 32; r += 8) {
-        const long i = i0 + tx;
-        const int m = m0 + r;
-        tile[r][tx] = (i < ml && m < nb) ? (double)psi[(long)m * ld + i] : 0.0;
+__global__ void __launch_bounds__(32 * SPC_KB) k_split_cols(const TI* __restrict__ psi, long ld, int nb, long ml,
+                                                           int nkb, __nv_bfloat16* __restrict__ out, int vec) {
+    const int lane = threadIdx.x & 31;
+    const int kb = blockIdx.x * SPC_KB + (threadIdx.x >> 5);
+    const int b = blockIdx.y * SPC_B + (lane >> 2);
+    if (kb >= nkb || b >= nb) return;
+    const long k0 = (long)kb * UB_K + (lane & 3) * 8;
+    const TI* src = psi + (long)b * ld + k0;
+    TI v[8];
+    constexpr int W = 16 / (int)sizeof(TI);  // elements per 16-byte load
+    if (vec && k0 + 8 <= ml) {
+#pragma unroll
+        for (int q = 0; q < 8 / W; ++q)
+            Vec16<TI>::get(*reinterpret_cast<const typename Vec16<TI>::t*>(src + W * q), v + W * q);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = k0 + q < ml ? src[q] : (TI)0;
     }
-    __syncthreads();
-    const long n = ml * mbk;
-    for (int r = ty; r < 32; r += 8) {
-        const long i = i0 + r;
-        const int m = m0 + tx;
-        if (i < ml && m < mbk) {
-            __nv_bfloat16 h, mm, l;
-            split_bf16(tile[tx][r], h, mm, l);
-            const long e = i * mbk + m;
-            out[e] = h;
-            out[n + e] = mm;
-            out[2 * n + e] = l;
-        }
-    }
+    __nv_bfloat16 h[8], m[8], l[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) split_bf16((double)v[q], h[q], m[q], l[q]);
+    const long n = (long)nkb * UB_K * nb;
+    __nv_bfloat16* o = out + ((long)kb * nb + b) * UB_K + (lane & 3) * 8;
+    *reinterpret_cast<uint4*>(o) = *reinterpret_cast<const uint4*>(h);
+    *reinterpret_cast<uint4*>(o + n) = *reinterpret_cast<const uint4*>(m);
+    *reinterpret_cast<uint4*>(o + 2 * n) = *reinterpret_cast<const uint4*>(l);
 }
 
 // slices[s][n][m] = term s of V(m, n) (V column-major mb x mb), padded to mbk
@@ -209,7 +182,7 @@ __global__ void k_split_small(const double* __restrict__ V, int mb, int ldv, int
 }
 
 struct UmmaMaps {
-    CUtensorMap a, b;  // 3-D: {K, rows, slice}
+    CUtensorMap a, b;
 };
 
 struct UmmaArgs {
@@ -257,7 +230,7 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_umma(const __grid_constant__ U
     constexpr int TCOLS = NACC * BN;  // 512 for BN = 128 (DRAIN) and BN = 256 (DIRECT)
     static_assert(TCOLS <= 512, "tensor memory holds 512 columns");
     constexpr uint32_t IDESC = TF ? umma_idesc_tf32(UB_M, BN) : umma_idesc_bf16(UB_M, BN, BMN);
-    // MN-major B (BMN): the tile is BN / 32 boxes of 32 N values x UB_K K rows
+    // MN-major B (BMN): the tile is BN / 32 pieces of 32 N values x UB_K K rows
     constexpr uint32_t B_LBO = 32 * UB_K * 2, B_SBO = 8 * 64;
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)NS * STAGE);
@@ -335,12 +308,19 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_umma(const __grid_constant__ U
                     const int k = kb * UKE;
 #pragma unroll
                     for (int t = 0; t < NT; ++t) {
-                        // the maps are rank 4 ({K, rows, slice, 1}): 4-D loads, w = 0
-                        tma_load_4d(st + t * ABYTES, &maps.a, k, tm * UB_M, t, 0, &full[s]);
-                        if (BMN)  // map {32, K, N / 32, slice}
-                            tma_load_4d(st + NT * ABYTES + t * BBYTES, &maps.b, 0, k, tn * (BN / 32), t, &full[s]);
+                        unsigned char *da = st + t * ABYTES, *db = st + NT * ABYTES + t * BBYTES;
+                        if (DRAIN && !TF) {  // blocked split, maps {32, rows, K blocks, slice}
+                            tma_load_4d(da, &maps.a, 0, tm * UB_M, kb, t, &full[s]);
+                            tma_load_4d(db, &maps.b, 0, tn * BN, kb, t, &full[s]);
+                            continue;
+                        }
+                        // row maps {K, rows, slice, 1}; MN-major B reads the
+                        // blocked split, its rows the K index
+                        tma_load_4d(da, &maps.a, k, tm * UB_M, t, 0, &full[s]);
+                        if (BMN)
+                            tma_load_4d(db, &maps.b, 0, k, tn * (BN / 32), t, &full[s]);
                         else
-                            tma_load_4d(st + NT * ABYTES + t * BBYTES, &maps.b, k, tn * BN, t, 0, &full[s]);
+                            tma_load_4d(db, &maps.b, k, tn * BN, t, 0, &full[s]);
                     }
                 }
             }
@@ -514,8 +494,8 @@ __global__ void k_reduce_tiles(const double* __restrict__ P, int nsplit, int npa
     C[(size_t)j * m + i] = alpha * v;
 }
 
-// Tensor map over the slices [s][rows][k] of a split (k fastest): 3 BF16 or
-// 2 TF32 slices, a 64-byte K block per row, 64-byte swizzle
+// Tensor map over the slices [s][rows][k] of a row split (k fastest): 3 BF16
+// or 2 TF32 slices, a 64-byte K block per row, 64-byte swizzle
 static int map3(CUtensorMap* mp, const void* base, long k, long rows, int box_rows, bool tf32 = false) {
     const unsigned long long eb = tf32 ? 4 : 2, ns = tf32 ? 2 : 3;
     const unsigned long long dims[4] = {(unsigned long long)k, (unsigned long long)rows, ns, 1ull};
@@ -524,6 +504,17 @@ static int map3(CUtensorMap* mp, const void* base, long k, long rows, int box_ro
     const unsigned int box[4] = {(unsigned)(UB_KB / eb), (unsigned)box_rows, 1u, 1u};
     return encode_tmap_4d(mp, tf32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, dims,
                           strides, box, CU_TENSOR_MAP_SWIZZLE_64B);
+}
+
+static int split_kblocks(long ml) { return (int)((ml + UB_K - 1) / UB_K); }
+
+// Tensor map over the blocked BF16 split [s][kb][rows][32] (k_split_cols)
+static int map_blocked(CUtensorMap* mp, const void* base, long ml, long rows, int box_rows, int box_kb) {
+    const unsigned long long nkb = (unsigned long long)split_kblocks(ml), r = (unsigned long long)rows;
+    const unsigned long long dims[4] = {(unsigned long long)UB_K, r, nkb, 3ull};
+    const unsigned long long strides[3] = {UB_KB, r * UB_KB, nkb * r * UB_KB};
+    const unsigned int box[4] = {(unsigned)UB_K, (unsigned)box_rows, (unsigned)box_kb, 1u};
+    return encode_tmap_4d(mp, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 template <int BN, int NT, int NS, bool DRAIN, bool BMN = false, bool TF = false>
@@ -545,8 +536,13 @@ static int gram_from_slices(void* sa, void* sb, bool same, int nb, double alpha,
     Context& c = ctx();
     const long ml = c.ml;
     UmmaMaps maps;
-    RS_CHECK(map3(&maps.a, sa, ml, nb, UB_M, sp.tf32));
-    RS_CHECK(map3(&maps.b, sb, ml, nb, 128, sp.tf32));
+    if (sp.tf32) {
+        RS_CHECK(map3(&maps.a, sa, ml, nb, UB_M, true));
+        RS_CHECK(map3(&maps.b, sb, ml, nb, 128, true));
+    } else {
+        RS_CHECK(map_blocked(&maps.a, sa, ml, nb, UB_M, 1));
+        RS_CHECK(map_blocked(&maps.b, sb, ml, nb, 128, 1));
+    }
     UmmaArgs g{};
     const int uke = sp.tf32 ? UB_KB / 4 : UB_K;
     g.kblocks = (int)((ml + uke - 1) / uke);
@@ -596,9 +592,11 @@ static int split_cols(const TI* A, long ld, int nb, const char* ws, Split sp, vo
         return RSDFT_OK;
     }
     __nv_bfloat16* o = nullptr;
-    RS_CHECK(workspace_t(ws, 3 * (size_t)ml * nb, &o));
+    const int nkb = split_kblocks(ml);
+    RS_CHECK(workspace_t(ws, 3 * (size_t)nkb * UB_K * nb, &o));
     const int vec = ((ld * (long)sizeof(TI)) % 16 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0) ? 1 : 0;
-    launch(k_split_cols<TI>, dim3(div_up(ml, 2048), nb), 256, 0, c.stream, A, ld, nb, ml, o, vec);
+    launch(k_split_cols<TI>, dim3(div_up(nkb, SPC_KB), div_up(nb, SPC_B)), 32 * SPC_KB, 0, c.stream, A, ld, nb, ml, nkb,
+           o, vec);
     RS_LAUNCH();
     *out = o;
     return RSDFT_OK;
@@ -674,67 +672,38 @@ static UmmaArgs rotate_args(long ml, int nb, int mbk, double* out, long ld, bool
     return g;
 }
 
-template <bool BMN>
-static int launch_rotate(const UmmaMaps& maps, const UmmaArgs& g, Split sp) {
-    Context& c = ctx();
-    const int sms = c.num_sms > 0 ? c.num_sms : 148;
-    const dim3 grid((unsigned)std::min(g.ntm * g.ntn, sms));
-    if constexpr (!BMN)
-        if (sp.tf32) return launch_umma<256, 2, 3, false, false, true>(maps, g, grid);
-    if (sp.terms == 3) return launch_umma<256, 3, 3, false, BMN>(maps, g, grid);
-    return launch_umma<256, 2, 3, false, BMN>(maps, g, grid);
-}
-
-// B operand from the split of psi as the Gram product leaves it (slices
-// [s][band][grid], grid fastest), read MN-major: the map views the grid
-// index as (32, ML / 32) so that one box is BN / 32 groups of 32 grid values
-// x UB_K bands.  Returns RSDFT_EUNSUP when that view is not available.
-static int rotate_from_split(const __nv_bfloat16* sp, double* out, long ld, int nb, const double* V, int ldv,
-                             Split spl) {
-    Context& c = ctx();
-    const long ml = c.ml;
-    if (ml % 32 != 0) return RSDFT_EUNSUP;
-    UmmaMaps maps;
-    const unsigned long long dims[4] = {32ull, (unsigned long long)nb, (unsigned long long)(ml / 32), 3ull};
-    const unsigned long long strides[3] = {(unsigned long long)ml * 2, 64ull, (unsigned long long)ml * nb * 2};
-    const unsigned int box[4] = {32u, (unsigned)UB_K, 256u / 32u, 1u};
-    if (encode_tmap_4d_swz64(&maps.b, sp, dims, strides, box) != RSDFT_OK) return RSDFT_EUNSUP;
-    const int mbk = (nb + 7) / 8 * 8;
-    RS_CHECK(split_v(V, nb, ldv, mbk, spl, &maps));
-    return launch_rotate<true>(maps, rotate_args(ml, nb, mbk, out, ld, false), spl);
-}
-
-// out (ML x nb, leading dimension ldo) = psi V, V (nb x nb, leading dimension ldv)
+// out (ML x nb, leading dimension ldo) = psi V, V (nb x nb, leading dimension
+// ldv).  BF16 forms: the B operand is the blocked split the Gram product made
+// (psi_split), read MN-major; TF32 splits psi transposed (slices[s][i][m], K =
+// band index fastest).
 template <typename TI>
 static int rotate(const TI* psi, double* out, long ld, int nb, const double* V, int ldv, int mode,
                   const void* psi_split) {
-    const Split sp = mode_split(mode);
-    if (psi_split && !sp.tf32) {
-        const int r = rotate_from_split(static_cast<const __nv_bfloat16*>(psi_split), out, ld, nb, V, ldv, sp);
-        if (r != RSDFT_EUNSUP) return r;
-    }
-    // transposed split: slices[s][i][m], K = band index fastest
     Context& c = ctx();
+    const Split sp = mode_split(mode);
     const long ml = c.ml;
     const int mbk = (nb + 7) / 8 * 8;
-    void* st = nullptr;
-    const dim3 sg(div_up(ml, 32), div_up(mbk, 32)), sb(32, 8);
+    const UmmaArgs g = rotate_args(ml, nb, mbk, out, ld, sp.tf32);
+    const int sms = c.num_sms > 0 ? c.num_sms : 148;
+    const dim3 grid((unsigned)std::min(g.ntm * g.ntn, sms));
+    UmmaMaps maps;
+    RS_CHECK(split_v(V, nb, ldv, mbk, sp, &maps));
     if (sp.tf32) {
         uint32_t* t = nullptr;
         RS_CHECK(workspace_t("umma_st", 2 * (size_t)ml * mbk, &t));
-        launch(k_split_rows_tf32<TI>, sg, sb, 0, c.stream, psi, ld, nb, ml, mbk, t);
-        st = t;
-    } else {
-        __nv_bfloat16* t = nullptr;
-        RS_CHECK(workspace_t("umma_st", 3 * (size_t)ml * mbk, &t));
-        launch(k_split_rows<TI>, sg, sb, 0, c.stream, psi, ld, nb, ml, mbk, t);
-        st = t;
+        launch(k_split_rows_tf32<TI>, dim3(div_up(ml, 32), div_up(mbk, 32)), dim3(32, 8), 0, c.stream, psi, ld, nb, ml,
+               mbk, t);
+        RS_LAUNCH();
+        RS_CHECK(map3(&maps.b, t, mbk, ml, 256, true));
+        return launch_umma<256, 2, 3, false, false, true>(maps, g, grid);
     }
-    RS_LAUNCH();
-    UmmaMaps maps;
-    RS_CHECK(split_v(V, nb, ldv, mbk, sp, &maps));
-    RS_CHECK(map3(&maps.b, st, mbk, ml, 256, sp.tf32));
-    return launch_rotate<false>(maps, rotate_args(ml, nb, mbk, out, ld, sp.tf32), sp);
+    if (!psi_split) {
+        set_error("rotate: no split of the bands");
+        return RSDFT_EINVAL;
+    }
+    RS_CHECK(map_blocked(&maps.b, psi_split, ml, nb, UB_K, 256 / UB_K));
+    if (sp.terms == 3) return launch_umma<256, 3, 3, false, true>(maps, g, grid);
+    return launch_umma<256, 2, 3, false, true>(maps, g, grid);
 }
 
 int rotate_mixed(const double* psi, double* out, long ld, int nb, const double* V, int ldv, int mode,
