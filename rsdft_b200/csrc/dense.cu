@@ -24,6 +24,7 @@
 #include "common.cuh"
 #include "kernels.cuh"
 #include "dmma.cuh"
+#include "imma.cuh"
 #include "mixed.cuh"
 
 namespace rsdft {
@@ -56,13 +57,74 @@ __global__ void k_reduce_partials(const double* __restrict__ P, int nch, int m, 
     C[(long)j * m + i] = alpha * s;
 }
 
-// C (m x n) = alpha A^T B with A, B tall (ML rows, leading dimension ld) on
-// the FP64 tensor cores (dmma.cu): split-K over the grid, partial tiles
-// reduced in a fixed order.  sym = 1 returns the symmetric part.
-// sym_op: B = H A with H symmetric, so only the upper tiles are formed.
-static int gemm_tn_splitk(const double* A, const double* B, long ld, int m, int n, double alpha, int sym,
-                          double* C, bool sym_op = false) {
-    return dmma_gram(A, B, ld, ctx().ml, m, n, alpha, sym, C, m, sym_op);
+// ------------------------------------------- FP64 products of tall blocks
+// A tall block (ml x nb) and how its FP64 products are formed: from its INT8
+// slices (imma.cu) where those suit, made once for every product it takes part
+// in, else straight on the FP64 tensor pipe (dmma.cu).  The INT8 launches
+// stand down when *bad is set on the device (a value that is not finite, or
+// out of the sliced range) and the DMMA launch behind each runs only then, so
+// NaNs and infinities come out as they do there, without a synchronisation.
+struct Fp64Block {
+    const double* x = nullptr;
+    long ld = 0, ml = 0;
+    int nb = 0;
+    int* bad = nullptr;  // null: DMMA only
+    ImmaSlices s;
+};
+
+static int fp64_flag(int** bad) {
+    RS_CHECK(workspace_t("imma_bad", 1, bad));
+    RS_CUDA(cudaMemsetAsync(*bad, 0, sizeof(int), ctx().stream));
+    return RSDFT_OK;
+}
+
+// rows / cols: slices for Gram products / for rotations.  bad: the operation's
+// flag (fp64_flag), shared by its blocks.
+static int fp64_block(const double* x, long ld, long ml, int nb, const char* ws, bool rows, bool cols, int* bad,
+                      Fp64Block* out) {
+    *out = Fp64Block{x, ld, ml, nb, nullptr, {}};
+    if (!imma_suits(ml, nb)) return RSDFT_OK;
+    const int r = imma_slice(x, ld, ml, nb, ws, rows, cols, bad, &out->s);
+    if (r == RSDFT_ENOMEM) return RSDFT_OK;  // no room for the slices
+    if (r == RSDFT_OK) out->bad = bad;
+    return r;
+}
+
+// C (nb x nb) = alpha a^T b for b = a or b = H a with H symmetric: the upper
+// half, mirrored; symmetrize averages what lies in the diagonal tiles
+static int fp64_gram(const Fp64Block& a, const Fp64Block& b, double alpha, int symmetrize, double* C) {
+    const int* bad = a.bad && b.bad ? a.bad : nullptr;
+    if (bad) RS_CHECK(imma_gram(a.s, b.s, alpha, symmetrize, bad, C, a.nb));
+    return dmma_gram(a.x, b.x, a.ld, a.ml, a.nb, a.nb, alpha, symmetrize, C, a.nb, true, bad);
+}
+
+__global__ void k_copy_cols_if(const double* __restrict__ src, long lds, double* __restrict__ dst, long ldd, long n,
+                               int nb, const int* __restrict__ flag) {
+    if (!*flag) return;
+    for (int b = blockIdx.y; b < nb; b += gridDim.y)
+        for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+            dst[(long)b * ldd + i] = src[(long)b * lds + i];
+}
+
+// out (ml x nb, leading dimension ldo) = a V.  out may be a itself, given tmp
+// (leading dimension ldt) for the DMMA form, which cannot work in place.
+static int fp64_rotate(const Fp64Block& a, const double* V, int ldv, double* out, long ldo, double* tmp = nullptr,
+                       long ldt = 0) {
+    Context& c = ctx();
+    if (a.bad) RS_CHECK(imma_rotate(a.s, V, ldv, a.bad, out, ldo));
+    const bool inplace = out == a.x;
+    RS_CHECK(dmma_gemm(false, a.ml, a.nb, a.nb, 1.0, a.x, a.ld, V, ldv, 0.0, inplace ? tmp : out,
+                       inplace ? ldt : ldo, a.bad));
+    if (!inplace) return RSDFT_OK;
+    if (a.bad) {
+        launch(k_copy_cols_if, dim3(64, std::min(a.nb, 64)), 256, 0, c.stream, (const double*)tmp, ldt, out, ldo, a.ml,
+               a.nb, (const int*)a.bad);
+        RS_LAUNCH();
+        return RSDFT_OK;
+    }
+    RS_CUDA(cudaMemcpy2DAsync(out, ldo * sizeof(double), tmp, ldt * sizeof(double), a.ml * sizeof(double), a.nb,
+                              cudaMemcpyDeviceToDevice, c.stream));
+    return RSDFT_OK;
 }
 
 static int check_info(int* dinfo, const char* what) {
@@ -168,14 +230,19 @@ static int trtri_upper(double* S, int nb, int* dinfo, const char* what) {
 static int cholqr_pass(const double* psi, double* out, long ld, int nb, double* S, int* dinfo, int mode) {
     Context& c = ctx();
     const void* split = nullptr;
-    if (mode == RSDFT_MODE_FP64)
-        RS_CHECK(gemm_tn_splitk(psi, psi, ld, nb, nb, c.dV, 0, S));
-    else
+    Fp64Block blk;
+    if (mode == RSDFT_MODE_FP64) {
+        int* bad = nullptr;
+        RS_CHECK(fp64_flag(&bad));
+        RS_CHECK(fp64_block(psi, ld, c.ml, nb, "imma_psi", true, true, bad, &blk));
+        RS_CHECK(fp64_gram(blk, blk, c.dV, 0, S));
+    } else {
         RS_CHECK(gram_mixed(psi, psi, ld, nb, c.dV, 0, mode, S, &split));
+    }
     RS_CHECK(potrf_upper(S, nb, dinfo, "gram_schmidt: overlap Cholesky"));
     RS_CHECK(trtri_upper(S, nb, dinfo, "gram_schmidt: triangular inverse"));
     if (mode == RSDFT_MODE_FP64)
-        RS_CHECK(dmma_gemm(false, c.ml, nb, nb, 1.0, psi, ld, S, nb, 0.0, out, ld));
+        RS_CHECK(fp64_rotate(blk, S, nb, out, ld));
     else
         RS_CHECK(rotate_mixed(psi, out, ld, nb, S, nb, mode, split));
     return RSDFT_OK;
@@ -216,24 +283,23 @@ int subspace_diag_device(double* psi, long ld, int mb, int spin, double* esp, in
     double *hpsi = nullptr, *H = nullptr;
     RS_CHECK(workspace_t("sub_hpsi", (size_t)ld * mb, &hpsi));
     RS_CHECK(workspace_t("sub_H", (size_t)mb * mb, &H));
+    RS_CHECK(hpsi_device<double>(psi, hpsi, ld, mb, spin, nullptr));
     if (mode == RSDFT_MODE_FP64) {
-        RS_CHECK(hpsi_device<double>(psi, hpsi, ld, mb, spin, nullptr));
+        int* bad = nullptr;
+        Fp64Block p, h;
+        RS_CHECK(fp64_flag(&bad));
+        RS_CHECK(fp64_block(psi, ld, c.ml, mb, "imma_psi", true, true, bad, &p));
+        RS_CHECK(fp64_block(hpsi, ld, c.ml, mb, "imma_hpsi", true, false, bad, &h));
         // Hsub = dV/2 (psi^T H psi + (H psi)^T psi): the symmetric part of dV psi^T (H psi)
-        RS_CHECK(gemm_tn_splitk(psi, hpsi, ld, mb, mb, c.dV, 1, H, true));
+        RS_CHECK(fp64_gram(p, h, c.dV, 1, H));
         RS_CHECK(syevd(H, mb, esp, CUBLAS_FILL_MODE_UPPER, "subspace_diag: syevd"));
-        RS_CHECK(dmma_gemm(false, c.ml, mb, mb, 1.0, psi, ld, H, mb, 0.0, hpsi, ld));
-    } else {
-        RS_CHECK(hpsi_device<double>(psi, hpsi, ld, mb, spin, nullptr));
-        const void* split = nullptr;
-        RS_CHECK(gram_mixed(psi, hpsi, ld, mb, c.dV, 1, mode, H, &split));
-        RS_CHECK(syevd(H, mb, esp, CUBLAS_FILL_MODE_UPPER, "subspace_diag: syevd"));
-        // reads only the BF16 split of psi: written in place
-        RS_CHECK(rotate_mixed(psi, psi, ld, mb, H, mb, mode, split));
-        return RSDFT_OK;
+        return fp64_rotate(p, H, mb, psi, ld, hpsi, ld);
     }
-    RS_CUDA(cudaMemcpy2DAsync(psi, ld * sizeof(double), hpsi, ld * sizeof(double), c.ml * sizeof(double), mb,
-                              cudaMemcpyDeviceToDevice, c.stream));
-    return RSDFT_OK;
+    const void* split = nullptr;
+    RS_CHECK(gram_mixed(psi, hpsi, ld, mb, c.dV, 1, mode, H, &split));
+    RS_CHECK(syevd(H, mb, esp, CUBLAS_FILL_MODE_UPPER, "subspace_diag: syevd"));
+    // reads only the BF16 split of psi: written in place
+    return rotate_mixed(psi, psi, ld, mb, H, mb, mode, split);
 }
 
 // The reduced eigenproblem of the fused Rayleigh-Ritz step: with Rinv = R^-1
@@ -313,9 +379,14 @@ int orth_subspace_diag_device(double* psi, long ld, int mb, int spin, double* es
     const void* split = nullptr;
     if (!hpsi_in) RS_CHECK(hpsi_device<double>(psi, hpsi, ld, mb, spin, nullptr));
     const double* hp = hpsi_in ? hpsi_in : hpsi;
+    Fp64Block p, h;
     if (mode == RSDFT_MODE_FP64) {
-        RS_CHECK(gemm_tn_splitk(psi, psi, ld, mb, mb, c.dV, 0, S));
-        RS_CHECK(gemm_tn_splitk(psi, hp, ld, mb, mb, c.dV, 1, H, true));
+        int* bad = nullptr;
+        RS_CHECK(fp64_flag(&bad));
+        RS_CHECK(fp64_block(psi, ld, c.ml, mb, "imma_psi", true, true, bad, &p));
+        RS_CHECK(fp64_block(hp, ld, c.ml, mb, "imma_hpsi", true, false, bad, &h));
+        RS_CHECK(fp64_gram(p, p, c.dV, 0, S));
+        RS_CHECK(fp64_gram(p, h, c.dV, 1, H));
     } else {
         RS_CHECK(gram_mixed_pair(psi, hp, ld, mb, c.dV, mode, S, H, &split));
     }
@@ -330,16 +401,10 @@ int orth_subspace_diag_device(double* psi, long ld, int mb, int spin, double* es
     }
     RS_CHECK(trtri_upper(S, mb, dinfo, "orth_subspace_diag: triangular inverse"));
     RS_CHECK(rr_reduced(S, H, T, mb, esp, "orth_subspace_diag: syevd"));
-    if (mode == RSDFT_MODE_FP64) {
-        RS_CHECK(dmma_gemm(false, c.ml, mb, mb, 1.0, psi, ld, T, mb, 0.0, hpsi, ld));
-        RS_CUDA(cudaMemcpy2DAsync(psi, ld * sizeof(double), hpsi, ld * sizeof(double), c.ml * sizeof(double), mb,
-                                  cudaMemcpyDeviceToDevice, c.stream));
-    } else {
-        // the tensor-core rotation reads only the BF16 split of psi, so it
-        // can write psi itself
-        RS_CHECK(rotate_mixed(psi, psi, ld, mb, T, mb, mode, split));
-    }
-    return RSDFT_OK;
+    if (mode == RSDFT_MODE_FP64) return fp64_rotate(p, T, mb, psi, ld, hpsi, ld);
+    // the tensor-core rotation reads only the BF16 split of psi, so it can
+    // write psi itself
+    return rotate_mixed(psi, psi, ld, mb, T, mb, mode, split);
 }
 
 // The same step on the FP32 bands of a mixed CG sweep: FP32 H psi, BF16
@@ -460,7 +525,7 @@ int rsdft_gpu_subspace_mate(int k, int s, const double* unk, long ld, int mb, do
     RS_CHECK(workspace_t("sub_hpsi", (size_t)ld * mb, &hpsi));
     RS_CHECK(workspace_t("sub_H", (size_t)mb * mb, &H));
     RS_CHECK(hpsi_device<double>(d, hpsi, ld, mb, s, nullptr));
-    RS_CHECK(gemm_tn_splitk(d, hpsi, ld, mb, mb, c.dV, 0, H));
+    RS_CHECK(dmma_gram(d, hpsi, ld, c.ml, mb, mb, c.dV, 0, H, mb));
     launch(k_zero_upper, dim3(div_up(mb, 128), mb), 128, 0, c.stream, H, mb, mb);
     RS_LAUNCH();
     RS_CUDA(cudaMemcpy2DAsync(hsub, (size_t)ldh * sizeof(double), H, (size_t)mb * sizeof(double),
@@ -506,9 +571,11 @@ int rsdft_gpu_subspace_rotv(int k, int s, double* unk, long ld, int mb, const do
     RS_CHECK(workspace_t("sub_hpsi", (size_t)ld * mb, &tmp));
     RS_CUDA(cudaMemcpy2DAsync(V, (size_t)mb * sizeof(double), vsub, (size_t)ldv * sizeof(double),
                               (size_t)mb * sizeof(double), mb, cudaMemcpyDefault, c.stream));
-    RS_CHECK(dmma_gemm(false, c.ml, mb, mb, 1.0, d, ld, V, mb, 0.0, tmp, ld));
-    RS_CUDA(cudaMemcpy2DAsync(d, ld * sizeof(double), tmp, ld * sizeof(double), c.ml * sizeof(double), mb,
-                              cudaMemcpyDeviceToDevice, c.stream));
+    int* bad = nullptr;
+    Fp64Block p;
+    RS_CHECK(fp64_flag(&bad));
+    RS_CHECK(fp64_block(d, ld, c.ml, mb, "imma_psi", false, true, bad, &p));
+    RS_CHECK(fp64_rotate(p, V, mb, d, ld, tmp, ld));
     RS_CHECK(wf_release(unk, d, ld, mb, st));
     return RSDFT_OK;
 }
@@ -611,10 +678,11 @@ int rsdft_gpu_rotate(double* unk, long ld, long rows, int mb, const double* v, i
     RS_CUDA(cudaMemcpy2DAsync(V, (size_t)mb * sizeof(double), v, (size_t)ldv * sizeof(double),
                               (size_t)mb * sizeof(double), mb, cudaMemcpyDefault, c.stream));
     double* d = static_cast<double*>(du);
-    RS_CHECK(dmma_gemm(false, rows, mb, mb, 1.0, d, ld, V, mb, 0.0, tmp, rows));
-    RS_CUDA(cudaMemcpy2DAsync(d, ld * sizeof(double), tmp, rows * sizeof(double), rows * sizeof(double), mb,
-                              cudaMemcpyDeviceToDevice, c.stream));
-    return RSDFT_OK;
+    int* bad = nullptr;
+    Fp64Block p;
+    RS_CHECK(fp64_flag(&bad));
+    RS_CHECK(fp64_block(d, ld, rows, mb, "imma_psi", false, true, bad, &p));
+    return fp64_rotate(p, V, mb, d, ld, tmp, rows);
 }
 
 int rsdft_gpu_eigensolver_sweep(int k, int s, double* unk, long ld, int mb, double* esp, double* res, int ncg,

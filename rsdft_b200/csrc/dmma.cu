@@ -43,6 +43,7 @@ struct DmmaArgs {
     double* partial;  // split-K: raw tile sums [split][tile][BM][BN], C unused; null: C written
     int sym;          // only tiles tm <= tn (a symmetric product)
     int ntm, ntiles;
+    const int* only_if;  // run only if this device flag is set (null: always)
 };
 
 constexpr int DM_BK = 16;  // K per stage (four m8n8k4 steps)
@@ -96,127 +97,133 @@ __global__ void __launch_bounds__(32 * WM * WN, CPS) k_dmma(DmmaArgs g) {
     constexpr int TM = BM / WM / 8, TN = BN / WN / 8;  // 8x8 tiles per warp
     static_assert(TM >= 1 && TN >= 1 && BM % (8 * WM) == 0 && BN % (8 * WN) == 0, "warp tiling");
     extern __shared__ __align__(16) double dsm[];
+    if (g.only_if && !*g.only_if) return;
     double* As = dsm;
     double* Bs = dsm + NS * AST;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wm0 = (warp % WM) * (BM / WM), wn0 = (warp / WM) * (BN / WN);
-    int tm, tn;
-    tile_of(g, blockIdx.x, tm, tn);
-    const int m0 = tm * BM, n0 = tn * BN;
-    const long k0 = (long)blockIdx.y * g.kchunk;
-    const long k1 = min(g.K, k0 + g.kchunk);
-    const int nkb = k1 > k0 ? (int)((k1 - k0 + BK - 1) / BK) : 0;
+    // one tile per CTA; a conditional launch, which as a rule does nothing,
+    // comes with a small grid that walks the tiles
+    for (int tile = blockIdx.x; tile < g.ntiles; tile += gridDim.x) {
+        if (tile != (int)blockIdx.x) __syncthreads();  // the last tile's stages are still read
+        int tm, tn;
+        tile_of(g, tile, tm, tn);
+        const int m0 = tm * BM, n0 = tn * BN;
+        const long k0 = (long)blockIdx.y * g.kchunk;
+        const long k1 = min(g.K, k0 + g.kchunk);
+        const int nkb = k1 > k0 ? (int)((k1 - k0 + BK - 1) / BK) : 0;
 
-    // operand tiles: 8-byte copies, or 16-byte ones (pairs of doubles along
-    // the contiguous dimension) when every row start is 16-byte aligned and
-    // the pair is wholly inside or outside the valid range (K, M, N even)
-    auto load_stage = [&](int s, int kb) {
-        const long kb0 = k0 + (long)kb * BK;
-        double* as = As + s * AST;
-        constexpr int V = VEC ? 2 : 1;
-        for (int e = threadIdx.x; e < BM * BK / V; e += NT) {
-            const int r = e / (BK / V), kk = (e % (BK / V)) * V;
-            const long k = kb0 + kk;
-            const bool ok = m0 + r < g.M && k < k1;
-            const double* src = ok ? g.A + (long)(m0 + r) * g.lda + k : g.A;
-            if (VEC) cp_async16(as + r * SA + kk, src, ok);
-            else cp_async8(as + r * SA + kk, src, ok);
-        }
-        double* bs = Bs + s * BST;
-        if (KMAJOR) {
-            for (int e = threadIdx.x; e < BN * BK / V; e += NT) {
+        // operand tiles: 8-byte copies, or 16-byte ones (pairs of doubles along
+        // the contiguous dimension) when every row start is 16-byte aligned and
+        // the pair is wholly inside or outside the valid range (K, M, N even)
+        auto load_stage = [&](int s, int kb) {
+            const long kb0 = k0 + (long)kb * BK;
+            double* as = As + s * AST;
+            constexpr int V = VEC ? 2 : 1;
+            for (int e = threadIdx.x; e < BM * BK / V; e += NT) {
                 const int r = e / (BK / V), kk = (e % (BK / V)) * V;
                 const long k = kb0 + kk;
-                const bool ok = n0 + r < g.N && k < k1;
-                const double* src = ok ? g.B + k + (long)(n0 + r) * g.ldb : g.B;
-                if (VEC) cp_async16(bs + r * SB + kk, src, ok);
-                else cp_async8(bs + r * SB + kk, src, ok);
+                const bool ok = m0 + r < g.M && k < k1;
+                const double* src = ok ? g.A + (long)(m0 + r) * g.lda + k : g.A;
+                if (VEC) cp_async16(as + r * SA + kk, src, ok);
+                else cp_async8(as + r * SA + kk, src, ok);
             }
-        } else {
-            for (int e = threadIdx.x; e < BN * BK / V; e += NT) {
-                const int kk = e / (BN / V), c = (e % (BN / V)) * V;
-                const long k = kb0 + kk;
-                const bool ok = n0 + c < g.N && k < k1;
-                const double* src = ok ? g.B + k * g.ldb + (n0 + c) : g.B;
-                if (VEC) cp_async16(bs + kk * SB + c, src, ok);
-                else cp_async8(bs + kk * SB + c, src, ok);
+            double* bs = Bs + s * BST;
+            if (KMAJOR) {
+                for (int e = threadIdx.x; e < BN * BK / V; e += NT) {
+                    const int r = e / (BK / V), kk = (e % (BK / V)) * V;
+                    const long k = kb0 + kk;
+                    const bool ok = n0 + r < g.N && k < k1;
+                    const double* src = ok ? g.B + k + (long)(n0 + r) * g.ldb : g.B;
+                    if (VEC) cp_async16(bs + r * SB + kk, src, ok);
+                    else cp_async8(bs + r * SB + kk, src, ok);
+                }
+            } else {
+                for (int e = threadIdx.x; e < BN * BK / V; e += NT) {
+                    const int kk = e / (BN / V), c = (e % (BN / V)) * V;
+                    const long k = kb0 + kk;
+                    const bool ok = n0 + c < g.N && k < k1;
+                    const double* src = ok ? g.B + k * g.ldb + (n0 + c) : g.B;
+                    if (VEC) cp_async16(bs + kk * SB + c, src, ok);
+                    else cp_async8(bs + kk * SB + c, src, ok);
+                }
+            }
+        };
+
+        double acc[TM][TN][2];
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+
+#pragma unroll
+        for (int s = 0; s < NS - 1; ++s) {
+            if (s < nkb) load_stage(s, s);
+            cp_async_commit();
+        }
+        const int fr = lane >> 2, fc = lane & 3;
+        for (int kb = 0; kb < nkb; ++kb) {
+            cp_async_wait<NS - 2>();
+            __syncthreads();  // stage kb has landed; every warp is done with stage kb - 1
+            if (kb + NS - 1 < nkb) load_stage((kb + NS - 1) % NS, kb + NS - 1);
+            cp_async_commit();
+            const double* as = As + (kb % NS) * AST + (wm0 + fr) * SA + fc;
+            const double* bs = Bs + (kb % NS) * BST + (KMAJOR ? (wn0 + fr) * SB + fc : fc * SB + wn0 + fr);
+#pragma unroll
+            for (int ks = 0; ks < BK; ks += 4) {
+                double a[TM], b[TN];
+#pragma unroll
+                for (int i = 0; i < TM; ++i) a[i] = as[8 * i * SA + ks];
+#pragma unroll
+                for (int j = 0; j < TN; ++j) b[j] = KMAJOR ? bs[8 * j * SB + ks] : bs[ks * SB + 8 * j];
+#pragma unroll
+                for (int i = 0; i < TM; ++i)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) dmma_884(acc[i][j], a[i], b[j]);
             }
         }
-    };
+        cp_async_wait<0>();
 
-    double acc[TM][TN][2];
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-
-#pragma unroll
-    for (int s = 0; s < NS - 1; ++s) {
-        if (s < nkb) load_stage(s, s);
-        cp_async_commit();
-    }
-    const int fr = lane >> 2, fc = lane & 3;
-    for (int kb = 0; kb < nkb; ++kb) {
-        cp_async_wait<NS - 2>();
-        __syncthreads();  // stage kb has landed; every warp is done with stage kb - 1
-        if (kb + NS - 1 < nkb) load_stage((kb + NS - 1) % NS, kb + NS - 1);
-        cp_async_commit();
-        const double* as = As + (kb % NS) * AST + (wm0 + fr) * SA + fc;
-        const double* bs = Bs + (kb % NS) * BST + (KMAJOR ? (wn0 + fr) * SB + fc : fc * SB + wn0 + fr);
-#pragma unroll
-        for (int ks = 0; ks < BK; ks += 4) {
-            double a[TM], b[TN];
-#pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = as[8 * i * SA + ks];
-#pragma unroll
-            for (int j = 0; j < TN; ++j) b[j] = KMAJOR ? bs[8 * j * SB + ks] : bs[ks * SB + 8 * j];
+        if (g.partial) {
+            double* P = g.partial + ((size_t)blockIdx.y * g.ntiles + tile) * (size_t)(BM * BN);
 #pragma unroll
             for (int i = 0; i < TM; ++i)
 #pragma unroll
-                for (int j = 0; j < TN; ++j) dmma_884(acc[i][j], a[i], b[j]);
+                for (int j = 0; j < TN; ++j) {
+                    const int r = wm0 + 8 * i + fr, c = wn0 + 8 * j + 2 * fc;
+                    *reinterpret_cast<double2*>(P + (size_t)r * BN + c) = make_double2(acc[i][j][0], acc[i][j][1]);
+                }
+            continue;
         }
-    }
-    cp_async_wait<0>();
-
-    if (g.partial) {
-        double* P = g.partial + ((size_t)blockIdx.y * g.ntiles + blockIdx.x) * (size_t)(BM * BN);
+        const bool pair = g.ldcn == 1 && (g.ldcm % 2) == 0 && (reinterpret_cast<uintptr_t>(g.C) % 16) == 0;
 #pragma unroll
         for (int i = 0; i < TM; ++i)
 #pragma unroll
             for (int j = 0; j < TN; ++j) {
-                const int r = wm0 + 8 * i + fr, c = wn0 + 8 * j + 2 * fc;
-                *reinterpret_cast<double2*>(P + (size_t)r * BN + c) = make_double2(acc[i][j][0], acc[i][j][1]);
+                const int m = m0 + wm0 + 8 * i + fr, n = n0 + wn0 + 8 * j + 2 * fc;
+                if (m >= g.M) continue;
+                double* o = g.C + (long)m * g.ldcm + (long)n * g.ldcn;
+                if (pair && n + 1 < g.N) {
+                    double2 v = make_double2(g.alpha * acc[i][j][0], g.alpha * acc[i][j][1]);
+                    if (g.beta != 0.0) {
+                        const double2 old = *reinterpret_cast<const double2*>(o);
+                        v.x = fma(g.beta, old.x, v.x);
+                        v.y = fma(g.beta, old.y, v.y);
+                    }
+                    *reinterpret_cast<double2*>(o) = v;
+                    continue;
+                }
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    if (n + e < g.N) {
+                        double* oe = o + (long)e * g.ldcn;
+                        const double v = g.alpha * acc[i][j][e];
+                        *oe = g.beta == 0.0 ? v : fma(g.beta, *oe, v);
+                    }
+                }
             }
-        return;
     }
-    const bool pair = g.ldcn == 1 && (g.ldcm % 2) == 0 && (reinterpret_cast<uintptr_t>(g.C) % 16) == 0;
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const int m = m0 + wm0 + 8 * i + fr, n = n0 + wn0 + 8 * j + 2 * fc;
-            if (m >= g.M) continue;
-            double* o = g.C + (long)m * g.ldcm + (long)n * g.ldcn;
-            if (pair && n + 1 < g.N) {
-                double2 v = make_double2(g.alpha * acc[i][j][0], g.alpha * acc[i][j][1]);
-                if (g.beta != 0.0) {
-                    const double2 old = *reinterpret_cast<const double2*>(o);
-                    v.x = fma(g.beta, old.x, v.x);
-                    v.y = fma(g.beta, old.y, v.y);
-                }
-                *reinterpret_cast<double2*>(o) = v;
-                continue;
-            }
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                if (n + e < g.N) {
-                    double* oe = o + (long)e * g.ldcn;
-                    const double v = g.alpha * acc[i][j][e];
-                    *oe = g.beta == 0.0 ? v : fma(g.beta, *oe, v);
-                }
-            }
-        }
 }
 
 // C(i, j) = alpha * sum over splits of the raw tile sums; a symmetric product
@@ -229,49 +236,53 @@ __global__ void __launch_bounds__(32 * WM * WN, CPS) k_dmma(DmmaArgs g) {
 template <int BT>
 __global__ void __launch_bounds__(1024) k_dmma_reduce(const double* __restrict__ P, int nsplit, int ntiles, int ntm,
                                                       int sym, int m, int n, double alpha, int symmetrize,
-                                                      double* __restrict__ C, long ldc) {
+                                                      double* __restrict__ C, long ldc, const int* __restrict__ only_if) {
     __shared__ double sh[2][32][33];
+    if (only_if && !*only_if) return;
     constexpr int CB = BT / 32;  // column blocks of a tile
     const int cx = threadIdx.x, y = threadIdx.y;
-    const int t = blockIdx.x / (BT * CB), rest = blockIdx.x % (BT * CB);
-    const int r = rest / CB, c = rest % CB * 32 + cx;
-    int tm, tn;
-    if (sym) {
-        tn = 0;
-        for (int u = t; u > tn; ++tn) u -= tn + 1;
-        tm = t - tn * (tn + 1) / 2;
-    } else {
-        tm = t % ntm;
-        tn = t / ntm;
-    }
-    const int i = tm * BT + r, j = tn * BT + c;
-    if (i >= m || j - cx >= n) return;  // uniform: the whole block is outside
-    // the transposed element is another one only on a diagonal tile of a
-    // symmetric product, or anywhere in a full one
-    const bool both = symmetrize && (!sym || tm == tn);
-    const size_t zs = (size_t)ntiles * (BT * BT);
-    const double* p = P + (size_t)t * (BT * BT) + (size_t)r * BT + c;
-    const double* q = P + (size_t)(sym ? t : tn + tm * ntm) * (BT * BT) + (size_t)c * BT + r;
-    double s = 0.0, u = 0.0;
+    for (int blk = blockIdx.x; blk < ntiles * BT * CB; blk += gridDim.x) {
+        const int t = blk / (BT * CB), rest = blk % (BT * CB);
+        const int r = rest / CB, c = rest % CB * 32 + cx;
+        int tm, tn;
+        if (sym) {
+            tn = 0;
+            for (int u = t; u > tn; ++tn) u -= tn + 1;
+            tm = t - tn * (tn + 1) / 2;
+        } else {
+            tm = t % ntm;
+            tn = t / ntm;
+        }
+        const int i = tm * BT + r, j = tn * BT + c;
+        if (i >= m || j - cx >= n) continue;  // uniform: the whole block is outside
+        // the transposed element is another one only on a diagonal tile of a
+        // symmetric product, or anywhere in a full one
+        const bool both = symmetrize && (!sym || tm == tn);
+        const size_t zs = (size_t)ntiles * (BT * BT);
+        const double* p = P + (size_t)t * (BT * BT) + (size_t)r * BT + c;
+        const double* q = P + (size_t)(sym ? t : tn + tm * ntm) * (BT * BT) + (size_t)c * BT + r;
+        double s = 0.0, u = 0.0;
 #pragma unroll 4
-    for (int z = y; z < nsplit; z += 32) {
-        s += p[z * zs];
-        if (both) u += q[z * zs];
+        for (int z = y; z < nsplit; z += 32) {
+            s += p[z * zs];
+            if (both) u += q[z * zs];
+        }
+        __syncthreads();
+        sh[0][y][cx] = s;
+        sh[1][y][cx] = u;
+        __syncthreads();
+        if (y > 0 || j >= n) continue;
+        const int nz = min(nsplit, 32);
+        double v = 0.0, w = 0.0;
+        for (int z = 0; z < nz; ++z) {
+            v += sh[0][z][cx];
+            w += sh[1][z][cx];
+        }
+        if (both) v = 0.5 * (v + w);
+        v *= alpha;
+        C[(long)j * ldc + i] = v;
+        if (sym && tm < tn) C[(long)i * ldc + j] = v;
     }
-    sh[0][y][cx] = s;
-    sh[1][y][cx] = u;
-    __syncthreads();
-    if (y > 0 || j >= n) return;
-    const int nz = min(nsplit, 32);
-    double v = 0.0, w = 0.0;
-    for (int z = 0; z < nz; ++z) {
-        v += sh[0][z][cx];
-        w += sh[1][z][cx];
-    }
-    if (both) v = 0.5 * (v + w);
-    v *= alpha;
-    C[(long)j * ldc + i] = v;
-    if (sym && tm < tn) C[(long)i * ldc + j] = v;
 }
 
 template <int BM, int BN, int WM, int WN, bool KMAJOR, int CPS>
@@ -282,11 +293,12 @@ int launch_dmma(const DmmaArgs& g, int nsplit, bool vec) {
     const void* fn = vec ? (const void*)k_dmma<BM, BN, WM, WN, KMAJOR, true, CPS>
                          : (const void*)k_dmma<BM, BN, WM, WN, KMAJOR, false, CPS>;
     RS_CHECK(set_smem_optin(fn, (int)smem));
+    const int sms = ctx().num_sms > 0 ? ctx().num_sms : 148;
+    const dim3 grid(g.only_if ? std::min(g.ntiles, 4 * sms) : g.ntiles, nsplit);
     if (vec)
-        launch(k_dmma<BM, BN, WM, WN, KMAJOR, true, CPS>, dim3(g.ntiles, nsplit), 32 * WM * WN, smem, ctx().stream, g);
+        launch(k_dmma<BM, BN, WM, WN, KMAJOR, true, CPS>, grid, 32 * WM * WN, smem, ctx().stream, g);
     else
-        launch(k_dmma<BM, BN, WM, WN, KMAJOR, false, CPS>, dim3(g.ntiles, nsplit), 32 * WM * WN, smem, ctx().stream,
-               g);
+        launch(k_dmma<BM, BN, WM, WN, KMAJOR, false, CPS>, grid, 32 * WM * WN, smem, ctx().stream, g);
     RS_LAUNCH();
     return RSDFT_OK;
 }
@@ -318,8 +330,9 @@ static int gram_tiles(DmmaArgs g, double alpha, int symmetrize, double* C, long 
     nsplit = (int)((g.K + g.kchunk - 1) / g.kchunk);
     RS_CHECK(workspace_t("dmma_partials", (size_t)nsplit * g.ntiles * BT * BT, &g.partial));
     RS_CHECK((launch_dmma<BT, BT, WM, WN, true, CPS>(g, nsplit, vec_ok(g))));
-    launch(k_dmma_reduce<BT>, g.ntiles * BT * (BT / 32), dim3(32, 32), 0, c.stream, (const double*)g.partial,
-           nsplit, g.ntiles, g.ntm, g.sym, g.M, g.N, alpha, symmetrize, C, ldc);
+    const int nblk = g.ntiles * BT * (BT / 32);
+    launch(k_dmma_reduce<BT>, g.only_if ? std::min(nblk, 512) : nblk, dim3(32, 32), 0, c.stream, (const double*)g.partial,
+           nsplit, g.ntiles, g.ntm, g.sym, g.M, g.N, alpha, symmetrize, C, ldc, g.only_if);
     RS_LAUNCH();
     return RSDFT_OK;
 }
@@ -327,8 +340,9 @@ static int gram_tiles(DmmaArgs g, double alpha, int symmetrize, double* C, long 
 // Tall Gram: C (m x n, column-major, ldc) = alpha A^T B for A (K x m), B
 // (K x n) column-major with leading dimension ld, K = kdim (the grid).
 int dmma_gram(const double* A, const double* B, long ld, long kdim, int m, int n, double alpha, int symmetrize,
-              double* C, long ldc, bool symmetric_product) {
+              double* C, long ldc, bool symmetric_product, const int* only_if) {
     DmmaArgs g{};
+    g.only_if = only_if;
     g.A = A;
     g.lda = ld;
     g.B = B;
@@ -360,8 +374,9 @@ int dmma_gram(const double* A, const double* B, long ld, long kdim, int m, int n
 // which is k-contiguous for op = T ([n][k] staging) and row-contiguous for
 // op = N ([k][n] staging).
 int dmma_gemm(bool transA, long m, int n, int k, double alpha, const double* A, long lda, const double* B, long ldb,
-              double beta, double* C, long ldc) {
+              double beta, double* C, long ldc, const int* only_if) {
     DmmaArgs g{};
+    g.only_if = only_if;
     g.A = B;  // A'(j, kk) = B[kk + j ldb]
     g.lda = ldb;
     g.B = A;  // B'(kk, i) = op(A)(i, kk)

@@ -3,6 +3,9 @@
 
 namespace rsdft {
 
+// only_if: the launch does nothing unless this device flag is set (null:
+// always runs).
+
 // C (m x n, column-major, leading dimension ldc) = alpha A^T B for tall A
 // (kdim x m) and B (kdim x n), column-major with leading dimension ld;
 // split-K over kdim, partial tiles added in a fixed order.  symmetrize: C =
@@ -11,11 +14,12 @@ namespace rsdft {
 // rounding), forms only the tiles on and above the diagonal: lower tiles are
 // mirrored, diagonal tiles symmetrised.
 int dmma_gram(const double* A, const double* B, long ld, long kdim, int m, int n, double alpha, int symmetrize,
-              double* C, long ldc, bool symmetric_product = false);
+              double* C, long ldc, bool symmetric_product = false,
+              const int* only_if = nullptr);
 
 // C = alpha op(A) B + beta C, column-major; op(A) = A (transA false) or A^T,
 // m x k; B k x n; C m x n.  C must not overlap A or B.
 int dmma_gemm(bool transA, long m, int n, int k, double alpha, const double* A, long lda, const double* B, long ldb,
-              double beta, double* C, long ldc);
+              double beta, double* C, long ldc, const int* only_if = nullptr);
 
 }  // namespace rsdft
