@@ -8,9 +8,9 @@
 //  3. k_nl_scatter: the nonlocal scatter-add (ps_nloc2_op_module.f90:
 //     255-263) turned into a per-point gather over a point-major CSR, so every
 //     sum is deterministic.
-//  Shapes the TMA kernel does not take (odd row widths, rows wider than 256
-//  elements) run k_stencil, a register-queue kernel with per-plane halo
-//  loads and the scatter fused in its epilogue.
+//  Row widths that tiled TMA cannot address run k_stencil_row, the same march
+//  fed by cp.async; what neither takes runs k_stencil, a register-queue kernel
+//  with per-plane halo loads and the scatter fused in its epilogue.
 #include <algorithm>
 
 #include "common.cuh"
@@ -310,23 +310,24 @@ struct Pk<float> {
 // U + m (first touch at m = Md) and U - m get cz_m c, slot U gets the in-plane
 // part when the plane is one of the tile's own, and slot U + Md + 1 (the
 // output completed by this arrival) is written when hp is set.  NK packs per
-// thread, two per row.
+// thread, two per row, written as one 16-byte vector, or (ROW: rows of any
+// width) pack by pack, npk of each of the first nrow rows.
 //
 // DOT adds this plane's share of <psi|(T + Vloc) psi>.  Slot U holds
 // sum_m cz_m psi(P - m) when plane P arrives; over the periodic grid the pairs
 // (P, P - m) and (P, P + m) give equal sums, so the z part is twice
 // psi(P) acc[U] and the dot needs no value that is not in registers here.
-template <typename T, int MD, int NK, int BY, bool DOT, int U>
+template <typename T, int MD, int NK, int BY, bool DOT, bool ROW, int U>
 __device__ __forceinline__ void push_body(typename Pk<T>::t (&acc)[2 * MD + 1][NK], const typename Pk<T>::t* c,
                                           const typename Pk<T>::t* in, bool inner, const CoefT<T>& cf, T* hp,
-                                          int n1, double& dot) {
+                                          int n1, double& dot, int nrow, int npk) {
     using P = Pk<T>;
     constexpr int Q = 2 * MD + 1;
     if constexpr (DOT) {
         if (inner) {
 #pragma unroll
             for (int i = 0; i < NK; ++i)
-                P::dot(c[i], P::fma(P::splat((T)2), acc[U][i], in[i]), dot);
+                if (!ROW || (i / 2 < nrow && i % 2 < npk)) P::dot(c[i], P::fma(P::splat((T)2), acc[U][i], in[i]), dot);
         }
     }
 #pragma unroll
@@ -341,21 +342,29 @@ __device__ __forceinline__ void push_body(typename Pk<T>::t (&acc)[2 * MD + 1][N
     }
     if (hp) {
 #pragma unroll
-        for (int r = 0; r < BY; ++r)
-            *reinterpret_cast<typename Vec16<T>::t*>(hp + (long)r * n1) = P::put2(&acc[(U + MD + 1) % Q][2 * r]);
+        for (int r = 0; r < BY; ++r) {
+            const typename P::t* o = &acc[(U + MD + 1) % Q][2 * r];
+            if constexpr (!ROW) {
+                *reinterpret_cast<typename Vec16<T>::t*>(hp + (long)r * n1) = P::put2(o);
+            } else if (r < nrow) {
+                *reinterpret_cast<typename P::t*>(hp + (long)r * n1) = o[0];
+                if (npk > 1) *reinterpret_cast<typename P::t*>(hp + (long)r * n1 + P::W) = o[1];
+            }
+        }
     }
 }
 
 // Runtime slot -> compile-time slot: only the short push runs per case, so
 // the loop body is not replicated 2 Md + 1 times.
-template <typename T, int MD, int NK, int BY, bool DOT>
+template <typename T, int MD, int NK, int BY, bool DOT, bool ROW>
 __device__ __forceinline__ void push_slot(int u, typename Pk<T>::t (&acc)[2 * MD + 1][NK], const typename Pk<T>::t* c,
                                           const typename Pk<T>::t* in, bool inner, const CoefT<T>& cf, T* hp,
-                                          int n1, double& dot) {
+                                          int n1, double& dot, int nrow = BY, int npk = 2) {
     constexpr int Q = 2 * MD + 1;
-#define RS_PUSH_CASE(K)                                                                            \
-    case K:                                                                                        \
-        if constexpr (K < Q) push_body<T, MD, NK, BY, DOT, K>(acc, c, in, inner, cf, hp, n1, dot); \
+#define RS_PUSH_CASE(K)                                                                             \
+    case K:                                                                                         \
+        if constexpr (K < Q)                                                                        \
+            push_body<T, MD, NK, BY, DOT, ROW, K>(acc, c, in, inner, cf, hp, n1, dot, nrow, npk);   \
         break;
     switch (u) {
         RS_PUSH_CASE(0) RS_PUSH_CASE(1) RS_PUSH_CASE(2) RS_PUSH_CASE(3) RS_PUSH_CASE(4) RS_PUSH_CASE(5)
@@ -551,7 +560,7 @@ __global__ void __launch_bounds__(384, 1) k_stencil_tma(const __grid_constant__ 
         // z pushes into the accumulator ring (slot = output arrival mod Q)
         // and, from arrival 2 Md on, the write of the completed output k - Md
         T* hp = (k >= 2 * MD && thr) ? hb + plane * (zs + k - 2 * MD) : nullptr;
-        push_slot<T, MD, NK, BY, DOT>(u, acc, c, in, inner, cf, hp, n1, dot);
+        push_slot<T, MD, NK, BY, DOT, false>(u, acc, c, in, inner, cf, hp, n1, dot);
         if (++s == S) {
             s = 0;
             ph ^= 1u;
@@ -573,6 +582,181 @@ __global__ void __launch_bounds__(384, 1) k_stencil_tma(const __grid_constant__ 
         }
     }
     if (!ok) atomicExch(err, 1);
+}
+
+// The same z march for row widths that tiled TMA cannot address (strides that
+// are no multiple of 16 bytes: odd widths in FP64, odd multiples of 2 in
+// FP32).  Planes come in by 8-byte cp.async of all threads, one barrier per
+// plane, into 16-byte aligned rows with the periodic x neighbours beside them,
+// so every window load is a vector at a constant offset; y and z wrap where the
+// rows are fetched, any n2 and n3.  The last vector of a row may stand half
+// outside the grid; what lies there is computed and not stored.  Bound, as the
+// TMA kernel's, by the shared-memory window loads and, with 10 to 12 warps per
+// SM, their latency.  H psi at 45^3 x 101 FP64: 394 us with k_stencil (16 x 32
+// tiles re-reading their halo every plane, a quarter of the tiles' points outside
+// the grid), 245 us with a thread on one x column (8-byte loads, 17 per point
+// against 7 here of 16 bytes), 216 us this way.
+constexpr int RS_STAGES = 3;  // planes of k_stencil_row's ring
+
+template <typename T, int MD, int BY, bool DOT>
+__global__ void __launch_bounds__(192, 2) k_stencil_row(StencilArgs<T> a, const CoefT<T> cf, int TY) {
+    using P = Pk<T>;
+    using PT = typename P::t;
+    using VT = Vec16<T>;
+    using V = typename VT::t;
+    constexpr int W = P::W;
+    constexpr int VX = 2 * W;                      // values per 16-byte vector
+    constexpr int HX = (MD + VX - 1) / VX * VX;    // x halo, whole vectors
+    constexpr int NV = 1 + 2 * HX / VX;            // vectors in the x window
+    constexpr int Q = 2 * MD + 1;
+    constexpr int S = RS_STAGES;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int n1 = a.n1, n2 = a.n2, n3 = a.n3;
+    const int nxv = (n1 + VX - 1) / VX;
+    const int PX = nxv * VX + 2 * HX;
+    const int ROWS = TY + 2 * MD;
+    const int SE = (ROWS + TY) * PX;  // elements per stage: psi rows, then Vloc rows
+    T* stages = reinterpret_cast<T*>(smem);
+    const int t = threadIdx.x;
+    const int nzc = a.nzc;
+    const int band = blockIdx.y / nzc;
+    const int zc = blockIdx.y - band * nzc;
+    if (a.band_active && !a.band_active[band]) return;  // uniform per CTA
+    const int y0 = blockIdx.x * TY;
+    const int ny = min(TY, n2 - y0);
+    const int zs = a.z0 + zc * a.zlen;
+    const int zlen = min(zs + a.zlen, a.z0 + a.nzo) - zs;
+    const int nk = zlen + 2 * MD;  // arrival k <-> plane zs - Md + k
+    const long plane = (long)n1 * n2;
+    const T* __restrict__ src = a.psi + (long)band * a.ld;
+    const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(stages));
+    // where each pack of a stage lies in its plane (the same for every plane;
+    // -1: not used), so that a plane's copies cost a table look-up each
+    int* goff = reinterpret_cast<int*>(smem + (size_t)S * SE * sizeof(T));
+    for (int e = t; e < SE / W; e += blockDim.x) {
+        const int r = e * W / PX, x = e * W - r * PX - HX;
+        int g = -1;
+        if (r < ROWS) {
+            if (r < ny + 2 * MD) g = n1 * pwrap(y0 - MD + r, n2) + pwrap(x, n1);
+        } else if (r - ROWS < ny && x >= 0 && x < n1) {
+            g = n1 * (y0 + r - ROWS) + x;
+        }
+        goff[e] = g;
+    }
+    // columns no copy ever fills (Vloc past the grid) hold zeros, not NaNs
+    for (int e = t; e < S * SE; e += blockDim.x) stages[e] = (T)0;
+    __syncthreads();
+    auto load_plane = [&](int k) {
+        if (k < nk) {
+            const uint32_t st = sbase + (uint32_t)((k % S) * SE) * (uint32_t)sizeof(T);
+            const int zp = pwrap(zs - MD + k, n3);
+            const bool inner = k >= MD && k < MD + zlen;
+            const T *pz = src + plane * zp, *vz = a.vloc + plane * zp;
+            // halo planes only feed the z accumulators: the own rows
+            const int e0 = inner ? 0 : MD * PX / W, e1 = inner ? SE / W : (MD + ny) * PX / W, ev = ROWS * PX / W;
+#pragma unroll 4
+            for (int e = e0 + t; e < e1; e += blockDim.x) {
+                const int g = goff[e];
+                if (g >= 0)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(st + (uint32_t)e * 8u),
+                                 "l"((e < ev ? pz : vz) + g)
+                                 : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    const bool thr = t < nxv * (TY / BY);
+    const int px = thr ? t % nxv : 0, py = thr ? t / nxv : 0;
+    const int x = VX * px, yl = BY * py;
+    const int nrow = thr ? max(0, min(BY, ny - yl)) : 0;  // rows of this thread inside the grid
+    const int npk = x + W < n1 ? 2 : 1;                    // packs of its vector inside the grid
+    T* __restrict__ hb = a.hpsi + (long)band * a.ld + (long)n1 * (y0 + yl) + x;
+
+    constexpr int NK = 2 * BY;
+    PT acc[Q][NK];
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+#pragma unroll
+        for (int i = 0; i < NK; ++i) acc[q][i] = P::splat((T)0);
+    double dot = 0.0;
+    // two planes in flight while one is used
+    load_plane(0);
+    load_plane(1);
+    int u = 0;
+    for (int k = 0; k < nk; ++k) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();  // plane k has landed for everyone; plane k - 1's stage is free
+        load_plane(k + 2);
+        const T* st = stages + (size_t)(k % S) * SE;
+        const bool inner = k >= MD && k < MD + zlen;  // uniform
+        const T* sp = st + (MD + yl) * PX + HX + x;    // the thread's first row
+        PT c[NK], in[NK];
+#pragma unroll
+        for (int r = 0; r < BY; ++r) P::get2(*reinterpret_cast<const V*>(sp + r * PX), c + 2 * r);
+        if (inner) {
+#pragma unroll
+            for (int i = 0; i < NK; ++i) in[i] = P::splat((T)0);
+#pragma unroll
+            for (int j = -MD; j < BY + MD; ++j) {
+                PT v[2];
+                if (j < 0 || j >= BY) {
+                    P::get2(*reinterpret_cast<const V*>(sp + j * PX), v);
+                } else {
+                    v[0] = c[2 * (j < 0 || j >= BY ? 0 : j)];
+                    v[1] = c[2 * (j < 0 || j >= BY ? 0 : j) + 1];
+                }
+#pragma unroll
+                for (int r = 0; r < BY; ++r) {
+                    const int m = j > r ? j - r : r - j;
+                    if (m >= 1 && m <= MD) {
+#pragma unroll
+                        for (int e = 0; e < 2; ++e)
+                            in[2 * r + e] = P::fma(P::splat(cf.cy[m - 1]), v[e], in[2 * r + e]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < BY; ++r) {
+                T w[NV * VX];
+#pragma unroll
+                for (int j = 0; j < NV; ++j) {
+                    if (j == HX / VX)
+                        P::unpack2(c + 2 * r, w + j * VX);
+                    else
+                        VT::get(*reinterpret_cast<const V*>(sp + r * PX - HX + VX * j), w + j * VX);
+                }
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+#pragma unroll
+                    for (int m = 1; m <= MD; ++m)
+                        in[2 * r + e] = P::fma(P::splat(cf.cx[m - 1]),
+                                               P::add(P::of(w + HX + W * e - m), P::of(w + HX + W * e + m)),
+                                               in[2 * r + e]);
+                PT vl[2];
+                P::get2(*reinterpret_cast<const V*>(sp + (ROWS - MD + r) * PX), vl);
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                    in[2 * r + e] = P::fma(P::add(P::splat(cf.c0), vl[e]), c[2 * r + e], in[2 * r + e]);
+            }
+        }
+        T* hp = (k >= 2 * MD && nrow > 0) ? hb + plane * (zs + k - 2 * MD) : nullptr;
+        push_slot<T, MD, NK, BY, DOT, true>(u, acc, c, in, inner, cf, hp, n1, dot, nrow, npk);
+        if (++u == Q) u = 0;
+    }
+    if constexpr (DOT) {
+        __shared__ double red[6];
+        const int warp = t >> 5, lane = t & 31, nw = blockDim.x >> 5;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        if (lane == 0) red[warp] = dot;
+        __syncthreads();
+        if (t == 0) {
+            double v = 0.0;
+            for (int w = 0; w < nw; ++w) v += red[w];
+            a.dot[(long)band * a.ndot + zc * gridDim.x + blockIdx.x] = v;
+        }
+    }
 }
 
 // Nonlocal scatter after the stencil: hpsi(p, b) += sum over the sphere
@@ -768,6 +952,60 @@ static int launch_tma(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStrea
     return RSDFT_OK;
 }
 
+// k_stencil_row: rows of whole packs (8 bytes), up to 192 vectors of 16, and
+// 8-byte aligned arrays.  The tile height and z split of least
+// march_cost, two CTAs per SM sharing its shared-memory bandwidth.
+template <typename T, int MD, int BY>
+static int launch_row(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStream_t st, HpsiDot* dot, bool* used) {
+    *used = false;
+    constexpr int W = Pk<T>::W, VX = 2 * W, S = RS_STAGES, HX = (MD + VX - 1) / VX * VX;
+    const int nxv = div_up(a.n1, VX);
+    if (a.n1 % W != 0 || nxv > 192) return RSDFT_OK;
+    if (W > 1 && (reinterpret_cast<uintptr_t>(a.psi) % 8 != 0 || reinterpret_cast<uintptr_t>(a.hpsi) % 8 != 0 ||
+                  reinterpret_cast<uintptr_t>(a.vloc) % 8 != 0 || a.ld % W != 0))
+        return RSDFT_OK;
+    const Context& c = ctx();
+    const int sms = c.num_sms > 0 ? c.num_sms : 148;
+    const double row = (nxv * VX + 2 * HX) * sizeof(T);
+    const int plan = dot && dot->plan_nb ? dot->plan_nb : nb;
+    int TY = 0, nzc = 1;
+    double best = 0.0;
+    for (int ty = BY; ty < a.n2 + BY; ty += BY) {
+        const int threads = (nxv * (ty / BY) + 31) / 32 * 32;
+        if (threads > 192) break;
+        if ((2 * ty + 2 * MD) * row * (S + 0.5) > 110.0 * 1024) break;
+        const int tiles = div_up(a.n2, ty);
+        const int zmax = std::min({std::max(1, a.nzo / 4), 65535 / plan, (dot ? dot->cap : 1 << 20) / tiles});
+        if (zmax < 1) continue;
+        const double loads = BY + 2 * MD + BY * (2.0 * HX / VX) + BY;
+        const double t = 700.0 + 2.0 * 1.4 * (4.0 * loads * (threads / 32) + 2.0 * (2.0 * ty + 2 * MD) * row / 128.0);
+        int n = 1;
+        const double cost = march_cost((long)tiles * plan, a.nzo, 2 * MD, zmax, 2L * sms, t, 0.3 * t, &n);
+        if (TY == 0 || cost <= 1.05 * best) {  // the taller tile at a near tie
+            best = TY == 0 ? cost : std::min(cost, best);
+            TY = ty;
+            nzc = n;
+        }
+    }
+    if (TY == 0) return RSDFT_OK;
+    a.zlen = div_up(a.nzo, nzc);
+    a.nzc = div_up(a.nzo, a.zlen);
+    const int tiles = div_up(a.n2, TY), threads = (nxv * (TY / BY) + 31) / 32 * 32;
+    const size_t se = (size_t)(2 * TY + 2 * MD) * (nxv * VX + 2 * HX);
+    const size_t smem = se * (S * sizeof(T) + sizeof(int) / W);
+    auto kern = dot ? k_stencil_row<T, MD, BY, true> : k_stencil_row<T, MD, BY, false>;
+    RS_CHECK(set_smem_optin((const void*)kern, (int)smem));
+    if (dot) {
+        dot->nch = a.ndot = tiles * a.nzc;
+        dot->with_nl = false;
+        a.dot = dot->part;
+    }
+    launch(kern, dim3(tiles, (unsigned)(nb * a.nzc)), threads, smem, st, a, coef_as<T>(cf), TY);
+    RS_LAUNCH();
+    *used = true;
+    return RSDFT_OK;
+}
+
 template <typename T, int MD>
 static int launch_stencil_md2(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStream_t st, HpsiDot* dot) {
     const Context& c = ctx();
@@ -775,6 +1013,7 @@ static int launch_stencil_md2(StencilArgs<T> a, const StencilCoef& cf, int nb, c
     // two rows per thread up to Md = 6; one above, where the 2 Md + 1
     // accumulators of two rows no longer fit the register budget
     RS_CHECK((launch_tma<T, MD, (MD <= 6 ? 2 : 1)>(a, cf, nb, st, dot, &used)));
+    if (!used) RS_CHECK((launch_row<T, MD, (MD <= 6 ? 2 : 1)>(a, cf, nb, st, dot, &used)));
     if (used) {
         if (a.gpt_ptr && c.nl_npt > 0) {
             const int bch = scatter_chunk(nb);
@@ -786,8 +1025,9 @@ static int launch_stencil_md2(StencilArgs<T> a, const StencilCoef& cf, int nb, c
         }
         return RSDFT_OK;
     }
-    // general shapes (odd widths, very wide rows): register-queue kernel with
-    // per-plane halo loads and the nonlocal scatter fused
+    // rows beyond both z marches (odd FP32 widths, more than 192 vectors):
+    // register-queue kernel with per-plane halo loads and the nonlocal scatter
+    // fused
     const int tx = (a.n1 % 32 == 0 || a.n1 > 24) ? 32 : (a.n1 % 24 == 0 ? 24 : 16);
     const long base = (long)div_up(a.n1, tx) * div_up(a.n2, 16) * (dot && dot->plan_nb ? dot->plan_nb : nb);
     const long want = 8L * (c.num_sms > 0 ? c.num_sms : 148);
