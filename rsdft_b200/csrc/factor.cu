@@ -20,9 +20,9 @@
 //    it needs, R(k, i) = X^T S(k, i) with X = R(k, k)^-1 published by the
 //    step before (so no CTA waits on another), and subtracts R(k, i)^T
 //    R(k, j) from S(i, j).  The CTA of (k+1, k+1) keeps its updated tile,
-//    factors it by one warp in dpotf2's order (r = d times 1 / sqrt(d),
-//    the row scaled by 1 / r, 1 / sqrt(d) by Newton-Raphson) and inverts
-//    the factor for the next step.  The panels go to a side buffer (S's row
+//    factors it in dpotf2's order (r = d times 1 / sqrt(d), the row scaled
+//    by 1 / r, 1 / sqrt(d) by Newton-Raphson) and inverts the factor beside
+//    it for the next step.  The panels go to a side buffer (S's row
 //    block k is still being read during step k) and into S at the end.  A
 //    pivot that is not positive (or NaN) sets info to its 1-based index as
 //    dpotrf does, and the later launches stop.
@@ -142,69 +142,54 @@ __device__ __forceinline__ double rsqrt_nr(double d) {
 }
 
 // Cholesky of the leading kk x kk block of the tile T (row-major, pitch
-// CF_P; its upper part read) by one warp, in dpotf2's order: step j,
+// CF_P; its upper part read) in dpotf2's order by the whole CTA: step j,
 // R(j, j) = sqrt(A(j, j)) (as d times 1/sqrt(d)), R(j, l) = A(j, l) times
-// 1 / R(j, j), then A(i, l) -= R(j, i) R(j, l) for j < i <= l (row by
-// row, lane l on column l).  dinv[j] receives 1 / R(j, j).  Returns
-// (in every lane) 0, or the 1-based index of the first pivot that is not
-// positive (or NaN).
-__device__ int chol_tile_warp(double* T, int kk, double* dinv) {
-    const int lane = threadIdx.x & 31;
-    for (int j = 0; j < kk; ++j) {
-        const double d = T[j * CF_P + j];
-        if (!(d > 0.0)) return j + 1;  // the same d in every lane
-        const double inv = rsqrt_nr(d);
-        const double rjl = (lane > j && lane < kk) ? T[j * CF_P + lane] * inv : 0.0;
-        __syncwarp();
-        if (lane == j) {
-            T[j * CF_P + j] = d * inv;
-            dinv[j] = inv;
-        } else if (lane > j && lane < kk) {
-            T[j * CF_P + lane] = rjl;
-        }
-        __syncwarp();
-        // the trailing triangle j < i <= l < kk: row by row, lane l on column
-        // l; R(j, i) comes from lane i's register (a shuffle, not a shared
-        // load, so no shared-memory access orders the rows' updates)
-#pragma unroll 4
-        for (int i = j + 1; i < kk; ++i) {
-            const double rji = __shfl_sync(FULL, rjl, i);
-            if (lane >= i && lane < kk) T[i * CF_P + lane] = fma(-rji, rjl, T[i * CF_P + lane]);
-        }
-        __syncwarp();
+// 1 / R(j, j), then A(i, l) -= R(j, i) R(j, l) for j < i <= l.  The same row
+// operations on an identity beside it leave R^-T, whose transpose R^-1 goes to
+// xg (32 x 32, row-major, zero below the diagonal and outside kk) when given.
+// Thread (l, g) keeps rows g, g + 4, .. of column l of [A | I] in registers;
+// the row a step divides by passes through one of two row buffers, one barrier
+// per step, and every thread forms 1/sqrt(d) for itself.  What bounds it is
+// that chain of 32 steps: 28 us for the factor and 15 us for the inverse by
+// one warp with the tile in shared memory, about 12 us for both this way.
+// Returns (in every thread) 0, or the 1-based index of the first pivot that is
+// not positive (or NaN).
+__device__ int chol_tile_cta(double* T, int kk, double (*row)[64], double* __restrict__ xg) {
+    const int l = threadIdx.x & 63, g = threadIdx.x >> 6;
+    const bool ident = l >= 32;
+    const int m = l - 32;
+    double v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int i = g + 4 * q;
+        v[q] = ident ? ((i == m && i < kk) ? 1.0 : 0.0) : T[i * CF_P + l];
     }
-    return 0;
-}
-
-// X = R^-1 of the kk x kk upper factor in T (dinv = 1 / diag) by one warp,
-// row by row from the last: X(i, i) = dinv[i], X(i, l) = -(sum_{m=i+1}^{l}
-// R(i, m) X(m, l)) dinv[i] (l > i), lane l forming X(i, l) with four
-// partial sums; written to xs (pitch CF_P) and xg (32 x 32, row-major),
-// zero below the diagonal and outside kk.
-__device__ void inv_tile_warp(const double* T, int kk, const double* dinv, double* xs, double* __restrict__ xg) {
-    const int l = threadIdx.x & 31;
-    for (int i = 31; i >= 0; --i) {
-        double x = 0.0;
-        if (i < kk && l < kk && i <= l) {
-            if (i == l) {
-                x = dinv[i];
-            } else {
-                double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-                int m = i + 1;
-                for (; m + 3 <= l; m += 4) {
-                    s0 = fma(T[i * CF_P + m], xs[m * CF_P + l], s0);
-                    s1 = fma(T[i * CF_P + m + 1], xs[(m + 1) * CF_P + l], s1);
-                    s2 = fma(T[i * CF_P + m + 2], xs[(m + 2) * CF_P + l], s2);
-                    s3 = fma(T[i * CF_P + m + 3], xs[(m + 3) * CF_P + l], s3);
-                }
-                for (; m <= l; ++m) s0 = fma(T[i * CF_P + m], xs[m * CF_P + l], s0);
-                x = -((s0 + s1) + (s2 + s3)) * dinv[i];
+    if (g == 0) row[0][l] = v[0];
+    __syncthreads();
+    for (int j = 0; j < kk; ++j) {
+        const double* rb = row[j & 1];
+        const double d = rb[j];
+        if (!(d > 0.0)) return j + 1;  // the same d in every thread
+        const double inv = rsqrt_nr(d);
+        const double rl = rb[l] * inv;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int i = g + 4 * q;
+            if (i > j && i < kk) {
+                v[q] = fma(-(rb[i] * inv), rl, v[q]);
+                if (i == j + 1) row[(j + 1) & 1][l] = v[q];
             }
         }
-        xs[i * CF_P + l] = x;
-        __syncwarp();
+        if (g == (j & 3)) {
+            if (!ident && l >= j && l < kk) T[j * CF_P + l] = l == j ? d * inv : rl;
+            if (ident && xg) xg[m * 32 + j] = rl;
+        }
+        __syncthreads();
     }
-    for (int r = 0; r < 32; ++r) xg[r * 32 + l] = xs[r * CF_P + l];
+    if (xg)
+        for (int j = kk; j < 32; ++j)
+            if (ident && g == 0) xg[m * 32 + j] = 0.0;
+    return 0;
 }
 
 // the upper part (r <= c, inside n) of tile T into tile (ti, tj) of the
@@ -227,50 +212,43 @@ __device__ __forceinline__ void tile_get(const double* __restrict__ S, int n, in
 
 // factor the diagonal tile held in sA (global tile index t) and publish it:
 // R into Rb, and (want_inv) R^-1 into xg; a bad pivot sets info and fail
-__device__ void chol_publish(double* sA, double* sX, double* dinv, int n, int t, bool want_inv,
-                             double* __restrict__ Rb, double* __restrict__ xg, int* __restrict__ info,
-                             int* __restrict__ fail) {
-    __shared__ int bad;
-    const int kk = min(32, n - 32 * t);
-    if (threadIdx.x < 32) {
-        const int b = chol_tile_warp(sA, kk, dinv);
-        if (b == 0 && want_inv) inv_tile_warp(sA, kk, dinv, sX, xg);
+__device__ void chol_publish(double* sA, int n, int t, bool want_inv, double* __restrict__ Rb,
+                             double* __restrict__ xg, int* __restrict__ info, int* __restrict__ fail) {
+    __shared__ double row[2][64];
+    const int b = chol_tile_cta(sA, min(32, n - 32 * t), row, want_inv ? xg : nullptr);
+    if (b) {
         if (threadIdx.x == 0) {
-            bad = b;
-            if (b) {
-                *info = 32 * t + b;
-                *fail = 1;
-            }
+            *info = 32 * t + b;
+            *fail = 1;
         }
+        return;
     }
-    __syncthreads();
-    if (!bad) tile_put_upper(sA, n, t, t, Rb);
+    tile_put_upper(sA, n, t, t, Rb);
 }
 
 // step -1: the first diagonal tile
 __global__ void __launch_bounds__(CH_T) k_chol_first(const double* __restrict__ S, int n, double* __restrict__ Rb,
                                                      double* __restrict__ xg, int* __restrict__ info,
                                                      int* __restrict__ fail) {
-    __shared__ double sA[32 * CF_P], sX[32 * CF_P], dinv[32];
+    __shared__ double sA[32 * CF_P];
     if (threadIdx.x == 0) {
         *info = 0;
         *fail = 0;
     }
     tile_get(S, n, 0, 0, sA);
     __syncthreads();
-    chol_publish(sA, sX, dinv, n, 0, n > 32, Rb, xg, info, fail);
+    chol_publish(sA, n, 0, n > 32, Rb, xg, info, fail);
 }
 
 // step k: one CTA per trailing tile (i, j), k < i <= j, the diagonal tile
 // (k+1, k+1) first.  Each CTA forms R(k, i) = X^T S(k, i) and R(k, j) with
 // X = R(k, k)^-1 (xin), writes R(k, i) to Rb when i == j, and subtracts
 // R(k, i)^T R(k, j) from S(i, j); the CTA of (k+1, k+1) keeps the updated
-// tile, factors it and publishes R(k+1, k+1) and its inverse (xout; sX is
-// free by then and serves as the inverse's scratch).
+// tile, factors it and publishes R(k+1, k+1) and its inverse (xout).
 __global__ void __launch_bounds__(CH_T) k_chol_step(double* __restrict__ S, int n, int k, double* __restrict__ Rb,
                                                     const double* __restrict__ xin, double* __restrict__ xout,
                                                     int* __restrict__ info, int* __restrict__ fail) {
-    __shared__ double sX[32 * CF_P], sA[32 * CF_P], sB[32 * CF_P], sC[32 * CF_P], dinv[32];
+    __shared__ double sX[32 * CF_P], sA[32 * CF_P], sB[32 * CF_P], sC[32 * CF_P];
     if (*(const volatile int*)fail) return;
     const int nt = (n + 31) / 32;
     int q = blockIdx.x, j = k + 1;
@@ -323,7 +301,7 @@ __global__ void __launch_bounds__(CH_T) k_chol_step(double* __restrict__ S, int 
 #pragma unroll
         for (int m = 0; m < 4; ++m) sC[r * CF_P + c0 + 8 * m] -= o[m];
         __syncthreads();
-        chol_publish(sC, sX, dinv, n, k + 1, k + 2 < nt, Rb, xout, info, fail);
+        chol_publish(sC, n, k + 1, k + 2 < nt, Rb, xout, info, fail);
     } else {
         const int gr = 32 * i + r;
 #pragma unroll
