@@ -375,6 +375,17 @@ __device__ __forceinline__ void push_slot(int u, typename Pk<T>::t (&acc)[2 * MD
 #undef RS_PUSH_CASE
 }
 
+// Order of the in-plane terms.  FP32: the y rows from the outermost inwards, x
+// likewise, the centre last, so that few roundings are at the size of the large
+// terms: the bands of a CG sweep (FP32, against FP64) at 24^3 were 4.4e-7 off
+// with the terms in the order the rows lie in and 3.9e-7 this way, at 26^3 4.1e-7
+// and 3.7e-7.  FP64 keeps the rows' order (72^3 x 480: 1625 us against 1667, and
+// H psi of smooth bands no better).
+template <typename T>
+__device__ __forceinline__ constexpr int term_order(int i, int n) {
+    return sizeof(T) == 8 ? i : (i % 2 == 0 ? i / 2 : n - 1 - i / 2);
+}
+
 // hpsi stencil + Vloc, TMA pipeline with a z "push" march.  A CTA owns TY
 // full-width rows of one band and marches along z over planes zs-Md ..
 // ze+Md-1.  One producer warp streams each plane (TY + 2 Md rows with the
@@ -502,7 +513,8 @@ __global__ void __launch_bounds__(384, 1) k_stencil_tma(const __grid_constant__ 
             for (int i = 0; i < NK; ++i) in[i] = P::splat((T)0);
             // y neighbours (the window also holds the thread's own rows)
 #pragma unroll
-            for (int j = 0; j < BY + 2 * MD; ++j) {
+            for (int jj = 0; jj < BY + 2 * MD; ++jj) {
+                const int j = term_order<T>(jj, BY + 2 * MD);
                 PT v[2];
                 P::get2(*reinterpret_cast<const V*>(sp + j * RS), v);
 #pragma unroll
@@ -537,10 +549,12 @@ __global__ void __launch_bounds__(384, 1) k_stencil_tma(const __grid_constant__ 
 #pragma unroll
                 for (int e = 0; e < 2; ++e)
 #pragma unroll
-                    for (int m = 1; m <= MD; ++m)
+                    for (int i = 1; i <= MD; ++i) {
+                        const int m = sizeof(T) == 8 ? i : MD + 1 - i;
                         in[2 * r + e] = P::fma(P::splat(cf.cx[m - 1]),
                                                P::add(P::of(w + MDX + W * e - m), P::of(w + MDX + W * e + m)),
                                                in[2 * r + e]);
+                    }
             }
             // centre and local potential
 #pragma unroll
@@ -698,7 +712,8 @@ __global__ void __launch_bounds__(192, 2) k_stencil_row(StencilArgs<T> a, const 
 #pragma unroll
             for (int i = 0; i < NK; ++i) in[i] = P::splat((T)0);
 #pragma unroll
-            for (int j = -MD; j < BY + MD; ++j) {
+            for (int jj = 0; jj < BY + 2 * MD; ++jj) {
+                const int j = term_order<T>(jj, BY + 2 * MD) - MD;
                 PT v[2];
                 if (j < 0 || j >= BY) {
                     P::get2(*reinterpret_cast<const V*>(sp + j * PX), v);
@@ -729,10 +744,12 @@ __global__ void __launch_bounds__(192, 2) k_stencil_row(StencilArgs<T> a, const 
 #pragma unroll
                 for (int e = 0; e < 2; ++e)
 #pragma unroll
-                    for (int m = 1; m <= MD; ++m)
+                    for (int i = 1; i <= MD; ++i) {
+                        const int m = sizeof(T) == 8 ? i : MD + 1 - i;
                         in[2 * r + e] = P::fma(P::splat(cf.cx[m - 1]),
                                                P::add(P::of(w + HX + W * e - m), P::of(w + HX + W * e + m)),
                                                in[2 * r + e]);
+                    }
                 PT vl[2];
                 P::get2(*reinterpret_cast<const V*>(sp + (ROWS - MD + r) * PX), vl);
 #pragma unroll
