@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(VT) k_cg_upd1(CGVec<T> v, long ld, long n, CGS
     const int items = vec_items<IT>(n);
     const long off = (long)b * ld, base = (long)blockIdx.x * (VT * items);
     const T u11 = (T)s.u11[b], u21 = (T)s.u21[b], w = (T)s.E[b];
-    const T xe = (T)(s.u11[b] * (s.E1[b] - s.E[b]));  // E1: the step's old quotient
+    const T xe = (T)(s.u11[b] * ((double)(T)s.E1[b] - (double)(T)s.E[b]));  // old and new shift, as g holds them
     const T* gin = FIRST ? v.hx : v.g;
     double acc = 0.0;
 #pragma unroll 4
@@ -554,7 +554,8 @@ __device__ void eig2(double a11, double a12, double a22, double b11, double b12,
 
 // 2x2 Rayleigh-Ritz, pair choice and sign fix (cg_module.f90:299-333) from the
 // five dots of the search-direction pass (the last two with g, or with H x in
-// the first step) and <p|H p>
+// the first step) and <p|H p>.  g was formed with the quotient rounded to T.
+template <typename T>
 __global__ void __launch_bounds__(SB) s_eig(CGScal s, const double* __restrict__ part, int nch, HpsiSum h, int nb,
                                             int first) {
     const int b = blockIdx.x * (SB / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -567,8 +568,9 @@ __global__ void __launch_bounds__(SB) s_eig(CGScal s, const double* __restrict__
     const double E = s.E[b];
     double W[2], X[4];
     int info;
-    const double xhx = first ? v[3] : fma(E, v[0], -0.5 * v[3]);
-    const double phx = first ? v[4] : fma(E, v[1], -0.5 * v[4]);
+    const double eg = (double)(T)E;
+    const double xhx = first ? v[3] : fma(eg, v[0], -0.5 * v[3]);
+    const double phx = first ? v[4] : fma(eg, v[1], -0.5 * v[4]);
     eig2(xhx, phx, php, v[0], v[1], v[2], W, X, &info);
     if (info != 0) {  // B not positive definite: keep x (no update)
         W[0] = E; X[0] = 1.0; X[1] = 0.0;
@@ -683,7 +685,7 @@ static int cg_run(T* x, long ld, int mb, int spin, double* esp, double* res, int
     hd.plan_nb = plan_mb;
     const int pcap = std::max(nchunk, 64);
     double* part = nullptr;
-    RS_CHECK(workspace_t("cg_part", (size_t)mb * ((size_t)nchunk * 6 + hd.cap + (size_t)(SS_MAXM + 1) * 2 * pcap),
+    RS_CHECK(workspace_t("cg_part", (size_t)mb * ((size_t)nchunk * 6 + hd.cap + (size_t)(SS_MAXM + 1) * 3 * pcap),
                          &part));
     double* pdots = part + (size_t)mb * nchunk;
     hd.part = pdots + (size_t)mb * nchunk * 5;
@@ -746,7 +748,7 @@ static int cg_run(T* x, long ld, int mb, int spin, double* esp, double* res, int
             RS_LAUNCH();
         }
         RS_CHECK(hpsi_device<T>(v.p, v.hp, ld, mb, spin, s.active, &hd));
-        launch(s_eig, wb, SB, 0, st, s, (const double*)pdots, nchunk, hpsi_sum_of(hd), mb, icg == 1);
+        launch(s_eig<T>, wb, SB, 0, st, s, (const double*)pdots, nchunk, hpsi_sum_of(hd), mb, icg == 1);
         launch(icg == 1 ? (full ? k_cg_upd1<T, true, 32> : k_cg_upd1<T, true, 0>)
                         : (full ? k_cg_upd1<T, false, 32> : k_cg_upd1<T, false, 0>),
                vg, VT, 0, st, v, ld, n, s, part, s.active, gv);

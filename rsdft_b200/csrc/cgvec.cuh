@@ -149,8 +149,8 @@ __device__ __forceinline__ void pc_step(const PcArgs& pa, int& i1, int& i2, int&
 // stays well conditioned) A acts on coefficients as the tridiagonal
 //   A w_0 = d (w_0 + w_1),  A w_k = d w_k + (d/2)(w_{k+1} + w_{k-1}),
 // and every dot the recurrences need is a bilinear form in the Gram matrix
-// G_ij = <w_i, w_j> (i < mloop, j <= mloop), which two dots per basis vector
-// determine (s_sstep).  So: mloop passes build the basis and its dots, the scalar recurrences of the reference run
+// G_ij = <w_i, w_j> (i < mloop, j <= mloop), which two or three dots per basis
+// vector determine (s_sstep).  So: mloop passes build the basis and its dots, the scalar recurrences of the reference run
 // per band on coefficient vectors (s_sstep), and one pass forms
 //   p = g + sum_j cz_j w_j + bk p
 // (Pg itself, the rb = <Pg|g> dot and cg_module.f90:247-261 folded in).
@@ -163,11 +163,11 @@ struct SSVec {
     T* w[SS_MAXM];
 };
 
-// per-CTA dot partials of the basis passes (pass k: nch[k] per band, two
-// values each, one in the last pass)
+// per-CTA dot partials of the basis passes (pass k: nch[k] per band, dots[k]
+// values each)
 struct SSPart {
     const double* part[SS_MAXM + 1];
-    int nch[SS_MAXM + 1];
+    int nch[SS_MAXM + 1], dots[SS_MAXM + 1];
 };
 
 // off-diagonal part of the 7-point operator at point i
@@ -187,7 +187,7 @@ __device__ __forceinline__ T pc_offdiag(const T* __restrict__ f, long i, int i1,
 // the line search's dots of x, p, g as per-CTA partials in dots (5 per chunk).
 // hx: H x in the first step, null later (k_ss_p).  plan_mb: the band count the
 // launch geometry is chosen for.
-// cz holds SS_MAXM doubles per band, part (SS_MAXM + 1) x 2 x part_cap per
+// cz holds SS_MAXM doubles per band, part (SS_MAXM + 1) x 3 x part_cap per
 // band.
 template <typename T>
 int sstep_precond(const T* g, const T* hx, const SSVec<T>& sv, T* p, T* x, long ld, int mb, int plan_mb, int mloop,

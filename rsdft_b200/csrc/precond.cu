@@ -14,13 +14,13 @@
 namespace rsdft {
 
 // Basis vector w_K (K = 0: r0 = g - A g, the reference's first residual) and
-// its dots: STORE, write w_K with <w_K, w_{K-1}> (K = 0: <g, w_0>) and
-// <w_K, w_K>; !STORE (K = mloop), only <S w_{K-1}, w_{K-1}> with S = B for
-// K = 1 and 2 B above.
-template <typename T, int K, bool STORE>
+// its D dots: D >= 2, write w_K with <w_K, w_{K-1}> (K = 0: <g, w_0>), <w_K, w_K>
+// and, with D = 3 (K >= 2), <w_K, w_{K-2}>; D = 1 (K = mloop), only
+// <S w_{K-1}, w_{K-1}> with S = B for K = 1 and 2 B above.
+template <typename T, int K, int D>
 __global__ void __launch_bounds__(VT) k_ss_basis(const T* __restrict__ g, SSVec<T> sv, long ld, long n, PcArgs pa,
                                                  double* __restrict__ part, const int* __restrict__ active) {
-    constexpr int D = STORE ? 2 : 1;
+    constexpr bool STORE = D > 1;
     __shared__ double sh[D * (VT / 32)];
     const int b = blockIdx.y;
     if (active && !active[b]) return;
@@ -45,12 +45,16 @@ __global__ void __launch_bounds__(VT) k_ss_basis(const T* __restrict__ g, SSVec<
                 wk = pc_offdiag<T>(src, i, i1, i2, i3, pa) * inv_d;
             } else {
                 wk = (T)2 * pc_offdiag<T>(src, i, i1, i2, i3, pa) * inv_d;
-                if constexpr (STORE) wk -= sv.w[K >= 2 ? K - 2 : 0][off + i];
+                if constexpr (STORE) {
+                    const T w2 = sv.w[K >= 2 ? K - 2 : 0][off + i];
+                    wk -= w2;
+                    if constexpr (D == 3) acc[2] = fma((double)wk, (double)w2, acc[2]);
+                }
             }
             acc[0] = fma((double)wk, (double)si, acc[0]);
             if constexpr (STORE) {
                 sv.w[K < SS_MAXM ? K : 0][off + i] = wk;
-                acc[D - 1] = fma((double)wk, (double)wk, acc[D - 1]);
+                acc[1] = fma((double)wk, (double)wk, acc[1]);
             }
         }
         pc_step(pa, i1, i2, i3);
@@ -69,16 +73,17 @@ __global__ void __launch_bounds__(VT) k_ss_basis(const T* __restrict__ g, SSVec<
 // <w_j|g> and the search-direction scalars bk = rb / gkgk, gkgk = rb
 // (cg_module.f90:232-250).
 //
-// w_j = T_j(B) w_0 with the Chebyshev polynomials T_j and B symmetric, so the
-// whole Gram matrix follows from the moments mu_k = <w_0, T_k(B) w_0>:
-//   <w_i, w_j> = (mu_{i+j} + mu_{|i-j|}) / 2,
-//   mu_{2k} = 2 <w_k, w_k> - mu_0,  mu_{2k+1} = 2 <w_{k+1}, w_k> - mu_1,
+// A basis pass dots what it has in hand: w_k with itself, with its source
+// w_{k-1} and, on small grids, with w_{k-2}.  The rest of the Gram matrix
+// follows from w_k = 2 B w_{k-1} - w_{k-2} with B symmetric, B w_0 = w_1 and
+// 2 B w_j = w_{j+1} + w_{j-1}:
+//   <w_k, w_j> = <w_{k-1}, w_{j+1}> + <w_{k-1}, w_{j-1}> - <w_{k-2}, w_j>,
+//   <w_k, w_0> = 2 <w_{k-1}, w_1> - <w_{k-2}, w_0>,
 // and, with B g = ((1 - d) g - w_0) / d (from w_0 = g - A g, A = d (I + B)),
-//   <g, w_1> = ((1 - d) <g, w_0> - mu_0) / d,
-//   <g, w_{j+1}> = 2 ((1 - d) <g, w_j> - mu_j) / d - <g, w_{j-1}>.
-// A basis pass therefore needs the dots of its source and its result only
-// (two per pass), and the last one a single dot of its source: it reads one
-// vector where a direct Gram matrix reads mloop + 1.
+//   <g, w_1> = ((1 - d) <g, w_0> - <w_0, w_0>) / d,
+//   <g, w_{j+1}> = 2 ((1 - d) <g, w_j> - <w_0, w_j>) / d - <g, w_{j-1}>.
+// The last pass needs one dot of its source, <S w_{m-1}, w_{m-1}>: it reads one
+// vector where dots with all of w_0 .. w_{m-1} and g read mloop + 1.
 // The order m is a template parameter, so that the small arrays stay in
 // registers (6.3 us a launch; 14.8 with run-time loops over local memory).
 template <int m>
@@ -86,36 +91,40 @@ __global__ void __launch_bounds__(128) s_sstep(CGScal s, SSPart pt, double* __re
                                                double dV, int first) {
     const int b = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (b >= nb || !s.active[b]) return;  // uniform per warp
-    double S[2 * (m + 1)];
+    double S[m + 1][3];
 #pragma unroll
     for (int k = 0; k <= m; ++k) {
-        const int D = k < m ? 2 : 1;
+        const int D = pt.dots[k];
         const double* p = pt.part[k] + (long)b * pt.nch[k] * D;
-        S[2 * k] = warp_strided_sum(p, pt.nch[k], D, lane);
-        S[2 * k + 1] = D == 2 ? warp_strided_sum(p + 1, pt.nch[k], D, lane) : 0.0;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) S[k][q] = q < D ? warp_strided_sum(p + q, pt.nch[k], D, lane) : 0.0;
     }
     if (lane != 0) return;
-    double mu[2 * m] = {}, gd[m] = {};
-    mu[0] = S[1];
-    gd[0] = S[0];
+    double G[m + 1][m + 1] = {}, gd[m] = {};
+    G[0][0] = S[0][1];
 #pragma unroll
     for (int k = 1; k <= m; ++k) {
-        // <w_k, w_{k-1}>; the last pass leaves <S w_{m-1}, w_{m-1}>
-        double c = S[2 * k];
-        if (k == m && k >= 2) c -= S[2 * (k - 1)];
-        mu[2 * k - 1] = k == 1 ? c : 2.0 * c - mu[1];
-        if (k < m) mu[2 * k] = 2.0 * S[2 * k + 1] - mu[0];
+        G[k][k] = S[k][1];
+#pragma unroll
+        for (int j = k - 1; j >= 0; --j) {
+            double v;
+            if (j == k - 1)  // the last pass leaves <S w_{m-1}, w_{m-1}>
+                v = k == m && k >= 2 ? S[k][0] - G[k >= 2 ? k - 2 : 0][j] : S[k][0];
+            else if (j == k - 2 && pt.dots[k] == 3)
+                v = S[k][2];
+            else if (j == 0)
+                v = 2.0 * G[k - 1][1] - G[k >= 2 ? k - 2 : 0][0];
+            else
+                v = G[k - 1][j + 1] + G[k - 1][j > 0 ? j - 1 : 0] - G[k >= 2 ? k - 2 : 0][j];
+            G[k][j] = G[j][k] = v;
+        }
     }
+    gd[0] = S[0][0];
 #pragma unroll
     for (int j = 1; j < m; ++j) {
-        const double t = ((1.0 - d) * gd[j - 1] - mu[j - 1]) / d;
-        gd[j] = j == 1 ? t : 2.0 * t - gd[j - 2];
+        const double t = ((1.0 - d) * gd[j - 1] - G[0][j - 1]) / d;
+        gd[j] = j == 1 ? t : 2.0 * t - gd[j >= 2 ? j - 2 : 0];
     }
-    double G[m + 1][m + 1] = {};
-#pragma unroll
-    for (int i = 0; i < m; ++i)
-    #pragma unroll
-    for (int j = 0; j <= m; ++j) G[i][j] = G[j][i] = 0.5 * (mu[i + j] + mu[i > j ? i - j : j - i]);
     double cz[m + 1] = {};
     double rr = G[0][0];
     if (!(rr < 1e-24)) {
@@ -266,29 +275,28 @@ __global__ void __launch_bounds__(VT) k_ss_p(const T* __restrict__ g, const T* _
     }
 }
 
+// element-wise basis step K with `dots` dots (one in the last pass)
 template <typename T>
-static int launch_ss_store(int k, dim3 vg, cudaStream_t st, const T* g, SSVec<T> sv, long ld, long n,
+static int launch_ss_basis(int K, int dots, dim3 vg, cudaStream_t st, const T* g, SSVec<T> sv, long ld, long n,
                            const PcArgs& pa, double* part, const int* act) {
-    switch (k) {
-        case 1: launch(k_ss_basis<T, 1, true>, vg, VT, 0, st, g, sv, ld, n, pa, part, act); break;
-        case 2: launch(k_ss_basis<T, 2, true>, vg, VT, 0, st, g, sv, ld, n, pa, part, act); break;
-        case 3: launch(k_ss_basis<T, 3, true>, vg, VT, 0, st, g, sv, ld, n, pa, part, act); break;
-        default: set_error("s-step basis index %d", k); return RSDFT_EUNSUP;
+#define RS_SS_CASE(KK, DD)                                                                    \
+    if (K == KK && dots == DD) {                                                              \
+        launch(k_ss_basis<T, KK, DD>, vg, VT, 0, st, g, sv, ld, n, pa, part, act);            \
+        return RSDFT_OK;                                                                      \
     }
-    return RSDFT_OK;
-}
-
-template <typename T>
-static int launch_ss_fly(int m, dim3 vg, cudaStream_t st, const T* g, SSVec<T> sv, long ld, long n,
-                         const PcArgs& pa, double* part, const int* act) {
-    switch (m) {
-        case 1: launch(k_ss_basis<T, 1, false>, vg, VT, 0, st, g, sv, ld, n, pa, part, act); break;
-        case 2: launch(k_ss_basis<T, 2, false>, vg, VT, 0, st, g, sv, ld, n, pa, part, act); break;
-        case 3: launch(k_ss_basis<T, 3, false>, vg, VT, 0, st, g, sv, ld, n, pa, part, act); break;
-        case 4: launch(k_ss_basis<T, 4, false>, vg, VT, 0, st, g, sv, ld, n, pa, part, act); break;
-        default: set_error("s-step mloop %d", m); return RSDFT_EUNSUP;
-    }
-    return RSDFT_OK;
+    RS_SS_CASE(0, 2)
+    RS_SS_CASE(1, 2)
+    RS_SS_CASE(2, 2)
+    RS_SS_CASE(3, 2)
+    RS_SS_CASE(2, 3)
+    RS_SS_CASE(3, 3)
+    RS_SS_CASE(1, 1)
+    RS_SS_CASE(2, 1)
+    RS_SS_CASE(3, 1)
+    RS_SS_CASE(4, 1)
+#undef RS_SS_CASE
+    set_error("s-step basis index %d", K);
+    return RSDFT_EUNSUP;
 }
 
 // ------------------------------------------- TMA z-march basis kernel
@@ -306,10 +314,9 @@ struct PcMaps {
     CUtensorMap aux[1];                 // epilogue operand, TY rows
 };
 
-template <int K, bool STORE>
+template <int K, int D>
 struct PcStep {
-    static constexpr int NA = (STORE && K >= 2) ? 1 : 0;  // w_{K-2}
-    static constexpr int D = STORE ? 2 : 1;
+    static constexpr int NA = (D > 1 && K >= 2) ? 1 : 0;  // w_{K-2}
     static constexpr int CTAS = 2;  // CTAs per SM (<= 85 registers, half the stage ring each)
 };
 
@@ -318,8 +325,8 @@ __device__ __forceinline__ int pc_pwrap(int i, int n) {
     return i < 0 ? i + n : i;
 }
 
-template <typename T, int K, bool STORE>
-__global__ void __launch_bounds__(384, PcStep<K, STORE>::CTAS) k_pc_tma(const __grid_constant__ PcMaps maps,
+template <typename T, int K, int D>
+__global__ void __launch_bounds__(384, PcStep<K, D>::CTAS) k_pc_tma(const __grid_constant__ PcMaps maps,
                                                                       T* __restrict__ wout,
                                                    StencilCoef cf, int n1, int n2, int n3, long ld, int zlen0,
                                                    int nzc, int TY, int RS, int S, int ncw,
@@ -331,8 +338,8 @@ __global__ void __launch_bounds__(384, PcStep<K, STORE>::CTAS) k_pc_tma(const __
     constexpr int BY = 2;
     constexpr int NP = VX * BY;
     constexpr int NV = 3;  // x window: x - VX .. x + 2 VX - 1
-    constexpr int NA = PcStep<K, STORE>::NA;
-    constexpr int D = PcStep<K, STORE>::D;
+    constexpr int NA = PcStep<K, D>::NA;
+    constexpr bool STORE = D > 1;
     extern __shared__ __align__(128) unsigned char smem[];
     const int ROWS = TY + 2;
     const int SE = (ROWS + NA * TY) * RS;
@@ -516,7 +523,8 @@ __global__ void __launch_bounds__(384, PcStep<K, STORE>::CTAS) k_pc_tma(const __
                         wk[e] = o[i] - av[0][e];
                     const double wd = (double)wk[e];
                     dots[0] = fma(wd, (double)cprev[i], dots[0]);
-                    if constexpr (STORE) dots[D - 1] = fma(wd, wd, dots[D - 1]);
+                    if constexpr (STORE) dots[1] = fma(wd, wd, dots[1]);
+                    if constexpr (D == 3) dots[2] = fma(wd, (double)av[0][e], dots[2]);
                 }
                 if constexpr (STORE) {
                     if (thr) *reinterpret_cast<V*>(ob + zo + (long)r * n1) = VT::make(wk);
@@ -608,16 +616,16 @@ static PcGeom pc_geometry(int n1, int n2, int n3, int mb, int sms, int part_cap,
 
 // Launch basis step K through k_pc_tma; *used = false when the shape or the
 // pointers do not suit it (the caller then takes the element-wise kernels).
-template <typename T, int K, bool STORE>
+template <typename T, int K, int D>
 static int pc_tma_step(const T* src, const T* const* aux, T* wout, const PcArgs& pa, long ld, int mb,
                        int plan_mb, const int* active, double* part, int part_cap, int* nchunk, bool* used) {
     Context& c = ctx();
     *used = false;
-    constexpr int NA = PcStep<K, STORE>::NA;
-    constexpr int D = PcStep<K, STORE>::D;
+    constexpr int NA = PcStep<K, D>::NA;
+    constexpr bool STORE = D > 1;
     const int n1 = pa.n1, n2 = pa.n2, n3 = pa.n3;
     const int sms = c.num_sms > 0 ? c.num_sms : 148;
-    const PcGeom g = pc_geometry<T>(n1, n2, n3, plan_mb, sms, part_cap, NA, D, PcStep<K, STORE>::CTAS);
+    const PcGeom g = pc_geometry<T>(n1, n2, n3, plan_mb, sms, part_cap, NA, D, PcStep<K, D>::CTAS);
     if (g.TY == 0 || (ld * sizeof(T)) % 16 != 0) return RSDFT_OK;
     if (STORE && reinterpret_cast<uintptr_t>(wout) % 16 != 0) return RSDFT_OK;
     const int zlen = div_up(n3, g.nzc);
@@ -639,7 +647,7 @@ static int pc_tma_step(const T* src, const T* const* aux, T* wout, const PcArgs&
         return RSDFT_OK;
     for (int a = 0; a < NA; ++a)
         if (encode_tmap_4d(&maps.aux[a], dt, aux[a], dims, strides, bm) != RSDFT_OK) return RSDFT_OK;
-    RS_CHECK(set_smem_optin((const void*)k_pc_tma<T, K, STORE>, 220 * 1024 + 8 * 16));
+    RS_CHECK(set_smem_optin((const void*)k_pc_tma<T, K, D>, 220 * 1024 + 8 * 16));
     // coefficients of the operator part: (A - I) for w_0, B = offdiag / d for
     // w_1, 2 B for the later steps
     StencilCoef cf{};
@@ -649,7 +657,7 @@ static int pc_tma_step(const T* src, const T* const* aux, T* wout, const PcArgs&
     cf.cy[0] = sc * pa.c2;
     cf.cz[0] = sc * pa.c3;
     dim3 grid(n2 / g.TY, (unsigned)(mb * nzc));
-    launch(k_pc_tma<T, K, STORE>, grid, g.threads, g.smem, c.stream, maps, wout, cf, n1, n2, n3, ld, zlen, nzc,
+    launch(k_pc_tma<T, K, D>, grid, g.threads, g.smem, c.stream, maps, wout, cf, n1, n2, n3, ld, zlen, nzc,
            g.TY, g.RS, g.S, g.ncw, part, active, c.err_flag);
     RS_LAUNCH();
     *nchunk = (n2 / g.TY) * nzc;
@@ -659,22 +667,24 @@ static int pc_tma_step(const T* src, const T* const* aux, T* wout, const PcArgs&
 
 // basis step K of the s-step form through the TMA kernel (runtime K)
 template <typename T>
-static int pc_tma_dispatch(int K, bool store, const T* g, const SSVec<T>& sv, const PcArgs& pa, long ld, int mb,
+static int pc_tma_dispatch(int K, int dots, const T* g, const SSVec<T>& sv, const PcArgs& pa, long ld, int mb,
                            int plan_mb, const int* active, double* part, int part_cap, int* nchunk, bool* used) {
     const T* src = K == 0 ? g : sv.w[K - 1];
     const T* aux[1] = {K >= 2 ? sv.w[K - 2] : nullptr};
-    T* wout = store ? sv.w[K] : nullptr;
-#define RS_PC_CASE(KK, ST)                                                                              \
-    if (K == KK && store == ST)                                                                         \
-        return pc_tma_step<T, KK, ST>(src, aux, wout, pa, ld, mb, plan_mb, active, part, part_cap, nchunk, used);
-    RS_PC_CASE(0, true)
-    RS_PC_CASE(1, true)
-    RS_PC_CASE(2, true)
-    RS_PC_CASE(3, true)
-    RS_PC_CASE(1, false)
-    RS_PC_CASE(2, false)
-    RS_PC_CASE(3, false)
-    RS_PC_CASE(4, false)
+    T* wout = dots > 1 ? sv.w[K] : nullptr;
+#define RS_PC_CASE(KK, DD)                                                                              \
+    if (K == KK && dots == DD)                                                                          \
+        return pc_tma_step<T, KK, DD>(src, aux, wout, pa, ld, mb, plan_mb, active, part, part_cap, nchunk, used);
+    RS_PC_CASE(0, 2)
+    RS_PC_CASE(1, 2)
+    RS_PC_CASE(2, 2)
+    RS_PC_CASE(3, 2)
+    RS_PC_CASE(2, 3)
+    RS_PC_CASE(3, 3)
+    RS_PC_CASE(1, 1)
+    RS_PC_CASE(2, 1)
+    RS_PC_CASE(3, 1)
+    RS_PC_CASE(4, 1)
 #undef RS_PC_CASE
     *used = false;
     return RSDFT_OK;
@@ -688,25 +698,28 @@ int sstep_precond(const T* g, const T* hx, const SSVec<T>& sv, T* p, T* x, long 
     const long n = c.ml;
     const int nchunk = vec_chunks(n, plan_mb, c.num_sms > 0 ? c.num_sms : 148);
     const dim3 vg(nchunk, mb);
+    // <w_k, w_{k-2}> as a dot or from the recurrence (s_sstep): w_0 .. w_2 of a
+    // smooth residual are nearly parallel, and the recurrence holds for the
+    // stored vectors to their rounding, whose effect on a dot falls as
+    // 1 / sqrt(n).  Residuals against 64 bits, FP64 48^3: 6.1e-14 by the
+    // recurrence, 3.8e-14 by the dot (85 | 103 us a pass at 160 bands); FP32,
+    // 72^3: 1.7e-6 either way (332 | 416 us at 480 bands).
+    const bool third = sizeof(T) == 8 || n <= 65536;
     SSPart pt{};
     // basis steps: TMA z march where the shape allows, element-wise otherwise
     for (int k = 0; k <= mloop; ++k) {
-        const bool store = k < mloop;
-        double* out = part + (size_t)k * 2 * part_cap * mb;
+        const int D = k == mloop ? 1 : (k >= 2 && third ? 3 : 2);
+        double* out = part + (size_t)k * 3 * part_cap * mb;
         bool used = false;
         int nch = 0;
-        RS_CHECK(pc_tma_dispatch<T>(k, store, g, sv, pa, ld, mb, plan_mb, s.active, out, part_cap, &nch, &used));
+        RS_CHECK(pc_tma_dispatch<T>(k, D, g, sv, pa, ld, mb, plan_mb, s.active, out, part_cap, &nch, &used));
         if (!used) {
-            if (k == 0)
-                launch(k_ss_basis<T, 0, true>, vg, VT, 0, st, g, sv, ld, n, pa, out, s.active);
-            else if (store)
-                RS_CHECK(launch_ss_store<T>(k, vg, st, g, sv, ld, n, pa, out, s.active));
-            else
-                RS_CHECK(launch_ss_fly<T>(k, vg, st, g, sv, ld, n, pa, out, s.active));
+            RS_CHECK(launch_ss_basis<T>(k, D, vg, st, g, sv, ld, n, pa, out, s.active));
             nch = nchunk;
         }
         pt.part[k] = out;
         pt.nch[k] = nch;
+        pt.dots[k] = D;
     }
     const int gv = grp16_ok<T>(ld, {g, hx, p, x, sv.w[0], sv.w[1], sv.w[2], sv.w[3]}) ? 1 : 0;
     auto launch_p = [&](auto M) {

@@ -1,6 +1,7 @@
 """CG sweep against the oracle where its kernels change form: the basis passes by TMA (even widths) and element-wise
-(odd ones), every s-step order, the literal preconditioner above it, no preconditioner, no line step, and bands that
-come in unnormalised (the first step then takes its dots from H x, not from g)."""
+(odd ones), every s-step order, the Gram matrix's second off-diagonal as dots (up to 65536 points) and from the
+recurrence, the literal preconditioner above it, no preconditioner, no line step, and bands that come in unnormalised
+(the first step then takes its dots from H x, not from g)."""
 import numpy as np
 import pytest
 import torch
@@ -20,6 +21,7 @@ def rel(a, b):
 @pytest.mark.parametrize("n,nb,mloop,ncg,scale", [
     (12, 16, 3, 4, 1.0), (12, 5, 1, 3, 1.0), (12, 3, 2, 2, 30.0), (16, 7, 4, 4, 1.0), (15, 9, 3, 4, 1.0),
     (13, 1, 4, 2, 1.0), (12, 4, 5, 3, 1.0), (12, 4, 0, 3, 1.0), (14, 6, 3, 0, 1.0), (15, 2, 2, 1, 30.0),
+    (40, 2, 4, 2, 1.0), (41, 2, 3, 2, 1.0), (42, 2, 4, 2, 1.0),
 ])
 def test_cg_forms(gpu, n, nb, mloop, ncg, scale):
     c = build_cell(Workload("cg_forms", 1, n, nb, nb, 0.03, 2000 + n))
