@@ -375,6 +375,10 @@ __device__ __forceinline__ void push_slot(int u, typename Pk<T>::t (&acc)[2 * MD
 #undef RS_PUSH_CASE
 }
 
+// Threads of a march CTA: the register budget of the 2 Md + 1 accumulators (168
+// per thread; three rows per thread take up to 255)
+constexpr int march_threads(int by) { return by == 3 ? 256 : 384; }
+
 // Order of the in-plane terms.  FP32: the y rows from the outermost inwards, x
 // likewise, the centre last, so that few roundings are at the size of the large
 // terms: the bands of a CG sweep (FP32, against FP64) at 24^3 were 4.4e-7 off
@@ -400,9 +404,9 @@ __device__ __forceinline__ constexpr int term_order(int i, int n) {
 // indices (a switch on the slot selects the push), so a stage is read only
 // while its own plane is current and the ring can stay shallow.
 template <typename T, int MD, int BY, bool DOT>
-__global__ void __launch_bounds__(384, 1) k_stencil_tma(const __grid_constant__ TmaMaps maps, StencilArgs<T> a,
-                                                       const CoefT<T> cf, int TY, int RS, int S, int ncw,
-                                                       int* __restrict__ err) {
+__global__ void __launch_bounds__(march_threads(BY), 1)
+    k_stencil_tma(const __grid_constant__ TmaMaps maps, StencilArgs<T> a, const CoefT<T> cf, int TY, int RS, int S,
+                  int ncw, int* __restrict__ err) {
     using VT = Vec16<T>;
     using V = typename VT::t;
     constexpr int VX = 16 / (int)sizeof(T);
@@ -867,6 +871,7 @@ static void launch_stencil_md(const StencilArgs<T>& a, const StencilCoef& cf, in
 struct TmaGeom {
     int TY = 0, RS = 0, S = 0, ncw = 0, threads = 0, nzc = 1;
     size_t smem = 0;
+    double cost = 0.0;
 };
 
 // The tile height and z split of least march_cost.  A plane costs about 500
@@ -888,7 +893,7 @@ static TmaGeom tma_geometry(int n1, int n2, int nz, int nb, int sms, int dot_cap
         if (n2 % TY != 0 || TY < MD || !(TY == n2 || n2 >= TY + MD)) continue;
         const int ncw = ((n1 / VX) * (TY / BY) + 31) / 32;
         const int threads = 32 * (ncw + 1);
-        if (threads > 384) continue;
+        if (threads > march_threads(BY)) continue;
         const size_t stage = (size_t)(2 * TY + 2 * MD) * RS * sizeof(T);
         const int S = (int)std::min<size_t>(budget / (stage + 16), 8);
         if (S < 3) continue;
@@ -909,6 +914,7 @@ static TmaGeom tma_geometry(int n1, int n2, int nz, int nb, int sms, int dot_cap
             best.ncw = ncw;
             best.threads = threads;
             best.nzc = nzc;
+            best.cost = cost;
             best.smem = (size_t)S * stage + (size_t)S * 16 + 12 * sizeof(double);
         }
     }
@@ -927,12 +933,10 @@ static int launch_tma_dot(const TmaMaps& maps, const StencilArgs<T>& a, const St
 }
 
 template <typename T, int MD, int BY>
-static int launch_tma(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStream_t st, HpsiDot* dot, bool* used) {
+static int launch_tma(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStream_t st, HpsiDot* dot,
+                      const TmaGeom& g, bool* used) {
     Context& c = ctx();
     *used = false;
-    const int sms = c.num_sms > 0 ? c.num_sms : 148;
-    const TmaGeom g = tma_geometry<T, MD, BY>(a.n1, a.n2, a.nzo, dot && dot->plan_nb ? dot->plan_nb : nb, sms,
-                                                dot ? dot->cap : 1 << 20);
     if (g.TY == 0) return RSDFT_OK;
     if (reinterpret_cast<uintptr_t>(a.hpsi) % 16 != 0 || (a.ld * sizeof(T)) % 16 != 0) return RSDFT_OK;
     a.zlen = div_up(a.nzo, g.nzc);
@@ -1027,9 +1031,24 @@ template <typename T, int MD>
 static int launch_stencil_md2(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStream_t st, HpsiDot* dot) {
     const Context& c = ctx();
     bool used = false;
-    // two rows per thread up to Md = 6; one above, where the 2 Md + 1
-    // accumulators of two rows no longer fit the register budget
-    RS_CHECK((launch_tma<T, MD, (MD <= 6 ? 2 : 1)>(a, cf, nb, st, dot, &used)));
+    // Rows per thread: two up to Md = 6, one above, where the 2 Md + 1
+    // accumulators of two rows no longer fit the register budget.  In FP64 also
+    // three (246 registers, 7 instead of 11 warps at 72^3): the window loads per
+    // point drop from 7 to 6, the stencil of 72^3 x 480 from 1113 to 1018 us.
+    // Only on the same tiles, for the long windows (Md >= 5) and with six warps
+    // left: 42^3 x 351 at Md = 4 took 283 us against 250.  In FP32, where a load
+    // serves twice the points and the warps' latency counts more, three rows
+    // took 660 us against 646.
+    constexpr int BY = MD <= 6 ? 2 : 1;
+    const int plan = dot && dot->plan_nb ? dot->plan_nb : nb, cap = dot ? dot->cap : 1 << 20;
+    const int nsm = c.num_sms > 0 ? c.num_sms : 148;
+    const TmaGeom g = tma_geometry<T, MD, BY>(a.n1, a.n2, a.nzo, plan, nsm, cap);
+    if constexpr (sizeof(T) == 8 && (MD == 5 || MD == 6)) {
+        const TmaGeom g3 = tma_geometry<T, MD, 3>(a.n1, a.n2, a.nzo, plan, nsm, cap);
+        if (g.TY != 0 && g3.TY == g.TY && g3.ncw >= 6 && g3.cost < 0.93 * g.cost)
+            RS_CHECK((launch_tma<T, MD, 3>(a, cf, nb, st, dot, g3, &used)));
+    }
+    if (!used) RS_CHECK((launch_tma<T, MD, BY>(a, cf, nb, st, dot, g, &used)));
     if (!used) RS_CHECK((launch_row<T, MD, (MD <= 6 ? 2 : 1)>(a, cf, nb, st, dot, &used)));
     if (used) {
         if (a.gpt_ptr && c.nl_npt > 0) {
