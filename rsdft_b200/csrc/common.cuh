@@ -119,7 +119,7 @@ struct Context {
     std::vector<char> host_ws;               // host scratch of cuSOLVER calls
     std::map<const void*, int> smem_optin;   // dynamic shared memory opted in, per kernel
     int max_smem_optin = -1;                 // device limit (cudaDevAttrMaxSharedMemoryPerBlockOptin)
-    int sytrd_clusters = -1;                 // active 16-CTA clusters of the eigensolver kernel
+    int sytrd_clusters[2] = {-1, -1};        // active clusters of the eigensolver kernel's two forms
     double* noalloc_scratch = nullptr;       // device address of the static scratch array
 };
 

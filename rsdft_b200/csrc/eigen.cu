@@ -4,14 +4,14 @@
 // orthonormal eigenvector basis), in three steps:
 //
 //  1. k_sytrd: Householder tridiagonalisation A = Q T Q^T (LAPACK dsytd2,
-//     lower form) by ONE thread-block cluster of 16 CTAs with the whole
-//     matrix resident in their shared memory: CTA c holds the full rows
-//     i = c, c + 16, ... .  Column j: every CTA holds the reflector v, forms
+//     lower form) by ONE thread-block cluster of C = 8 or 16 CTAs with the
+//     whole matrix resident in their shared memory: CTA c holds the full rows
+//     i = c, c + C, ... .  Column j: every CTA holds the reflector v, forms
 //     p = tau A v on its own rows and its part of p^T v, pulls the rest of p
 //     and the look-ahead row j+1 over distributed shared memory, applies the
 //     rank-2 update A -= v w^T + w v^T (w = p - tau/2 (p^T v) v) to its own
 //     rows and to that row, and forms the next reflector itself.  One
-//     cluster barrier per column; nothing leaves the SMs until T and the
+//     exchange per column; nothing leaves the SMs until T and the
 //     reflectors are written.
 //  2. k_tri_bisect: eigenvalues of T by multisection on Sturm counts (one
 //     warp per eigenvalue, 32 trial points per round; LAPACK dstebz's count
@@ -33,7 +33,7 @@
 //
 // cuSOLVER's one-stage syevd spends ~80 % of its time in sytrd for these
 // sizes (3.9 of 5.0 ms at n = 480 on B200), one short kernel per column;
-// here each column costs one cluster barrier.
+// here each column costs one exchange within the cluster.
 #include <cfloat>
 
 #include "common.cuh"
@@ -44,21 +44,23 @@
 
 namespace rsdft {
 
-constexpr int TD_C = 16;          // CTAs in the cluster
-constexpr int TD_T = 512;         // threads per CTA
-constexpr int TD_W = TD_T / 32;
-
+// k_sytrd's cluster: 16 CTAs of 512 threads, or up to n = TD_SMALL 8 of 256,
+// whose barriers and exchange cost less (8 x 256 | 16 x 512, us: n = 32 49.5 |
+// 56, 101 171 | 189, 160 346 | 310)
+constexpr int TD_SMALL = 128;
 
 // Shared-memory layout of k_sytrd (doubles; every array an even count, so
-// each starts 16-byte aligned for the bulk copies): own rows R x np, the
+// each starts 16-byte aligned for the exchange): own rows R x np, the
 // reflectors v_j / v_{j+1}, w, p, the look-ahead row, and the exchange
-// buffers: per parity what each CTA sent, px[16][PR], and this CTA's
+// buffers: per parity what each CTA sent, px[C][PR], and this CTA's
 // outgoing block sb[PR] = [its R pieces of p, its part of p^T v, its rows'
 // entries of the look-ahead column, padding]; reduction slots, scalars, and
 // the two receive mbarriers.
+template <int TD_C, int TD_T>
 struct TdLayout {
+    static constexpr int TD_W = TD_T / 32;
     int R, np, PR;
-    size_t rows, vl, wf, pf, rr, px, sb, red, sc, bar, total;
+    size_t rows, vl, wf, pf, rr, px, sb, red, rsg, sc, bar, total;
     __host__ __device__ TdLayout(int n) {
         R = (n + TD_C - 1) / TD_C;
         np = (n + 1) & ~1;
@@ -71,7 +73,8 @@ struct TdLayout {
         px = rr + np;                       // [2][TD_C][PR]
         sb = px + 2 * (size_t)TD_C * PR;    // [2][PR]
         red = sb + 2 * (size_t)PR;
-        sc = red + TD_W;
+        rsg = red + TD_W;
+        sc = rsg + TD_W;
         bar = sc + 8;  // 2 x uint64_t
         total = bar + 2;
     }
@@ -85,23 +88,20 @@ __device__ __forceinline__ uint32_t cl_addr(const void* p, uint32_t rank) {
     return r;
 }
 
-// Bulk copy (TMA engine, point to point, no multicast) of `bytes` from this
-// CTA's shared memory to the buffer at the same offset as `dst` in CTA
-// `rank`, completion counted on that CTA's mbarrier at the offset of `bar`.
-// Addresses 16-byte aligned, bytes a multiple of 16.
-__device__ __forceinline__ void bulk_to_peer(const void* dst, const void* src, uint32_t bytes, const uint64_t* bar,
-                                             uint32_t rank) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            cl_addr(dst, rank)),
-        "r"((uint32_t)__cvta_generic_to_shared(src)), "r"(bytes), "r"(cl_addr(bar, rank))
-        : "memory");
+// Asynchronous 16-byte store to another CTA's shared memory (point to point),
+// counted on that CTA's mbarrier; both are shared::cluster addresses (cl_addr).
+__device__ __forceinline__ void st_to_peer(uint32_t dst, double x, double y, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(dst),
+                 "d"(x), "d"(y), "r"(bar)
+                 : "memory");
 }
 
 // dlarfg on x[0..len): v (v_0 = 1) into vl, sc[0] = tau, sc[1] = beta.  All
 // threads of the CTA; fixed reduction order, so every CTA that runs it on
 // the same x gets the same bits.
+template <int TD_T>
 __device__ __forceinline__ void td_reflector(const double* x, int len, double* vl, double* red, double* sc) {
+    constexpr int TD_W = TD_T / 32;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     double s = 0.0;
     for (int k = 1 + tid; k < len; k += TD_T) s = fma(x[k], x[k], s);
@@ -134,8 +134,8 @@ __device__ __forceinline__ void td_reflector(const double* x, int len, double* v
 // tau (n-1) and the reflectors in the strict lower part of Q (n x n, ld n;
 // Q(j+1+k, j) = v_k for k >= 1, dsytrd's 'L' storage).
 //
-// Column j: every CTA holds v_j and has pushed, with bulk copies into every
-// CTA of the cluster, its pieces of p_j = tau_j A v_j and of p_j^T v_j and
+// Column j: every CTA holds v_j and has pushed, into every CTA of the
+// cluster, its pieces of p_j = tau_j A v_j and of p_j^T v_j and
 // its rows' entries of column j+1 as they stand (the look-ahead row, by
 // symmetry; gathered from all CTAs, so no SM serves a one-to-all broadcast).
 // Each CTA waits on its own mbarrier for those bytes, forms w_j, brings its
@@ -146,12 +146,20 @@ __device__ __forceinline__ void td_reflector(const double* x, int len, double* v
 // ordering: exchange buffers are double-buffered by column parity, and the
 // block a CTA must hold before reusing a buffer was sent after that buffer's
 // previous use, so no cluster barrier is needed per column.
+//
+// Bound by the latency of a column's chain (n = 480: 2.8 us).  The exchange is
+// by 16-byte asynchronous stores, a warp per receiver, straight from the block's
+// elements: with a bulk copy per receiver, issued one after the other by one
+// thread behind a proxy fence and one more barrier, n = 32 took 69 us, 160 377
+// and 480 1499; this way 49.5, 310 and 1323.
+template <int TD_C, int TD_T>
 __global__ void __launch_bounds__(TD_T, 1) k_sytrd(const double* __restrict__ A, int lda, int n, int upper,
                                                   double* __restrict__ Q, double* __restrict__ d,
                                                   double* __restrict__ e, double* __restrict__ tau,
                                                   int* __restrict__ err) {
+    constexpr int TD_W = TD_T / 32;
     extern __shared__ __align__(16) double sm[];
-    const TdLayout L(n);
+    const TdLayout<TD_C, TD_T> L(n);
     const int R = L.R, np = L.np, PR = L.PR;
     double* rows = sm + L.rows;
     double* vb = sm + L.vl;  // [2][np]
@@ -161,6 +169,7 @@ __global__ void __launch_bounds__(TD_T, 1) k_sytrd(const double* __restrict__ A,
     double* px = sm + L.px;
     double* sb = sm + L.sb;
     double* red = sm + L.red;
+    double* rsg = sm + L.rsg;  // its own array: a slow warp of send may still read red
     double* sc = sm + L.sc;
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm + L.bar);
     const int cr = (int)cluster_rank();
@@ -183,24 +192,47 @@ __global__ void __launch_bounds__(TD_T, 1) k_sytrd(const double* __restrict__ A,
     __syncthreads();
     cluster_sync();  // rows loaded and receive barriers initialised everywhere
 
-    // push this CTA's block for column jn from sb[buf] into every CTA; arm
-    // this CTA's own barrier for the 16 blocks it will receive
+    // push this CTA's block for a column from sb[buf], with the sum of red (its
+    // share of <p, v>) as element R, into every CTA, a warp per receiver and 16
+    // bytes per lane; arm this CTA's own barrier for the blocks it will receive
     auto send = [&](int buf) {
-        fence_proxy_async_smem();
+        const double* sbb = sb + (size_t)buf * PR;
+        auto red_sum = [&] {  // fixed order
+            double v[TD_W];
+#pragma unroll
+            for (int w = 0; w < TD_W; w += 2) {
+                const double2 q = *reinterpret_cast<const double2*>(red + w);
+                v[w] = q.x;
+                v[w + 1] = q.y;
+            }
+#pragma unroll
+            for (int h = TD_W / 2; h >= 1; h >>= 1)
+#pragma unroll
+                for (int w = 0; w < h; ++w) v[w] = v[2 * w] + v[2 * w + 1];
+            return v[0];
+        };
         __syncthreads();
-        if (tid == 0) {
-            const uint32_t pb = (uint32_t)(PR * sizeof(double));
-            mbar_arrive_expect_tx(&bar[buf], TD_C * pb);
-            for (int dst = 0; dst < TD_C; ++dst)
-                bulk_to_peer(px + ((size_t)buf * TD_C + cr) * PR, sb + (size_t)buf * PR, pb, &bar[buf],
-                             (uint32_t)dst);
+        if (tid == 0) mbar_arrive_expect_tx(&bar[buf], (uint32_t)(TD_C * PR * sizeof(double)));
+        const double* to = px + ((size_t)buf * TD_C + cr) * PR;
+        for (int dst = warp; dst < TD_C; dst += TD_W) {
+            const uint32_t da = cl_addr(to, (uint32_t)dst), ba = cl_addr(&bar[buf], (uint32_t)dst);
+            for (int k = 2 * lane; k < PR; k += 64)
+                if (k != (R & ~1)) {
+                    const double2 q = *reinterpret_cast<const double2*>(sbb + k);
+                    st_to_peer(da + 8 * k, q.x, q.y, ba);
+                }
+            if (lane == 0) {
+                const int k = R & ~1;
+                const double v = red_sum();
+                st_to_peer(da + 8 * k, k == R ? v : sbb[k], k == R ? sbb[k + 1] : v, ba);
+            }
         }
     };
 
     // v_0 from row 0 (CTA 0, local row 0)
     for (int k = tid; k < n; k += TD_T) rr[k] = dsmem_ld(rows + k, 0);
     __syncthreads();
-    td_reflector(rr + 1, n - 1, vb, red, sc);
+    td_reflector<TD_T>(rr + 1, n - 1, vb, red, sc);
     if (cr == 0 && tid == 0) {
         d[0] = rr[0];
         e[0] = sc[1];
@@ -232,11 +264,6 @@ __global__ void __launch_bounds__(TD_T, 1) k_sytrd(const double* __restrict__ A,
             }
         }
         if (lane == 0) red[warp] = kacc;
-        __syncthreads();
-        if (warp == 0) {
-            const double s1 = warp_sum_d(lane < TD_W ? red[lane] : 0.0);
-            if (lane == 0) sb[R] = s1;
-        }
         send(0);
     }
 
@@ -248,14 +275,11 @@ __global__ void __launch_bounds__(TD_T, 1) k_sytrd(const double* __restrict__ A,
         const double t = tcur;
         // no cluster barrier: a CTA copies into px[par] of a peer for column
         // j+2 only after it has received that peer's block for column j+1,
-        // which the peer sends after its reads of px[par] for column j; and a
-        // peer's copies out of sb[par] for column j have all landed once this
-        // CTA holds every block for column j+1 (each sender waited for its
-        // column-j blocks before sending those)
+        // which the peer sends after its reads of px[par] for column j
         if (!mbar_wait(&bar[par], (uint32_t)((j >> 1) & 1))) ok = false;
         {
             // p_j and the look-ahead row j+1 (= column j+1: A(i, j+1) from the
-            // owner of row i), both spread over the 16 blocks
+            // owner of row i), both spread over the CTAs' blocks
             const double* xp = px + (size_t)par * TD_C * PR;
             for (int k = tid; k < m; k += TD_T) {
                 const int i = j + 1 + k;
@@ -267,13 +291,13 @@ __global__ void __launch_bounds__(TD_T, 1) k_sytrd(const double* __restrict__ A,
         // w = p + alpha v (into wf), row j+1 up to date; its columns j+3..
         // give sigma of v_{j+1}
         double sg = 0.0;
-        {
+        if (warp * 32 < m) {
             const double* xp = px + (size_t)par * TD_C * PR;
-            double kp[TD_C / 2];  // pairwise sum of the 16 partial dots (fixed order)
+            double kp[TD_C];  // pairwise sum of the CTAs' partial dots (fixed order)
 #pragma unroll
-            for (int c = 0; c < TD_C / 2; ++c) kp[c] = xp[(size_t)(2 * c) * PR + R] + xp[(size_t)(2 * c + 1) * PR + R];
+            for (int c = 0; c < TD_C; ++c) kp[c] = xp[(size_t)c * PR + R];
 #pragma unroll
-            for (int h = TD_C / 4; h >= 1; h >>= 1)
+            for (int h = TD_C / 2; h >= 1; h >>= 1)
 #pragma unroll
                 for (int c = 0; c < h; ++c) kp[c] = kp[2 * c] + kp[2 * c + 1];
             const double al = -0.5 * t * kp[0];
@@ -289,7 +313,7 @@ __global__ void __launch_bounds__(TD_T, 1) k_sytrd(const double* __restrict__ A,
             }
         }
         sg = warp_sum_d(sg);
-        if (lane == 0) red[warp] = sg;
+        if (lane == 0) rsg[warp] = sg;
         __syncthreads();
         if (j + 1 > n - 2) {
             if (cr == 0 && tid == 0) {
@@ -303,7 +327,7 @@ __global__ void __launch_bounds__(TD_T, 1) k_sytrd(const double* __restrict__ A,
         double tn, scal;
         bool nontriv;
         {
-            const double sig = warp_sum_d(lane < TD_W ? red[lane] : 0.0);
+            const double sig = warp_sum_d(lane < TD_W ? rsg[lane] : 0.0);
             const double alpha = rr[1];
             double tt = 0.0, beta = alpha, sl = 0.0;
             if (sig > 0.0) {
@@ -372,11 +396,6 @@ __global__ void __launch_bounds__(TD_T, 1) k_sytrd(const double* __restrict__ A,
             }
         }
         if (lane == 0) red[warp] = kacc;
-        __syncthreads();
-        if (warp == 0) {
-            const double s1 = warp_sum_d(lane < TD_W ? red[lane] : 0.0);
-            if (lane == 0) sbn[R] = s1;
-        }
         send(nxt);
         tcur = tn;
     }
@@ -430,6 +449,9 @@ __global__ void __launch_bounds__(32 * BS_WARPS) k_tri_bisect(const double* __re
     const double tnorm = fmax(fabs(glo), fabs(ghi));
     double lo = glo - 2.0 * DBL_EPSILON * tnorm * n - 2.0 * pivmin;
     double hi = ghi + 2.0 * DBL_EPSILON * tnorm * n + 2.0 * pivmin;
+    // the pivots' floor, up to the next value of the high word
+    const int pivhi = __double2hiint(pivmin);
+    const double pivmin2 = __hiloint2double(pivhi + 1, 0);
     constexpr int NPT = 32 * BS_PTS;
     for (int round = 0; round < 64; ++round) {
         if (hi - lo <= 2.0 * DBL_EPSILON * tnorm + pivmin) break;  // dstebz's absolute tolerance
@@ -440,16 +462,28 @@ __global__ void __launch_bounds__(32 * BS_WARPS) k_tri_bisect(const double* __re
         for (int u = 0; u < BS_PTS; ++u) {
             x[u] = lo + h * ((double)(lane * BS_PTS + u + 1) / (double)(NPT + 1));
             q[u] = sd[0] - x[u];
-            if (fabs(q[u]) <= pivmin) q[u] = -pivmin;
+            if ((__double2hiint(q[u]) & 0x7fffffff) <= pivhi) q[u] = -pivmin2;
             c[u] = q[u] < 0.0 ? 1 : 0;
         }
         for (int i = 1; i < n; ++i) {
             const double di = sd[i], ei = se2[i - 1];
 #pragma unroll
             for (int u = 0; u < BS_PTS; ++u) {
-                q[u] = di - x[u] - ei * rcp_nr(q[u]);  // |q| > pivmin >= DBL_MIN: normal
-                if (fabs(q[u]) <= pivmin) q[u] = -pivmin;
-                c[u] += q[u] < 0.0 ? 1 : 0;
+                // q <- d - x - e^2 / q (|q| > pivmin >= DBL_MIN: normal).  With
+                // y ~ 1 / q to 2^-22 and err = 1 - q y, 1 / q = y (1 + err +
+                // err^2) to 2^-66 (Householder's third-order iteration), and
+                // e^2 y and d - x - e^2 y do not wait for err: three dependent
+                // operations after the seed, where a rounded reciprocal, the
+                // product and the difference are six.  Sign and the test
+                // against pivmin on the high word.
+                double y;
+                asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(q[u]));
+                const double err = fma(-q[u], y, 1.0);
+                const double r = ei * y, base = di - x[u] - r;
+                q[u] = fma(-r, fma(err, err, err), base);
+                const int hi = __double2hiint(q[u]);
+                if ((hi & 0x7fffffff) <= pivhi) q[u] = -pivmin2;
+                c[u] += (unsigned)__double2hiint(q[u]) >> 31;
             }
         }
         // first trial point (in x order) with more than k eigenvalues below it
@@ -646,39 +680,40 @@ __global__ void __launch_bounds__(32 * IV_WARPS) k_tri_invit(const double* __res
     }
 }
 
-static size_t td_smem_bytes(int n) { return TdLayout(n).total * sizeof(double); }
-
 int syevd_fast(double* A, int n, double* W, cublasFillMode_t uplo) {
     Context& c = ctx();
     if (n < 3 || n > 32 * IV_RPL) return RSDFT_EUNSUP;
-    const size_t smem = td_smem_bytes(n);
+    const bool small = n <= TD_SMALL;
+    const size_t smem = (small ? TdLayout<8, 256>(n).total : TdLayout<16, 512>(n).total) * sizeof(double);
+    auto kern = small ? k_sytrd<8, 256> : k_sytrd<16, 512>;
+    int& clusters = c.sytrd_clusters[small ? 0 : 1];
     if (c.max_smem_optin < 0)
         RS_CUDA(cudaDeviceGetAttribute(&c.max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c.device));
     if (smem > (size_t)c.max_smem_optin || ormtr_smem_bytes(n) > (size_t)c.max_smem_optin) return RSDFT_EUNSUP;
-    if ((int)smem > c.smem_optin[(const void*)k_sytrd]) {
-        RS_CUDA(cudaFuncSetAttribute(k_sytrd, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        RS_CHECK(set_smem_optin((const void*)k_sytrd, (int)smem));
-        c.sytrd_clusters = -1;
+    if ((int)smem > c.smem_optin[(const void*)kern]) {
+        if (!small) RS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        RS_CHECK(set_smem_optin((const void*)kern, (int)smem));
+        clusters = -1;
     }
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = TD_C;
+    attr[0].val.clusterDim.x = small ? 8 : 16;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(TD_C);
-    cfg.blockDim = dim3(TD_T);
+    cfg.gridDim = dim3(small ? 8 : 16);
+    cfg.blockDim = dim3(small ? 256 : 512);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = c.stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (c.sytrd_clusters < 0) {
-        if (cudaOccupancyMaxActiveClusters(&c.sytrd_clusters, k_sytrd, &cfg) != cudaSuccess) {
+    if (clusters < 0) {
+        if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
             cudaGetLastError();
-            c.sytrd_clusters = 0;
+            clusters = 0;
         }
     }
-    if (c.sytrd_clusters < 1) return RSDFT_EUNSUP;
+    if (clusters < 1) return RSDFT_EUNSUP;
 
     double *Q = nullptr, *dd = nullptr, *ws = nullptr;
     RS_CHECK(workspace_t("eig_Q", (size_t)n * n, &Q));
@@ -689,7 +724,7 @@ int syevd_fast(double* A, int n, double* W, cublasFillMode_t uplo) {
     double* tau = dd + 2 * n;
     double* aux = dd + 3 * n;
     ++g_kernel_launches;
-    RS_CUDA(cudaLaunchKernelEx(&cfg, k_sytrd, (const double*)A, n, n, uplo == CUBLAS_FILL_MODE_UPPER ? 1 : 0, Q, d,
+    RS_CUDA(cudaLaunchKernelEx(&cfg, kern, (const double*)A, n, n, uplo == CUBLAS_FILL_MODE_UPPER ? 1 : 0, Q, d,
                                e, tau, c.err_flag));
     RS_LAUNCH();
     launch(k_tri_bisect, div_up(n, BS_WARPS), 32 * BS_WARPS, (size_t)2 * n * sizeof(double), c.stream,

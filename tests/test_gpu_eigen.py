@@ -60,6 +60,13 @@ def test_subspace_solv_matches_lapack(gpu, n, kind):
     assert np.abs(a @ v - v * w).max() <= 1e-13 * n * scale
 
 
+@pytest.mark.parametrize("n", [5, 8, 9, 31, 64, 127, 128, 129, 130])
+@pytest.mark.parametrize("kind", ["random", "degenerate", "scaled"])
+def test_tridiagonalisation_clusters(gpu, n, kind):
+    """Both sides of the line between the two clusters at n = 128, and remainders of their row blocks."""
+    test_subspace_solv_matches_lapack(gpu, n, kind)
+
+
 def test_subspace_solv_repeatable(gpu):
     """Same input, same bits (fixed reduction orders, seeded start vectors)."""
     a = spectrum_matrix(480, "near_diagonal", np.random.default_rng(7))
