@@ -19,7 +19,7 @@
 // Why: the FP64 tensor pipe gives 37 TFLOP/s, the INT8 pipe 34 digit products
 // per FP64 product at up to 4.5 POP/s, an FP64 rate of about 130 TFLOP/s.
 // 72^3 x 480, psi^T psi: 1170 us against 4365 us (DMMA, upper tiles);
-// psi V: 2100 us against 6360 us; slicing psi for both 1080 us
+// psi V: 2000 us against 6360 us; slicing psi for both 960 us
 // (exponents included).
 //
 // k_imma, one CTA per 128 x 64 tile of D(m, n) = sum_k A(m, k) B(n, k):
@@ -131,7 +131,10 @@ __device__ __forceinline__ void byte_transpose(uint32_t a, uint32_t b, uint32_t 
 __global__ void __launch_bounds__(256) k_imma_slice(const double* __restrict__ A, long ld, long ml, int nb, int nkb,
                                                     const int* __restrict__ exps, int8_t* __restrict__ rows,
                                                     int8_t* __restrict__ cols, const int* __restrict__ bad, int vec) {
-    __shared__ __align__(16) uint32_t sm[IM_S][64][20];
+    // pitch 17: the transposed words of a half warp (rows 4 apart) fall on 8
+    // banks (at a pitch of 20, which 16-byte reads want, on 2: 872 us per
+    // 72^3 x 480 block instead of 753)
+    __shared__ uint32_t sm[IM_S][64][17];
     if (*bad) return;
     const int p = threadIdx.x & 15, q = threadIdx.x >> 4;
     const int kb = blockIdx.x, mb = blockIdx.y;
@@ -175,7 +178,7 @@ __global__ void __launch_bounds__(256) k_imma_slice(const double* __restrict__ A
             const int s = t >> 8, r = (t >> 2) & 63, w = t & 3;
             if (mb * 64 + r < nb)
                 *reinterpret_cast<uint4*>(rows + (((size_t)s * nkb + kb) * nb + mb * 64 + r) * 64 + 16 * w) =
-                    *reinterpret_cast<const uint4*>(&sm[s][r][4 * w]);
+                    make_uint4(sm[s][r][4 * w], sm[s][r][4 * w + 1], sm[s][r][4 * w + 2], sm[s][r][4 * w + 3]);
         }
         __syncthreads();
     }
@@ -195,14 +198,15 @@ __global__ void __launch_bounds__(256) k_imma_slice(const double* __restrict__ A
         const long gi = (long)kb * 64 + i;
         if (gi < ml)
             *reinterpret_cast<uint4*>(cols + (((size_t)s * nmb + mb) * ml + gi) * 64 + 16 * w) =
-                *reinterpret_cast<const uint4*>(&sm[s][i][4 * w]);
+                make_uint4(sm[s][i][4 * w], sm[s][i][4 * w + 1], sm[s][i][4 * w + 2], sm[s][i][4 * w + 3]);
     }
 }
 
-// V'(m, n) = V(m, n) 2^exps[m] per column n: its exponent vexp[n] and slices
+// V'(m, n) = V(m, n) 2^exps[m] per column n: its exponent e, as the product's
+// scale 2^(e - 12), and its slices
 // [s][mb][n][64], one warp per column
 __global__ void __launch_bounds__(128) k_imma_slice_v(const double* __restrict__ V, int ldv, int nb, int nmb,
-                                                      const int* __restrict__ exps, int* __restrict__ vexp,
+                                                      const int* __restrict__ exps, double* __restrict__ vscale,
                                                       int8_t* __restrict__ out, int* __restrict__ bad) {
     const int n = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (n >= nb || *bad) return;
@@ -225,7 +229,7 @@ __global__ void __launch_bounds__(128) k_imma_slice_v(const double* __restrict__
         if (lane == 0) *bad = 1;
         return;
     }
-    if (lane == 0) vexp[n] = e;
+    if (lane == 0) vscale[n] = scalbn(1.0, e - 12);
     for (int m = lane; m < nmb * 64; m += 32) {
         const double x = m < nb ? scalbn(v[m], exps[m] - e) : 0.0;
         uint32_t lo, hi;
@@ -252,7 +256,7 @@ struct ImmaArgs {
     long ldo;
     long mrows;
     int nrows;
-    const int* vexp;
+    const double* vscale;  // rotation: 2^(exponent of V's column - 12)
     const int* bad;
     int* err;
 };
@@ -432,31 +436,30 @@ __global__ void __launch_bounds__(IM_THREADS, 1) k_imma(const __grid_constant__ 
                 break;
             }
             tc_fence_after();
-            // sum_d D_d 256^-d from two exact 64-bit sums, D_0..D_3 and D_4..D_7
+            // sum_d D_d 256^-d from two exact 64-bit sums, D_0..D_3 and D_4..D_7.
+            // The MMAs of the next tile wait for these reads (the accumulators
+            // take all of TMEM), so four loads are issued per wait.
 #pragma unroll
             for (int c0 = 0; c0 < 32; c0 += 16) {
-                long long t[16];
-                uint32_t r[16];
-#pragma unroll
-                for (int d = 0; d < 4; ++d) {
-                    tmem_ld_x16(tq + (uint32_t)(d * IM_N + c0), r);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int c = 0; c < 16; ++c) t[c] = d == 0 ? (long long)(int)r[c] : t[c] * 256 + (int)r[c];
-                }
                 double v[16];
 #pragma unroll
-                for (int c = 0; c < 16; ++c) v[c] = (double)t[c] * 5.9604644775390625e-08;  // 256^-3
+                for (int d0 = 0; d0 < IM_D; d0 += 4) {
+                    uint32_t r[4][16];
 #pragma unroll
-                for (int d = 4; d < IM_D; ++d) {
-                    tmem_ld_x16(tq + (uint32_t)(d * IM_N + c0), r);
+                    for (int d = 0; d < 4; ++d) tmem_ld_x16(tq + (uint32_t)((d0 + d) * IM_N + c0), r[d]);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int c = 0; c < 16; ++c) t[c] = d == 4 ? (long long)(int)r[c] : t[c] * 256 + (int)r[c];
+                    for (int c = 0; c < 16; ++c) {
+                        const long long t = (((long long)(int)r[0][c] * 256 + (int)r[1][c]) * 256 + (int)r[2][c]) * 256 +
+                                            (int)r[3][c];
+                        if (d0 == 0)
+                            v[c] = (double)t * 5.9604644775390625e-08;  // 256^-3
+                        else
+                            v[c] = fma((double)t, 1.3877787807814457e-17, v[c]);  // 256^-7
+                    }
                 }
 #pragma unroll
                 for (int c = 0; c < 16; ++c) {
-                    v[c] = fma((double)t[c], 1.3877787807814457e-17, v[c]);  // 256^-7
                     if (GRAM)
                         acc[c0 + c] += v[c];
                     else
@@ -473,7 +476,7 @@ __global__ void __launch_bounds__(IM_THREADS, 1) k_imma(const __grid_constant__ 
                     double* o = g.out + (size_t)n0 * g.ldo + m;
 #pragma unroll
                     for (int c = 0; c < 32; ++c)
-                        if (n0 + c < g.nrows) o[(size_t)c * g.ldo] = acc[c] * scalbn(1.0, __ldg(g.vexp + n0 + c) - 12);
+                        if (n0 + c < g.nrows) o[(size_t)c * g.ldo] = acc[c] * __ldg(g.vscale + n0 + c);
                 }
             }
         }
@@ -602,10 +605,10 @@ int imma_rotate(const ImmaSlices& a, const double* V, int ldv, int* bad, double*
     Context& c = ctx();
     const int nb = a.nb, nmb = div_up(nb, 64);
     int8_t* sv = nullptr;
-    int* vexp = nullptr;
+    double* vscale = nullptr;
     RS_CHECK(workspace_t("imma_v", (size_t)IM_S * nmb * nb * 64, &sv));
-    RS_CHECK(workspace_t("imma_vexp", (size_t)nb, &vexp));
-    launch(k_imma_slice_v, div_up(nb, 4), 128, 0, c.stream, V, ldv, nb, nmb, a.exps, vexp, sv, bad);
+    RS_CHECK(workspace_t("imma_vscale", (size_t)nb, &vscale));
+    launch(k_imma_slice_v, div_up(nb, 4), 128, 0, c.stream, V, ldv, nb, nmb, a.exps, vscale, sv, bad);
     RS_LAUNCH();
     ImmaMaps maps;
     RS_CHECK(imma_map(&maps.a, a.cols, a.ml, nmb, IM_M));
@@ -619,7 +622,7 @@ int imma_rotate(const ImmaSlices& a, const double* V, int ldv, int* bad, double*
     g.ldo = ld;
     g.mrows = a.ml;
     g.nrows = nb;
-    g.vexp = vexp;
+    g.vscale = vscale;
     g.bad = bad;
     g.err = c.err_flag;
     const int sms = c.num_sms > 0 ? c.num_sms : 148;
