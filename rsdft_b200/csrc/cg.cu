@@ -21,6 +21,7 @@ namespace rsdft {
 // ----------------------------------------------------------- reductions
 __global__ void k_finish(const double* __restrict__ part, int nchunk, int K, int nb, double scale,
                          double* __restrict__ out, const int* __restrict__ active) {
+    grid_dependency();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nb * K) return;
     int b = i / K, k = i - b * K;
@@ -84,6 +85,7 @@ template <typename T, int NV, class P>
 __global__ void __launch_bounds__(VT) k_multidot(const T* v0, const T* v1, const T* v2, const T* v3, long ld,
                                                  long n, double* __restrict__ part, const int* __restrict__ active,
                                                  int vec) {
+    grid_dependency();
     constexpr int K = P::K;
     using G = Grp16<T>;
     constexpr int W = G::W;
@@ -130,6 +132,7 @@ __global__ void __launch_bounds__(VT) k_multidot(const T* v0, const T* v1, const
 template <typename T, int IT>
 __global__ void __launch_bounds__(VT) k_cg_g(CGVec<T> v, long ld, long n, const double* __restrict__ E,
                                              double* __restrict__ part, int vec) {
+    grid_dependency();
     using G = Grp16<T>;
     constexpr int W = G::W;
     __shared__ double sh[VT / 32];
@@ -167,6 +170,7 @@ __global__ void __launch_bounds__(VT) k_cg_g(CGVec<T> v, long ld, long n, const 
 template <typename T>
 __global__ void __launch_bounds__(VT) k_pc0(CGVec<T> v, long ld, long n, PcArgs pa, double* __restrict__ part,
                                             const int* __restrict__ active) {
+    grid_dependency();
     __shared__ double sh[VT / 32];
     const int b = blockIdx.y;
     if (active && !active[b]) return;
@@ -198,6 +202,7 @@ __global__ void __launch_bounds__(VT) k_pc0(CGVec<T> v, long ld, long n, PcArgs 
 template <typename T>
 __global__ void __launch_bounds__(VT) k_pc1(CGVec<T> v, long ld, long n, PcArgs pa, double* __restrict__ part,
                                             const int* __restrict__ active) {
+    grid_dependency();
     __shared__ double sh[VT / 32];
     const int b = blockIdx.y;
     if (active && !active[b]) return;
@@ -225,6 +230,7 @@ __global__ void __launch_bounds__(VT) k_pc1(CGVec<T> v, long ld, long n, PcArgs 
 template <typename T>
 __global__ void __launch_bounds__(VT) k_pc2(CGVec<T> v, long ld, long n, const double* __restrict__ pa_,
                                             int last, double* __restrict__ part, const int* __restrict__ active) {
+    grid_dependency();
     __shared__ double sh[VT / 32];
     const int b = blockIdx.y;
     if (active && !active[b]) return;
@@ -255,6 +261,7 @@ __global__ void __launch_bounds__(VT) k_pc2(CGVec<T> v, long ld, long n, const d
 template <typename T>
 __global__ void __launch_bounds__(VT) k_pc3(CGVec<T> v, long ld, long n, const double* __restrict__ pb_,
                                             const int* __restrict__ active) {
+    grid_dependency();
     const int b = blockIdx.y;
     if (active && !active[b]) return;
     const int items = vec_items(n);
@@ -271,6 +278,7 @@ __global__ void __launch_bounds__(VT) k_pc3(CGVec<T> v, long ld, long n, const d
 template <typename T>
 __global__ void __launch_bounds__(VT) k_cg_p(CGVec<T> v, long ld, long n, const double* __restrict__ bk_,
                                              int first, const int* __restrict__ active) {
+    grid_dependency();
     const int b = blockIdx.y;
     if (active && !active[b]) return;
     const int items = vec_items(n);
@@ -299,6 +307,7 @@ __device__ __forceinline__ T cg_g_elem(T g, T hp, T x, T p, T u11, T u21, T w, T
 template <typename T, bool FIRST, int IT>
 __global__ void __launch_bounds__(VT) k_cg_upd1(CGVec<T> v, long ld, long n, CGScal s, double* __restrict__ part,
                                                 const int* __restrict__ active, int vec) {
+    grid_dependency();
     using G = Grp16<T>;
     constexpr int W = G::W;
     __shared__ double sh[VT / 32];
@@ -341,6 +350,7 @@ __global__ void __launch_bounds__(VT) k_cg_upd1(CGVec<T> v, long ld, long n, CGS
 // x = u11 x + u21 p unless rejected (:366-369), for the bands with pend set
 template <typename T>
 __global__ void __launch_bounds__(VT) k_cg_upd2(CGVec<T> v, long ld, long n, CGScal s, int vec) {
+    grid_dependency();
     using G = Grp16<T>;
     constexpr int W = G::W;
     const int b = blockIdx.y;
@@ -370,6 +380,7 @@ __global__ void __launch_bounds__(VT) k_cg_upd2(CGVec<T> v, long ld, long n, CGS
 template <typename T, int IT>
 __global__ void __launch_bounds__(VT) k_cg_end(CGVec<T> v, long ld, long n, CGScal s, int apply, T* __restrict__ hx,
                                                double* __restrict__ out64, int vec) {
+    grid_dependency();
     using G = Grp16<T>;
     constexpr int W = G::W;
     const int b = blockIdx.y;
@@ -426,6 +437,7 @@ constexpr int SB = 128;  // threads of a scalar CTA: four bands
 
 // start of a sweep: E = dV <x|H x>
 __global__ void __launch_bounds__(SB) s_start(CGScal s, HpsiSum h, int nb) {
+    grid_dependency();
     const int b = blockIdx.x * (SB / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (b >= nb) return;
     const double v = hpsi_sum(h, b, lane);
@@ -448,6 +460,7 @@ __global__ void __launch_bounds__(SB) s_start(CGScal s, HpsiSum h, int nb) {
 __global__ void __launch_bounds__(SB) s_step(CGScal s, const double* __restrict__ part, int nch, double dV, int nb,
                                              int first, int last, double tol_e, double* __restrict__ esp,
                                              double* __restrict__ res) {
+    grid_dependency();
     const int b = blockIdx.x * (SB / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (b >= nb) return;
     const int act = s.active[b];
@@ -488,25 +501,29 @@ constexpr double cg_stop_tol() {
 }
 
 __global__ void s_pc0(CGScal s, int nb) {
+    grid_dependency();
     int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nb) return;
     s.pc_active[b] = s.active[b] && !(s.rr1[b] < 1e-24);
 }
 
-__global__ void s_pc1(CGScal s, int nb) {  // rr0 = rr1; a = rr0/pAp (pAp in dots[b])
+__global__ void s_pc1(CGScal s, int nb) {
+    grid_dependency();  // rr0 = rr1; a = rr0/pAp (pAp in dots[b])
     int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nb || !s.pc_active[b]) return;
     s.rr0[b] = s.rr1[b];
     s.pa[b] = s.rr0[b] / s.dots[b];
 }
 
-__global__ void s_pc2(CGScal s, int nb) {  // b = rr1/rr0
+__global__ void s_pc2(CGScal s, int nb) {
+    grid_dependency();  // b = rr1/rr0
     int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nb || !s.pc_active[b]) return;
     s.pb[b] = s.rr1[b] / s.rr0[b];
 }
 
-__global__ void s_p(CGScal s, int nb, int first) {  // bk = rb/gkgk; gkgk = rb
+__global__ void s_p(CGScal s, int nb, int first) {
+    grid_dependency();  // bk = rb/gkgk; gkgk = rb
     int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nb || !s.active[b]) return;
     s.bk[b] = first ? 0.0 : s.rb[b] / s.gkgk[b];
@@ -558,6 +575,7 @@ __device__ void eig2(double a11, double a12, double a22, double b11, double b12,
 template <typename T>
 __global__ void __launch_bounds__(SB) s_eig(CGScal s, const double* __restrict__ part, int nch, HpsiSum h, int nb,
                                             int first) {
+    grid_dependency();
     const int b = blockIdx.x * (SB / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (b >= nb || !s.active[b]) return;  // uniform per warp
     double v[5];
@@ -586,6 +604,7 @@ __global__ void __launch_bounds__(SB) s_eig(CGScal s, const double* __restrict__
 
 template <typename T>
 __global__ void k_convert(const double* __restrict__ a, T* __restrict__ b, long n) {
+    grid_dependency();
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     for (; i < n; i += (long)gridDim.x * blockDim.x) b[i] = (T)a[i];
 }
@@ -593,6 +612,7 @@ __global__ void k_convert(const double* __restrict__ a, T* __restrict__ b, long 
 // sum_i (hx - e x)^2 per band (residual norms after the eigenvalues are known)
 __global__ void __launch_bounds__(VT) k_resid(const double* __restrict__ x, const double* __restrict__ hx, long ld,
                                               long n, const double* __restrict__ e, double* __restrict__ part) {
+    grid_dependency();
     __shared__ double sh[VT / 32];
     const int b = blockIdx.y;
     const int items = vec_items(n);
@@ -612,6 +632,7 @@ __global__ void __launch_bounds__(VT) k_resid(const double* __restrict__ x, cons
 }
 
 __global__ void __launch_bounds__(SB) s_esp(HpsiSum h, int nb, double* __restrict__ e) {
+    grid_dependency();
     const int b = blockIdx.x * (SB / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (b >= nb) return;
     const double v = hpsi_sum(h, b, lane);
@@ -794,6 +815,7 @@ int cg_device_f32(const double* unk, long ld, int mb, int spin, double* esp, dou
 }
 
 __global__ void k_or_flag(int* __restrict__ dst, const int* __restrict__ src) {
+    grid_dependency();
     if (*src) *dst = 1;
 }
 

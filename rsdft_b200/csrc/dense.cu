@@ -12,8 +12,8 @@
 // solv / rotv entries cover the ScaLAPACK route on a 1x1 process grid
 // (subspace_mate_sl, subspace_solv_sl, subspace_rotv_sl).
 //
-// FP64 form: the Gram matrices and rotations on the FP64 tensor pipe
-// (dmma.cu), the overlap's Cholesky factor and its inverse by the tile-step
+// FP64 form: the Gram matrices and rotations from INT8 slices (imma.cu; small
+// blocks on the FP64 tensor pipe, dmma.cu), the overlap's Cholesky factor and its inverse by the tile-step
 // and staged-column kernels of factor.cu, the eigensolve in eigen.cu
 // (cuSOLVER DSYEVD only above its shared-memory limit).  Mixed forms: the contractions go to the split-BF16 /
 // split-TF32 tensor-core kernels of mixed.cu; FP64 stays in the Cholesky
@@ -30,12 +30,14 @@
 namespace rsdft {
 
 __global__ void k_zero_upper(double* a, int n, int lda) {
+    grid_dependency();
     int i = blockIdx.x * blockDim.x + threadIdx.x;  // row
     int j = blockIdx.y;                              // column
     if (i < n && i < j) a[(long)j * lda + i] = 0.0;
 }
 
 __global__ void k_widen(const float* __restrict__ a, double* __restrict__ b, long n) {
+    grid_dependency();
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
         b[i] = (double)a[i];
 }
@@ -43,6 +45,7 @@ __global__ void k_widen(const float* __restrict__ a, double* __restrict__ b, lon
 // C = alpha * sum_c P[c] (sym: alpha/2 (G + G^T)), fixed summation order
 __global__ void k_reduce_partials(const double* __restrict__ P, int nch, int m, int n, double alpha, int sym,
                                   double* __restrict__ C) {
+    grid_dependency();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
     if (i >= m) return;
@@ -100,6 +103,7 @@ static int fp64_gram(const Fp64Block& a, const Fp64Block& b, double alpha, int s
 
 __global__ void k_copy_cols_if(const double* __restrict__ src, long lds, double* __restrict__ dst, long ldd, long n,
                                int nb, const int* __restrict__ flag) {
+    grid_dependency();
     if (!*flag) return;
     for (int b = blockIdx.y; b < nb; b += gridDim.y)
         for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
@@ -173,6 +177,7 @@ constexpr int TI_W = 4;  // rows (warps) per CTA
 
 __global__ void __launch_bounds__(32 * TI_W) k_trtri_rows(const double* __restrict__ R, int n,
                                                          double* __restrict__ X) {
+    grid_dependency();
     extern __shared__ double ti_sm[];
     double* dinv = ti_sm;                // 1 / R(j, j)
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -314,6 +319,7 @@ static int rr_reduced(const double* Rinv, double* H, double* T, int mb, double* 
 
 // min and max of the diagonal of an n x n matrix (one block)
 __global__ void k_diag_minmax(const double* __restrict__ a, int n, int lda, double* __restrict__ out) {
+    grid_dependency();
     __shared__ double smin[256], smax[256];
     double lo = 1e300, hi = 0.0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {

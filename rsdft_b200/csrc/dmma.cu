@@ -89,6 +89,7 @@ __device__ __forceinline__ void tile_of(const DmmaArgs& g, int t, int& tm, int& 
 
 template <int BM, int BN, int WM, int WN, bool KMAJOR, bool VEC, int CPS>
 __global__ void __launch_bounds__(32 * WM * WN, CPS) k_dmma(DmmaArgs g) {
+    grid_dependency();
     constexpr int BK = DM_BK, NS = DM_NS, NT = 32 * WM * WN;
     constexpr int SA = BK + 4;
     constexpr int SB = KMAJOR ? BK + 4 : BN + 8;
@@ -237,6 +238,7 @@ template <int BT>
 __global__ void __launch_bounds__(1024) k_dmma_reduce(const double* __restrict__ P, int nsplit, int ntiles, int ntm,
                                                       int sym, int m, int n, double alpha, int symmetrize,
                                                       double* __restrict__ C, long ldc, const int* __restrict__ only_if) {
+    grid_dependency();
     __shared__ double sh[2][32][33];
     if (only_if && !*only_if) return;
     constexpr int CB = BT / 32;  // column blocks of a tile

@@ -157,6 +157,7 @@ __global__ void __launch_bounds__(TD_T, 1) k_sytrd(const double* __restrict__ A,
                                                   double* __restrict__ Q, double* __restrict__ d,
                                                   double* __restrict__ e, double* __restrict__ tau,
                                                   int* __restrict__ err) {
+    grid_dependency();
     constexpr int TD_W = TD_T / 32;
     extern __shared__ __align__(16) double sm[];
     const TdLayout<TD_C, TD_T> L(n);
@@ -418,6 +419,7 @@ constexpr int BS_PTS = 4;  // trial points per lane (independent Sturm chains)
 __global__ void __launch_bounds__(32 * BS_WARPS) k_tri_bisect(const double* __restrict__ d,
                                                              const double* __restrict__ e, int n,
                                                              double* __restrict__ w, double* __restrict__ aux) {
+    grid_dependency();
     extern __shared__ double bsh[];
     double* sd = bsh;
     double* se2 = bsh + n;
@@ -526,6 +528,7 @@ __global__ void __launch_bounds__(32 * IV_WARPS) k_tri_invit(const double* __res
                                                             const double* __restrict__ w,
                                                             const double* __restrict__ aux, int n,
                                                             double* __restrict__ Z, int ldz) {
+    grid_dependency();
     extern __shared__ double ish[];  // d, e of T for the block's warps
     double* sd = ish;
     double* se = ish + n;

@@ -56,6 +56,7 @@ constexpr int TR_G = 8;  // columns per reduction group
 
 __global__ void __launch_bounds__(32 * TR_W) k_trtri(const double* __restrict__ R, int n, int cwmax,
                                                      double* __restrict__ X) {
+    grid_dependency();
     extern __shared__ double tr_sm[];
     const int i0 = blockIdx.x * TR_W;
     const int rows = n - i0;           // pitch of a staged column: rows i0 .. n-1 at most
@@ -230,6 +231,7 @@ __device__ void chol_publish(double* sA, int n, int t, bool want_inv, double* __
 __global__ void __launch_bounds__(CH_T) k_chol_first(const double* __restrict__ S, int n, double* __restrict__ Rb,
                                                      double* __restrict__ xg, int* __restrict__ info,
                                                      int* __restrict__ fail) {
+    grid_dependency();
     __shared__ double sA[32 * CF_P];
     if (threadIdx.x == 0) {
         *info = 0;
@@ -248,6 +250,7 @@ __global__ void __launch_bounds__(CH_T) k_chol_first(const double* __restrict__ 
 __global__ void __launch_bounds__(CH_T) k_chol_step(double* __restrict__ S, int n, int k, double* __restrict__ Rb,
                                                     const double* __restrict__ xin, double* __restrict__ xout,
                                                     int* __restrict__ info, int* __restrict__ fail) {
+    grid_dependency();
     __shared__ double sX[32 * CF_P], sA[32 * CF_P], sB[32 * CF_P], sC[32 * CF_P];
     if (*(const volatile int*)fail) return;
     const int nt = (n + 31) / 32;
@@ -316,6 +319,7 @@ __global__ void __launch_bounds__(CH_T) k_chol_step(double* __restrict__ S, int 
 // left as it was
 __global__ void k_chol_copy(double* __restrict__ S, int n, const double* __restrict__ Rb,
                             const int* __restrict__ fail) {
+    grid_dependency();
     if (*fail) return;
     const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (long)n * n) return;
@@ -356,6 +360,7 @@ int potrf_upper_device(double* S, int n, int* dinfo) {
 // G(l, j).
 __global__ void __launch_bounds__(256) k_larft(const double* __restrict__ Q, int n, const double* __restrict__ tau,
                                                double* __restrict__ T) {
+    grid_dependency();
     __shared__ double sV[64 * CF_P], sG[32 * CF_P], sT[32 * CF_P];
     const int b = blockIdx.x, j0 = 32 * b;
     const int nr = min(32, n - 1 - j0), R = n - 1 - j0;
@@ -405,6 +410,7 @@ constexpr int OW = 8;  // columns of C (one per warp) per CTA of k_apply_wy
 __global__ void __launch_bounds__(32 * OW) k_apply_wy(const double* __restrict__ Q, int n,
                                                       const double* __restrict__ T, double* __restrict__ C,
                                                       int ldc) {
+    grid_dependency();
     extern __shared__ double ow_sm[];
     double* sV = ow_sm;                 // V(rr, j) at sV[j * n + rr]
     double* sT = ow_sm + (size_t)32 * n;  // the block's T (32 x 32, row-major)

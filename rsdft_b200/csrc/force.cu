@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(FW * 32) k_nl_grad(const double* __restrict__ 
                                                      const double* __restrict__ uv, const double* __restrict__ duv,
                                                      const int* __restrict__ iuv, double dV, int nzlma,
                                                      double* __restrict__ part, int* __restrict__ err) {
+    grid_dependency();
     extern __shared__ __align__(16) double fg_sm[];  // 16 x FG_CH values, FG_CH indices
     double(*s_c)[FG_CH] = reinterpret_cast<double(*)[FG_CH]>(fg_sm);
     int* s_j = reinterpret_cast<int*>(fg_sm + 16 * FG_CH);
@@ -146,6 +147,7 @@ __global__ void __launch_bounds__(FW * 32) k_nl_grad(const double* __restrict__ 
 // order; one warp per atom component (the lanes take the chunks)
 __global__ void k_atom_sum(const double* __restrict__ part, int nchunk, int nzlma, const int* __restrict__ atom_ptr,
                            const int* __restrict__ atom_lma, int natom, double* __restrict__ f) {
+    grid_dependency();
     const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (i >= natom * 3) return;
     const int a = i / 3, k = i % 3;
@@ -168,6 +170,7 @@ template <int W, bool CHI>
 __global__ void __launch_bounds__(256) k_vloc_adjoint(const double* __restrict__ psi, const double* __restrict__ chi,
                                                       long ld, int nb, const double* __restrict__ occ, double dV,
                                                       long n, double* __restrict__ out) {
+    grid_dependency();
     __shared__ int s_b[VA_LIST];
     __shared__ double s_o[VA_LIST];
     __shared__ int s_n;

@@ -48,6 +48,7 @@ __global__ void __launch_bounds__(256) k_nl_project(const T* __restrict__ psi, l
                                                     const int* __restrict__ iuv, double dV,
                                                     double* __restrict__ uvunk, int nzlma,
                                                     const int* __restrict__ band_active, int* __restrict__ err) {
+    grid_dependency();
     __shared__ int s_j[PJ_CH];
     __shared__ double s_u[4][PJ_CH];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -150,6 +151,7 @@ struct StencilArgs {
 
 template <typename T, int MD, int TX>
 __global__ void __launch_bounds__(TX * 16) k_stencil(StencilArgs<T> a, StencilCoef cf) {
+    grid_dependency();
     constexpr int TY = 16, SX = TX + 2 * MD, SY = TY + 2 * MD, NT = TX * TY;
     __shared__ T tile[SY * SX];
     const int t = threadIdx.x;
@@ -407,6 +409,7 @@ template <typename T, int MD, int BY, bool DOT>
 __global__ void __launch_bounds__(march_threads(BY), 1)
     k_stencil_tma(const __grid_constant__ TmaMaps maps, StencilArgs<T> a, const CoefT<T> cf, int TY, int RS, int S,
                   int ncw, int* __restrict__ err) {
+    grid_dependency();
     using VT = Vec16<T>;
     using V = typename VT::t;
     constexpr int VX = 16 / (int)sizeof(T);
@@ -618,6 +621,7 @@ constexpr int RS_STAGES = 3;  // planes of k_stencil_row's ring
 
 template <typename T, int MD, int BY, bool DOT>
 __global__ void __launch_bounds__(192, 2) k_stencil_row(StencilArgs<T> a, const CoefT<T> cf, int TY) {
+    grid_dependency();
     using P = Pk<T>;
     using PT = typename P::t;
     using VT = Vec16<T>;
@@ -795,6 +799,7 @@ __global__ void __launch_bounds__(128) k_nl_scatter(T* __restrict__ hpsi, long l
                                                    const T* __restrict__ gpt_uv4, const double* __restrict__ uvunk,
                                                    int nzlma, const int* __restrict__ band_active,
                                                    int* __restrict__ err) {
+    grid_dependency();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= npt) return;
     const int p = nl_pts[i];

@@ -68,6 +68,7 @@ constexpr int IM_EMAX = 400;
 // value.
 __global__ void __launch_bounds__(256) k_imma_exp(const double* __restrict__ A, long ld, long ml,
                                                   int* __restrict__ exps, int* __restrict__ bad) {
+    grid_dependency();
     const double* p = A + (long)blockIdx.y * ld;
     const long per = (ml + gridDim.x - 1) / gridDim.x;
     const long i1 = min(ml, (blockIdx.x + 1) * per);
@@ -98,6 +99,7 @@ __global__ void __launch_bounds__(256) k_imma_exp(const double* __restrict__ A, 
 // A zero vector has every digit zero whatever its exponent; a tiny one is out
 // of range.
 __global__ void k_imma_exp_check(int* __restrict__ exps, int n, int* __restrict__ bad) {
+    grid_dependency();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= n) return;
     if (exps[b] < -100000)
@@ -131,6 +133,7 @@ __device__ __forceinline__ void byte_transpose(uint32_t a, uint32_t b, uint32_t 
 __global__ void __launch_bounds__(256) k_imma_slice(const double* __restrict__ A, long ld, long ml, int nb, int nkb,
                                                     const int* __restrict__ exps, int8_t* __restrict__ rows,
                                                     int8_t* __restrict__ cols, const int* __restrict__ bad, int vec) {
+    grid_dependency();
     // pitch 17: the transposed words of a half warp (rows 4 apart) fall on 8
     // banks (at a pitch of 20, which 16-byte reads want, on 2: 872 us per
     // 72^3 x 480 block instead of 753)
@@ -208,6 +211,7 @@ __global__ void __launch_bounds__(256) k_imma_slice(const double* __restrict__ A
 __global__ void __launch_bounds__(128) k_imma_slice_v(const double* __restrict__ V, int ldv, int nb, int nmb,
                                                       const int* __restrict__ exps, double* __restrict__ vscale,
                                                       int8_t* __restrict__ out, int* __restrict__ bad) {
+    grid_dependency();
     const int n = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (n >= nb || *bad) return;
     const double* v = V + (long)n * ldv;
@@ -291,6 +295,7 @@ __host__ __device__ inline void imma_sym_tile(int t, int& tm, int& tn) {
 
 template <bool GRAM>
 __global__ void __launch_bounds__(IM_THREADS, 1) k_imma(const __grid_constant__ ImmaMaps maps, ImmaArgs g) {
+    grid_dependency();
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)IM_NS * IM_STAGE);
     uint64_t* empty = full + IM_NS;
@@ -503,6 +508,7 @@ __global__ void __launch_bounds__(256) k_imma_reduce(const double* __restrict__ 
                                                      const int* __restrict__ ea, const int* __restrict__ eb,
                                                      double alpha, int symmetrize, const int* __restrict__ bad,
                                                      double* __restrict__ C, long ldc) {
+    grid_dependency();
     if (*bad) return;
     const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
     if (i >= nb || j >= nb) return;

@@ -101,8 +101,8 @@ inline double march_cost(long nwork, int nz, int extra, int zmax, long conc, dou
 }
 
 // Symmetric-positive-definite orthonormalisation (CholeskyQR2 in the dV
-// metric) of nb columns, FP64 (DMMA Gram and rotation, the Cholesky factor
-// and its inverse by factor.cu) or mixed (tcgen05 tensor cores).
+// metric) of nb columns, FP64 (INT8-slice or DMMA Gram and rotation, the
+// Cholesky factor and its inverse by factor.cu) or mixed (split BF16 / TF32).
 int gram_schmidt_device(double* psi, long ld, int nb, int mode);
 
 // Rayleigh-Ritz (subspace_diag_la) on device data.

@@ -74,6 +74,7 @@ __device__ __forceinline__ void split_tf32(double x, uint32_t& h, uint32_t& l) {
 template <typename TI>
 __global__ void __launch_bounds__(256) k_split_cols_tf32(const TI* __restrict__ psi, long ld, int nb, long ml,
                                                          uint32_t* __restrict__ out) {
+    grid_dependency();
     const long n = ml * nb;
     const int b = blockIdx.y;
     const long k0 = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
@@ -91,6 +92,7 @@ __global__ void __launch_bounds__(256) k_split_cols_tf32(const TI* __restrict__ 
 template <typename TI>
 __global__ void k_split_rows_tf32(const TI* __restrict__ psi, long ld, int nb, long ml, int mbk,
                                   uint32_t* __restrict__ out) {
+    grid_dependency();
     __shared__ double tile[32][33];
     const long i0 = (long)blockIdx.x * 32;
     const int m0 = blockIdx.y * 32;
@@ -116,6 +118,7 @@ __global__ void k_split_rows_tf32(const TI* __restrict__ psi, long ld, int nb, l
 }
 
 __global__ void k_split_small_tf32(const double* __restrict__ V, int mb, int ldv, int mbk, uint32_t* __restrict__ out) {
+    grid_dependency();
     const long n = (long)mb * mbk;
     for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
         const int col = (int)(e / mbk), m = (int)(e - (long)col * mbk);
@@ -141,6 +144,7 @@ constexpr int SPC_B = 8;   // bands per warp
 template <typename TI>
 __global__ void __launch_bounds__(32 * SPC_KB) k_split_cols(const TI* __restrict__ psi, long ld, int nb, long ml,
                                                            int nkb, __nv_bfloat16* __restrict__ out, int vec) {
+    grid_dependency();
     const int lane = threadIdx.x & 31;
     const int kb = blockIdx.x * SPC_KB + (threadIdx.x >> 5);
     const int b = blockIdx.y * SPC_B + (lane >> 2);
@@ -169,6 +173,7 @@ __global__ void __launch_bounds__(32 * SPC_KB) k_split_cols(const TI* __restrict
 
 // slices[s][n][m] = term s of V(m, n) (V column-major mb x mb), padded to mbk
 __global__ void k_split_small(const double* __restrict__ V, int mb, int ldv, int mbk, __nv_bfloat16* __restrict__ out) {
+    grid_dependency();
     const long n = (long)mb * mbk;
     for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
         const int col = (int)(e / mbk), m = (int)(e - (long)col * mbk);
@@ -215,6 +220,7 @@ __device__ __forceinline__ void pair_tiles(const UmmaArgs& g, int pair, int& tm,
 
 template <int BN, int NT, int NS, bool DRAIN, bool BMN, bool TF = false>
 __global__ void __launch_bounds__(U_THREADS, 1) k_umma(const __grid_constant__ UmmaMaps maps, UmmaArgs g) {
+    grid_dependency();
     static_assert(!(TF && BMN), "TF32 operands are K-major");
     constexpr int ABYTES = UB_M * UB_KB;  // one A slice tile
     constexpr int BBYTES = BN * UB_KB;
@@ -469,6 +475,7 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_umma(const __grid_constant__ U
 // symmetric product are read transposed from tile (tn, tm)
 __global__ void k_reduce_tiles(const double* __restrict__ P, int nsplit, int npairs, int ntm, int sym, int bn, int m,
                                double alpha, int symmetrize, double* __restrict__ C) {
+    grid_dependency();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
     if (i >= m) return;

@@ -20,6 +20,7 @@ namespace rsdft {
 template <typename T, int K, int D>
 __global__ void __launch_bounds__(VT) k_ss_basis(const T* __restrict__ g, SSVec<T> sv, long ld, long n, PcArgs pa,
                                                  double* __restrict__ part, const int* __restrict__ active) {
+    grid_dependency();
     constexpr bool STORE = D > 1;
     __shared__ double sh[D * (VT / 32)];
     const int b = blockIdx.y;
@@ -89,6 +90,7 @@ __global__ void __launch_bounds__(VT) k_ss_basis(const T* __restrict__ g, SSVec<
 template <int m>
 __global__ void __launch_bounds__(128) s_sstep(CGScal s, SSPart pt, double* __restrict__ cz_out, int nb, double d,
                                                double dV, int first) {
+    grid_dependency();
     const int b = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (b >= nb || !s.active[b]) return;  // uniform per warp
     double S[m + 1][3];
@@ -190,6 +192,7 @@ __global__ void __launch_bounds__(VT) k_ss_p(const T* __restrict__ g, const T* _
                                              const int* __restrict__ active, const int* __restrict__ pend,
                                              const double* __restrict__ u11_, const double* __restrict__ u21_,
                                              double* __restrict__ part, int vec) {
+    grid_dependency();
     using G = Grp16<T>;
     constexpr int W = G::W;
     __shared__ double sh[5 * (VT / 32)];
@@ -332,6 +335,7 @@ __global__ void __launch_bounds__(384, PcStep<K, D>::CTAS) k_pc_tma(const __grid
                                                    int nzc, int TY, int RS, int S, int ncw,
                                                    double* __restrict__ part, const int* __restrict__ active,
                                                    int* __restrict__ err) {
+    grid_dependency();
     using VT = Vec16<T>;
     using V = typename VT::t;
     constexpr int VX = 16 / (int)sizeof(T);

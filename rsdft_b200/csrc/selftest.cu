@@ -14,6 +14,7 @@
 namespace rsdft {
 
 __global__ void k_wait_for_nothing(long long cycles, int* __restrict__ err) {
+    grid_dependency();
     __shared__ uint64_t bar;
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
@@ -33,6 +34,7 @@ __global__ void k_wait_for_nothing(long long cycles, int* __restrict__ err) {
 // out of range, so the check records itself and the read is skipped.
 __global__ void k_check_probe(const double* __restrict__ buf, int n, int i, double* __restrict__ out,
                               int* __restrict__ err) {
+    grid_dependency();
     double v = 0.0;
     if (RS_DCHECK(i >= 0 && i < n, CK_SELFTEST, i, err)) v = buf[i];
     out[0] = v;

@@ -122,6 +122,7 @@ __device__ double fermi_bisect(const double* esp, double* occ, int mb, int s0, i
 __global__ void __launch_bounds__(FM_T) k_calc_fermi(const double* __restrict__ esp, double* __restrict__ occ, int mb,
                                                      int msp, double znel, double dspn, int fixed, double ekbt,
                                                      int kinteg, double* __restrict__ out) {
+    grid_dependency();
     __shared__ double sh[FM_T / 32 + 1];
     int ok = 1;
     double ef;
@@ -146,6 +147,7 @@ __global__ void __launch_bounds__(FM_T) k_calc_fermi(const double* __restrict__ 
 __global__ void __launch_bounds__(FM_T) k_conv_check(const double* __restrict__ esp, const double* __restrict__ esp0,
                                                      double* __restrict__ res, int mb, int msp, int mb_ref, int mode,
                                                      double tol, double* __restrict__ out) {
+    grid_dependency();
     __shared__ double sh[FM_T / 32 + 1];
     double m = 0.0;
     for (int i = threadIdx.x; i < msp * mb; i += FM_T) {
