@@ -320,7 +320,10 @@ struct PcMaps {
 template <int K, int D>
 struct PcStep {
     static constexpr int NA = (D > 1 && K >= 2) ? 1 : 0;  // w_{K-2}
-    static constexpr int CTAS = 2;  // CTAs per SM (<= 85 registers, half the stage ring each)
+    // CTAs per SM: two (<= 85 registers, half the stage ring each); one with three
+    // dots, which spill at 80 registers (48^3 x 160 FP64 103 us a pass with two,
+    // 88 with one; 72^3 x 480 695 and 643)
+    static constexpr int CTAS = D == 3 ? 1 : 2;
 };
 
 __device__ __forceinline__ int pc_pwrap(int i, int n) {
@@ -706,7 +709,7 @@ int sstep_precond(const T* g, const T* hx, const SSVec<T>& sv, T* p, T* x, long 
     // smooth residual are nearly parallel, and the recurrence holds for the
     // stored vectors to their rounding, whose effect on a dot falls as
     // 1 / sqrt(n).  Residuals against 64 bits, FP64 48^3: 6.1e-14 by the
-    // recurrence, 3.8e-14 by the dot (85 | 103 us a pass at 160 bands); FP32,
+    // recurrence, 3.8e-14 by the dot (85 | 88 us a pass at 160 bands); FP32,
     // 72^3: 1.7e-6 either way (332 | 416 us at 480 bands).
     const bool third = sizeof(T) == 8 || n <= 65536;
     SSPart pt{};
