@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(VT) k_multidot(const T* v0, const T* v1, const
 
 // g = -c1 (hx - E x); partial |g|^2 (cg_module.f90:186-190)
 template <typename T, int IT>
-__global__ void __launch_bounds__(VT) k_cg_g(CGVec<T> v, long ld, long n, const double* __restrict__ E,
+__global__ void __launch_bounds__(VT) k_cg_g(CGVec<T> v, long ld, long n, const double* E,
                                              double* __restrict__ part, int vec) {
     grid_dependency();
     using G = Grp16<T>;
@@ -306,7 +306,7 @@ __device__ __forceinline__ T cg_g_elem(T g, T hp, T x, T p, T u11, T u21, T w, T
 
 template <typename T, bool FIRST, int IT>
 __global__ void __launch_bounds__(VT) k_cg_upd1(CGVec<T> v, long ld, long n, CGScal s, double* __restrict__ part,
-                                                const int* __restrict__ active, int vec) {
+                                                const int* active, int vec) {
     grid_dependency();
     using G = Grp16<T>;
     constexpr int W = G::W;
@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(SB) s_start(CGScal s, HpsiSum h, int nb) {
 // moved by less than tol_e in the last line step (the reference's 1e-15,
 // cg_module.f90:218, in FP64); a rejected one stops here too, its quotient
 // being put back.
-__global__ void __launch_bounds__(SB) s_step(CGScal s, const double* __restrict__ part, int nch, double dV, int nb,
+__global__ void __launch_bounds__(SB) s_step(CGScal s, const double* part, int nch, double dV, int nb,
                                              int first, int last, double tol_e, double* __restrict__ esp,
                                              double* __restrict__ res) {
     grid_dependency();
@@ -573,7 +573,7 @@ __device__ void eig2(double a11, double a12, double a22, double b11, double b12,
 // five dots of the search-direction pass (the last two with g, or with H x in
 // the first step) and <p|H p>.  g was formed with the quotient rounded to T.
 template <typename T>
-__global__ void __launch_bounds__(SB) s_eig(CGScal s, const double* __restrict__ part, int nch, HpsiSum h, int nb,
+__global__ void __launch_bounds__(SB) s_eig(CGScal s, const double* part, int nch, HpsiSum h, int nb,
                                             int first) {
     grid_dependency();
     const int b = blockIdx.x * (SB / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -654,7 +654,7 @@ int esp_device(const double* x, long ld, int nb, int spin, double* e, double* re
     RS_CHECK(workspace_t("esp_dot", (size_t)nb * dot.cap, &dot.part));
     RS_CHECK(hpsi_device<double>(x, hx, ld, nb, spin, nullptr, &dot));
     const dim3 vg(nchunk, nb);
-    launch(s_esp, div_up(nb, SB / 32), SB, 0, st, hpsi_sum_of(dot), nb, e);
+    launch_dependent(s_esp, div_up(nb, SB / 32), SB, 0, st, hpsi_sum_of(dot), nb, e);
     if (res) {
         launch(k_resid, vg, VT, 0, st, x, hx, ld, n, e, part);
         launch(k_finish, div_up(nb, 128), 128, 0, st, part, nchunk, 1, nb, c.dV, res, nullptr);
@@ -724,9 +724,9 @@ static int cg_run(T* x, long ld, int mb, int spin, double* esp, double* res, int
     };
 
     RS_CHECK(hpsi_device<T>(x, v.hx, ld, mb, spin, nullptr, &hd));
-    launch(s_start, wb, SB, 0, st, s, hpsi_sum_of(hd), mb);
-    launch(full ? k_cg_g<T, 32> : k_cg_g<T, 0>, vg, VT, 0, st, v, ld, n, s.E, part, gv);
-    launch(s_step, wb, SB, 0, st, s, (const double*)part, nchunk, dV, mb, 1, ncg == 0, tol, esp, res);
+    launch_dependent(s_start, wb, SB, 0, st, s, hpsi_sum_of(hd), mb);
+    launch_dependent(full ? k_cg_g<T, 32> : k_cg_g<T, 0>, vg, VT, 0, st, v, ld, n, s.E, part, gv);
+    launch_dependent(s_step, wb, SB, 0, st, s, (const double*)part, nchunk, dV, mb, 1, ncg == 0, tol, esp, res);
     RS_LAUNCH();
 
     const bool sstep = ipc == 4 && mloop >= 1 && mloop <= SS_MAXM;
@@ -769,17 +769,17 @@ static int cg_run(T* x, long ld, int mb, int spin, double* esp, double* res, int
             RS_LAUNCH();
         }
         RS_CHECK(hpsi_device<T>(v.p, v.hp, ld, mb, spin, s.active, &hd));
-        launch(s_eig<T>, wb, SB, 0, st, s, (const double*)pdots, nchunk, hpsi_sum_of(hd), mb, icg == 1);
-        launch(icg == 1 ? (full ? k_cg_upd1<T, true, 32> : k_cg_upd1<T, true, 0>)
+        launch_dependent(s_eig<T>, wb, SB, 0, st, s, (const double*)pdots, nchunk, hpsi_sum_of(hd), mb, icg == 1);
+        launch_dependent(icg == 1 ? (full ? k_cg_upd1<T, true, 32> : k_cg_upd1<T, true, 0>)
                         : (full ? k_cg_upd1<T, false, 32> : k_cg_upd1<T, false, 0>),
                vg, VT, 0, st, v, ld, n, s, part, s.active, gv);
-        launch(s_step, wb, SB, 0, st, s, (const double*)part, nchunk, dV, mb, 0, icg == ncg, tol, esp, res);
+        launch_dependent(s_step, wb, SB, 0, st, s, (const double*)part, nchunk, dV, mb, 0, icg == ncg, tol, esp, res);
         if (!sstep) launch(k_cg_upd2<T>, vg, VT, 0, st, v, ld, n, s, gv);
         RS_LAUNCH();
     }
     T* hx = hx_out && ncg > 0 ? v.hx : nullptr;
     if (hx_out) *hx_out = v.hx;
-    launch(full ? k_cg_end<T, 32> : k_cg_end<T, 0>, vg, VT, 0, st, v, ld, n, s, sstep ? 1 : 0, hx, out64, gv);
+    launch_dependent(full ? k_cg_end<T, 32> : k_cg_end<T, 0>, vg, VT, 0, st, v, ld, n, s, sstep ? 1 : 0, hx, out64, gv);
     RS_LAUNCH();
     return RSDFT_OK;
 }

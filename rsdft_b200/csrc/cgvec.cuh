@@ -86,7 +86,7 @@ struct CGVec {
 
 // Fixed-order sum by one warp of n values p[0], p[stride], ...: lane l takes
 // l, l + 32, ..., then a shuffle tree; the result is valid in every lane.
-__device__ __forceinline__ double warp_strided_sum(const double* __restrict__ p, int n, int stride, int lane) {
+__device__ __forceinline__ double warp_strided_sum(const double* p, int n, int stride, int lane) {
     double v = 0.0;
     for (int c = lane; c < n; c += 32) v += p[(long)c * stride];
 #pragma unroll

@@ -193,22 +193,25 @@ __device__ __forceinline__ bool dev_check(bool ok, int site, long idx, int* err)
 // Number of this library's kernel launches since load (diagnostics).
 extern long long g_kernel_launches;
 
-// The first statement of every kernel.  A small launch is a programmatic
-// dependent of the kernel before it (launch below): its CTAs may be set up as
-// soon as those of that kernel have all started, and wait here until everything
-// it wrote is visible, so the kernels still run one after the other and only the
-// launch latency overlaps (24^3 x 32 iteration, about 90 launches: 733 us
-// without and 685 us with).  Large launches are ordinary ones: their
-// waiting CTAs would crowd the SMs that drain first (72^3 x 480 CG sweep with
-// every launch a dependent: 19.8 ms against 18.6).
+// The first statement of every kernel: wait until everything the kernel before
+// it wrote is visible, then let the next one be set up.  An ordinary launch
+// does not overlap its predecessor at all and the wait is over at once.
+//
+// A dependent launch (launch_dependent) is set up while the kernel before it
+// runs, so its lifetime overlaps that one kernel's, and no other's, since the
+// kernel before lets it in only after its own wait.  What the kernel before
+// writes is thus not read-only for the dependent's lifetime: it must not read
+// that through the non-coherent path (const __restrict__ parameters, __ldg),
+// which neither the wait nor its memory clobber orders.  Struct members and
+// plain pointers are read coherently; TMA loads come after the wait.
 __device__ __forceinline__ void grid_dependency() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// Launch one of this library's kernels and count it (errors: RS_LAUNCH).
 template <typename... KArgs, typename... Args>
-inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+inline void launch_as(bool dependent, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                      Args&&... args) {
     ++g_kernel_launches;
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[1];
@@ -220,13 +223,33 @@ inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 0;
-    if ((long)grid.x * grid.y * grid.z <= 512) {
+    if (dependent && (long)grid.x * grid.y * grid.z <= 512) {
         // a captured launch stays an ordinary one: programmatic edges make a
         // graph that not every caller's query of the capture can describe
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) cfg.numAttrs = 1;
     }
     (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+// Launch one of this library's kernels and count it (errors: RS_LAUNCH).
+template <typename... KArgs, typename... Args>
+inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+    launch_as(false, kernel, grid, block, smem, st, std::forward<Args>(args)...);
+}
+
+// The same as a programmatic dependent of the launch before it, for kernels
+// that read what that one writes coherently (above), in chains of short
+// kernels, where the launch latency is what there is to save.  Above 512 CTAs
+// an ordinary launch: the waiting CTAs would crowd the SMs that drain first
+// (72^3 x 480 CG sweep with every launch a dependent: 19.8 ms against 18.6).  Not
+// behind long kernels of few CTAs either, whose L1 a waiting CTA's shared memory
+// takes away: 128^3 x 1 band in a cell of 8 wide spheres, the H psi stencil
+// waiting for the projection, 688 us against 569.
+template <typename... KArgs, typename... Args>
+inline void launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                             Args&&... args) {
+    launch_as(true, kernel, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
 int require_init();

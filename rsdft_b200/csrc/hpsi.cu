@@ -789,11 +789,12 @@ __global__ void __launch_bounds__(192, 2) k_stencil_row(StencilArgs<T> a, const 
 // (ps_nloc2_op_module.f90:255-263), one thread per covered point and a chunk
 // of bands, SC_BU bands in flight at once (2: measured faster than 4 and 8).
 // A point's entries are taken in projector order, so every sum has a fixed
-// order.
+// order.  Launched as a dependent of the stencil, whose H psi it reads through a
+// plain pointer; uVunk is the projection's, complete before the stencil began.
 constexpr int SC_BU = 2;
 
 template <typename T>
-__global__ void __launch_bounds__(128) k_nl_scatter(T* __restrict__ hpsi, long ld, int nb, int bchunk,
+__global__ void __launch_bounds__(128) k_nl_scatter(T* hpsi, long ld, int nb, int bchunk,
                                                    const int* __restrict__ nl_pts, const int* __restrict__ nl_ptr,
                                                    int npt, const int* __restrict__ gpt_grp,
                                                    const T* __restrict__ gpt_uv4, const double* __restrict__ uvunk,
@@ -850,6 +851,17 @@ static int scatter_chunk(int nb) {
     int bch = 32;
     while (bch > SC_BU && (long)div_up(c.nl_npt, 128) * div_up(nb, bch) < 8 * sms) bch /= 2;
     return bch;
+}
+
+// Whether the stencil is launched as a dependent of the projection (of which
+// it reads nothing): where the spheres are of ordinary size, so that the
+// projection is short.  Behind a long one the waiting stencil CTAs' shared memory
+// costs it its L1 (launch_dependent).  24^3 x 32, about 500 points per sphere:
+// 24.6 us without; 256^3 x 1 band in an 8-atom cell, 57,000 points: 6070 us
+// without, 6580 with.
+static bool stencil_dependent() {
+    const Context& c = ctx();
+    return c.nl_set && c.nnz <= 1024L * c.nzlma;
 }
 
 template <typename T, int MD, int TX>
@@ -931,8 +943,8 @@ static int launch_tma_dot(const TmaMaps& maps, const StencilArgs<T>& a, const St
                           const TmaGeom& g, cudaStream_t st) {
     RS_CHECK(set_smem_optin((const void*)k_stencil_tma<T, MD, BY, DOT>, 220 * 1024 + 8 * 16 + 12 * 8));
     dim3 grid(a.n2 / g.TY, (unsigned)(nb * a.nzc));
-    launch(k_stencil_tma<T, MD, BY, DOT>, grid, g.threads, g.smem, st, maps, a, coef_as<T>(cf), g.TY, g.RS, g.S, g.ncw,
-           ctx().err_flag);
+    launch_as(stencil_dependent(), k_stencil_tma<T, MD, BY, DOT>, grid, g.threads, g.smem, st, maps, a, coef_as<T>(cf),
+              g.TY, g.RS, g.S, g.ncw, ctx().err_flag);
     RS_LAUNCH();
     return RSDFT_OK;
 }
@@ -1026,7 +1038,7 @@ static int launch_row(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStrea
         dot->with_nl = false;
         a.dot = dot->part;
     }
-    launch(kern, dim3(tiles, (unsigned)(nb * a.nzc)), threads, smem, st, a, coef_as<T>(cf), TY);
+    launch_as(stencil_dependent(), kern, dim3(tiles, (unsigned)(nb * a.nzc)), threads, smem, st, a, coef_as<T>(cf), TY);
     RS_LAUNCH();
     *used = true;
     return RSDFT_OK;
@@ -1059,7 +1071,7 @@ static int launch_stencil_md2(StencilArgs<T> a, const StencilCoef& cf, int nb, c
         if (a.gpt_ptr && c.nl_npt > 0) {
             const int bch = scatter_chunk(nb);
             dim3 grid(div_up(c.nl_npt, 128), div_up(nb, bch));
-            launch(k_nl_scatter<T>, grid, 128, 0, st, a.hpsi, a.ld, nb, bch, (const int*)c.nl_pts,
+            launch_dependent(k_nl_scatter<T>, grid, 128, 0, st, a.hpsi, a.ld, nb, bch, (const int*)c.nl_pts,
                    (const int*)c.nl_ptr, c.nl_npt, a.gpt_grp, a.gpt_uv4, a.uvunk, a.nzlma, a.band_active,
                    c.err_flag);
             RS_LAUNCH();

@@ -187,10 +187,10 @@ __global__ void __launch_bounds__(128) s_sstep(CGScal s, SSPart pt, double* __re
 // the residuals of a band of norm 27, against 1e-15 this way).
 template <typename T, int M, int IT>
 __global__ void __launch_bounds__(VT) k_ss_p(const T* __restrict__ g, const T* __restrict__ hx, SSVec<T> sv,
-                                             T* __restrict__ p, T* __restrict__ x, long ld, long n, const double* __restrict__ cz,
-                                             const double* __restrict__ bk_,
-                                             const int* __restrict__ active, const int* __restrict__ pend,
-                                             const double* __restrict__ u11_, const double* __restrict__ u21_,
+                                             T* __restrict__ p, T* __restrict__ x, long ld, long n, const double* cz,
+                                             const double* bk_,
+                                             const int* active, const int* pend,
+                                             const double* u11_, const double* u21_,
                                              double* __restrict__ part, int vec) {
     grid_dependency();
     using G = Grp16<T>;
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(384, PcStep<K, D>::CTAS) k_pc_tma(const __grid
                                                                       T* __restrict__ wout,
                                                    StencilCoef cf, int n1, int n2, int n3, long ld, int zlen0,
                                                    int nzc, int TY, int RS, int S, int ncw,
-                                                   double* __restrict__ part, const int* __restrict__ active,
+                                                   double* __restrict__ part, const int* active,
                                                    int* __restrict__ err) {
     grid_dependency();
     using VT = Vec16<T>;
@@ -664,7 +664,7 @@ static int pc_tma_step(const T* src, const T* const* aux, T* wout, const PcArgs&
     cf.cy[0] = sc * pa.c2;
     cf.cz[0] = sc * pa.c3;
     dim3 grid(n2 / g.TY, (unsigned)(mb * nzc));
-    launch(k_pc_tma<T, K, D>, grid, g.threads, g.smem, c.stream, maps, wout, cf, n1, n2, n3, ld, zlen, nzc,
+    launch_dependent(k_pc_tma<T, K, D>, grid, g.threads, g.smem, c.stream, maps, wout, cf, n1, n2, n3, ld, zlen, nzc,
            g.TY, g.RS, g.S, g.ncw, part, active, c.err_flag);
     RS_LAUNCH();
     *nchunk = (n2 / g.TY) * nzc;
@@ -731,8 +731,8 @@ int sstep_precond(const T* g, const T* hx, const SSVec<T>& sv, T* p, T* x, long 
     const int gv = grp16_ok<T>(ld, {g, hx, p, x, sv.w[0], sv.w[1], sv.w[2], sv.w[3]}) ? 1 : 0;
     auto launch_p = [&](auto M) {
         constexpr int MM = decltype(M)::value;
-        launch(s_sstep<MM>, div_up(mb, 4), 128, 0, st, s, pt, cz, mb, pa.d, dV, hx ? 1 : 0);
-        launch(vec_full(n, nchunk) ? k_ss_p<T, MM, 32> : k_ss_p<T, MM, 0>, vg, VT, 0, st, g, hx, sv, p, x, ld, n, (const double*)cz,
+        launch_dependent(s_sstep<MM>, div_up(mb, 4), 128, 0, st, s, pt, cz, mb, pa.d, dV, hx ? 1 : 0);
+        launch_dependent(vec_full(n, nchunk) ? k_ss_p<T, MM, 32> : k_ss_p<T, MM, 0>, vg, VT, 0, st, g, hx, sv, p, x, ld, n, (const double*)cz,
                (const double*)s.bk, (const int*)s.active, (const int*)(hx ? nullptr : s.pend),
                (const double*)s.u11, (const double*)s.u21, dots, gv);
     };
