@@ -12,6 +12,7 @@
 //  fed by cp.async; what neither takes runs k_stencil, a register-queue kernel
 //  with per-plane halo loads and the scatter fused in its epilogue.
 #include <algorithm>
+#include <cmath>
 
 #include "common.cuh"
 #include "kernels.cuh"
@@ -240,6 +241,7 @@ struct TmaMaps {
 template <typename T>
 struct CoefT {
     T c0;
+    T c0x, c0yz;  // c0 = c0x + c0yz exactly: x's own share of it, rounded to half the digits
     T cx[MAXMD], cy[MAXMD], cz[MAXMD];
 };
 
@@ -252,6 +254,13 @@ static CoefT<T> coef_as(const StencilCoef& cf) {
         o.cy[m] = (T)cf.cy[m];
         o.cz[m] = (T)cf.cz[m];
     }
+    double share = 0.0;
+    for (int m = 0; m < MAXMD; ++m) share -= 2.0 * cf.cx[m];
+    int e = 0;
+    const double f = std::frexp(share, &e);
+    constexpr int half = sizeof(T) == 8 ? 24 : 11;
+    o.c0x = (T)std::ldexp(std::rint(std::ldexp(f, half)), e - half);
+    o.c0yz = o.c0 - o.c0x;
     return o;
 }
 
@@ -611,12 +620,20 @@ __global__ void __launch_bounds__(march_threads(BY), 1)
 // plane, into 16-byte aligned rows with the periodic x neighbours beside them,
 // so every window load is a vector at a constant offset; y and z wrap where the
 // rows are fetched, any n2 and n3.  The last vector of a row may stand half
-// outside the grid; what lies there is computed and not stored.  Bound, as the
-// TMA kernel's, by the shared-memory window loads and, with 10 to 12 warps per
-// SM, their latency.  H psi at 45^3 x 101 FP64: 394 us with k_stencil (16 x 32
-// tiles re-reading their halo every plane, a quarter of the tiles' points outside
-// the grid), 245 us with a thread on one x column (8-byte loads, 17 per point
-// against 7 here of 16 bytes), 216 us this way.
+// outside the grid; what lies there is computed and not stored.
+//
+// Order of the sum: symmetric pairs from the outermost inwards, x with its own
+// share of the centre weight and Vloc, y with the rest of it, so that the large
+// terms cancel before the sums meet.  Relative error of H psi against 80 bits,
+// smooth bands at 45^3, Md = 6: 7.7e-16 with k_stencil (pairs, the innermost
+// first), 6.6e-16 this way, 1.5e-15 with the y rows one by one and c0 + Vloc as one
+// factor.
+//
+// Bound, as the TMA kernel's, by the shared-memory window loads and, with 10 to
+// 12 warps per SM, their latency.  H psi at 45^3 x 101 FP64: 394 us with
+// k_stencil (16 x 32 tiles re-reading their halo every plane, a quarter of the
+// tiles' points outside the grid), 245 us with a thread on one x column (8-byte
+// loads, 17 per point against 7 here of 16 bytes), 220 us this way.
 constexpr int RS_STAGES = 3;  // planes of k_stencil_row's ring
 
 template <typename T, int MD, int BY, bool DOT>
@@ -717,28 +734,25 @@ __global__ void __launch_bounds__(192, 2) k_stencil_row(StencilArgs<T> a, const 
 #pragma unroll
         for (int r = 0; r < BY; ++r) P::get2(*reinterpret_cast<const V*>(sp + r * PX), c + 2 * r);
         if (inner) {
+            // y pairs (row r - m + row r + m), each row loaded where the order
+            // first meets it
+            PT v[BY + 2 * MD][2];
+            auto row = [&](int j, bool first, int e) -> PT {
+                if (j >= 0 && j < BY) return c[2 * (j >= 0 && j < BY ? j : 0) + e];
+                if (first && e == 0) P::get2(*reinterpret_cast<const V*>(sp + j * PX), v[j + MD]);
+                return v[j + MD][e];
+            };
 #pragma unroll
             for (int i = 0; i < NK; ++i) in[i] = P::splat((T)0);
 #pragma unroll
-            for (int jj = 0; jj < BY + 2 * MD; ++jj) {
-                const int j = term_order<T>(jj, BY + 2 * MD) - MD;
-                PT v[2];
-                if (j < 0 || j >= BY) {
-                    P::get2(*reinterpret_cast<const V*>(sp + j * PX), v);
-                } else {
-                    v[0] = c[2 * (j < 0 || j >= BY ? 0 : j)];
-                    v[1] = c[2 * (j < 0 || j >= BY ? 0 : j) + 1];
-                }
+            for (int m = MD; m >= 1; --m)
 #pragma unroll
-                for (int r = 0; r < BY; ++r) {
-                    const int m = j > r ? j - r : r - j;
-                    if (m >= 1 && m <= MD) {
+                for (int r = 0; r < BY; ++r)
 #pragma unroll
-                        for (int e = 0; e < 2; ++e)
-                            in[2 * r + e] = P::fma(P::splat(cf.cy[m - 1]), v[e], in[2 * r + e]);
+                    for (int e = 0; e < 2; ++e) {
+                        const PT lo = row(r - m, r == BY - 1 || m == MD, e), hi = row(r + m, r == 0 || m == MD, e);
+                        in[2 * r + e] = P::fma(P::splat(cf.cy[m - 1]), P::add(lo, hi), in[2 * r + e]);
                     }
-                }
-            }
 #pragma unroll
             for (int r = 0; r < BY; ++r) {
                 T w[NV * VX];
@@ -749,20 +763,18 @@ __global__ void __launch_bounds__(192, 2) k_stencil_row(StencilArgs<T> a, const 
                     else
                         VT::get(*reinterpret_cast<const V*>(sp + r * PX - HX + VX * j), w + j * VX);
                 }
-#pragma unroll
-                for (int e = 0; e < 2; ++e)
-#pragma unroll
-                    for (int i = 1; i <= MD; ++i) {
-                        const int m = sizeof(T) == 8 ? i : MD + 1 - i;
-                        in[2 * r + e] = P::fma(P::splat(cf.cx[m - 1]),
-                                               P::add(P::of(w + HX + W * e - m), P::of(w + HX + W * e + m)),
-                                               in[2 * r + e]);
-                    }
                 PT vl[2];
                 P::get2(*reinterpret_cast<const V*>(sp + (ROWS - MD + r) * PX), vl);
 #pragma unroll
-                for (int e = 0; e < 2; ++e)
-                    in[2 * r + e] = P::fma(P::add(P::splat(cf.c0), vl[e]), c[2 * r + e], in[2 * r + e]);
+                for (int e = 0; e < 2; ++e) {
+                    PT ix = P::splat((T)0);
+#pragma unroll
+                    for (int m = MD; m >= 1; --m)
+                        ix = P::fma(P::splat(cf.cx[m - 1]), P::add(P::of(w + HX + W * e - m), P::of(w + HX + W * e + m)),
+                                    ix);
+                    ix = P::fma(vl[e], c[2 * r + e], P::fma(P::splat(cf.c0x), c[2 * r + e], ix));
+                    in[2 * r + e] = P::add(ix, P::fma(P::splat(cf.c0yz), c[2 * r + e], in[2 * r + e]));
+                }
             }
         }
         T* hp = (k >= 2 * MD && nrow > 0) ? hb + plane * (zs + k - 2 * MD) : nullptr;

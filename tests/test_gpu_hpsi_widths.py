@@ -52,3 +52,42 @@ def test_fp32_widths(gpu, n, nb):
     assert np.abs(u.cpu().numpy() - ru).max() <= 2e-5 * np.abs(ru).max()
     assert np.abs(esp.cpu().numpy() - resp).max() <= 2e-4 * np.abs(resp).max()
     assert np.abs(res.cpu().numpy() - rres).max() <= 2e-4 * np.abs(rres).max()
+
+
+def smooth_bands(n, nb, a, seed):
+    """Rows of Gaussian noise damped above 1 Ha, as bands are after the first iterations."""
+    rng = np.random.default_rng(seed)
+    k = 2.0 * np.pi * np.fft.fftfreq(n, 1.0 / n) / a
+    e = 0.5 * (k[:, None, None] ** 2 + k[None, :, None] ** 2 + k[None, None, :] ** 2)
+    noise = np.fft.fftn(rng.normal(size=(nb, n, n, n)), axes=(1, 2, 3))
+    return np.fft.ifftn(noise / (1.0 + e * e), axes=(1, 2, 3)).real
+
+
+@pytest.mark.parametrize("n,md", [(15, 2), (15, 6), (21, 4), (27, 5), (33, 6), (45, 4), (45, 6), (45, 8)])
+def test_odd_width_rounding(gpu, n, md):
+    """The stencil at odd widths rounds no worse than the register-queue kernel's sum: the centre, then for each distance
+    the three axes' symmetric pairs by one multiply-add each, then Vloc."""
+    ld = np.longdouble
+    c = build_cell(Workload("w", max(1, round(n / 24)), n, 2, 2, 0.02, 1003, md))
+    c.uv[:] = 0.0
+    gpu.setup(c)
+    x = smooth_bands(n, 2, c.a, n)
+    v = c.vloc.reshape(-1)[:c.ML].reshape(n, n, n)
+
+    def pair(f, axis, m):
+        return np.roll(f, m, 3 - axis) + np.roll(f, -m, 3 - axis)
+
+    xl = x.astype(ld)
+    ref = (ld(c.coef_lap0) + v.astype(ld)) * xl
+    q = c.coef_lap0 * x
+    for m in range(1, md + 1):
+        for axis in range(3):
+            w = c.coef_lap[axis, m - 1]
+            ref += ld(w) * pair(xl, axis, m)
+            q = (ld(w) * pair(x, axis, m) + q).astype(np.float64)
+    q = (v.astype(ld) * x + q).astype(np.float64)
+    out = api.fortran_empty(c.ML, 2)
+    gpu.hamiltonian(1, 1, dev(x.reshape(2, -1).T), out, 1, c.ML, 1, 2)
+    gpu.synchronize()
+    got = out.cpu().numpy().T.reshape(x.shape)
+    assert np.sqrt(((got - ref) ** 2).sum()) <= np.sqrt(((q - ref) ** 2).sum())
