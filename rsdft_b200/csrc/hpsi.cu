@@ -1003,8 +1003,17 @@ static int launch_tma(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStrea
 }
 
 // k_stencil_row: rows of whole packs (8 bytes), up to 192 vectors of 16, and
-// 8-byte aligned arrays.  The tile height and z split of least
-// march_cost, two CTAs per SM sharing its shared-memory bandwidth.
+// 8-byte aligned arrays.
+//
+// The tile height and z split of least modelled time.  A plane takes 1350 plus
+// 31 per copy a thread issues plus 0.8 per shared-memory wavefront (window loads
+// and fill) of the CTAs that share the SM; a halo plane 0.23 of that; a CTA 1740
+// plus 410 per copy to set up its offsets; whole waves.  Fitted (in SM cycles)
+// to the times of all tiles and splits of 9^3 .. 111^3, 1 to 640 bands, Md 4, 6,
+// 8: the choice is within 1.4 % (rms) of the best.  Two CTAs per SM throughout and
+// no term for the copies, as suits the TMA march, splits small blocks into tiles
+// of two rows and few z chunks: 45^3 x 1 band 30.3 us against 23.4, Md = 8 x 8 bands 49.4 against 33.3
+// (projectors aside).
 template <typename T, int MD, int BY>
 static int launch_row(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStream_t st, HpsiDot* dot, bool* used) {
     *used = false;
@@ -1028,13 +1037,22 @@ static int launch_row(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStrea
         const int zmax = std::min({std::max(1, a.nzo / 4), 65535 / plan, (dot ? dot->cap : 1 << 20) / tiles});
         if (zmax < 1) continue;
         const double loads = BY + 2 * MD + BY * (2.0 * HX / VX) + BY;
-        const double t = 700.0 + 2.0 * 1.4 * (4.0 * loads * (threads / 32) + 2.0 * (2.0 * ty + 2 * MD) * row / 128.0);
-        int n = 1;
-        const double cost = march_cost((long)tiles * plan, a.nzo, 2 * MD, zmax, 2L * sms, t, 0.3 * t, &n);
-        if (TY == 0 || cost <= 1.05 * best) {  // the taller tile at a near tie
-            best = TY == 0 ? cost : std::min(cost, best);
-            TY = ty;
-            nzc = n;
+        const double lds = 4.0 * loads * (threads / 32) + 2.0 * (2.0 * ty + 2 * MD) * row / 128.0;
+        const double copies = (2.0 * ty + 2 * MD) * row / 8.0 / threads;
+        const double smem = (2.0 * ty + 2 * MD) * row * (S + 0.5);
+        const int per_sm = std::max(1, (int)std::min(227.0 * 1024 / (smem + 1024), 65536.0 / (168 * threads)));
+        for (int z = 1; z <= zmax; ++z) {
+            const int zlen = div_up(a.nzo, z), n = div_up(a.nzo, zlen);
+            const long ctas = (long)tiles * plan * n;
+            const int share = (int)std::min<long>(per_sm, (ctas + sms - 1) / sms);
+            const double t = 1350.0 + 31.0 * copies + 0.8 * share * lds;
+            const double cost = (double)((ctas + (long)per_sm * sms - 1) / ((long)per_sm * sms)) *
+                                (zlen * t + 2 * MD * 0.23 * t + 1740.0 + 410.0 * copies);
+            if (TY == 0 || cost < best || (ty > TY && cost <= 1.02 * best)) {  // the taller tile at a near tie
+                best = TY == 0 ? cost : std::min(cost, best);
+                TY = ty;
+                nzc = n;
+            }
         }
     }
     if (TY == 0) return RSDFT_OK;

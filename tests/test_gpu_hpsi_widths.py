@@ -21,7 +21,7 @@ def dev(a):
 @pytest.mark.parametrize("n,nb,md", [
     (5, 3, 6), (7, 1, 8), (9, 2, 6), (13, 5, 6), (15, 40, 4), (17, 3, 8), (21, 2, 7), (27, 9, 6), (45, 3, 6), (12, 1, 6),
     (12, 200, 6), (20, 7, 2), (26, 3, 6), (36, 5, 6), (40, 30, 8),
-    (36, 100, 6), (48, 20, 5), (48, 3, 6),
+    (36, 100, 6), (48, 20, 5), (48, 3, 6), (27, 1, 6), (33, 2, 8), (39, 1, 5),
 ])
 def test_hpsi_widths(gpu, n, nb, md):
     c = build_cell(Workload("w", 1, n, nb, nb, 0.03, 5000 + n, md))
