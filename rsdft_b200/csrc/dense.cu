@@ -64,8 +64,8 @@ __global__ void k_reduce_partials(const double* __restrict__ P, int nch, int m, 
 // A tall block (ml x nb) and how its FP64 products are formed: from its INT8
 // slices (imma.cu) where those suit, made once for every product it takes part
 // in, else straight on the FP64 tensor pipe (dmma.cu).  The INT8 launches
-// stand down when *bad is set on the device (a value that is not finite, or
-// out of the sliced range) and the DMMA launch behind each runs only then, so
+// stand down when *bad is set on the device (a value that is not finite or out of
+// the sliced range, or a decaying band) and the DMMA launch behind each runs only then, so
 // NaNs and infinities come out as they do there, without a synchronisation.
 struct Fp64Block {
     const double* x = nullptr;

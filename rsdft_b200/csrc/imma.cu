@@ -4,33 +4,40 @@
 // Yokota, "DGEMM on integer matrix multiplication unit", 2024).
 //
 // A vector (a band, or a column of the rotation matrix) is scaled by a power
-// of two to 54-bit integers, q = rint(x 2^(54 - e)) with |x| < 2^e, and q is
-// written in seven balanced base-256 digits, q = sum_s d_s 256^(6 - s), each
-// an int8.  A product of two values is the sum of the digit products d_s d'_t
-// with s + t <= 7 (up to 6, the dropped products of a 480-term rotation sum up
-// to 4e-15 of the bands; up to 7, to 3e-17).  Digit products of equal s + t
-// share an INT32 accumulator: 7 pairs x 2^14 x 16,384 terms < 2^31, so a chain
-// of IM_SEG K blocks is exact, after which the eight accumulators are folded
-// into FP64.  An element is thus represented to
-// 2^-55 of its vector's largest, where FP64 keeps 2^-53 of the element itself:
-// the error of a product is a share of the vectors' norms, as it is in FP64
-// (tests: no larger than the DMMA kernels' against 64-bit references).
+// of two to 62-bit integers, q = rint(x 2^(62 - e)) with |x| < 2^e, and q is
+// written in eight balanced base-256 digits, q = sum_s d_s 256^(7 - s), each
+// an int8, the first at most 64.  A product of two values is the sum of the
+// digit products d_s d'_t with s + t <= 7.  Digit products of equal s + t share
+// an INT32 accumulator: at most (6 x 2^14 + 2 x 2^13) x 16,384 terms < 2^31, so a
+// chain of IM_SEG K blocks is exact, after which the eight accumulators are
+// folded into FP64.
 //
-// Why: the FP64 tensor pipe gives 37 TFLOP/s, the INT8 pipe 34 digit products
+// Precision.  An element is held to 2^-63 of its vector's largest, and the
+// products left out come to 2^-62 of the largest (rms) per term, so the error of
+// a sum of k terms is at most about 2^-60 k of the vectors' largest values, where
+// FP64 arithmetic gives 2^-53 of each partial sum.  It is the smaller one as long
+// as the terms reach 2^-9 or so of the largest, but unlike FP64's it does not
+// shrink with them: where a band decays (vacuum, a localised band) its tail
+// would lose digits.  Such blocks go to the FP64 tensor pipe whole
+// (k_imma_slice: a grid point at which 64 bands, or 32 points in a row at which
+// one band, stay below 2^-12 of their largest).  What is left are the isolated
+// values near a band's nodes, good to 2^-60 of its largest.
+//
+// Why: the FP64 tensor pipe gives 37 TFLOP/s, the INT8 pipe 36 digit products
 // per FP64 product at up to 4.5 POP/s, an FP64 rate of about 130 TFLOP/s.
 // 72^3 x 480, psi^T psi: 1170 us against 4365 us (DMMA, upper tiles);
 // psi V: 2000 us against 6360 us; slicing psi for both 960 us
 // (exponents included).
 //
 // k_imma, one CTA per 128 x 64 tile of D(m, n) = sum_k A(m, k) B(n, k):
-//   warp 0    TMA producer: per K block of 64 the seven slices of both tiles
+//   warp 0    TMA producer: per K block of 64 the eight slices of both tiles
 //             (64-byte swizzle), one box each, into a ring of IM_NS stages;
-//   warp 1    allocates TMEM; one lane issues the MMAs.  The seven slices of B
+//   warp 1    allocates TMEM; one lane issues the MMAs.  The eight slices of B
 //             lie one after the other in shared memory and the accumulators
 //             of s + t = 0..7 one after the other in TMEM, so A's slice s
 //             meets B's slices t, t + 1, .. as one MMA of N = 64 x (slices),
-//             at most 256: 13 MMAs per K step instead of 34, and A is read
-//             from shared memory once per MMA (34 MMAs of N = 64 would be
+//             at most 256: 12 MMAs per K step instead of 36, and A is read
+//             from shared memory once per MMA (36 MMAs of N = 64 would be
 //             bound by that, 48 cycles of shared memory for 32 of MMA);
 //   warps 2-9 fold the accumulators (two warps per TMEM lane quadrant).
 // What bounds it is the operand stream from L2: 86 KB per 2176 cycles of MMA.
@@ -46,7 +53,7 @@ namespace rsdft {
 
 namespace {
 
-constexpr int IM_S = 7;        // slices
+constexpr int IM_S = 8;        // slices
 constexpr int IM_M = 128;      // tile rows (TMEM lanes)
 constexpr int IM_N = 64;       // tile columns
 constexpr int IM_K = 64;       // K block: one 64-byte row
@@ -58,7 +65,9 @@ constexpr int IM_EPI = 8;      // epilogue warps
 constexpr int IM_THREADS = 32 * (2 + IM_EPI);
 constexpr int IM_D = 8;        // accumulators, s + t = 0 .. 7
 constexpr int IM_TCOLS = IM_D * IM_N;  // all of TMEM
-constexpr int IM_BITS = 54;    // integer bits of a scaled value
+static_assert(IM_S == IM_D, "slice 0 of A opens every accumulator");
+constexpr int IM_BITS = 62;    // integer bits of a scaled value
+constexpr int IM_TINY = 12;    // values below 2^-IM_TINY of the largest may come singly only
 // exponents beyond which 2^(IM_BITS - e) or the products leave the range
 constexpr int IM_EMAX = 400;
 
@@ -96,24 +105,24 @@ __global__ void __launch_bounds__(256) k_imma_exp(const double* __restrict__ A, 
     }
 }
 
-// A zero vector has every digit zero whatever its exponent; a tiny one is out
-// of range.
+// A zero vector has every digit zero whatever its exponent (-IM_EMAX marks it);
+// a tiny one is out of range.
 __global__ void k_imma_exp_check(int* __restrict__ exps, int n, int* __restrict__ bad) {
     grid_dependency();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= n) return;
     if (exps[b] < -100000)
-        exps[b] = 0;
-    else if (exps[b] < -IM_EMAX)
+        exps[b] = -IM_EMAX;
+    else if (exps[b] <= -IM_EMAX)
         *bad = 1;
 }
 
-// the seven digits of x: lo holds the bytes of slices 6, 5, 4, 3, hi those of
-// 2, 1, 0
+// the eight digits of x: lo holds the bytes of slices 7, 6, 5, 4, hi those of
+// 3, 2, 1, 0
 __device__ __forceinline__ void imma_digits(double x, double scale, uint32_t& lo, uint32_t& hi) {
-    const long long q = __double2ll_rn(x * scale) + 0x80808080808080ll;
+    const unsigned long long q = (unsigned long long)__double2ll_rn(x * scale) + 0x8080808080808080ull;
     lo = (uint32_t)q ^ 0x80808080u;
-    hi = (uint32_t)((unsigned long long)q >> 32) ^ 0x00808080u;
+    hi = (uint32_t)(q >> 32) ^ 0x80808080u;
 }
 
 // 4 x 4 byte transpose: row j of the result holds byte j of a, b, c, d
@@ -130,27 +139,36 @@ __device__ __forceinline__ void byte_transpose(uint32_t a, uint32_t b, uint32_t 
 // transposes the digits in registers both ways, and each layout goes out
 // through shared memory in 16-byte stores.  rows: [s][kb][nb][64 points]; cols:
 // [s][mb][ml][64 bands].
+//
+// Sets *bad when the block decays (file header): at one of the CTA's points all
+// its bands (if at least 32), or over 32 aligned points one band, below 2^-IM_TINY
+// of the bands' largest.  Bands that are zero throughout are left out.
 __global__ void __launch_bounds__(256) k_imma_slice(const double* __restrict__ A, long ld, long ml, int nb, int nkb,
                                                     const int* __restrict__ exps, int8_t* __restrict__ rows,
-                                                    int8_t* __restrict__ cols, const int* __restrict__ bad, int vec) {
+                                                    int8_t* __restrict__ cols, int* bad, int vec) {
     grid_dependency();
     // pitch 17: the transposed words of a half warp (rows 4 apart) fall on 8
     // banks (at a pitch of 20, which 16-byte reads want, on 2: 872 us per
     // 72^3 x 480 block instead of 753)
     __shared__ uint32_t sm[IM_S][64][17];
-    if (*bad) return;
+    __shared__ uint32_t s_row[8][4];  // per warp: the points (16 x 4) where its 8 bands are tiny
+    if (__syncthreads_or(*bad)) return;  // one answer for the CTA: another may set it meanwhile
     const int p = threadIdx.x & 15, q = threadIdx.x >> 4;
     const int kb = blockIdx.x, mb = blockIdx.y;
     const long i0 = (long)kb * 64 + 4 * p;
     const int b0 = mb * 64 + 4 * q;
     uint32_t lo[4][4], hi[4][4];  // [band][point]
+    uint32_t tiny = 0, run = 0;   // bit 4 r + e: tiny or no value; bit r: four tiny values
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const int b = b0 + r;
         double x[4] = {0.0, 0.0, 0.0, 0.0};
         double scale = 0.0;
+        uint32_t floor_hi = 0xffffffffu;  // no value: below any
         if (b < nb) {
-            scale = scalbn(1.0, IM_BITS - exps[b]);
+            const int ex = exps[b];
+            scale = scalbn(1.0, IM_BITS - ex);
+            if (ex != -IM_EMAX) floor_hi = (uint32_t)(ex - IM_TINY + 1023) << 20;
             const double* src = A + (long)b * ld + i0;
             if (vec && i0 + 4 <= ml) {
                 const double2 u = *reinterpret_cast<const double2*>(src), v = *reinterpret_cast<const double2*>(src + 2);
@@ -165,8 +183,33 @@ __global__ void __launch_bounds__(256) k_imma_slice(const double* __restrict__ A
             }
         }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) imma_digits(x[e], scale, lo[r][e], hi[r][e]);
+        for (int e = 0; e < 4; ++e) {
+            imma_digits(x[e], scale, lo[r][e], hi[r][e]);
+            if ((uint32_t)(__double2hiint(x[e]) & 0x7fffffff) < floor_hi) tiny |= 1u << (4 * r + e);
+        }
+        if (floor_hi != 0xffffffffu && ((tiny >> (4 * r)) & 15u) == 15u && i0 + 4 <= ml) run |= 1u << r;
     }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t runs = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        uint32_t m = __ballot_sync(0xffffffffu, ((tiny >> e) & 0x1111u) == 0x1111u && i0 + e < ml);
+        m &= m >> 16;
+        if (lane == 0) s_row[warp][e] = m & 0xffffu;
+        uint32_t n = __ballot_sync(0xffffffffu, (run >> e) & 1u);  // here e is the band
+        n &= n >> 4;
+        n &= n >> 2;
+        runs |= n & (n >> 1) & 0x01010101u;
+    }
+    if (runs && lane == 0) *bad = 1;
+    auto check_rows = [&] {
+        if (threadIdx.x < 4 && nb - mb * 64 >= 32) {
+            uint32_t m = 0xffffu;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) m &= s_row[w][threadIdx.x];
+            if (m) *bad = 1;
+        }
+    };
     if (rows) {
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -174,9 +217,10 @@ __global__ void __launch_bounds__(256) k_imma_slice(const double* __restrict__ A
             byte_transpose(lo[r][0], lo[r][1], lo[r][2], lo[r][3], tl);
             byte_transpose(hi[r][0], hi[r][1], hi[r][2], hi[r][3], th);
 #pragma unroll
-            for (int s = 0; s < IM_S; ++s) sm[s][4 * q + r][p] = s < 3 ? th[2 - s] : tl[6 - s];
+            for (int s = 0; s < IM_S; ++s) sm[s][4 * q + r][p] = s < 4 ? th[3 - s] : tl[7 - s];
         }
         __syncthreads();
+        check_rows();
         for (int t = threadIdx.x; t < IM_S * 64 * 4; t += 256) {
             const int s = t >> 8, r = (t >> 2) & 63, w = t & 3;
             if (mb * 64 + r < nb)
@@ -192,9 +236,10 @@ __global__ void __launch_bounds__(256) k_imma_slice(const double* __restrict__ A
         byte_transpose(lo[0][e], lo[1][e], lo[2][e], lo[3][e], tl);
         byte_transpose(hi[0][e], hi[1][e], hi[2][e], hi[3][e], th);
 #pragma unroll
-        for (int s = 0; s < IM_S; ++s) sm[s][4 * p + e][q] = s < 3 ? th[2 - s] : tl[6 - s];
+        for (int s = 0; s < IM_S; ++s) sm[s][4 * p + e][q] = s < 4 ? th[3 - s] : tl[7 - s];
     }
     __syncthreads();
+    if (!rows) check_rows();
     const int nmb = gridDim.y;
     for (int t = threadIdx.x; t < IM_S * 64 * 4; t += 256) {
         const int s = t >> 8, i = (t >> 2) & 63, w = t & 3;
@@ -210,10 +255,10 @@ __global__ void __launch_bounds__(256) k_imma_slice(const double* __restrict__ A
 // [s][mb][n][64], one warp per column
 __global__ void __launch_bounds__(128) k_imma_slice_v(const double* __restrict__ V, int ldv, int nb, int nmb,
                                                       const int* __restrict__ exps, double* __restrict__ vscale,
-                                                      int8_t* __restrict__ out, int* __restrict__ bad) {
+                                                      int8_t* __restrict__ out, int* bad) {
     grid_dependency();
     const int n = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (n >= nb || *bad) return;
+    if (n >= nb || __any_sync(0xffffffffu, *bad)) return;
     const double* v = V + (long)n * ldv;
     int e = INT_MIN;
     bool fin = true;
@@ -242,7 +287,7 @@ __global__ void __launch_bounds__(128) k_imma_slice_v(const double* __restrict__
         const size_t ss = (size_t)nmb * nb * 64;
 #pragma unroll
         for (int s = 0; s < IM_S; ++s)
-            o[s * ss] = (int8_t)((s < 3 ? hi >> (8 * (2 - s)) : lo >> (8 * (6 - s))) & 255u);
+            o[s * ss] = (int8_t)((s < 4 ? hi >> (8 * (3 - s)) : lo >> (8 * (7 - s))) & 255u);
     }
 }
 
@@ -401,22 +446,15 @@ __global__ void __launch_bounds__(IM_THREADS, 1) k_imma(const __grid_constant__ 
 #pragma unroll
                         for (int i = 0; i < IM_S; ++i) {
                             const uint64_t ad = umma_desc_sw64(sa + i * IM_ABYTES + kk * 32);
-                            // slices t of B with s + t <= 7, four at a time;
-                            // A's slice 1 meets slice 6 apart, as the first
-                            // product of its accumulator
-                            constexpr int NB = IM_S;
-                            const int nt = i == 1 ? NB - 1 : (IM_D - i < NB ? IM_D - i : NB);
+                            // slices t of B with s + t <= 7, four at a time
 #pragma unroll
-                            for (int j = 0; j < nt; j += 4) {
-                                const int nj = nt - j < 4 ? nt - j : 4;
+                            for (int j = 0; j < IM_D - i; j += 4) {
+                                const int nj = IM_D - i - j < 4 ? IM_D - i - j : 4;
                                 const uint64_t bd = umma_desc_sw64(sb + j * IM_BBYTES + kk * 32);
-                                // a chain's first products overwrite
+                                // a chain's first products, slice 0 with all, overwrite
                                 const uint32_t acc = (kb == ka && kk == 0 && i == 0) ? 0u : 1u;
                                 imma_mma(tbase + (uint32_t)((i + j) * IM_N), ad, bd, imma_idesc(IM_N * nj), acc);
                             }
-                            if (i == 1)
-                                imma_mma(tbase + (uint32_t)(7 * IM_N), ad, umma_desc_sw64(sb + 6 * IM_BBYTES + kk * 32),
-                                         imma_idesc(IM_N), (kb == ka && kk == 0) ? 0u : 1u);
                         }
                     }
                     umma_commit(&empty[s]);
@@ -573,7 +611,7 @@ int imma_slice(const double* A, long ld, long ml, int nb, const char* ws, bool n
     launch(k_imma_exp_check, div_up(nb, 128), 128, 0, c.stream, exps, nb, bad);
     const int vec = (ld % 2 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0) ? 1 : 0;
     launch(k_imma_slice, dim3(nkb, nmb), 256, 0, c.stream, A, ld, ml, nb, nkb, (const int*)exps, rows, cols,
-           (const int*)bad, vec);
+           bad, vec);
     RS_LAUNCH();
     *out = ImmaSlices{rows, cols, exps, nb, ml};
     return RSDFT_OK;

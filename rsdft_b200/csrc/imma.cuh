@@ -20,8 +20,9 @@ bool imma_suits(long ml, int nb);
 
 // Slice A (ml x nb, leading dimension ld) into the workspaces named after ws:
 // rows for Gram products, cols for rotations.  *bad (device, cleared by the
-// caller) is set when a value is not finite or out of the sliced range: the
-// products below then leave their results to a DMMA launch conditional on it.
+// caller) is set when a value is not finite or out of the sliced range, or when a
+// band decays so far that its tail would lose digits: the products below then
+// leave their results to a DMMA launch conditional on it.
 // RSDFT_ENOMEM when the slices do not fit (error cleared).
 int imma_slice(const double* A, long ld, long ml, int nb, const char* ws, bool need_rows, bool need_cols, int* bad,
                ImmaSlices* out);
