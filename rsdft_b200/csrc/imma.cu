@@ -589,7 +589,9 @@ int launch_imma(const ImmaMaps& maps, const ImmaArgs& g, dim3 grid) {
 
 }  // namespace
 
-bool imma_suits(long ml, int nb) { return nb >= 96 && ml >= 4096; }
+// A rotation runs over all bands in one chain, which is exact up to IM_SEG K
+// blocks; a larger set takes the DMMA form, as it did before there were slices.
+bool imma_suits(long ml, int nb) { return nb >= 96 && nb <= IM_SEG * IM_K && ml >= 4096; }
 
 int imma_slice(const double* A, long ld, long ml, int nb, const char* ws, bool need_rows, bool need_cols, int* bad,
                ImmaSlices* out) {

@@ -90,3 +90,15 @@ def test_every_entry_is_defined_once_and_opens_a_trace_range():
     for name, first in defs:
         if name not in getters:
             assert first == "RS_ENTRY();", f"{name} does not open with RS_ENTRY()"
+
+
+def test_int8_chains_stay_exact():
+    """A rotation of nb bands is one INT32 chain of nb terms: the INT8 form is not taken where it could wrap."""
+    L = _lib.load()
+    suits = getattr(L, "_ZN5rsdft10imma_suitsEli")
+    suits.restype, suits.argtypes = ctypes.c_bool, [ctypes.c_long, ctypes.c_int]
+    # digit products of equal weight: eight pairs, two of them with a first digit of at most 64
+    per_term = 6 * 128 * 128 + 2 * 64 * 128
+    largest = max(nb for nb in range(64, 1 << 16, 64) if suits(1 << 20, nb))
+    assert largest >= 8192 and largest * per_term < 2 ** 31
+    assert not suits(1 << 20, largest + 1) and not suits(1 << 20, 1 << 20)
