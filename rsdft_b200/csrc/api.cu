@@ -58,6 +58,52 @@ char* host_workspace(size_t bytes) {
     return g_ctx.host_ws.data();
 }
 
+bool release_optional(const char* name) {
+    if (!name && g_ctx.optional_held) return false;
+    bool any = false;
+    for (auto& kv : g_ctx.ws) {
+        Buf& b = kv.second;
+        if (!b.optional || !b.p || (name && kv.first != name)) continue;
+        if (!any && cudaStreamSynchronize(g_ctx.stream) != cudaSuccess) return false;
+        cudaFree(b.p);
+        b.p = nullptr;
+        b.bytes = 0;
+        any = true;
+    }
+    return any;
+}
+
+cudaError_t device_malloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        if (release_optional()) e = cudaMalloc(p, bytes);
+        if (e != cudaSuccess) cudaGetLastError();
+    }
+    return e;
+}
+
+int workspace_optional(const char* name, size_t bytes, void** out) {
+    Buf& b = g_ctx.ws[name];
+    b.optional = true;
+    if (b.bytes < bytes) {
+        if (b.p) release_optional(name);
+        size_t held = 0, free_bytes = 0, total = 0;
+        for (const auto& kv : g_ctx.ws)
+            if (kv.second.optional) held += kv.second.bytes;
+        const size_t want = std::max<size_t>(bytes, 256);
+        if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || held + want > (free_bytes + held) / 2 ||
+            cudaMalloc(&b.p, want) != cudaSuccess) {
+            cudaGetLastError();
+            b.p = nullptr;
+            return RSDFT_ENOMEM;
+        }
+        b.bytes = want;
+    }
+    *out = b.p;
+    return RSDFT_OK;
+}
+
 int workspace(const char* name, size_t bytes, void** out) {
     Buf& b = g_ctx.ws[name];
     if (b.bytes < bytes) {
@@ -68,8 +114,9 @@ int workspace(const char* name, size_t bytes, void** out) {
             b.bytes = 0;
         }
         size_t want = std::max<size_t>(bytes, 256);
-        cudaError_t e = cudaMalloc(&b.p, want);
+        cudaError_t e = device_malloc(&b.p, want);
         if (e != cudaSuccess) {
+            b.p = nullptr;
             set_error("workspace '%s': cudaMalloc(%zu) failed: %s", name, want, cudaGetErrorString(e));
             return RSDFT_ENOMEM;
         }
@@ -204,7 +251,7 @@ static int upload(T** dst, const T* src, size_t n) {
         *dst = nullptr;
     }
     if (n == 0) return RSDFT_OK;
-    if (cudaMalloc(dst, n * sizeof(T)) != cudaSuccess) {
+    if (device_malloc(reinterpret_cast<void**>(dst), n * sizeof(T)) != cudaSuccess) {
         set_error("cudaMalloc(%zu) failed", n * sizeof(T));
         return RSDFT_ENOMEM;
     }
@@ -548,7 +595,7 @@ int rsdft_gpu_register_wf(double* unk, long ml, int mb) {
     WfReg r;
     r.host = h;
     r.bytes = bytes;
-    if (cudaMalloc(&r.dev, bytes) != cudaSuccess) {
+    if (device_malloc(reinterpret_cast<void**>(&r.dev), bytes) != cudaSuccess) {
         set_error("register_wf: cudaMalloc(%zu) failed", bytes);
         return RSDFT_ENOMEM;
     }

@@ -47,6 +47,7 @@ struct PrecondCoef {
 struct Buf {
     void* p = nullptr;
     size_t bytes = 0;
+    bool optional = false;  // may be freed when something else needs the memory
 };
 
 struct WfReg {
@@ -115,6 +116,7 @@ struct Context {
 
     // workspace
     std::map<std::string, Buf> ws;
+    int optional_held = 0;  // OptionalHold objects alive
     std::vector<WfReg> regs;
     std::vector<char> host_ws;               // host scratch of cuSOLVER calls
     std::map<const void*, int> smem_optin;   // dynamic shared memory opted in, per kernel
@@ -270,6 +272,30 @@ template <typename T>
 inline int workspace_t(const char* name, size_t count, T** out) {
     return workspace(name, count * sizeof(T), reinterpret_cast<void**>(out));
 }
+
+// The same for a buffer that its caller can do without.  All of them together
+// take at most half of the memory not otherwise in use (RSDFT_ENOMEM beyond
+// that, no error kept), and they are freed when any other allocation of the
+// library fails, unless an OptionalHold is alive: an operation holds one
+// while it uses such buffers.
+int workspace_optional(const char* name, size_t bytes, void** out);
+template <typename T>
+inline int workspace_optional_t(const char* name, size_t count, T** out) {
+    return workspace_optional(name, count * sizeof(T), reinterpret_cast<void**>(out));
+}
+struct OptionalHold {
+    OptionalHold() { ++ctx().optional_held; }
+    ~OptionalHold() { --ctx().optional_held; }
+    OptionalHold(const OptionalHold&) = delete;
+    OptionalHold& operator=(const OptionalHold&) = delete;
+};
+
+// Free the optional buffers (only one of them if a name is given); whether any
+// memory came free.  Waits for the stream.
+bool release_optional(const char* name = nullptr);
+
+// cudaMalloc, tried again without the optional buffers when it fails.
+cudaError_t device_malloc(void** p, size_t bytes);
 
 // ------------------------------------------------- pointer resolution
 // Classify a caller pointer and the `bytes` that follow it: device memory of

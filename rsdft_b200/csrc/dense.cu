@@ -75,18 +75,35 @@ struct Fp64Block {
     ImmaSlices s;
 };
 
-static int fp64_flag(int** bad) {
+static int fp64_flag(bool slices, int** bad) {
+    *bad = nullptr;
+    if (!slices) return RSDFT_OK;
     RS_CHECK(workspace_t("imma_bad", 1, bad));
     RS_CUDA(cudaMemsetAsync(*bad, 0, sizeof(int), ctx().stream));
     return RSDFT_OK;
 }
 
+// An operation on FP64 blocks: op(true) may use slices, which are held meanwhile;
+// where that leaves too little memory for the rest of it, op(false) runs again
+// without them.  op must leave its inputs alone until its last step, the rotation,
+// which needs no memory of its own.
+template <class Op>
+static int with_slices(Op op) {
+    int r;
+    {
+        const OptionalHold hold;
+        r = op(true);
+    }
+    if (r == RSDFT_ENOMEM && release_optional()) r = op(false);
+    return r;
+}
+
 // rows / cols: slices for Gram products / for rotations.  bad: the operation's
-// flag (fp64_flag), shared by its blocks.
+// flag (fp64_flag), shared by its blocks; null: no slices.
 static int fp64_block(const double* x, long ld, long ml, int nb, const char* ws, bool rows, bool cols, int* bad,
                       Fp64Block* out) {
     *out = Fp64Block{x, ld, ml, nb, nullptr, {}};
-    if (!imma_suits(ml, nb)) return RSDFT_OK;
+    if (!bad || !imma_suits(ml, nb)) return RSDFT_OK;
     const int r = imma_slice(x, ld, ml, nb, ws, rows, cols, bad, &out->s);
     if (r == RSDFT_ENOMEM) return RSDFT_OK;  // no room for the slices
     if (r == RSDFT_OK) out->bad = bad;
@@ -97,7 +114,13 @@ static int fp64_block(const double* x, long ld, long ml, int nb, const char* ws,
 // half, mirrored; symmetrize averages what lies in the diagonal tiles
 static int fp64_gram(const Fp64Block& a, const Fp64Block& b, double alpha, int symmetrize, double* C) {
     const int* bad = a.bad && b.bad ? a.bad : nullptr;
-    if (bad) RS_CHECK(imma_gram(a.s, b.s, alpha, symmetrize, bad, C, a.nb));
+    if (bad) {
+        const int r = imma_gram(a.s, b.s, alpha, symmetrize, bad, C, a.nb);
+        if (r == RSDFT_ENOMEM)
+            bad = nullptr;
+        else
+            RS_CHECK(r);
+    }
     return dmma_gram(a.x, b.x, a.ld, a.ml, a.nb, a.nb, alpha, symmetrize, C, a.nb, true, bad);
 }
 
@@ -115,14 +138,21 @@ __global__ void k_copy_cols_if(const double* __restrict__ src, long lds, double*
 static int fp64_rotate(const Fp64Block& a, const double* V, int ldv, double* out, long ldo, double* tmp = nullptr,
                        long ldt = 0) {
     Context& c = ctx();
-    if (a.bad) RS_CHECK(imma_rotate(a.s, V, ldv, a.bad, out, ldo));
+    int* bad = a.bad;
+    if (bad) {
+        const int r = imma_rotate(a.s, V, ldv, bad, out, ldo);
+        if (r == RSDFT_ENOMEM)
+            bad = nullptr;
+        else
+            RS_CHECK(r);
+    }
     const bool inplace = out == a.x;
     RS_CHECK(dmma_gemm(false, a.ml, a.nb, a.nb, 1.0, a.x, a.ld, V, ldv, 0.0, inplace ? tmp : out,
-                       inplace ? ldt : ldo, a.bad));
+                       inplace ? ldt : ldo, bad));
     if (!inplace) return RSDFT_OK;
-    if (a.bad) {
+    if (bad) {
         launch(k_copy_cols_if, dim3(64, std::min(a.nb, 64)), 256, 0, c.stream, (const double*)tmp, ldt, out, ldo, a.ml,
-               a.nb, (const int*)a.bad);
+               a.nb, (const int*)bad);
         RS_LAUNCH();
         return RSDFT_OK;
     }
@@ -234,23 +264,24 @@ static int trtri_upper(double* S, int nb, int* dinfo, const char* what) {
 // product is one DGEMM (in and out are different buffers).
 static int cholqr_pass(const double* psi, double* out, long ld, int nb, double* S, int* dinfo, int mode) {
     Context& c = ctx();
-    const void* split = nullptr;
-    Fp64Block blk;
-    if (mode == RSDFT_MODE_FP64) {
-        int* bad = nullptr;
-        RS_CHECK(fp64_flag(&bad));
-        RS_CHECK(fp64_block(psi, ld, c.ml, nb, "imma_psi", true, true, bad, &blk));
-        RS_CHECK(fp64_gram(blk, blk, c.dV, 0, S));
-    } else {
-        RS_CHECK(gram_mixed(psi, psi, ld, nb, c.dV, 0, mode, S, &split));
-    }
-    RS_CHECK(potrf_upper(S, nb, dinfo, "gram_schmidt: overlap Cholesky"));
-    RS_CHECK(trtri_upper(S, nb, dinfo, "gram_schmidt: triangular inverse"));
+    auto factor = [&] {
+        RS_CHECK(potrf_upper(S, nb, dinfo, "gram_schmidt: overlap Cholesky"));
+        return trtri_upper(S, nb, dinfo, "gram_schmidt: triangular inverse");
+    };
     if (mode == RSDFT_MODE_FP64)
-        RS_CHECK(fp64_rotate(blk, S, nb, out, ld));
-    else
-        RS_CHECK(rotate_mixed(psi, out, ld, nb, S, nb, mode, split));
-    return RSDFT_OK;
+        return with_slices([&](bool slices) {
+            int* bad = nullptr;
+            Fp64Block blk;
+            RS_CHECK(fp64_flag(slices, &bad));
+            RS_CHECK(fp64_block(psi, ld, c.ml, nb, "imma_psi", true, true, bad, &blk));
+            RS_CHECK(fp64_gram(blk, blk, c.dV, 0, S));
+            RS_CHECK(factor());
+            return fp64_rotate(blk, S, nb, out, ld);
+        });
+    const void* split = nullptr;
+    RS_CHECK(gram_mixed(psi, psi, ld, nb, c.dV, 0, mode, S, &split));
+    RS_CHECK(factor());
+    return rotate_mixed(psi, out, ld, nb, S, nb, mode, split);
 }
 
 int gram_schmidt_device(double* psi, long ld, int nb, int mode) {
@@ -289,17 +320,18 @@ int subspace_diag_device(double* psi, long ld, int mb, int spin, double* esp, in
     RS_CHECK(workspace_t("sub_hpsi", (size_t)ld * mb, &hpsi));
     RS_CHECK(workspace_t("sub_H", (size_t)mb * mb, &H));
     RS_CHECK(hpsi_device<double>(psi, hpsi, ld, mb, spin, nullptr));
-    if (mode == RSDFT_MODE_FP64) {
-        int* bad = nullptr;
-        Fp64Block p, h;
-        RS_CHECK(fp64_flag(&bad));
-        RS_CHECK(fp64_block(psi, ld, c.ml, mb, "imma_psi", true, true, bad, &p));
-        RS_CHECK(fp64_block(hpsi, ld, c.ml, mb, "imma_hpsi", true, false, bad, &h));
-        // Hsub = dV/2 (psi^T H psi + (H psi)^T psi): the symmetric part of dV psi^T (H psi)
-        RS_CHECK(fp64_gram(p, h, c.dV, 1, H));
-        RS_CHECK(syevd(H, mb, esp, CUBLAS_FILL_MODE_UPPER, "subspace_diag: syevd"));
-        return fp64_rotate(p, H, mb, psi, ld, hpsi, ld);
-    }
+    if (mode == RSDFT_MODE_FP64)
+        return with_slices([&](bool slices) {
+            int* bad = nullptr;
+            Fp64Block p, h;
+            RS_CHECK(fp64_flag(slices, &bad));
+            RS_CHECK(fp64_block(psi, ld, c.ml, mb, "imma_psi", true, true, bad, &p));
+            RS_CHECK(fp64_block(hpsi, ld, c.ml, mb, "imma_hpsi", true, false, bad, &h));
+            // Hsub = dV/2 (psi^T H psi + (H psi)^T psi): the symmetric part of dV psi^T (H psi)
+            RS_CHECK(fp64_gram(p, h, c.dV, 1, H));
+            RS_CHECK(syevd(H, mb, esp, CUBLAS_FILL_MODE_UPPER, "subspace_diag: syevd"));
+            return fp64_rotate(p, H, mb, psi, ld, hpsi, ld);
+        });
     const void* split = nullptr;
     RS_CHECK(gram_mixed(psi, hpsi, ld, mb, c.dV, 1, mode, H, &split));
     RS_CHECK(syevd(H, mb, esp, CUBLAS_FILL_MODE_UPPER, "subspace_diag: syevd"));
@@ -385,32 +417,42 @@ int orth_subspace_diag_device(double* psi, long ld, int mb, int spin, double* es
     const void* split = nullptr;
     if (!hpsi_in) RS_CHECK(hpsi_device<double>(psi, hpsi, ld, mb, spin, nullptr));
     const double* hp = hpsi_in ? hpsi_in : hpsi;
-    Fp64Block p, h;
+    // factor S and, unless the overlap is too ill-conditioned for one step, T =
+    // R^-1 V; *fused says which
+    auto reduce = [&](bool* fused) {
+        RS_CHECK(potrf_upper(S, mb, dinfo, "orth_subspace_diag: overlap Cholesky", false));
+        launch(k_diag_minmax, 1, 256, 0, c.stream, S, mb, mb, mm);
+        RS_LAUNCH();
+        double hmm[2] = {0.0, 0.0};
+        RS_CHECK(read_cholesky(dinfo, mm, hmm, "orth_subspace_diag: overlap Cholesky"));
+        *fused = hmm[0] > 0.0 && !((hmm[1] / hmm[0]) * (hmm[1] / hmm[0]) > fused_rr_kappa_max(mode));
+        if (!*fused) return RSDFT_OK;
+        RS_CHECK(trtri_upper(S, mb, dinfo, "orth_subspace_diag: triangular inverse"));
+        return rr_reduced(S, H, T, mb, esp, "orth_subspace_diag: syevd");
+    };
+    bool fused = false;
     if (mode == RSDFT_MODE_FP64) {
-        int* bad = nullptr;
-        RS_CHECK(fp64_flag(&bad));
-        RS_CHECK(fp64_block(psi, ld, c.ml, mb, "imma_psi", true, true, bad, &p));
-        RS_CHECK(fp64_block(hp, ld, c.ml, mb, "imma_hpsi", true, false, bad, &h));
-        RS_CHECK(fp64_gram(p, p, c.dV, 0, S));
-        RS_CHECK(fp64_gram(p, h, c.dV, 1, H));
+        RS_CHECK(with_slices([&](bool slices) {
+            int* bad = nullptr;
+            Fp64Block p, h;
+            RS_CHECK(fp64_flag(slices, &bad));
+            RS_CHECK(fp64_block(psi, ld, c.ml, mb, "imma_psi", true, true, bad, &p));
+            RS_CHECK(fp64_block(hp, ld, c.ml, mb, "imma_hpsi", true, false, bad, &h));
+            RS_CHECK(fp64_gram(p, p, c.dV, 0, S));
+            RS_CHECK(fp64_gram(p, h, c.dV, 1, H));
+            RS_CHECK(reduce(&fused));
+            return fused ? fp64_rotate(p, T, mb, psi, ld, hpsi, ld) : RSDFT_OK;
+        }));
     } else {
         RS_CHECK(gram_mixed_pair(psi, hp, ld, mb, c.dV, mode, S, H, &split));
+        RS_CHECK(reduce(&fused));
+        // the tensor-core rotation reads only the BF16 split of psi, so it can
+        // write psi itself
+        if (fused) return rotate_mixed(psi, psi, ld, mb, T, mb, mode, split);
     }
-    RS_CHECK(potrf_upper(S, mb, dinfo, "orth_subspace_diag: overlap Cholesky", false));
-    launch(k_diag_minmax, 1, 256, 0, c.stream, S, mb, mb, mm);
-    RS_LAUNCH();
-    double hmm[2] = {0.0, 0.0};
-    RS_CHECK(read_cholesky(dinfo, mm, hmm, "orth_subspace_diag: overlap Cholesky"));
-    if (!(hmm[0] > 0.0) || (hmm[1] / hmm[0]) * (hmm[1] / hmm[0]) > fused_rr_kappa_max(mode)) {
-        RS_CHECK(gram_schmidt_device(psi, ld, mb, mode));
-        return subspace_diag_device(psi, ld, mb, spin, esp, mode);
-    }
-    RS_CHECK(trtri_upper(S, mb, dinfo, "orth_subspace_diag: triangular inverse"));
-    RS_CHECK(rr_reduced(S, H, T, mb, esp, "orth_subspace_diag: syevd"));
-    if (mode == RSDFT_MODE_FP64) return fp64_rotate(p, T, mb, psi, ld, hpsi, ld);
-    // the tensor-core rotation reads only the BF16 split of psi, so it can
-    // write psi itself
-    return rotate_mixed(psi, psi, ld, mb, T, mb, mode, split);
+    if (fused) return RSDFT_OK;
+    RS_CHECK(gram_schmidt_device(psi, ld, mb, mode));
+    return subspace_diag_device(psi, ld, mb, spin, esp, mode);
 }
 
 // The same step on the FP32 bands of a mixed CG sweep: FP32 H psi, BF16
@@ -577,11 +619,13 @@ int rsdft_gpu_subspace_rotv(int k, int s, double* unk, long ld, int mb, const do
     RS_CHECK(workspace_t("sub_hpsi", (size_t)ld * mb, &tmp));
     RS_CUDA(cudaMemcpy2DAsync(V, (size_t)mb * sizeof(double), vsub, (size_t)ldv * sizeof(double),
                               (size_t)mb * sizeof(double), mb, cudaMemcpyDefault, c.stream));
-    int* bad = nullptr;
-    Fp64Block p;
-    RS_CHECK(fp64_flag(&bad));
-    RS_CHECK(fp64_block(d, ld, c.ml, mb, "imma_psi", false, true, bad, &p));
-    RS_CHECK(fp64_rotate(p, V, mb, d, ld, tmp, ld));
+    RS_CHECK(with_slices([&](bool slices) {
+        int* bad = nullptr;
+        Fp64Block p;
+        RS_CHECK(fp64_flag(slices, &bad));
+        RS_CHECK(fp64_block(d, ld, c.ml, mb, "imma_psi", false, true, bad, &p));
+        return fp64_rotate(p, V, mb, d, ld, tmp, ld);
+    }));
     RS_CHECK(wf_release(unk, d, ld, mb, st));
     return RSDFT_OK;
 }
@@ -684,11 +728,13 @@ int rsdft_gpu_rotate(double* unk, long ld, long rows, int mb, const double* v, i
     RS_CUDA(cudaMemcpy2DAsync(V, (size_t)mb * sizeof(double), v, (size_t)ldv * sizeof(double),
                               (size_t)mb * sizeof(double), mb, cudaMemcpyDefault, c.stream));
     double* d = static_cast<double*>(du);
-    int* bad = nullptr;
-    Fp64Block p;
-    RS_CHECK(fp64_flag(&bad));
-    RS_CHECK(fp64_block(d, ld, rows, mb, "imma_psi", false, true, bad, &p));
-    return fp64_rotate(p, V, mb, d, ld, tmp, rows);
+    return with_slices([&](bool slices) {
+        int* bad = nullptr;
+        Fp64Block p;
+        RS_CHECK(fp64_flag(slices, &bad));
+        RS_CHECK(fp64_block(d, ld, rows, mb, "imma_psi", false, true, bad, &p));
+        return fp64_rotate(p, V, mb, d, ld, tmp, rows);
+    });
 }
 
 int rsdft_gpu_eigensolver_sweep(int k, int s, double* unk, long ld, int mb, double* esp, double* res, int ncg,

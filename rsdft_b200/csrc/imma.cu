@@ -600,12 +600,14 @@ int imma_slice(const double* A, long ld, long ml, int nb, const char* ws, bool n
     int8_t *rows = nullptr, *cols = nullptr;
     int* exps = nullptr;
     const std::string name(ws);
-    if ((need_rows && workspace_t((name + "_r").c_str(), (size_t)IM_S * nkb * nb * 64, &rows) != RSDFT_OK) ||
-        (need_cols && workspace_t((name + "_c").c_str(), (size_t)IM_S * nmb * ml * 64, &cols) != RSDFT_OK)) {
-        cudaGetLastError();
+    if ((need_rows && workspace_optional_t((name + "_r").c_str(), (size_t)IM_S * nkb * nb * 64, &rows) != RSDFT_OK) ||
+        (need_cols && workspace_optional_t((name + "_c").c_str(), (size_t)IM_S * nmb * ml * 64, &cols) != RSDFT_OK) ||
+        workspace_optional_t((name + "_e").c_str(), (size_t)nb, &exps) != RSDFT_OK) {
+        // one layout without the other is of no use
+        release_optional((name + "_r").c_str());
+        release_optional((name + "_c").c_str());
         return RSDFT_ENOMEM;
     }
-    RS_CHECK(workspace_t((name + "_e").c_str(), (size_t)nb, &exps));
     RS_CUDA(cudaMemsetAsync(exps, 0x80, sizeof(int) * nb, c.stream));
     const int sms = c.num_sms > 0 ? c.num_sms : 148;
     const int chunks = (int)std::max<long>(1, std::min<long>(div_up(ml, 4096), div_up(16L * sms, nb) + 7));
@@ -637,7 +639,7 @@ int imma_gram(const ImmaSlices& a, const ImmaSlices& b, double alpha, int symmet
     int nsplit = std::max(1, std::min(nkb, sms / g.ntiles));
     g.kb_per_split = div_up(nkb, nsplit);
     nsplit = div_up(nkb, g.kb_per_split);
-    RS_CHECK(workspace_t("imma_part", (size_t)nsplit * g.ntiles * IM_M * IM_N, &g.partial));
+    RS_CHECK(workspace_optional_t("imma_part", (size_t)nsplit * g.ntiles * IM_M * IM_N, &g.partial));
     g.bad = bad;
     g.err = c.err_flag;
     RS_CHECK(launch_imma<true>(maps, g, dim3(g.ntiles, nsplit)));
@@ -652,8 +654,8 @@ int imma_rotate(const ImmaSlices& a, const double* V, int ldv, int* bad, double*
     const int nb = a.nb, nmb = div_up(nb, 64);
     int8_t* sv = nullptr;
     double* vscale = nullptr;
-    RS_CHECK(workspace_t("imma_v", (size_t)IM_S * nmb * nb * 64, &sv));
-    RS_CHECK(workspace_t("imma_vscale", (size_t)nb, &vscale));
+    RS_CHECK(workspace_optional_t("imma_v", (size_t)IM_S * nmb * nb * 64, &sv));
+    RS_CHECK(workspace_optional_t("imma_vscale", (size_t)nb, &vscale));
     launch(k_imma_slice_v, div_up(nb, 4), 128, 0, c.stream, V, ldv, nb, nmb, a.exps, vscale, sv, bad);
     RS_LAUNCH();
     ImmaMaps maps;

@@ -23,17 +23,20 @@ bool imma_suits(long ml, int nb);
 // caller) is set when a value is not finite or out of the sliced range, or when a
 // band decays so far that its tail would lose digits: the products below then
 // leave their results to a DMMA launch conditional on it.
-// RSDFT_ENOMEM when the slices do not fit (error cleared).
+// RSDFT_ENOMEM when the slices do not fit.  All buffers are optional ones
+// (workspace_optional): the caller holds them while it uses the slices.
 int imma_slice(const double* A, long ld, long ml, int nb, const char* ws, bool need_rows, bool need_cols, int* bad,
                ImmaSlices* out);
 
 // C (nb x nb, ldc) = alpha A^T B, symmetric: only the tiles on and above the
 // diagonal are formed, symmetrize averages the 128 x 128 diagonal blocks.
+// RSDFT_ENOMEM, and nothing launched, when the partial sums do not fit.
 int imma_gram(const ImmaSlices& a, const ImmaSlices& b, double alpha, int symmetrize, const int* bad, double* C,
               long ldc);
 
 // out (ml x nb, leading dimension ld) = A V; V (nb x nb, leading dimension
-// ldv).  Reads only A's slices, so out may be A itself.
+// ldv).  Reads only A's slices, so out may be A itself.  RSDFT_ENOMEM, and
+// nothing launched, when V's slices do not fit.
 int imma_rotate(const ImmaSlices& a, const double* V, int ldv, int* bad, double* out, long ld);
 
 }  // namespace rsdft
