@@ -591,7 +591,17 @@ int launch_imma(const ImmaMaps& maps, const ImmaArgs& g, dim3 grid) {
 
 // A rotation runs over all bands in one chain, which is exact up to IM_SEG K
 // blocks; a larger set takes the DMMA form, as it did before there were slices.
-bool imma_suits(long ml, int nb) { return nb >= 96 && nb <= IM_SEG * IM_K && ml >= 4096; }
+//
+// Below, the lower end: the slicing, the reductions and the conditional launches
+// behind (40 to 60 us an operation, slices 8 us per 10^6 values) against what the
+// faster products save.  DMMA | INT8, us, Gram-Schmidt: 24^3 x 160 507 | 507, x 192
+// 591 | 568, 20^3 x 192 532 | 530, 30^3 x 128 436 | 459, x 144 602 | 561, 42^3 x 128
+// 640 | 637, 48^3 x 96 672 | 663, x 64 413 | 438; subspace_diag: 24^3 x 160 813 | 826,
+// x 192 954 | 956, x 256 1270 | 1246, 36^3 x 128 761 | 782, x 160 1074 | 1019, 48^3 x 96
+// 884 | 883.  Up to 128 bands the DMMA form has 64 x 64 tiles to match.
+bool imma_suits(long ml, int nb) {
+    return (double)ml * nb * nb >= 5e8 && (nb > 128 || (nb >= 96 && ml >= 100000)) && nb <= IM_SEG * IM_K;
+}
 
 int imma_slice(const double* A, long ld, long ml, int nb, const char* ws, bool need_rows, bool need_cols, int* bad,
                ImmaSlices* out) {

@@ -1,14 +1,23 @@
 """The FP64 products of tall blocks (Gram, rotation) and the overlap's Cholesky factor where their kernels change form:
 tile edges, remainders, the INT8-slice form against the DMMA one, and values that the slices cannot hold."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
-from rsdft_b200 import api
+from rsdft_b200 import _lib, api
 from rsdft_b200.cell import Workload, build_cell
 
 pytestmark = pytest.mark.gpu
 EPS = 2.0 ** -53
+
+
+def sliced(ml, nb):
+    """Whether the library takes the INT8 slices for a product of this size."""
+    f = getattr(_lib.load(), "_ZN5rsdft10imma_suitsEli")
+    f.restype, f.argtypes = ctypes.c_bool, [ctypes.c_long, ctypes.c_int]
+    return f(ml, nb)
 
 
 def dev(a):
@@ -37,9 +46,12 @@ def test_gram(gpu, ml, m, n, sym):
 
 @pytest.mark.parametrize("ml,nb", [
     (4096, 96), (4097, 97), (4160, 127), (5000, 128), (4159, 129), (8192, 192), (4500, 200), (4095, 96), (5000, 95),
+    (30001, 129), (13824, 191), (13000, 197), (100001, 96), (100000, 97), (100002, 127), (100063, 128), (4096, 352),
+    (29000, 192),
 ])
 def test_rotate(gpu, ml, nb):
-    """nb >= 96 and ml >= 4096 take the INT8 slices, the last two the DMMA kernel.  Bands of very different scale."""
+    """The second half of the sizes takes the INT8 slices, the others the DMMA kernel.  Bands of very different scale."""
+    assert sliced(ml, nb) == (ml * nb * nb >= 5e8)
     rng = np.random.default_rng(nb)
     u = rng.normal(size=(ml, nb)) * 10.0 ** rng.uniform(-6, 6, nb)
     u[:, nb // 2] = 0.0
@@ -50,18 +62,19 @@ def test_rotate(gpu, ml, nb):
     ref = u.astype(np.longdouble) @ v.astype(np.longdouble)
     # nb terms and additions, each within EPS of sum_m |u(i, m)| |v(m, n)|; the slices: within 2^-60 of the bands' largest
     bound = nb * EPS * (np.abs(u) @ np.abs(v))
-    if nb >= 96 and ml >= 4096:
+    if sliced(ml, nb):
         bound += nb * 2.0 ** -60 * (np.abs(u).max(0) @ np.abs(v))
     assert (np.abs(t.cpu().numpy() - ref) <= bound).all()
 
 
 @pytest.mark.parametrize("kind", ["vacuum", "slab", "localised", "one band"])
-@pytest.mark.parametrize("ml,nb", [(4096, 96), (5000, 130), (6000, 200), (4095, 96)])
+@pytest.mark.parametrize("ml,nb", [(4096, 96), (30000, 130), (13824, 200), (4096, 352), (100000, 96)])
 def test_rotate_decaying_bands(gpu, kind, ml, nb):
     """Bands that fall off by many decades keep the digits of their tails: every element within FP64's own bound."""
     rng = np.random.default_rng(nb)
     u, i, m = rng.normal(size=(ml, nb)), np.arange(ml)[:, None], np.arange(nb)[None, :]
     v = np.linalg.qr(rng.normal(size=(nb, nb)))[0]
+    assert sliced(ml, nb) == (ml * nb * nb >= 5e8)
     if kind == "vacuum":    # the whole set, along the grid
         u *= 10.0 ** (-20.0 * i / ml)
     elif kind == "slab":    # the whole set, a few points of every row of 64
@@ -82,45 +95,47 @@ def test_rotate_decaying_bands(gpu, kind, ml, nb):
 
 def test_second_block_decays(gpu):
     """subspace_diag where only H psi leaves the slices' range: both products go to the DMMA kernel."""
-    c = build_cell(Workload("sd", 1, 18, 96, 96, 0.03, 3100))
+    c = build_cell(Workload("sd", 1, 24, 192, 192, 0.03, 3100))
+    assert sliced(c.ML, 192)
     c.coef_lap[:], c.coef_lap0, c.uv[:] = 0.0, 0.0, 0.0
     c.vloc[:] = (10.0 ** (-20.0 * np.arange(c.vloc.size) / c.vloc.size)).reshape(c.vloc.shape)
     gpu.setup(c)
-    u = np.linalg.qr(np.random.default_rng(1).normal(size=(c.ML, 96)))[0] / np.sqrt(c.dV)
-    t, esp = dev(u), torch.zeros(96, dtype=torch.float64, device="cuda")
+    u = np.linalg.qr(np.random.default_rng(1).normal(size=(c.ML, 192)))[0] / np.sqrt(c.dV)
+    t, esp = dev(u), torch.zeros(192, dtype=torch.float64, device="cuda")
     gpu.subspace_diag(1, 1, t, esp)
     gpu.synchronize()
     h = u.T @ (c.vloc.reshape(-1, 1)[:c.ML] * u) * c.dV
     w, z = np.linalg.eigh(0.5 * (h + h.T))
-    assert np.abs(esp.cpu().numpy() - w).max() <= 96 * EPS * np.abs(w).max()
+    assert np.abs(esp.cpu().numpy() - w).max() <= 192 * EPS * np.abs(w).max()
     g = t.cpu().numpy()
-    assert np.abs(g.T @ g * c.dV - np.eye(96)).max() <= 1e-13
+    assert np.abs(g.T @ g * c.dV - np.eye(192)).max() <= 1e-13
     assert np.abs(np.abs((u @ z * g).sum(0) * c.dV) - 1.0).max() <= 1e-10
 
 
+@pytest.mark.parametrize("ml,nb", [(4096, 96), (4096, 352)])
 @pytest.mark.parametrize("bad", [np.nan, np.inf, 1e300, 1e-300])
-def test_rotate_out_of_range(gpu, bad):
+def test_rotate_out_of_range(gpu, bad, ml, nb):
     """A value the slices cannot hold sends the whole product to the DMMA kernel, on the device."""
     rng = np.random.default_rng(5)
-    u = rng.normal(size=(4096, 96))
+    u = rng.normal(size=(ml, nb))
     if abs(bad) < 1.0:
         u[:, 3] *= bad
     else:
         u[17, 3] = bad
-    v = rng.normal(size=(96, 96))
+    v = rng.normal(size=(nb, nb))
     t = dev(u)
     gpu.rotate(t, dev(v))
     gpu.synchronize()
     with np.errstate(all="ignore"):
         ref = u @ v
     got = t.cpu().numpy()
-    rows = np.arange(4096) != 17
-    assert np.isfinite(got[rows]).all() and np.abs(got[rows] - ref[rows]).max() <= 96 * EPS * np.abs(ref).max(where=rows[:, None], initial=0) * 8
+    rows = np.arange(ml) != 17
+    assert np.isfinite(got[rows]).all() and np.abs(got[rows] - ref[rows]).max() <= nb * EPS * np.abs(ref).max(where=rows[:, None], initial=0) * 8
     np.testing.assert_array_equal(np.isnan(got[17]), np.isnan(ref[17]))
     np.testing.assert_array_equal(np.isinf(got[17]), np.isinf(ref[17]))
 
 
-@pytest.mark.parametrize("n,nb", [(16, 96), (17, 128), (18, 131), (20, 190)])
+@pytest.mark.parametrize("n,nb", [(16, 96), (17, 128), (18, 131), (20, 190), (16, 352), (24, 191), (25, 180), (26, 200)])
 def test_gram_schmidt_slices(gpu, n, nb):
     c = build_cell(Workload("gs", 1, n, nb, nb, 0.03, 3000 + n))
     gpu.setup(c)
