@@ -19,8 +19,8 @@
 namespace rsdft {
 
 // ----------------------------------------------------------- reductions
-__global__ void k_finish(const double* __restrict__ part, int nchunk, int K, int nb, double scale,
-                         double* __restrict__ out, const int* __restrict__ active) {
+__global__ void k_finish(const double* part, int nchunk, int K, int nb, double scale,
+                         double* __restrict__ out, const int* active) {
     grid_dependency();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nb * K) return;
@@ -83,7 +83,7 @@ static HpsiSum hpsi_sum_of(const HpsiDot& d) {
 // K dot products per band among up to 4 vectors, one read of each vector.
 template <typename T, int NV, class P>
 __global__ void __launch_bounds__(VT) k_multidot(const T* v0, const T* v1, const T* v2, const T* v3, long ld,
-                                                 long n, double* __restrict__ part, const int* __restrict__ active,
+                                                 long n, double* __restrict__ part, const int* active,
                                                  int vec) {
     grid_dependency();
     constexpr int K = P::K;
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(VT) k_cg_g(CGVec<T> v, long ld, long n, const 
 // P0: Pg = g; r = g - A g; q = r; partial |r|^2  (cgpc_hprsdft_module.f90:161-175)
 template <typename T>
 __global__ void __launch_bounds__(VT) k_pc0(CGVec<T> v, long ld, long n, PcArgs pa, double* __restrict__ part,
-                                            const int* __restrict__ active) {
+                                            const int* active) {
     grid_dependency();
     __shared__ double sh[VT / 32];
     const int b = blockIdx.y;
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(VT) k_pc0(CGVec<T> v, long ld, long n, PcArgs 
 // P1: ft = A q; partial q.ft  (ft stored in hp, which is free until hpsi(p))
 template <typename T>
 __global__ void __launch_bounds__(VT) k_pc1(CGVec<T> v, long ld, long n, PcArgs pa, double* __restrict__ part,
-                                            const int* __restrict__ active) {
+                                            const int* active) {
     grid_dependency();
     __shared__ double sh[VT / 32];
     const int b = blockIdx.y;
@@ -228,8 +228,8 @@ __global__ void __launch_bounds__(VT) k_pc1(CGVec<T> v, long ld, long n, PcArgs 
 
 // P2: Pg += a q; (not last) r -= a ft; partial |r|^2
 template <typename T>
-__global__ void __launch_bounds__(VT) k_pc2(CGVec<T> v, long ld, long n, const double* __restrict__ pa_,
-                                            int last, double* __restrict__ part, const int* __restrict__ active) {
+__global__ void __launch_bounds__(VT) k_pc2(CGVec<T> v, long ld, long n, const double* pa_,
+                                            int last, double* __restrict__ part, const int* active) {
     grid_dependency();
     __shared__ double sh[VT / 32];
     const int b = blockIdx.y;
@@ -259,8 +259,8 @@ __global__ void __launch_bounds__(VT) k_pc2(CGVec<T> v, long ld, long n, const d
 
 // P3: q = r + b q
 template <typename T>
-__global__ void __launch_bounds__(VT) k_pc3(CGVec<T> v, long ld, long n, const double* __restrict__ pb_,
-                                            const int* __restrict__ active) {
+__global__ void __launch_bounds__(VT) k_pc3(CGVec<T> v, long ld, long n, const double* pb_,
+                                            const int* active) {
     grid_dependency();
     const int b = blockIdx.y;
     if (active && !active[b]) return;
@@ -276,8 +276,8 @@ __global__ void __launch_bounds__(VT) k_pc3(CGVec<T> v, long ld, long n, const d
 
 // p = Pg + bk p (icg > 1) or p = Pg (cg_module.f90:247-261)
 template <typename T>
-__global__ void __launch_bounds__(VT) k_cg_p(CGVec<T> v, long ld, long n, const double* __restrict__ bk_,
-                                             int first, const int* __restrict__ active) {
+__global__ void __launch_bounds__(VT) k_cg_p(CGVec<T> v, long ld, long n, const double* bk_,
+                                             int first, const int* active) {
     grid_dependency();
     const int b = blockIdx.y;
     if (active && !active[b]) return;
@@ -610,8 +610,8 @@ __global__ void k_convert(const double* __restrict__ a, T* __restrict__ b, long 
 }
 
 // sum_i (hx - e x)^2 per band (residual norms after the eigenvalues are known)
-__global__ void __launch_bounds__(VT) k_resid(const double* __restrict__ x, const double* __restrict__ hx, long ld,
-                                              long n, const double* __restrict__ e, double* __restrict__ part) {
+__global__ void __launch_bounds__(VT) k_resid(const double* x, const double* hx, long ld,
+                                              long n, const double* e, double* __restrict__ part) {
     grid_dependency();
     __shared__ double sh[VT / 32];
     const int b = blockIdx.y;
@@ -654,7 +654,7 @@ int esp_device(const double* x, long ld, int nb, int spin, double* e, double* re
     RS_CHECK(workspace_t("esp_dot", (size_t)nb * dot.cap, &dot.part));
     RS_CHECK(hpsi_device<double>(x, hx, ld, nb, spin, nullptr, &dot));
     const dim3 vg(nchunk, nb);
-    launch_dependent(s_esp, div_up(nb, SB / 32), SB, 0, st, hpsi_sum_of(dot), nb, e);
+    launch(s_esp, div_up(nb, SB / 32), SB, 0, st, hpsi_sum_of(dot), nb, e);
     if (res) {
         launch(k_resid, vg, VT, 0, st, x, hx, ld, n, e, part);
         launch(k_finish, div_up(nb, 128), 128, 0, st, part, nchunk, 1, nb, c.dV, res, nullptr);
@@ -724,9 +724,9 @@ static int cg_run(T* x, long ld, int mb, int spin, double* esp, double* res, int
     };
 
     RS_CHECK(hpsi_device<T>(x, v.hx, ld, mb, spin, nullptr, &hd));
-    launch_dependent(s_start, wb, SB, 0, st, s, hpsi_sum_of(hd), mb);
-    launch_dependent(full ? k_cg_g<T, 32> : k_cg_g<T, 0>, vg, VT, 0, st, v, ld, n, s.E, part, gv);
-    launch_dependent(s_step, wb, SB, 0, st, s, (const double*)part, nchunk, dV, mb, 1, ncg == 0, tol, esp, res);
+    launch(s_start, wb, SB, 0, st, s, hpsi_sum_of(hd), mb);
+    launch(full ? k_cg_g<T, 32> : k_cg_g<T, 0>, vg, VT, 0, st, v, ld, n, s.E, part, gv);
+    launch(s_step, wb, SB, 0, st, s, (const double*)part, nchunk, dV, mb, 1, ncg == 0, tol, esp, res);
     RS_LAUNCH();
 
     const bool sstep = ipc == 4 && mloop >= 1 && mloop <= SS_MAXM;
@@ -769,17 +769,17 @@ static int cg_run(T* x, long ld, int mb, int spin, double* esp, double* res, int
             RS_LAUNCH();
         }
         RS_CHECK(hpsi_device<T>(v.p, v.hp, ld, mb, spin, s.active, &hd));
-        launch_dependent(s_eig<T>, wb, SB, 0, st, s, (const double*)pdots, nchunk, hpsi_sum_of(hd), mb, icg == 1);
-        launch_dependent(icg == 1 ? (full ? k_cg_upd1<T, true, 32> : k_cg_upd1<T, true, 0>)
+        launch(s_eig<T>, wb, SB, 0, st, s, (const double*)pdots, nchunk, hpsi_sum_of(hd), mb, icg == 1);
+        launch(icg == 1 ? (full ? k_cg_upd1<T, true, 32> : k_cg_upd1<T, true, 0>)
                         : (full ? k_cg_upd1<T, false, 32> : k_cg_upd1<T, false, 0>),
                vg, VT, 0, st, v, ld, n, s, part, s.active, gv);
-        launch_dependent(s_step, wb, SB, 0, st, s, (const double*)part, nchunk, dV, mb, 0, icg == ncg, tol, esp, res);
+        launch(s_step, wb, SB, 0, st, s, (const double*)part, nchunk, dV, mb, 0, icg == ncg, tol, esp, res);
         if (!sstep) launch(k_cg_upd2<T>, vg, VT, 0, st, v, ld, n, s, gv);
         RS_LAUNCH();
     }
     T* hx = hx_out && ncg > 0 ? v.hx : nullptr;
     if (hx_out) *hx_out = v.hx;
-    launch_dependent(full ? k_cg_end<T, 32> : k_cg_end<T, 0>, vg, VT, 0, st, v, ld, n, s, sstep ? 1 : 0, hx, out64, gv);
+    launch(full ? k_cg_end<T, 32> : k_cg_end<T, 0>, vg, VT, 0, st, v, ld, n, s, sstep ? 1 : 0, hx, out64, gv);
     RS_LAUNCH();
     return RSDFT_OK;
 }
@@ -802,7 +802,7 @@ int cg_device_f32(const double* unk, long ld, int mb, int spin, double* esp, dou
     float* x32 = nullptr;
     const long n = ld * (long)mb;
     RS_CHECK(workspace_t("cg_x32", (size_t)n, &x32));
-    launch(k_convert<float>, 4 * c.num_sms, 256, 0, c.stream, unk, x32, n);
+    launch_ordinary(k_convert<float>, 4 * c.num_sms, 256, 0, c.stream, unk, x32, n);
     RS_LAUNCH();
     RS_CHECK(cg_run<float>(x32, ld, mb, spin, esp, res, ncg, mloop, ipc, hx_out));
     *x32_out = x32;
@@ -814,7 +814,7 @@ int cg_device_f32(const double* unk, long ld, int mb, int spin, double* esp, dou
     return RSDFT_OK;
 }
 
-__global__ void k_or_flag(int* __restrict__ dst, const int* __restrict__ src) {
+__global__ void k_or_flag(int* __restrict__ dst, const int* src) {
     grid_dependency();
     if (*src) *dst = 1;
 }
@@ -843,7 +843,7 @@ int cg_device_f32_staged(const double* unk_host, double* unk_dev, long ld, int m
         const long n = ld * (long)nb;
         RS_CUDA(cudaStreamWaitEvent(c.stream, c.ev[k], 0));
         float* xb = x32 + (size_t)b0 * ld;
-        launch(k_convert<float>, 4 * c.num_sms, 256, 0, c.stream, (const double*)(unk_dev + (size_t)b0 * ld), xb, n);
+        launch_ordinary(k_convert<float>, 4 * c.num_sms, 256, 0, c.stream, (const double*)(unk_dev + (size_t)b0 * ld), xb, n);
         RS_LAUNCH();
         const float* hx = nullptr;
         RS_CHECK(cg_run<float>(xb, ld, nb, spin, esp + b0, res + b0, ncg, mloop, ipc, &hx, nullptr, mb));
@@ -878,7 +878,7 @@ int cg_device(double* unk, long ld, int mb, int spin, double* esp, double* res, 
     float* x32 = nullptr;
     const long n = ld * (long)mb;
     RS_CHECK(workspace_t("cg_x32", (size_t)n, &x32));
-    launch(k_convert<float>, 4 * c.num_sms, 256, 0, c.stream, unk, x32, n);
+    launch_ordinary(k_convert<float>, 4 * c.num_sms, 256, 0, c.stream, unk, x32, n);
     RS_LAUNCH();
     return cg_run<float>(x32, ld, mb, spin, esp, res, ncg, mloop, ipc, nullptr, unk);
 }

@@ -199,13 +199,15 @@ extern long long g_kernel_launches;
 // it wrote is visible, then let the next one be set up.  An ordinary launch
 // does not overlap its predecessor at all and the wait is over at once.
 //
-// A dependent launch (launch_dependent) is set up while the kernel before it
-// runs, so its lifetime overlaps that one kernel's, and no other's, since the
-// kernel before lets it in only after its own wait.  What the kernel before
-// writes is thus not read-only for the dependent's lifetime: it must not read
-// that through the non-coherent path (const __restrict__ parameters, __ldg),
-// which neither the wait nor its memory clobber orders.  Struct members and
-// plain pointers are read coherently; TMA loads come after the wait.
+// A dependent launch (launch) is set up while the kernel before it runs, so its
+// lifetime overlaps that one kernel's, and no other's, since the kernel before
+// lets it in only after its own wait.  What the kernel before writes is thus
+// not read-only for the dependent's lifetime: it must not read that through the
+// non-coherent path (const __restrict__ parameters, __ldg), which neither the
+// wait nor its memory clobber orders.  That path is for the cell's tables, which
+// their set-up calls upload before they return; what kernels write is read
+// through plain pointers and struct members, and by TMA and cp.async after the
+// wait.
 __device__ __forceinline__ void grid_dependency() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -234,24 +236,24 @@ inline void launch_as(bool dependent, void (*kernel)(KArgs...), dim3 grid, dim3 
     (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-// Launch one of this library's kernels and count it (errors: RS_LAUNCH).
+// Launch one of this library's kernels and count it (errors: RS_LAUNCH), as a
+// programmatic dependent of the launch before it where it has up to 512 CTAs
+// (iteration of 24^3 x 32, about 90 launches: 727 us without dependents, 658 with;
+// CG of 48^3 x 160: 3615 and 3598).  Above that an ordinary launch: waiting CTAs
+// crowd the SMs that drain first (72^3 x 480 CG sweep with every launch a
+// dependent: 19.8 ms against 18.6).
 template <typename... KArgs, typename... Args>
 inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
-    launch_as(false, kernel, grid, block, smem, st, std::forward<Args>(args)...);
+    launch_as(true, kernel, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
-// The same as a programmatic dependent of the launch before it, for kernels
-// that read what that one writes coherently (above), in chains of short
-// kernels, where the launch latency is what there is to save.  Above 512 CTAs
-// an ordinary launch: the waiting CTAs would crowd the SMs that drain first
-// (72^3 x 480 CG sweep with every launch a dependent: 19.8 ms against 18.6).  Not
-// behind long kernels of few CTAs either, whose L1 a waiting CTA's shared memory
-// takes away: 128^3 x 1 band in a cell of 8 wide spheres, the H psi stencil
-// waiting for the projection, 688 us against 569.
+// The same, after the kernel before it has ended: for kernels that read its
+// output through the non-coherent path, or that must not wait beside it
+// (stencil_dependent in hpsi.cu).
 template <typename... KArgs, typename... Args>
-inline void launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                             Args&&... args) {
-    launch_as(true, kernel, grid, block, smem, st, std::forward<Args>(args)...);
+inline void launch_ordinary(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                            Args&&... args) {
+    launch_as(false, kernel, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
 int require_init();

@@ -43,7 +43,7 @@ __global__ void k_widen(const float* __restrict__ a, double* __restrict__ b, lon
 }
 
 // C = alpha * sum_c P[c] (sym: alpha/2 (G + G^T)), fixed summation order
-__global__ void k_reduce_partials(const double* __restrict__ P, int nch, int m, int n, double alpha, int sym,
+__global__ void k_reduce_partials(const double* P, int nch, int m, int n, double alpha, int sym,
                                   double* __restrict__ C) {
     grid_dependency();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -124,8 +124,8 @@ static int fp64_gram(const Fp64Block& a, const Fp64Block& b, double alpha, int s
     return dmma_gram(a.x, b.x, a.ld, a.ml, a.nb, a.nb, alpha, symmetrize, C, a.nb, true, bad);
 }
 
-__global__ void k_copy_cols_if(const double* __restrict__ src, long lds, double* __restrict__ dst, long ldd, long n,
-                               int nb, const int* __restrict__ flag) {
+__global__ void k_copy_cols_if(const double* src, long lds, double* __restrict__ dst, long ldd, long n,
+                               int nb, const int* flag) {
     grid_dependency();
     if (!*flag) return;
     for (int b = blockIdx.y; b < nb; b += gridDim.y)
@@ -205,7 +205,7 @@ static int read_cholesky(const int* dinfo, const double* mm, double* hmm, const 
 // diagonal is positive.
 constexpr int TI_W = 4;  // rows (warps) per CTA
 
-__global__ void __launch_bounds__(32 * TI_W) k_trtri_rows(const double* __restrict__ R, int n,
+__global__ void __launch_bounds__(32 * TI_W) k_trtri_rows(const double* R, int n,
                                                          double* __restrict__ X) {
     grid_dependency();
     extern __shared__ double ti_sm[];
@@ -350,7 +350,7 @@ static int rr_reduced(const double* Rinv, double* H, double* T, int mb, double* 
 }
 
 // min and max of the diagonal of an n x n matrix (one block)
-__global__ void k_diag_minmax(const double* __restrict__ a, int n, int lda, double* __restrict__ out) {
+__global__ void k_diag_minmax(const double* a, int n, int lda, double* __restrict__ out) {
     grid_dependency();
     __shared__ double smin[256], smax[256];
     double lo = 1e300, hi = 0.0;
@@ -483,7 +483,7 @@ int orth_subspace_diag_f32(const float* x32, const float* hx, double* psi, long 
     double hmm[2] = {0.0, 0.0};
     RS_CHECK(read_cholesky(dinfo, mm, hmm, "eigensolver_sweep: overlap Cholesky"));
     if (!(hmm[0] > 0.0) || (hmm[1] / hmm[0]) * (hmm[1] / hmm[0]) > fused_rr_kappa_max(mode)) {
-        launch(k_widen, 4 * c.num_sms, 256, 0, c.stream, x32, psi, ld * (long)mb);
+        launch_ordinary(k_widen, 4 * c.num_sms, 256, 0, c.stream, x32, psi, ld * (long)mb);
         RS_LAUNCH();
         RS_CHECK(gram_schmidt_device(psi, ld, mb, mode));
         return subspace_diag_device(psi, ld, mb, spin, esp, mode);

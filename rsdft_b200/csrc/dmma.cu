@@ -235,9 +235,9 @@ __global__ void __launch_bounds__(32 * WM * WN, CPS) k_dmma(DmmaArgs g) {
 // thread added 296 splits by itself with its neighbours a tile row apart,
 // about 5 us this way).
 template <int BT>
-__global__ void __launch_bounds__(1024) k_dmma_reduce(const double* __restrict__ P, int nsplit, int ntiles, int ntm,
+__global__ void __launch_bounds__(1024) k_dmma_reduce(const double* P, int nsplit, int ntiles, int ntm,
                                                       int sym, int m, int n, double alpha, int symmetrize,
-                                                      double* __restrict__ C, long ldc, const int* __restrict__ only_if) {
+                                                      double* __restrict__ C, long ldc, const int* only_if) {
     grid_dependency();
     __shared__ double sh[2][32][33];
     if (only_if && !*only_if) return;

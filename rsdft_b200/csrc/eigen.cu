@@ -416,8 +416,8 @@ constexpr int BS_PTS = 4;  // trial points per lane (independent Sturm chains)
 // trial points per round, each counted with dlaebz's Sturm recurrence
 // q_i = d_i - x - e_{i-1}^2 / q_{i-1} (eigenvalues below x = negative q,
 // |q| <= pivmin replaced by -pivmin); aux[0] = |T|_1
-__global__ void __launch_bounds__(32 * BS_WARPS) k_tri_bisect(const double* __restrict__ d,
-                                                             const double* __restrict__ e, int n,
+__global__ void __launch_bounds__(32 * BS_WARPS) k_tri_bisect(const double* d,
+                                                             const double* e, int n,
                                                              double* __restrict__ w, double* __restrict__ aux) {
     grid_dependency();
     extern __shared__ double bsh[];
@@ -523,10 +523,10 @@ __device__ __forceinline__ double start_entry(int j, int i) {
 constexpr int IV_RPL = 20;  // rows per lane: n <= 640
 constexpr int IV_WARPS = 4;
 
-__global__ void __launch_bounds__(32 * IV_WARPS) k_tri_invit(const double* __restrict__ d,
-                                                            const double* __restrict__ e,
-                                                            const double* __restrict__ w,
-                                                            const double* __restrict__ aux, int n,
+__global__ void __launch_bounds__(32 * IV_WARPS) k_tri_invit(const double* d,
+                                                            const double* e,
+                                                            const double* w,
+                                                            const double* aux, int n,
                                                             double* __restrict__ Z, int ldz) {
     grid_dependency();
     extern __shared__ double ish[];  // d, e of T for the block's warps

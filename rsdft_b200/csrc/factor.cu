@@ -54,7 +54,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_al
 constexpr int TR_W = 8;  // rows of X (one per warp) per CTA
 constexpr int TR_G = 8;  // columns per reduction group
 
-__global__ void __launch_bounds__(32 * TR_W) k_trtri(const double* __restrict__ R, int n, int cwmax,
+__global__ void __launch_bounds__(32 * TR_W) k_trtri(const double* R, int n, int cwmax,
                                                      double* __restrict__ X) {
     grid_dependency();
     extern __shared__ double tr_sm[];
@@ -228,7 +228,7 @@ __device__ void chol_publish(double* sA, int n, int t, bool want_inv, double* __
 }
 
 // step -1: the first diagonal tile
-__global__ void __launch_bounds__(CH_T) k_chol_first(const double* __restrict__ S, int n, double* __restrict__ Rb,
+__global__ void __launch_bounds__(CH_T) k_chol_first(const double* S, int n, double* __restrict__ Rb,
                                                      double* __restrict__ xg, int* __restrict__ info,
                                                      int* __restrict__ fail) {
     grid_dependency();
@@ -247,8 +247,8 @@ __global__ void __launch_bounds__(CH_T) k_chol_first(const double* __restrict__ 
 // X = R(k, k)^-1 (xin), writes R(k, i) to Rb when i == j, and subtracts
 // R(k, i)^T R(k, j) from S(i, j); the CTA of (k+1, k+1) keeps the updated
 // tile, factors it and publishes R(k+1, k+1) and its inverse (xout).
-__global__ void __launch_bounds__(CH_T) k_chol_step(double* __restrict__ S, int n, int k, double* __restrict__ Rb,
-                                                    const double* __restrict__ xin, double* __restrict__ xout,
+__global__ void __launch_bounds__(CH_T) k_chol_step(double* S, int n, int k, double* __restrict__ Rb,
+                                                    const double* xin, double* __restrict__ xout,
                                                     int* __restrict__ info, int* __restrict__ fail) {
     grid_dependency();
     __shared__ double sX[32 * CF_P], sA[32 * CF_P], sB[32 * CF_P], sC[32 * CF_P];
@@ -317,8 +317,8 @@ __global__ void __launch_bounds__(CH_T) k_chol_step(double* __restrict__ S, int 
 
 // R (the upper triangle of Rb) into S; the strictly lower triangle of S is
 // left as it was
-__global__ void k_chol_copy(double* __restrict__ S, int n, const double* __restrict__ Rb,
-                            const int* __restrict__ fail) {
+__global__ void k_chol_copy(double* __restrict__ S, int n, const double* Rb,
+                            const int* fail) {
     grid_dependency();
     if (*fail) return;
     const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -358,7 +358,7 @@ int potrf_upper_device(double* S, int n, int* dinfo) {
 // reflectors): G = V^T V over the block's rows j0+1 .. n-1, then dlarft's
 // recurrence T(j, j) = tau_j, T(i, j) = -tau_j sum_{i <= l < j} T(i, l)
 // G(l, j).
-__global__ void __launch_bounds__(256) k_larft(const double* __restrict__ Q, int n, const double* __restrict__ tau,
+__global__ void __launch_bounds__(256) k_larft(const double* Q, int n, const double* tau,
                                                double* __restrict__ T) {
     grid_dependency();
     __shared__ double sV[64 * CF_P], sG[32 * CF_P], sT[32 * CF_P];
@@ -407,8 +407,8 @@ constexpr int OW = 8;  // columns of C (one per warp) per CTA of k_apply_wy
 
 // dynamic shared memory: the block's V (32 columns, pitch n) and the CTA's
 // columns of C (n each)
-__global__ void __launch_bounds__(32 * OW) k_apply_wy(const double* __restrict__ Q, int n,
-                                                      const double* __restrict__ T, double* __restrict__ C,
+__global__ void __launch_bounds__(32 * OW) k_apply_wy(const double* Q, int n,
+                                                      const double* T, double* C,
                                                       int ldc) {
     grid_dependency();
     extern __shared__ double ow_sm[];

@@ -34,8 +34,8 @@ constexpr int FG_CH = 512;    // sphere points staged at a time
 
 // part[chunk][lma * 3 + k] = the chunk's band sum of each projector
 template <bool CHI>
-__global__ void __launch_bounds__(FW * 32) k_nl_grad(const double* __restrict__ psi, const double* __restrict__ chi,
-                                                     long ld, int nb, const double* __restrict__ occ, double cscale,
+__global__ void __launch_bounds__(FW * 32) k_nl_grad(const double* psi, const double* chi,
+                                                     long ld, int nb, const double* occ, double cscale,
                                                      const int* __restrict__ grp_lma0, const int* __restrict__ grp_cnt,
                                                      const int* __restrict__ lma_ptr, const int* __restrict__ jjp,
                                                      const double* __restrict__ uv, const double* __restrict__ duv,
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(FW * 32) k_nl_grad(const double* __restrict__ 
                 const bool in = RS_DCHECK(jj >= 0 && jj < ld, CK_NL_GRAD_POINT, jj, err);
                 double x[2];
 #pragma unroll
-                for (int w = 0; w < 2; ++w) x[w] = act[w] && in ? __ldg(v[w] + jj) : 0.0;
+                for (int w = 0; w < 2; ++w) x[w] = act[w] && in ? v[w][jj] : 0.0;
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     const double u = s_c[i][j];
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(FW * 32) k_nl_grad(const double* __restrict__ 
 
 // f(3 a + k): the projectors of atom a in order, each over its band chunks in
 // order; one warp per atom component (the lanes take the chunks)
-__global__ void k_atom_sum(const double* __restrict__ part, int nchunk, int nzlma, const int* __restrict__ atom_ptr,
+__global__ void k_atom_sum(const double* part, int nchunk, int nzlma, const int* __restrict__ atom_ptr,
                            const int* __restrict__ atom_lma, int natom, double* __restrict__ f) {
     grid_dependency();
     const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -167,8 +167,8 @@ __global__ void k_atom_sum(const double* __restrict__ part, int nchunk, int nzlm
 constexpr int VA_LIST = 1024;  // bands listed at a time
 
 template <int W, bool CHI>
-__global__ void __launch_bounds__(256) k_vloc_adjoint(const double* __restrict__ psi, const double* __restrict__ chi,
-                                                      long ld, int nb, const double* __restrict__ occ, double dV,
+__global__ void __launch_bounds__(256) k_vloc_adjoint(const double* psi, const double* chi,
+                                                      long ld, int nb, const double* occ, double dV,
                                                       long n, double* __restrict__ out) {
     grid_dependency();
     __shared__ int s_b[VA_LIST];
@@ -182,11 +182,11 @@ __global__ void __launch_bounds__(256) k_vloc_adjoint(const double* __restrict__
     for (int e = 0; e < W; ++e) s[e] = 0.0;
     auto load = [](const double* p, double (&v)[W]) {
         if constexpr (W == 2) {
-            const double2 t = __ldg(reinterpret_cast<const double2*>(p));
+            const double2 t = *reinterpret_cast<const double2*>(p);
             v[0] = t.x;
             v[1] = t.y;
         } else {
-            v[0] = __ldg(p);
+            v[0] = *p;
         }
     };
     for (int b0 = 0; b0 < nb; b0 += VA_LIST) {

@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(256) k_nl_project(const T* __restrict__ psi, l
                                                     const double* __restrict__ uv,
                                                     const int* __restrict__ iuv, double dV,
                                                     double* __restrict__ uvunk, int nzlma,
-                                                    const int* __restrict__ band_active, int* __restrict__ err) {
+                                                    const int* band_active, int* __restrict__ err) {
     grid_dependency();
     __shared__ int s_j[PJ_CH];
     __shared__ double s_u[4][PJ_CH];
@@ -120,7 +120,7 @@ template <typename T>
 static int launch_project(const T* psi, long ld, int nb, double* uvunk, const int* band_active, cudaStream_t st) {
     const Context& c = ctx();
     dim3 grid(c.ngroup, div_up(nb, PJ_WARPS * PJ_BW));
-    launch(k_nl_project<T>, grid, 256, 0, st, psi, ld, nb, c.grp_lma0, c.grp_cnt, c.lma_ptr, c.jjp, c.uv, c.iuv,
+    launch_ordinary(k_nl_project<T>, grid, 256, 0, st, psi, ld, nb, c.grp_lma0, c.grp_cnt, c.lma_ptr, c.jjp, c.uv, c.iuv,
            c.dV, uvunk, c.nzlma, band_active, c.err_flag);
     RS_LAUNCH();
     return RSDFT_OK;
@@ -868,7 +868,7 @@ static int scatter_chunk(int nb) {
 // Whether the stencil is launched as a dependent of the projection (of which
 // it reads nothing): where the spheres are of ordinary size, so that the
 // projection is short.  Behind a long one the waiting stencil CTAs' shared memory
-// costs it its L1 (launch_dependent).  24^3 x 32, about 500 points per sphere:
+// costs it its L1.  24^3 x 32, about 500 points per sphere:
 // 24.6 us without; 256^3 x 1 band in an 8-atom cell, 57,000 points: 6070 us
 // without, 6580 with.
 static bool stencil_dependent() {
@@ -879,7 +879,7 @@ static bool stencil_dependent() {
 template <typename T, int MD, int TX>
 static void launch_stencil_tx(const StencilArgs<T>& a, const StencilCoef& cf, int nb, cudaStream_t st) {
     dim3 grid(div_up(a.n1, TX), div_up(a.n2, 16), nb * a.nzc);
-    launch(k_stencil<T, MD, TX>, grid, TX * 16, 0, st, a, cf);
+    launch_ordinary(k_stencil<T, MD, TX>, grid, TX * 16, 0, st, a, cf);
 }
 
 template <typename T, int MD>
@@ -1101,7 +1101,7 @@ static int launch_stencil_md2(StencilArgs<T> a, const StencilCoef& cf, int nb, c
         if (a.gpt_ptr && c.nl_npt > 0) {
             const int bch = scatter_chunk(nb);
             dim3 grid(div_up(c.nl_npt, 128), div_up(nb, bch));
-            launch_dependent(k_nl_scatter<T>, grid, 128, 0, st, a.hpsi, a.ld, nb, bch, (const int*)c.nl_pts,
+            launch(k_nl_scatter<T>, grid, 128, 0, st, a.hpsi, a.ld, nb, bch, (const int*)c.nl_pts,
                    (const int*)c.nl_ptr, c.nl_npt, a.gpt_grp, a.gpt_uv4, a.uvunk, a.nzlma, a.band_active,
                    c.err_flag);
             RS_LAUNCH();
@@ -1326,7 +1326,7 @@ extern "C" int rsdft_gpu_op_nonlocal_add(const double* uvunk, double* htpsi, lon
     RS_CHECK(wf_acquire(htpsi, ld, nb, "ham_out", &dh, &sh));
     const int bch = scatter_chunk(nb);
     dim3 grid(div_up(c.nl_npt, 128), div_up(nb, bch));
-    launch(k_nl_scatter<double>, grid, 128, 0, c.stream, dh, ld, nb, bch, (const int*)c.nl_pts, (const int*)c.nl_ptr,
+    launch_ordinary(k_nl_scatter<double>, grid, 128, 0, c.stream, dh, ld, nb, bch, (const int*)c.nl_pts, (const int*)c.nl_ptr,
            c.nl_npt, (const int*)c.gpt_grp, (const double*)c.gpt_uv4, (const double*)du, c.nzlma, (const int*)nullptr,
            c.err_flag);
     RS_LAUNCH();

@@ -72,7 +72,7 @@ __device__ __forceinline__ void split_tf32(double x, uint32_t& h, uint32_t& l) {
 // TF32 versions of the three split kernels below: two slices of 4-byte
 // values in the same layouts
 template <typename TI>
-__global__ void __launch_bounds__(256) k_split_cols_tf32(const TI* __restrict__ psi, long ld, int nb, long ml,
+__global__ void __launch_bounds__(256) k_split_cols_tf32(const TI* psi, long ld, int nb, long ml,
                                                          uint32_t* __restrict__ out) {
     grid_dependency();
     const long n = ml * nb;
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(256) k_split_cols_tf32(const TI* __restrict__ 
 }
 
 template <typename TI>
-__global__ void k_split_rows_tf32(const TI* __restrict__ psi, long ld, int nb, long ml, int mbk,
+__global__ void k_split_rows_tf32(const TI* psi, long ld, int nb, long ml, int mbk,
                                   uint32_t* __restrict__ out) {
     grid_dependency();
     __shared__ double tile[32][33];
@@ -117,7 +117,7 @@ __global__ void k_split_rows_tf32(const TI* __restrict__ psi, long ld, int nb, l
     }
 }
 
-__global__ void k_split_small_tf32(const double* __restrict__ V, int mb, int ldv, int mbk, uint32_t* __restrict__ out) {
+__global__ void k_split_small_tf32(const double* V, int mb, int ldv, int mbk, uint32_t* __restrict__ out) {
     grid_dependency();
     const long n = (long)mb * mbk;
     for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
@@ -142,7 +142,7 @@ constexpr int SPC_KB = 8;  // K blocks (warps) per CTA
 constexpr int SPC_B = 8;   // bands per warp
 
 template <typename TI>
-__global__ void __launch_bounds__(32 * SPC_KB) k_split_cols(const TI* __restrict__ psi, long ld, int nb, long ml,
+__global__ void __launch_bounds__(32 * SPC_KB) k_split_cols(const TI* psi, long ld, int nb, long ml,
                                                            int nkb, __nv_bfloat16* __restrict__ out, int vec) {
     grid_dependency();
     const int lane = threadIdx.x & 31;
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(32 * SPC_KB) k_split_cols(const TI* __restrict
 }
 
 // slices[s][n][m] = term s of V(m, n) (V column-major mb x mb), padded to mbk
-__global__ void k_split_small(const double* __restrict__ V, int mb, int ldv, int mbk, __nv_bfloat16* __restrict__ out) {
+__global__ void k_split_small(const double* V, int mb, int ldv, int mbk, __nv_bfloat16* __restrict__ out) {
     grid_dependency();
     const long n = (long)mb * mbk;
     for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_umma(const __grid_constant__ U
 
 // C(i, j) = alpha * sum_split P (sym: symmetric part); tiles with tm > tn of a
 // symmetric product are read transposed from tile (tn, tm)
-__global__ void k_reduce_tiles(const double* __restrict__ P, int nsplit, int npairs, int ntm, int sym, int bn, int m,
+__global__ void k_reduce_tiles(const double* P, int nsplit, int npairs, int ntm, int sym, int bn, int m,
                                double alpha, int symmetrize, double* __restrict__ C) {
     grid_dependency();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;

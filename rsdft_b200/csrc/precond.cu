@@ -18,8 +18,8 @@ namespace rsdft {
 // and, with D = 3 (K >= 2), <w_K, w_{K-2}>; D = 1 (K = mloop), only
 // <S w_{K-1}, w_{K-1}> with S = B for K = 1 and 2 B above.
 template <typename T, int K, int D>
-__global__ void __launch_bounds__(VT) k_ss_basis(const T* __restrict__ g, SSVec<T> sv, long ld, long n, PcArgs pa,
-                                                 double* __restrict__ part, const int* __restrict__ active) {
+__global__ void __launch_bounds__(VT) k_ss_basis(const T* g, SSVec<T> sv, long ld, long n, PcArgs pa,
+                                                 double* __restrict__ part, const int* active) {
     grid_dependency();
     constexpr bool STORE = D > 1;
     __shared__ double sh[D * (VT / 32)];
@@ -664,7 +664,7 @@ static int pc_tma_step(const T* src, const T* const* aux, T* wout, const PcArgs&
     cf.cy[0] = sc * pa.c2;
     cf.cz[0] = sc * pa.c3;
     dim3 grid(n2 / g.TY, (unsigned)(mb * nzc));
-    launch_dependent(k_pc_tma<T, K, D>, grid, g.threads, g.smem, c.stream, maps, wout, cf, n1, n2, n3, ld, zlen, nzc,
+    launch(k_pc_tma<T, K, D>, grid, g.threads, g.smem, c.stream, maps, wout, cf, n1, n2, n3, ld, zlen, nzc,
            g.TY, g.RS, g.S, g.ncw, part, active, c.err_flag);
     RS_LAUNCH();
     *nchunk = (n2 / g.TY) * nzc;
@@ -731,8 +731,8 @@ int sstep_precond(const T* g, const T* hx, const SSVec<T>& sv, T* p, T* x, long 
     const int gv = grp16_ok<T>(ld, {g, hx, p, x, sv.w[0], sv.w[1], sv.w[2], sv.w[3]}) ? 1 : 0;
     auto launch_p = [&](auto M) {
         constexpr int MM = decltype(M)::value;
-        launch_dependent(s_sstep<MM>, div_up(mb, 4), 128, 0, st, s, pt, cz, mb, pa.d, dV, hx ? 1 : 0);
-        launch_dependent(vec_full(n, nchunk) ? k_ss_p<T, MM, 32> : k_ss_p<T, MM, 0>, vg, VT, 0, st, g, hx, sv, p, x, ld, n, (const double*)cz,
+        launch(s_sstep<MM>, div_up(mb, 4), 128, 0, st, s, pt, cz, mb, pa.d, dV, hx ? 1 : 0);
+        launch(vec_full(n, nchunk) ? k_ss_p<T, MM, 32> : k_ss_p<T, MM, 0>, vg, VT, 0, st, g, hx, sv, p, x, ld, n, (const double*)cz,
                (const double*)s.bk, (const int*)s.active, (const int*)(hx ? nullptr : s.pend),
                (const double*)s.u11, (const double*)s.u21, dots, gv);
     };

@@ -32,7 +32,7 @@ __global__ void k_wait_for_nothing(long long cycles, int* __restrict__ err) {
 #ifdef RSDFT_GPU_CHECK
 // Reads buf[i] only where the debug build's index check passes; i = n is
 // out of range, so the check records itself and the read is skipped.
-__global__ void k_check_probe(const double* __restrict__ buf, int n, int i, double* __restrict__ out,
+__global__ void k_check_probe(const double* buf, int n, int i, double* __restrict__ out,
                               int* __restrict__ err) {
     grid_dependency();
     double v = 0.0;

@@ -119,7 +119,7 @@ __device__ double fermi_bisect(const double* esp, double* occ, int mb, int s0, i
 // mb2 = MB): one bisection over all spins (MSP = 1, or iter > nfixed), else
 // one per spin with the fixed moment dspn; occ = 2 ff / MSP.  out[0] = ef,
 // out[1] = 1 if the electron count was matched.
-__global__ void __launch_bounds__(FM_T) k_calc_fermi(const double* __restrict__ esp, double* __restrict__ occ, int mb,
+__global__ void __launch_bounds__(FM_T) k_calc_fermi(const double* esp, double* occ, int mb,
                                                      int msp, double znel, double dspn, int fixed, double ekbt,
                                                      int kinteg, double* __restrict__ out) {
     grid_dependency();
@@ -144,8 +144,8 @@ __global__ void __launch_bounds__(FM_T) k_calc_fermi(const double* __restrict__ 
 // conv_check_2/3 (sweep_module.f90:255-280): the largest |esp - esp0| over
 // bands 1..mb_ref of every spin; mode 3 also writes res = |esp - esp0|, with
 // -1 where it is below tol.
-__global__ void __launch_bounds__(FM_T) k_conv_check(const double* __restrict__ esp, const double* __restrict__ esp0,
-                                                     double* __restrict__ res, int mb, int msp, int mb_ref, int mode,
+__global__ void __launch_bounds__(FM_T) k_conv_check(const double* esp, const double* esp0,
+                                                     double* res, int mb, int msp, int mb_ref, int mode,
                                                      double tol, double* __restrict__ out) {
     grid_dependency();
     __shared__ double sh[FM_T / 32 + 1];

@@ -1,20 +1,21 @@
 """The rules that programmatic dependent launches rest on, read off the CUDA sources (common.cuh, grid_dependency): every
-kernel waits for its predecessor first and lets its successor in only then, only launch_dependent makes a dependent, and a
-kernel launched that way reads what its predecessor writes coherently, that is not through const __restrict__ parameters
-or __ldg."""
+kernel waits for its predecessor first and lets its successor in only then, launches go through launch_as, and a kernel
+that may be a dependent reads only the cell's tables, and what its predecessor does not write, through const
+__restrict__ parameters or __ldg."""
 import glob
 import os
 import re
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "rsdft_b200", "csrc")
 
-# const __restrict__ parameters of dependents, none written by the launch before: k_ss_p follows s_sstep, which writes
-# per-band scalars (g and hx come from the line step before); k_nl_scatter follows the stencil, which writes H psi (the
-# tables are the cell's, uVunk the projection's, the band flags the line step's)
-READ_ONLY = {
-    "k_ss_p": {"g", "hx"},
-    "k_nl_scatter": {"nl_pts", "nl_ptr", "gpt_grp", "gpt_uv4", "uvunk", "band_active"},
-}
+# uploaded by rsdft_gpu_set_nonlocal, which returns after the copies
+TABLES = {"grp_lma0", "grp_cnt", "lma_ptr", "jjp", "uv", "iuv", "duv", "nl_pts", "nl_ptr", "gpt_grp", "gpt_uv4",
+          "atom_ptr", "atom_lma"}
+# written by kernels, but not by the launch before: k_ss_p follows s_sstep, which writes per-band scalars (g and hx come
+# from the line step before); k_nl_scatter follows the stencil, which writes H psi (uVunk is the projection's, the band
+# flags the line step's; rsdft_gpu_op_nonlocal_add, where uVunk may be the launch before's, makes an ordinary launch)
+EARLIER = {"k_ss_p": {"g", "hx"}, "k_nl_scatter": {"uvunk", "band_active"}}
+ORDINARY = {"k_convert", "k_imma", "k_nl_project", "k_stencil", "k_sytrd", "k_widen"}  # never dependents
 
 
 def _sources():
@@ -44,12 +45,6 @@ def _kernels(text):
         yield head.group(1), text[p0 + 1:p1], text[b0 + 1:_closing(text, b0, "{}")]
 
 
-def _dependents(text):
-    for m in re.finditer(r"\blaunch_(?:dependent|as)\(", text):
-        args = text[m.end():_closing(text, m.end() - 1, "()")]
-        yield from re.findall(r"\b([ks]_[a-z]\w*)\b", args.split("vg,")[0].split("dim3")[0][:160])
-
-
 def test_every_kernel_waits_first():
     names = []
     for name, text in _sources().items():
@@ -61,24 +56,21 @@ def test_every_kernel_waits_first():
     assert wait.index("griddepcontrol.wait") < wait.index("griddepcontrol.launch_dependents")
 
 
-def test_only_asked_for_launches_are_dependents():
-    text = _sources()["common.cuh"]
-    plain = text.split("inline void launch(")[1].split("inline void")[0]
-    assert "launch_as(false," in plain and "numAttrs" not in plain
-    uses = sum(t.count("cudaLaunchAttributeProgrammaticStreamSerialization") for t in _sources().values())
-    assert uses == 1
+def test_launches_go_through_one_place():
+    text = "".join(_sources().values())
+    assert text.count("cudaLaunchAttributeProgrammaticStreamSerialization") == 1 and "<<<" not in text
+    # k_sytrd's cluster launch is the one other, without that attribute
+    assert text.count("cudaLaunchKernelEx(&cfg") == 2
+    for kernel in ORDINARY - {"k_sytrd"}:
+        assert re.search(r"\blaunch_ordinary\(%s\b" % kernel, text) and not re.search(r"\blaunch\(%s\b" % kernel, text)
 
 
 def test_dependents_read_coherently():
-    kernels, dependents = {}, set()
-    for text in _sources().values():
-        kernels.update({k: (p, b) for k, p, b in _kernels(text)})
-        dependents.update(_dependents(text))
-    dependents &= set(kernels)
-    assert {"s_step", "s_eig", "s_sstep", "k_ss_p", "k_pc_tma", "k_cg_upd1", "k_stencil_tma", "k_nl_scatter"} <= dependents
-    dependents.add("k_stencil_row")  # launched through a function pointer
-    for k in dependents:
-        params, body = kernels[k]
-        nc = set(re.findall(r"const\s+\w+\s*\*\s*__restrict__\s+(\w+)", params))
-        assert nc <= READ_ONLY.get(k, set()), (k, nc)
-        assert "__ldg" not in body or k in READ_ONLY, k
+    for name, text in _sources().items():
+        for kernel, params, body in _kernels(text):
+            if kernel in ORDINARY:
+                continue
+            allowed = TABLES | EARLIER.get(kernel, set())
+            assert set(re.findall(r"const\s+\w+\s*\*\s*__restrict__\s+(\w+)", params)) <= allowed, (name, kernel)
+            if kernel not in EARLIER:
+                assert set(re.findall(r"__ldg\(\s*(\w+)", body)) <= allowed, (name, kernel)
