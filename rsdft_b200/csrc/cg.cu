@@ -7,9 +7,10 @@
 // sign fix, 1e8 rejection, preconditioner early exit) is kept per band in
 // device arrays; the loop needs no host synchronisation.
 //
-// Vector kernels share one decomposition (CTA = 2048 points of one band) so
-// that dot products leave per-CTA partial sums that k_finish adds in a fixed
-// order: results are bit-reproducible run to run.
+// Vector kernels share one decomposition (a CTA takes a chunk of one band's
+// points, vec_chunks) and leave per-CTA partial sums of their dot products, which
+// the per-band scalar kernels (one warp per band) add in a fixed order: results are
+// bit-reproducible run to run.
 #include <cmath>
 
 #include "cgvec.cuh"

@@ -65,7 +65,7 @@ inline bool grp16_ok(long ld, std::initializer_list<const void*> ptrs) {
 
 struct CGScal {
     double *E, *E1, *rb, *gkgk, *res, *u11, *u21, *rr0, *rr1, *pa, *pb, *bk, *dots;
-    int *active, *pc_active, *reject;
+    int *active, *pc_active;
     int* pend;     // x = u11 x + u21 p still to be applied (s-step form: by the next p pass)
     int* rej_any;  // set when any band's update was rejected (its hx then no longer equals H x)
 };

@@ -42,24 +42,6 @@ __global__ void k_widen(const float* __restrict__ a, double* __restrict__ b, lon
         b[i] = (double)a[i];
 }
 
-// C = alpha * sum_c P[c] (sym: alpha/2 (G + G^T)), fixed summation order
-__global__ void k_reduce_partials(const double* P, int nch, int m, int n, double alpha, int sym,
-                                  double* __restrict__ C) {
-    grid_dependency();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y;
-    if (i >= m) return;
-    const long mn = (long)m * n;
-    double s = 0.0;
-    for (int c = 0; c < nch; ++c) s += P[c * mn + (long)j * m + i];
-    if (sym) {
-        double t = 0.0;
-        for (int c = 0; c < nch; ++c) t += P[c * mn + (long)i * m + j];
-        s = 0.5 * (s + t);
-    }
-    C[(long)j * m + i] = alpha * s;
-}
-
 // ------------------------------------------- FP64 products of tall blocks
 // A tall block (ml x nb) and how its FP64 products are formed: from its INT8
 // slices (imma.cu) where those suit, made once for every product it takes part

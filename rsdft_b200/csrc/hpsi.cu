@@ -1012,8 +1012,8 @@ static int launch_tma(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStrea
 // to the times of all tiles and splits of 9^3 .. 111^3, 1 to 640 bands, Md 4, 6,
 // 8: the choice is within 1.4 % (rms) of the best.  Two CTAs per SM throughout and
 // no term for the copies, as suits the TMA march, splits small blocks into tiles
-// of two rows and few z chunks: 45^3 x 1 band 30.3 us against 23.4, Md = 8 x 8 bands 49.4 against 33.3
-// (projectors aside).
+// of two rows and few z chunks: 45^3 x 1 band 30.3 us against 23.4, Md = 8 x 8
+// bands 49.4 against 33.3 (projectors aside).
 template <typename T, int MD, int BY>
 static int launch_row(StencilArgs<T> a, const StencilCoef& cf, int nb, cudaStream_t st, HpsiDot* dot, bool* used) {
     *used = false;
@@ -1083,7 +1083,11 @@ static int launch_stencil_md2(StencilArgs<T> a, const StencilCoef& cf, int nb, c
     // three (246 registers, 7 instead of 11 warps at 72^3): the window loads per
     // point drop from 7 to 6, the stencil of 72^3 x 480 from 1113 to 1018 us.
     // Only on the same tiles, for the long windows (Md >= 5) and with six warps
-    // left: 42^3 x 351 at Md = 4 took 283 us against 250.  In FP32, where a load
+    // left: 42^3 x 351 at Md = 4 took 283 us against 250.  H psi at Md = 6, two |
+    // three rows, us: same tiles 36^3 x 320 211 | 192, 48^3 404 | 393, 54^3 584 | 585,
+    // 72^3 x 240 888 | 823, 96^3 x 101 911 | 872; other tiles 60^3 x 320 711 | 780, 84^3
+    // 962 | 980, 90^3 993 | 1096 (42^3 385 | 326: the cost, fitted to two rows, does
+    // not tell these apart).  In FP32, where a load
     // serves twice the points and the warps' latency counts more, three rows
     // took 660 us against 646.
     constexpr int BY = MD <= 6 ? 2 : 1;

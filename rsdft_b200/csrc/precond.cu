@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(VT) k_ss_basis(const T* g, SSVec<T> sv, long l
 // (cg_module.f90:232-250).
 //
 // A basis pass dots what it has in hand: w_k with itself, with its source
-// w_{k-1} and, on small grids, with w_{k-2}.  The rest of the Gram matrix
+// w_{k-1} and, in FP64 and on small FP32 grids, with w_{k-2}.  The rest of the Gram matrix
 // follows from w_k = 2 B w_{k-1} - w_{k-2} with B symmetric, B w_0 = w_1 and
 // 2 B w_j = w_{j+1} + w_{j-1}:
 //   <w_k, w_j> = <w_{k-1}, w_{j+1}> + <w_{k-1}, w_{j-1}> - <w_{k-2}, w_j>,
@@ -132,37 +132,37 @@ __global__ void __launch_bounds__(128) s_sstep(CGScal s, SSPart pt, double* __re
     if (!(rr < 1e-24)) {
         double r[m + 1] = {}, q[m + 1] = {}, ft[m + 1];
         r[0] = q[0] = 1.0;
-    #pragma unroll
-    for (int il = 1; il <= m; ++il) {
+#pragma unroll
+        for (int il = 1; il <= m; ++il) {
             // ft = A q in the basis
-        #pragma unroll
-    for (int i = 0; i <= m; ++i) ft[i] = d * q[i];
+#pragma unroll
+            for (int i = 0; i <= m; ++i) ft[i] = d * q[i];
             ft[1] += d * q[0];
-        #pragma unroll
-    for (int j = 1; j < m; ++j) {
+#pragma unroll
+            for (int j = 1; j < m; ++j) {
                 ft[j + 1] += 0.5 * d * q[j];
                 ft[j - 1] += 0.5 * d * q[j];
             }
             double pAp = 0.0;
-        #pragma unroll
-    for (int i = 0; i <= m; ++i)
-            #pragma unroll
-    for (int j = 0; j <= m; ++j) pAp += q[i] * G[i][j] * ft[j];
+#pragma unroll
+            for (int i = 0; i <= m; ++i)
+#pragma unroll
+                for (int j = 0; j <= m; ++j) pAp += q[i] * G[i][j] * ft[j];
             const double a = rr / pAp;
-        #pragma unroll
-    for (int i = 0; i <= m; ++i) cz[i] += a * q[i];
+#pragma unroll
+            for (int i = 0; i <= m; ++i) cz[i] += a * q[i];
             if (il == m) break;
-        #pragma unroll
-    for (int i = 0; i <= m; ++i) r[i] -= a * ft[i];
+#pragma unroll
+            for (int i = 0; i <= m; ++i) r[i] -= a * ft[i];
             double rn = 0.0;
-        #pragma unroll
-    for (int i = 0; i <= m; ++i)
-            #pragma unroll
-    for (int j = 0; j <= m; ++j) rn += r[i] * G[i][j] * r[j];
+#pragma unroll
+            for (int i = 0; i <= m; ++i)
+#pragma unroll
+                for (int j = 0; j <= m; ++j) rn += r[i] * G[i][j] * r[j];
             const double bb = rn / rr;
             rr = rn;
-        #pragma unroll
-    for (int i = 0; i <= m; ++i) q[i] = r[i] + bb * q[i];
+#pragma unroll
+            for (int i = 0; i <= m; ++i) q[i] = r[i] + bb * q[i];
         }
     }
     double gz = 0.0;
@@ -282,10 +282,13 @@ __global__ void __launch_bounds__(VT) k_ss_p(const T* __restrict__ g, const T* _
 template <typename T>
 static int launch_ss_basis(int K, int dots, dim3 vg, cudaStream_t st, const T* g, SSVec<T> sv, long ld, long n,
                            const PcArgs& pa, double* part, const int* act) {
+    // FP64 takes three dots from K = 2 on (sstep_precond)
 #define RS_SS_CASE(KK, DD)                                                                    \
-    if (K == KK && dots == DD) {                                                              \
-        launch(k_ss_basis<T, KK, DD>, vg, VT, 0, st, g, sv, ld, n, pa, part, act);            \
-        return RSDFT_OK;                                                                      \
+    if constexpr (sizeof(T) == 4 || KK < 2 || DD != 2) {                                      \
+        if (K == KK && dots == DD) {                                                          \
+            launch(k_ss_basis<T, KK, DD>, vg, VT, 0, st, g, sv, ld, n, pa, part, act);        \
+            return RSDFT_OK;                                                                  \
+        }                                                                                     \
     }
     RS_SS_CASE(0, 2)
     RS_SS_CASE(1, 2)
@@ -679,9 +682,12 @@ static int pc_tma_dispatch(int K, int dots, const T* g, const SSVec<T>& sv, cons
     const T* src = K == 0 ? g : sv.w[K - 1];
     const T* aux[1] = {K >= 2 ? sv.w[K - 2] : nullptr};
     T* wout = dots > 1 ? sv.w[K] : nullptr;
-#define RS_PC_CASE(KK, DD)                                                                              \
-    if (K == KK && dots == DD)                                                                          \
-        return pc_tma_step<T, KK, DD>(src, aux, wout, pa, ld, mb, plan_mb, active, part, part_cap, nchunk, used);
+#define RS_PC_CASE(KK, DD)                                                                                  \
+    if constexpr (sizeof(T) == 4 || KK < 2 || DD != 2) {                                                    \
+        if (K == KK && dots == DD)                                                                          \
+            return pc_tma_step<T, KK, DD>(src, aux, wout, pa, ld, mb, plan_mb, active, part, part_cap, nchunk, \
+                                          used);                                                            \
+    }
     RS_PC_CASE(0, 2)
     RS_PC_CASE(1, 2)
     RS_PC_CASE(2, 2)
@@ -709,8 +715,11 @@ int sstep_precond(const T* g, const T* hx, const SSVec<T>& sv, T* p, T* x, long 
     // smooth residual are nearly parallel, and the recurrence holds for the
     // stored vectors to their rounding, whose effect on a dot falls as
     // 1 / sqrt(n).  Residuals against 64 bits, FP64 48^3: 6.1e-14 by the
-    // recurrence, 3.8e-14 by the dot (85 | 88 us a pass at 160 bands); FP32,
-    // 72^3: 1.7e-6 either way (332 | 416 us at 480 bands).
+    // recurrence, 3.8e-14 by the dot (85 | 88 us a pass at 160 bands).  FP32, time of
+    // a sweep and error of its residuals by the recurrence | by the dot: 24^3 x 32
+    // 329 us, 1.8e-6 | 335, 1.9e-6; 36^3 x 80 752, 1.6e-6 | 774, 1.4e-6; 48^3 x 160
+    // 2231, 1.6e-6 | 2283, 1.5e-6; 64^3 x 300 8127, 1.2e-6 | 8295, 1.2e-6: within the
+    // scatter of the errors, so only small grids, where it is cheap, keep the dot.
     const bool third = sizeof(T) == 8 || n <= 65536;
     SSPart pt{};
     // basis steps: TMA z march where the shape allows, element-wise otherwise

@@ -1,9 +1,8 @@
 // Bulk-copy (TMA) and mbarrier helpers for sm_100a, inline PTX.
 //
-// Only plain (non-multicast) bulk copies are used: from this GPU's global
-// memory into the issuing CTA's own shared memory, and (eigen.cu) from a
-// CTA's shared memory into one CTA of its cluster.  Every wait is bounded: a
-// wait that runs out reports failure and the caller aborts the CTA cleanly.
+// Only plain (non-multicast) tiled loads are used, from this GPU's global memory
+// into the issuing CTA's own shared memory.  Every wait is bounded: a wait that
+// runs out reports failure and the caller aborts the CTA cleanly.
 #pragma once
 
 #include <cstdint>
@@ -53,20 +52,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
-
-// 1-D bulk copy global -> own shared memory, completion counted on bar.
-// dst, src 16-byte aligned; bytes a multiple of 16.
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
-
-}  // namespace rsdft
-
-namespace rsdft {
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
