@@ -106,40 +106,46 @@ static int fp64_gram(const Fp64Block& a, const Fp64Block& b, double alpha, int s
     return dmma_gram(a.x, b.x, a.ld, a.ml, a.nb, a.nb, alpha, symmetrize, C, a.nb, true, bad);
 }
 
-__global__ void k_copy_cols_if(const double* src, long lds, double* __restrict__ dst, long ldd, long n,
-                               int nb, const int* flag) {
+__global__ void k_copy_cols_if(const double* src, long lds, double* __restrict__ dst, long ldd, long n, int nb,
+                               const int* flag, const int* need) {
     grid_dependency();
-    if (!*flag) return;
-    for (int b = blockIdx.y; b < nb; b += gridDim.y)
+    const bool all = *flag;
+    if (!all && !need[(nb + 127) / 128]) return;
+    for (int b = blockIdx.y; b < nb; b += gridDim.y) {
+        if (!all && !need[b / 128]) continue;
         for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
             dst[(long)b * ldd + i] = src[(long)b * lds + i];
+    }
 }
 
 // out (ml x nb, leading dimension ldo) = a V.  out may be a itself, given tmp
-// (leading dimension ldt) for the DMMA form, which cannot work in place.
+// (leading dimension ldt) for the DMMA form, which cannot work in place and
+// therefore comes before the INT8 form overwrites a.
 static int fp64_rotate(const Fp64Block& a, const double* V, int ldv, double* out, long ldo, double* tmp = nullptr,
                        long ldt = 0) {
     Context& c = ctx();
-    int* bad = a.bad;
-    if (bad) {
-        const int r = imma_rotate(a.s, V, ldv, bad, out, ldo);
-        if (r == RSDFT_ENOMEM)
-            bad = nullptr;
-        else
-            RS_CHECK(r);
-    }
     const bool inplace = out == a.x;
-    RS_CHECK(dmma_gemm(false, a.ml, a.nb, a.nb, 1.0, a.x, a.ld, V, ldv, 0.0, inplace ? tmp : out,
-                       inplace ? ldt : ldo, bad));
-    if (!inplace) return RSDFT_OK;
-    if (bad) {
-        launch(k_copy_cols_if, dim3(64, std::min(a.nb, 64)), 256, 0, c.stream, (const double*)tmp, ldt, out, ldo, a.ml,
-               a.nb, (const int*)bad);
-        RS_LAUNCH();
+    if (!inplace) {
+        tmp = out;
+        ldt = ldo;
+    }
+    ImmaV v;
+    const int r = a.bad ? imma_slice_v(a.s, V, ldv, a.bad, &v) : RSDFT_ENOMEM;
+    if (r == RSDFT_ENOMEM) {
+        RS_CHECK(dmma_gemm(false, a.ml, a.nb, a.nb, 1.0, a.x, a.ld, V, ldv, 0.0, tmp, ldt));
+        if (inplace)
+            RS_CUDA(cudaMemcpy2DAsync(out, ldo * sizeof(double), tmp, ldt * sizeof(double), a.ml * sizeof(double),
+                                      a.nb, cudaMemcpyDeviceToDevice, c.stream));
         return RSDFT_OK;
     }
-    RS_CUDA(cudaMemcpy2DAsync(out, ldo * sizeof(double), tmp, ldt * sizeof(double), a.ml * sizeof(double), a.nb,
-                              cudaMemcpyDeviceToDevice, c.stream));
+    RS_CHECK(r);
+    if (!inplace) RS_CHECK(imma_rotate(a.s, v, a.bad, out, ldo));
+    RS_CHECK(dmma_gemm(false, a.ml, a.nb, a.nb, 1.0, a.x, a.ld, V, ldv, 0.0, tmp, ldt, a.bad, a.s.need));
+    if (!inplace) return RSDFT_OK;
+    RS_CHECK(imma_rotate(a.s, v, a.bad, out, ldo));
+    launch(k_copy_cols_if, dim3(64, std::min(a.nb, 64)), 256, 0, c.stream, (const double*)tmp, ldt, out, ldo, a.ml,
+           a.nb, (const int*)a.bad, (const int*)a.s.need);
+    RS_LAUNCH();
     return RSDFT_OK;
 }
 

@@ -44,6 +44,7 @@ struct DmmaArgs {
     int sym;          // only tiles tm <= tn (a symmetric product)
     int ntm, ntiles;
     const int* only_if;  // run only if this device flag is set (null: always)
+    const int* need;     // else the row tiles with need[tm] (null: none); need[ntm]: any
 };
 
 constexpr int DM_BK = 16;  // K per stage (four m8n8k4 steps)
@@ -98,7 +99,8 @@ __global__ void __launch_bounds__(32 * WM * WN, CPS) k_dmma(DmmaArgs g) {
     constexpr int TM = BM / WM / 8, TN = BN / WN / 8;  // 8x8 tiles per warp
     static_assert(TM >= 1 && TN >= 1 && BM % (8 * WM) == 0 && BN % (8 * WN) == 0, "warp tiling");
     extern __shared__ __align__(16) double dsm[];
-    if (g.only_if && !*g.only_if) return;
+    const bool all = !g.only_if || *g.only_if;
+    if (!all && !(g.need && g.need[g.ntm])) return;
     double* As = dsm;
     double* Bs = dsm + NS * AST;
 
@@ -110,6 +112,7 @@ __global__ void __launch_bounds__(32 * WM * WN, CPS) k_dmma(DmmaArgs g) {
         if (tile != (int)blockIdx.x) __syncthreads();  // the last tile's stages are still read
         int tm, tn;
         tile_of(g, tile, tm, tn);
+        if (!all && !g.need[tm]) continue;  // the same for the CTA
         const int m0 = tm * BM, n0 = tn * BN;
         const long k0 = (long)blockIdx.y * g.kchunk;
         const long k1 = min(g.K, k0 + g.kchunk);
@@ -376,7 +379,7 @@ int dmma_gram(const double* A, const double* B, long ld, long kdim, int m, int n
 // which is k-contiguous for op = T ([n][k] staging) and row-contiguous for
 // op = N ([k][n] staging).
 int dmma_gemm(bool transA, long m, int n, int k, double alpha, const double* A, long lda, const double* B, long ldb,
-              double beta, double* C, long ldc, const int* only_if) {
+              double beta, double* C, long ldc, const int* only_if, const int* need) {
     DmmaArgs g{};
     g.only_if = only_if;
     g.A = B;  // A'(j, kk) = B[kk + j ldb]
@@ -404,6 +407,7 @@ int dmma_gemm(bool transA, long m, int n, int k, double alpha, const double* A, 
         constexpr int BM = 128, BN = 64;
         g.ntm = div_up(n, BM);
         g.ntiles = g.ntm * div_up(m, BN);
+        g.need = need;
         return transA ? launch_dmma<BM, BN, 4, 2, true, 2>(g, 1, vec) : launch_dmma<BM, BN, 4, 2, false, 2>(g, 1, vec);
     }
     // small dense products: 32 x 32 tiles, four warps

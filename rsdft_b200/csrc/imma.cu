@@ -18,10 +18,17 @@
 // FP64 arithmetic gives 2^-53 of each partial sum.  It is the smaller one as long
 // as the terms reach 2^-9 or so of the largest, but unlike FP64's it does not
 // shrink with them: where a band decays (vacuum, a localised band) its tail
-// would lose digits.  Such blocks go to the FP64 tensor pipe whole
-// (k_imma_slice: a grid point at which 64 bands, or 32 points in a row at which
-// one band, stay below 2^-12 of their largest).  What is left are the isolated
-// values near a band's nodes, good to 2^-60 of its largest.
+// would lose digits.  So k_imma_slice looks for points at which 64 bands, and
+// stretches of 32 points over which one band, stay below 2^-12 of their largest:
+//   the first, or a band below 2^-20 over such a stretch: the whole block goes to
+//     the FP64 tensor pipe;
+//   a tail band between 2^-12 and 2^-20 (the lowest bands of the 216-atom cell reach
+//     2^-13): the Gram products stay (sums over the whole grid, good to 2^-60 of the
+//     norms, FP64's bound being 2^-53 x points x the overlap of the moduli), and of a
+//     rotation the columns made up of tail bands (k_imma_slice_v) go to the FP64
+//     pipe, in tiles of 128.
+// What is left are isolated values near a band's nodes, good to 2^-60 of its
+// largest.
 //
 // Why: the FP64 tensor pipe gives 37 TFLOP/s, the INT8 pipe 36 digit products
 // per FP64 product at up to 4.5 POP/s, an FP64 rate of about 130 TFLOP/s.
@@ -67,7 +74,9 @@ constexpr int IM_D = 8;        // accumulators, s + t = 0 .. 7
 constexpr int IM_TCOLS = IM_D * IM_N;  // all of TMEM
 static_assert(IM_S == IM_D, "slice 0 of A opens every accumulator");
 constexpr int IM_BITS = 62;    // integer bits of a scaled value
-constexpr int IM_TINY = 12;    // values below 2^-IM_TINY of the largest may come singly only
+constexpr int IM_TINY = 12;    // values below 2^-IM_TINY of the largest: singly, or the band is a tail band
+constexpr int IM_DEEP = 20;    // below 2^-IM_DEEP: singly only
+constexpr int IM_OWN = 10;     // a column whose other weights are below 2^-IM_OWN of its tail bands' is theirs
 // exponents beyond which 2^(IM_BITS - e) or the products leave the range
 constexpr int IM_EMAX = 400;
 
@@ -106,10 +115,11 @@ __global__ void __launch_bounds__(256) k_imma_exp(const double* A, long ld, long
 }
 
 // A zero vector has every digit zero whatever its exponent (-IM_EMAX marks it);
-// a tiny one is out of range.
-__global__ void k_imma_exp_check(int* exps, int n, int* bad) {
+// a tiny one is out of range.  Also clears the tail and column flags.
+__global__ void k_imma_exp_check(int* exps, int n, int* tail, int nflags, int* bad) {
     grid_dependency();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b < nflags) tail[b] = 0;
     if (b >= n) return;
     if (exps[b] < -100000)
         exps[b] = -IM_EMAX;
@@ -140,12 +150,13 @@ __device__ __forceinline__ void byte_transpose(uint32_t a, uint32_t b, uint32_t 
 // through shared memory in 16-byte stores.  rows: [s][kb][nb][64 points]; cols:
 // [s][mb][ml][64 bands].
 //
-// Sets *bad when the block decays (file header): at one of the CTA's points all
-// its bands (if at least 32), or over 32 aligned points one band, below 2^-IM_TINY
-// of the bands' largest.  Bands that are zero throughout are left out.
+// Looks for decaying bands (file header): *bad when at one of the CTA's points all
+// its bands (if at least 32) are below 2^-IM_TINY of their largest, or over 32
+// aligned points one band below 2^-IM_DEEP; tail[band] when it is below 2^-IM_TINY
+// there.  Bands that are zero throughout are left out.
 __global__ void __launch_bounds__(256) k_imma_slice(const double* A, long ld, long ml, int nb, int nkb,
                                                     const int* exps, int8_t* __restrict__ rows,
-                                                    int8_t* __restrict__ cols, int* bad, int vec) {
+                                                    int8_t* __restrict__ cols, int* tail, int* bad, int vec) {
     grid_dependency();
     // pitch 17: the transposed words of a half warp (rows 4 apart) fall on 8
     // banks (at a pitch of 20, which 16-byte reads want, on 2: 872 us per
@@ -158,7 +169,7 @@ __global__ void __launch_bounds__(256) k_imma_slice(const double* A, long ld, lo
     const long i0 = (long)kb * 64 + 4 * p;
     const int b0 = mb * 64 + 4 * q;
     uint32_t lo[4][4], hi[4][4];  // [band][point]
-    uint32_t tiny = 0, run = 0;   // bit 4 r + e: tiny or no value; bit r: four tiny values
+    uint32_t tiny = 0, run = 0;   // bit 4 r + e: tiny or no value; bit r (4 + r): four tiny (deep) values
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const int b = b0 + r;
@@ -187,21 +198,33 @@ __global__ void __launch_bounds__(256) k_imma_slice(const double* A, long ld, lo
             imma_digits(x[e], scale, lo[r][e], hi[r][e]);
             if ((uint32_t)(__double2hiint(x[e]) & 0x7fffffff) < floor_hi) tiny |= 1u << (4 * r + e);
         }
-        if (floor_hi != 0xffffffffu && ((tiny >> (4 * r)) & 15u) == 15u && i0 + 4 <= ml) run |= 1u << r;
+        if (floor_hi != 0xffffffffu && ((tiny >> (4 * r)) & 15u) == 15u && i0 + 4 <= ml) {
+            run |= 1u << r;
+            uint32_t big = 0;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) big = max(big, (uint32_t)(__double2hiint(x[e]) & 0x7fffffff));
+            if (big < floor_hi - ((uint32_t)(IM_DEEP - IM_TINY) << 20)) run |= 16u << r;
+        }
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint32_t runs = 0;
+    // bits 0, 8 (16, 24): a run of eight lanes' points of the half warp's band
+    auto runs_of = [&](int bit) {
+        uint32_t n = __ballot_sync(0xffffffffu, (run >> bit) & 1u);
+        n &= n >> 4;
+        n &= n >> 2;
+        return n & (n >> 1) & 0x01010101u;
+    };
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         uint32_t m = __ballot_sync(0xffffffffu, ((tiny >> e) & 0x1111u) == 0x1111u && i0 + e < ml);
         m &= m >> 16;
         if (lane == 0) s_row[warp][e] = m & 0xffffu;
-        uint32_t n = __ballot_sync(0xffffffffu, (run >> e) & 1u);  // here e is the band
-        n &= n >> 4;
-        n &= n >> 2;
-        runs |= n & (n >> 1) & 0x01010101u;
+        const uint32_t n = runs_of(e);  // here e is the band
+        if (n) {                        // the same for the warp
+            if ((lane & 15) == 0 && ((n >> lane) & 0x0101u)) tail[b0 + e] = 1;
+            if (runs_of(4 + e) && lane == 0) *bad = 1;
+        }
     }
-    if (runs && lane == 0) *bad = 1;
     auto check_rows = [&] {
         if (threadIdx.x < 4 && nb - mb * 64 >= 32) {
             uint32_t m = 0xffffu;
@@ -251,16 +274,17 @@ __global__ void __launch_bounds__(256) k_imma_slice(const double* A, long ld, lo
 }
 
 // V'(m, n) = V(m, n) 2^exps[m] per column n: its exponent e, as the product's
-// scale 2^(e - 12), and its slices
-// [s][mb][n][64], one warp per column
+// scale 2^(e - 12), and its slices [s][mb][n][64], one warp per column.  need[n /
+// 128] (and need[all groups]) is set for a column whose weights on other than tail
+// bands are below 2^-IM_OWN of its largest: it may come out as a tail.
 __global__ void __launch_bounds__(128) k_imma_slice_v(const double* V, int ldv, int nb, int nmb,
-                                                      const int* exps, double* __restrict__ vscale,
-                                                      int8_t* __restrict__ out, int* bad) {
+                                                      const int* exps, const int* tail, int* need,
+                                                      double* __restrict__ vscale, int8_t* __restrict__ out, int* bad) {
     grid_dependency();
     const int n = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (n >= nb || __any_sync(0xffffffffu, *bad)) return;
     const double* v = V + (long)n * ldv;
-    int e = INT_MIN;
+    int e = INT_MIN, eo = INT_MIN;  // largest exponent over all bands, over those without tails
     bool fin = true;
     for (int m = lane; m < nb; m += 32) {
         const double x = fabs(v[m]);
@@ -269,14 +293,20 @@ __global__ void __launch_bounds__(128) k_imma_slice_v(const double* V, int ldv, 
         if (fin && x > 0.0) {
             frexp(x, &k);
             e = max(e, k + exps[m]);
+            if (!tail[m]) eo = max(eo, k + exps[m]);
         }
     }
     e = __reduce_max_sync(0xffffffffu, e);
+    eo = __reduce_max_sync(0xffffffffu, eo);
     fin = __all_sync(0xffffffffu, fin);
-    if (e == INT_MIN) e = 0;
+    if (e == INT_MIN) e = eo = 0;
     if (!fin || e > IM_EMAX || e < -IM_EMAX) {
         if (lane == 0) *bad = 1;
         return;
+    }
+    if (lane == 0 && (eo == INT_MIN || eo < e - IM_OWN)) {
+        need[n / 128] = 1;
+        need[(nb + 127) / 128] = 1;
     }
     if (lane == 0) vscale[n] = scalbn(1.0, e - 12);
     for (int m = lane; m < nmb * 64; m += 32) {
@@ -602,7 +632,7 @@ int launch_imma(const ImmaMaps& maps, const ImmaArgs& g, dim3 grid) {
 // x 192 954 | 956, x 256 1270 | 1246, 36^3 x 128 761 | 782, x 160 1074 | 1019, 48^3 x 96
 // 884 | 883.  Up to 128 bands the DMMA form has 64 x 64 tiles to match.
 bool imma_suits(long ml, int nb) {
-    return (double)ml * nb * nb >= 5e8 && (nb > 128 || (nb >= 96 && ml >= 100000)) && nb <= IM_SEG * IM_K;
+    return ml >= 4096 && (double)ml * nb * nb >= 5e8 && (nb > 128 || (nb >= 96 && ml >= 100000)) && nb <= IM_SEG * IM_K;
 }
 
 int imma_slice(const double* A, long ld, long ml, int nb, const char* ws, bool need_rows, bool need_cols, int* bad,
@@ -611,10 +641,11 @@ int imma_slice(const double* A, long ld, long ml, int nb, const char* ws, bool n
     const int nkb = div_up(ml, 64), nmb = div_up(nb, 64);
     int8_t *rows = nullptr, *cols = nullptr;
     int* exps = nullptr;
+    const int nflags = nb + div_up(nb, 128) + 1;  // tail bands, column groups
     const std::string name(ws);
     if ((need_rows && workspace_optional_t((name + "_r").c_str(), (size_t)IM_S * nkb * nb * 64, &rows) != RSDFT_OK) ||
         (need_cols && workspace_optional_t((name + "_c").c_str(), (size_t)IM_S * nmb * ml * 64, &cols) != RSDFT_OK) ||
-        workspace_optional_t((name + "_e").c_str(), (size_t)nb, &exps) != RSDFT_OK) {
+        workspace_optional_t((name + "_e").c_str(), (size_t)nb + nflags, &exps) != RSDFT_OK) {
         // one layout without the other is of no use
         release_optional((name + "_r").c_str());
         release_optional((name + "_c").c_str());
@@ -624,12 +655,13 @@ int imma_slice(const double* A, long ld, long ml, int nb, const char* ws, bool n
     const int sms = c.num_sms > 0 ? c.num_sms : 148;
     const int chunks = (int)std::max<long>(1, std::min<long>(div_up(ml, 4096), div_up(16L * sms, nb) + 7));
     launch(k_imma_exp, dim3(chunks, nb), 256, 0, c.stream, A, ld, ml, exps, bad);
-    launch(k_imma_exp_check, div_up(nb, 128), 128, 0, c.stream, exps, nb, bad);
+    int* tail = exps + nb;
+    launch(k_imma_exp_check, div_up(nflags, 128), 128, 0, c.stream, exps, nb, tail, nflags, bad);
     const int vec = (ld % 2 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0) ? 1 : 0;
     launch(k_imma_slice, dim3(nkb, nmb), 256, 0, c.stream, A, ld, ml, nb, nkb, (const int*)exps, rows, cols,
-           bad, vec);
+           tail, bad, vec);
     RS_LAUNCH();
-    *out = ImmaSlices{rows, cols, exps, nb, ml};
+    *out = ImmaSlices{rows, cols, exps, tail, tail + nb, nb, ml};
     return RSDFT_OK;
 }
 
@@ -661,18 +693,25 @@ int imma_gram(const ImmaSlices& a, const ImmaSlices& b, double alpha, int symmet
     return RSDFT_OK;
 }
 
-int imma_rotate(const ImmaSlices& a, const double* V, int ldv, int* bad, double* out, long ld) {
+int imma_slice_v(const ImmaSlices& a, const double* V, int ldv, int* bad, ImmaV* out) {
     Context& c = ctx();
     const int nb = a.nb, nmb = div_up(nb, 64);
     int8_t* sv = nullptr;
     double* vscale = nullptr;
     RS_CHECK(workspace_optional_t("imma_v", (size_t)IM_S * nmb * nb * 64, &sv));
     RS_CHECK(workspace_optional_t("imma_vscale", (size_t)nb, &vscale));
-    launch(k_imma_slice_v, div_up(nb, 4), 128, 0, c.stream, V, ldv, nb, nmb, a.exps, vscale, sv, bad);
+    launch(k_imma_slice_v, div_up(nb, 4), 128, 0, c.stream, V, ldv, nb, nmb, a.exps, a.tail, a.need, vscale, sv, bad);
     RS_LAUNCH();
+    *out = ImmaV{sv, vscale};
+    return RSDFT_OK;
+}
+
+int imma_rotate(const ImmaSlices& a, const ImmaV& v, const int* bad, double* out, long ld) {
+    Context& c = ctx();
+    const int nb = a.nb, nmb = div_up(nb, 64);
     ImmaMaps maps;
     RS_CHECK(imma_map(&maps.a, a.cols, a.ml, nmb, IM_M));
-    RS_CHECK(imma_map(&maps.b, sv, nb, nmb, IM_N));
+    RS_CHECK(imma_map(&maps.b, v.slices, nb, nmb, IM_N));
     ImmaArgs g{};
     g.kblocks = nmb;
     g.ntm = div_up(a.ml, IM_M);
@@ -682,7 +721,7 @@ int imma_rotate(const ImmaSlices& a, const double* V, int ldv, int* bad, double*
     g.ldo = ld;
     g.mrows = a.ml;
     g.nrows = nb;
-    g.vscale = vscale;
+    g.vscale = v.scale;
     g.bad = bad;
     g.err = c.err_flag;
     const int sms = c.num_sms > 0 ? c.num_sms : 148;

@@ -10,6 +10,8 @@ struct ImmaSlices {
     const int8_t* rows = nullptr;  // [slice][K block of 64 grid points][band][64]
     const int8_t* cols = nullptr;  // [slice][K block of 64 bands][grid point][64]
     const int* exps = nullptr;     // per band: |x| < 2^exps
+    const int* tail = nullptr;     // per band: set when it decays (imma.cu)
+    int* need = nullptr;           // per 128 columns of a rotation, and for all: set when the DMMA form has to make them
     int nb = 0;
     long ml = 0;
 };
@@ -34,9 +36,18 @@ int imma_slice(const double* A, long ld, long ml, int nb, const char* ws, bool n
 int imma_gram(const ImmaSlices& a, const ImmaSlices& b, double alpha, int symmetrize, const int* bad, double* C,
               long ldc);
 
-// out (ml x nb, leading dimension ld) = A V; V (nb x nb, leading dimension
-// ldv).  Reads only A's slices, so out may be A itself.  RSDFT_ENOMEM, and
-// nothing launched, when V's slices do not fit.
-int imma_rotate(const ImmaSlices& a, const double* V, int ldv, int* bad, double* out, long ld);
+// The INT8 slices of a rotation matrix V (nb x nb, leading dimension ldv) and
+// its columns' scales.  Sets a.need for the columns that the DMMA form has to make
+// (they come out right to 2^-60 of their largest only).  RSDFT_ENOMEM, and nothing
+// launched, when they do not fit.
+struct ImmaV {
+    const int8_t* slices = nullptr;
+    const double* scale = nullptr;
+};
+int imma_slice_v(const ImmaSlices& a, const double* V, int ldv, int* bad, ImmaV* out);
+
+// out (ml x nb, leading dimension ld) = A V.  Reads only A's slices, so out may be
+// A itself.
+int imma_rotate(const ImmaSlices& a, const ImmaV& v, const int* bad, double* out, long ld);
 
 }  // namespace rsdft

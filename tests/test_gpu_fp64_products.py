@@ -93,6 +93,42 @@ def test_rotate_decaying_bands(gpu, kind, ml, nb):
     assert (np.abs(t.cpu().numpy() - ref) <= nb * EPS * (np.abs(u) @ np.abs(v))).all()
 
 
+@pytest.mark.parametrize("ml,nb", [(30000, 130), (13824, 200), (20000, 290)])
+@pytest.mark.parametrize("mix", [1e-14, 1e-6, 1e-2])
+@pytest.mark.parametrize("inplace", [True, False])
+def test_rotate_tail_bands(gpu, ml, nb, mix, inplace):
+    """A few bands that fall to 2^-17 among bands that do not: columns made of them keep FP64's bound, by tiles of 128
+    columns from the DMMA kernel, the others by either form.  Out of place through the Gram-Schmidt of nearly
+    orthonormal bands, whose second rotation is by I + rounding."""
+    rng = np.random.default_rng(nb)
+    u, i = rng.normal(size=(ml, nb)), np.arange(ml) / ml
+    tails = np.array([1, nb - 2])
+    u[:, tails] = rng.uniform(0.5, 1.5, size=(ml, 2)) * 2.0 ** (-24.0 * np.abs(i[:, None] - np.array([0.3, 0.6])))
+    v = np.eye(nb) + mix * np.linalg.qr(rng.normal(size=(nb, nb)))[0]
+    assert sliced(ml, nb)
+    if inplace:
+        t = dev(u)
+        gpu.rotate(t, dev(v))
+        gpu.synchronize()
+        ref = u.astype(np.longdouble) @ v.astype(np.longdouble)
+        err, bound = np.abs(t.cpu().numpy() - ref), nb * EPS * (np.abs(u) @ np.abs(v))
+        assert (err[:, tails] <= bound[:, tails]).all()
+        assert (err <= bound + nb * 2.0 ** -60 * (np.abs(u).max(0) @ np.abs(v))).all()
+        return
+    n = round(ml ** (1 / 3))
+    c = build_cell(Workload("tails", 1, n, nb, nb, 0.03, 3300 + n))
+    gpu.setup(c)
+    w = np.linalg.qr(np.column_stack([u[:n ** 3, tails], np.delete(u[:n ** 3], tails, 1)]))[0] / np.sqrt(c.dV)
+    t = dev(w)
+    gpu.gram_schmidt(1, nb, 1, 1, t)
+    gpu.synchronize()
+    g = t.cpu().numpy()
+    assert np.abs(g.T @ g * c.dV - np.eye(nb)).max() <= 1e-14
+    # the first two columns stay themselves, to the rounding of a norm and of the pair's overlap
+    err = np.abs(g[:, :2] - w[:, :2])
+    assert (err <= 1e-14 * (np.abs(w[:, :1]) + np.abs(w[:, :2]))).all()
+
+
 def test_second_block_decays(gpu):
     """subspace_diag where only H psi leaves the slices' range: both products go to the DMMA kernel."""
     c = build_cell(Workload("sd", 1, 24, 192, 192, 0.03, 3100))
