@@ -43,7 +43,10 @@ extern "C" {
  * split of the tensor-core contractions (CG sweeps run in FP32 in every
  * mixed mode; Cholesky, the subspace eigensolve and the closing residuals
  * stay FP64) */
-#define RSDFT_MODE_FP64 0          /* plain all-FP64 form */
+#define RSDFT_MODE_FP64 0          /* plain FP64 form: large Gram matrices and rotations of bands
+                                    * that do not decay are formed in 62-bit fixed point per band
+                                    * (error of an element 2^-60 of the band's largest, below
+                                    * FP64's except at isolated near-zeros); decaying ones in FP64 */
 #define RSDFT_MODE_MIXED_BF16X3 1  /* 3-term split-BF16 (6 products, 24 significant bits) */
 #define RSDFT_MODE_MIXED_TF32 2    /* 2-term split-TF32, kind::tf32 (3 products, ~22 bits: FP32 accuracy) */
 #define RSDFT_MODE_MIXED_BF16X2 3  /* 2-term split-BF16 (3 products, 16 bits) */

@@ -31,10 +31,10 @@
 // largest.
 //
 // Why: the FP64 tensor pipe gives 37 TFLOP/s, the INT8 pipe 36 digit products
-// per FP64 product at up to 4.5 POP/s, an FP64 rate of about 130 TFLOP/s.
-// 72^3 x 480, psi^T psi: 1170 us against 4365 us (DMMA, upper tiles);
-// psi V: 2000 us against 6360 us; slicing psi for both 960 us
-// (exponents included).
+// per FP64 product at 3.2 to 3.4 POP/s measured, an FP64 rate of about 90 TFLOP/s.
+// 72^3 x 480, psi^T psi: 1255 us against 4365 us (DMMA, upper tiles); psi V: 2090 us
+// against 6360 us; slicing psi for both 1040 us (exponents included).  With seven
+// digits, 34 products, 1170, 2000 and 960 us.
 //
 // k_imma, one CTA per 128 x 64 tile of D(m, n) = sum_k A(m, k) B(n, k):
 //   warp 0    TMA producer: per K block of 64 the eight slices of both tiles
@@ -47,7 +47,9 @@
 //             from shared memory once per MMA (36 MMAs of N = 64 would be
 //             bound by that, 48 cycles of shared memory for 32 of MMA);
 //   warps 2-9 fold the accumulators (two warps per TMEM lane quadrant).
-// What bounds it is the operand stream from L2: 86 KB per 2176 cycles of MMA.
+// What bounds the Gram form is the tensor pipe (88 to 93 % active at 110,592 x 480).
+// The rotation's reaches 75 %: its tiles are nb / 64 K blocks long, and the next
+// one's MMAs wait for the fold's TMEM reads, the accumulators taking all of TMEM.
 #include <algorithm>
 #include <climits>
 
